@@ -504,9 +504,8 @@ int alloc_state(Solve& sv, DStateT<R>& s) {
   s.adp_piv = m.adp_piv;
   s.adp_pmap = m.adp_pmap;
   s.adp_rhs = nullptr;
-  if (m.adp_lu) {
-    const size_t rsz = m.adp_pmap ? sizeof(R) : sizeof(double);  // panel-shared factors: the state's type
-    s.adp_rhs = dalloc(sv, (size_t)adp_range_count(d) * 36 * rsz, e);
+  if (m.adp_lu && !m.adp_pmap) {  // k_adp6 keeps its right-hand sides in shared memory
+    s.adp_rhs = dalloc(sv, (size_t)adp_range_count(d) * 36 * sizeof(double), e);
     if (!s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP right-hand sides)");
   }
   s.giveup = (int32_t*)dalloc(sv, S6 * sizeof(int32_t), e);
@@ -741,7 +740,8 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
   cudaError_t e = cudaSuccess;
   // ADP: the KKT matrix of every zone depends on the geometry only, so its
   // factors are computed once here and each stage only substitutes.  They
-  // take 10.4 KB per zone per panel (1.7 KB shared by the panels); without
+  // take 10.4 KB per zone per panel (shared by the panels: the inverse's rows,
+  // 0.86 KB); without
   // room for them (or with CS_FLAG_NO_ADP_CACHE) every stage assembles and
   // factors in place.  The least-squares solution operators of STEPS
   // 7.b / 9.c are geometry-only as well: the row weights Minv A_row^T
@@ -788,21 +788,24 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
   if (!(sv.p.flags & CS_FLAG_NO_ADP_CACHE)) {
     int8_t pmap[6 * 72];
     const bool shared = !(sv.p.flags & CS_FLAG_ADP_PER_PANEL) && adp_panel_maps(m.host, pmap);
-    // panel-shared factors and right-hand sides in the state's type (the
-    // precision form substitutes in FP32), per-panel ones in FP64
+    // panel-shared inverses in the state's type (the precision form applies
+    // them in FP32), per-panel factors and their right-hand sides in FP64
     const size_t esz = shared ? sizeof(R) : sizeof(double);
     const long long nf = adp_factor_doubles(d, shared);
-    const size_t lu_bytes = (size_t)nf * esz, pv_bytes = (size_t)nf / 36;
-    const size_t rhs_bytes = (size_t)adp_range_count(d) * 36 * esz;
+    const size_t lu_bytes = (size_t)nf * esz, pv_bytes = shared ? 0 : (size_t)nf / 36;
+    const size_t rhs_bytes = shared ? 0 : (size_t)adp_range_count(d) * 36 * esz;
     size_t fr = 0, tot = 0;
     // room left after them and their right-hand sides: the FP32 form's state
     // staging (one FP64 word per point, cs_state_put / cs_state_get) and 2 GB
     if (cudaMemGetInfo(&fr, &tot) == cudaSuccess &&
         lu_bytes + pv_bytes + rhs_bytes + (size_t)8 * S6 + ((size_t)2 << 30) < fr) {
       m.adp_lu = mdalloc(sv, m, lu_bytes, e);
-      m.adp_piv = m.adp_lu ? (int8_t*)mdalloc(sv, m, pv_bytes, e) : nullptr;
-      s.adp_rhs = m.adp_piv ? dalloc(sv, (size_t)adp_range_count(d) * 36 * esz, e) : nullptr;
-      if (!m.adp_lu || !m.adp_piv || !s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP factors)");
+      if (!m.adp_lu) return cuda_fail(sv, e, "cudaMalloc(ADP operators)");
+      if (!shared) {
+        m.adp_piv = (int8_t*)mdalloc(sv, m, pv_bytes, e);
+        s.adp_rhs = m.adp_piv ? dalloc(sv, rhs_bytes, e) : nullptr;
+        if (!m.adp_piv || !s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP factors)");
+      }
       if (shared) {
         m.adp_pmap = (int8_t*)mdalloc(sv, m, sizeof pmap, e);
         if (!m.adp_pmap) return cuda_fail(sv, e, "cudaMalloc(ADP panel maps)");

@@ -73,11 +73,11 @@ struct DStateT {
   R* op_p2v;                             // CS_FLAG_P2 STEP 7.a stencil inverses, [8 x 9 x 9][zones of shrink(2)], or null
   R* op_p2e;                             // CS_FLAG_P2 STEP 9.b stencil inverses, [8 x 10 x 10][zones of shrink(2)], or null
   const LsqPanelMap* p2_map;             // op_p2v / op_p2e shared by the panels, or null
-  void* adp_lu;                          // ADP KKT factors, per block of zones [1296 in use order][block], or null:
-                                         // FP64 per panel; panel 1's (adp_pmap set) in the state's type R
-  int8_t* adp_piv;                       // their row permutation, per block [36][block]
-  void* adp_rhs;                         // ADP right-hand sides, [36][zones of the ADP range], typed as adp_lu
-  const int8_t* adp_pmap;                // factors shared by the panels: per panel [unknown map 36][sign 36], or null
+  void* adp_lu;                          // ADP operators per block of zones, or null: the KKT factors (FP64, [1296 in use
+                                         // order]), or panel 1's packed inverse (adp_pmap set, in the state's type R)
+  int8_t* adp_piv;                       // the factors' row permutation, per block [36][block]
+  void* adp_rhs;                         // the factors' right-hand sides, [36][zones of the ADP range]
+  const int8_t* adp_pmap;                // inverse shared by the panels: per panel [unknown map 36][sign 36], or null
   int* err_flag;                         // device-side error bits (bounded waits that gave up)
   int32_t* giveup;                       // positivity give-up flags per zone
   unsigned long long* dtmin;             // CFL reduction target (bit pattern of a positive double)
@@ -442,6 +442,7 @@ void launch_flattener(Solve& s);
 void launch_weno(Solve& s);
 void launch_positivity(Solve& s);
 void launch_faceB_adp(Solve& s);
+void launch_adp(Solve& s);
 void launch_adp_factor(Solve& s);
 void set_adp_smem_limits();
 long long adp_range_count(const Dims& d);

@@ -9,22 +9,11 @@
 // each kernel names the reference step it implements.  One thread per zone
 // or face; the ADP solve uses one warp per zone with the 36x36 KKT system
 // in shared memory.
-#include <algorithm>
-
-#include <utility>
-
-#include "cs_solve.h"
+#include "cs_recon.cuh"
 
 namespace cs {
 
 namespace {
-
-constexpr int TPB = 128;
-
-template <typename R>
-__device__ __forceinline__ R& Vat(const DStateT<R>& s, const Dims& d, int comp, int mode, int p, int i, int j, int k) {
-  return s.V[d.at(mode * NVAR + comp, p, i, j, k)];
-}
 
 // STEP 2 (zone part, 421:597-635) and STEP 5 (421:1497-1628).
 template <typename R>
@@ -234,40 +223,6 @@ __device__ __forceinline__ Nbr12 load_nbr(const DGeom& g, const Dims& d, int p, 
   return n;
 }
 
-// ---- bulk asynchronous copies (cp.async.bulk) and mbarriers ----
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred P;\n mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n selp.u32 %0, 1, 0, P;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-// Bounded wait on an mbarrier phase: after 2^23 polls (seconds, far beyond
-// any copy) it records an error in *err and returns, so no wait can hang.
-__device__ __noinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int* err) {
-  for (int it = 0; it < (1 << 23); ++it)
-    if (mbar_try_wait(bar, parity)) return;
-  atomicOr(err, 1);
-}
-
 // STEP 7.a (kE false) and STEP 9.b (kE true, the WENO-AO slopes of the
 // three E components, 421:6840-8400) with the work of a zone spread over
 // three threads: a block takes 32 zones; warp w first forms stencils w,
@@ -390,12 +345,6 @@ __global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_ao_
     }
     __syncthreads();
   }
-}
-
-template <typename R>
-__device__ __forceinline__ void coef10(const DGeom& g, const Dims& d, int p, int i, int j, int k, R* c) {
-#pragma unroll
-  for (int t = 0; t < 10; ++t) c[t] = geoR<R>(g, d, CS_G_COEF, t, p, i, j, k);
 }
 
 // Row rr of the 18 x 9 least-squares matrix of STEP 7.b (421:3869-4001)
@@ -871,485 +820,6 @@ __global__ void __launch_bounds__(TPB) k_faceB(Dims d, PhysC ph, DGeom g, DState
 #pragma unroll
     for (int q = 0; q < 5; ++q) Bq[d.at(q, p, i, j, k)] = (double)bq[q] + bd;
   }
-}
-
-// STEP 8.d ADP (421:5617-6677): constrained least squares for the 30
-// quadratic B modes matching the 6 face means exactly, solved per zone as
-// the 36x36 KKT system by one warp with Gaussian elimination (scaled
-// partial pivoting) in shared memory.
-constexpr int ADP_WARPS = 4;
-// Resident ADP factors are stored as one stream per block of ADP_ZB zones
-// (zone fastest), in the order the substitution consumes them: the strict
-// lower triangle row by row (630), then for rows 35..0 the entries right of
-// the diagonal followed by the diagonal (666).
-constexpr int ADP_ZB = 128;
-__host__ __device__ constexpr int adp_stream_pos(int a, int b) {
-  return b < a ? a * (a - 1) / 2 + b : 630 + (35 - a) * (36 - a) / 2 + (b == a ? 35 - a : b - a - 1);
-}
-// Factor stream of the panel-shared cache: blocks of ADP6_ZB zones; the
-// strict lower triangle column by column (630: column b, rows b+1..35),
-// then for rows 35..0 the entries right of the diagonal followed by the
-// diagonal (666).  Column order lets the forward pass update 35 - b rows
-// independently per column; each row still receives its terms in
-// ascending column order, so the arithmetic is that of the row order.
-constexpr int ADP6_ZB = 32;
-__host__ __device__ constexpr int adp6_stream_pos(int a, int b) {
-  return b < a ? b * 35 - b * (b - 1) / 2 + (a - b - 1)
-               : 630 + (35 - a) * (36 - a) / 2 + (b == a ? 35 - a : b - a - 1);
-}
-struct AdpSmem {
-  double K[36][37];
-  double Q[30][31];
-  double bq[30], wt[30], C[6][30], D[6], rhs[36], sol[36], sc[36], vB[30];
-  int piv[36];
-};
-
-// kFactorOnly: assemble and factor the geometry-only KKT matrix and store
-// the factors and the row permutation for k_adp_solve (once per mesh).
-// tmax: zones of the range handled (all of it, or panel 1's share when the
-// factors are shared by the six panels); zb: zones per factor block.
-template <bool kFactorOnly, typename R>
-__global__ void __launch_bounds__(32 * ADP_WARPS) k_adp(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r,
-                                                        long long tmax, int zb) {
-  extern __shared__ unsigned char smem_raw[];
-  AdpSmem& S = reinterpret_cast<AdpSmem*>(smem_raw)[threadIdx.x / 32];
-  const int lane = threadIdx.x & 31;
-  const long long nw = (long long)gridDim.x * ADP_WARPS;
-  for (long long t = blockIdx.x * (long long)ADP_WARPS + threadIdx.x / 32; t < tmax; t += nw) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    if (mask_at(g, d, p, i, j) == 0) continue;
-    const double obl0 = 1.0 / fmax(geo(g, d, CS_G_V_SCALE, 0, p, i, j, k), ph.smallnum);
-    const double vc0 = geo(g, d, CS_G_V_CEN, 0, p, i, j, k), vc1 = geo(g, d, CS_G_V_CEN, 1, p, i, j, k),
-                 vc2 = geo(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    double c0[10];
-    coef10(g, d, p, i, j, k, c0);
-    // 1. the 30 quadrature rows, one per lane
-    if (lane < 30) {
-      const int f = lane / 5, q = lane % 5, dir = f / 2;
-      const int fx = (f == 1) ? i - 1 : i, fy = (f == 3) ? j - 1 : j, fz = (f == 5) ? k - 1 : k;
-      const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-      const int BW = dir == 0 ? CS_G_XB_QW : (dir == 1 ? CS_G_YB_QW : CS_G_ZB_QW);
-      const int NF = dir == 0 ? CS_G_XF_N : (dir == 1 ? CS_G_YF_N : CS_G_ZF_N);
-      const int nq = dir == 2 ? q : 0, ns = dir == 2 ? 5 : 1;
-      const double nx = geo(g, d, NF, nq, p, fx, fy, fz), ny = geo(g, d, NF, ns + nq, p, fx, fy, fz),
-                   nz = geo(g, d, NF, 2 * ns + nq, p, fx, fy, fz);
-      const double x = (geo(g, d, QP, q, p, fx, fy, fz) - vc0) * obl0;
-      const double y = (geo(g, d, QP, 5 + q, p, fx, fy, fz) - vc1) * obl0;
-      const double z = (geo(g, d, QP, 10 + q, p, fx, fy, fz) - vc2) * obl0;
-      const double bfn[10] = {1.0, x, y, z, x * x - c0[4], y * y - c0[5], z * z - c0[6], x * y - c0[7], y * z - c0[8], x * z - c0[9]};
-#pragma unroll
-      for (int m = 0; m < 10; ++m) {
-        S.Q[lane][m] = m == 0 ? nx : nx * bfn[m];
-        S.Q[lane][10 + m] = m == 0 ? ny : ny * bfn[m];
-        S.Q[lane][20 + m] = m == 0 ? nz : nz * bfn[m];
-      }
-      S.wt[lane] = geo(g, d, BW, q, p, fx, fy, fz);
-      if (!kFactorOnly) {
-        S.bq[lane] = s.Bq[dir][d.at(q, p, fx, fy, fz)];
-        S.vB[lane] = Vat(s, d, 5 + lane / 10, lane % 10, p, i, j, k);
-      } else {
-        S.bq[lane] = 0.0;
-        S.vB[lane] = 0.0;
-      }
-    }
-    __syncwarp();
-    // 2. constraint rows C, D and the KKT matrix
-    for (int e = lane; e < 180; e += 32) {
-      const int f = e / 30, m = e % 30;
-      double acc = 0.0;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) acc = acc + S.wt[f * 5 + q] * S.Q[f * 5 + q][m];
-      S.C[f][m] = acc;
-    }
-    if (lane < 6) {
-      double acc = 0.0;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) acc = acc + S.wt[lane * 5 + q] * S.bq[lane * 5 + q];
-      S.D[lane] = acc;
-    }
-    __syncwarp();
-    // divergence-free rows (421:6586-6600) as (column, value) pairs
-    const int dcol[4][3] = {{1, 12, 23}, {4, 17, 29}, {7, 15, 28}, {9, 18, 26}};
-    const double dval[4][3] = {{1.0, 1.0, 1.0}, {2.0, 1.0, 1.0}, {1.0, 2.0, 1.0}, {1.0, 1.0, 2.0}};
-    for (int e = lane; e < 900; e += 32) {
-      const int a = e / 30, b = e % 30;
-      double acc = 0.0;
-      for (int q = 0; q < 30; ++q) acc = acc + S.Q[q][a] * S.Q[q][b];
-      if (a == b) acc = acc + 1.0;
-      for (int rr = 0; rr < 4; ++rr) {
-        double va = 0.0, vb = 0.0;
-        for (int c = 0; c < 3; ++c) {
-          if (dcol[rr][c] == a) va = dval[rr][c];
-          if (dcol[rr][c] == b) vb = dval[rr][c];
-        }
-        acc = acc + va * vb;
-      }
-      S.K[a][b] = acc;
-    }
-    for (int e = lane; e < 180; e += 32) {
-      const int f = e / 30, m = e % 30;
-      S.K[m][30 + f] = S.C[f][m];
-      S.K[30 + f][m] = S.C[f][m];
-    }
-    for (int e = lane; e < 36; e += 32) {
-      S.K[30 + e / 6][30 + e % 6] = 0.0;
-    }
-    if (lane < 30) {
-      double acc = 0.0;
-      for (int q = 0; q < 30; ++q) acc = acc + S.Q[q][lane] * S.bq[q];
-      S.rhs[lane] = acc + S.vB[lane];
-    } else {
-      for (int f = lane - 30; f < 6; f += 2) S.rhs[30 + f] = S.D[f];
-    }
-    __syncwarp();
-    // 3. elimination with scaled partial pivoting
-    for (int row = lane; row < 36; row += 32) {
-      double m = 0.0;
-      for (int c = 0; c < 36; ++c) m = fmax(m, fabs(S.K[row][c]));
-      S.sc[row] = (m == 0.0) ? 0.0 : 1.0 / m;
-      S.piv[row] = row;
-    }
-    __syncwarp();
-    for (int kk = 0; kk < 36; ++kk) {
-      double best = -1.0;
-      int bi = kk;
-      for (int row = kk + lane; row < 36; row += 32) {
-        const double v = fabs(S.K[row][kk]) * S.sc[row];
-        if (v > best) {
-          best = v;
-          bi = row;
-        }
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (bi != kk) {
-        for (int c = lane; c < 36; c += 32) {
-          const double tmp = S.K[kk][c];
-          S.K[kk][c] = S.K[bi][c];
-          S.K[bi][c] = tmp;
-        }
-        if (lane == 0) {
-          const double ts = S.sc[kk];
-          S.sc[kk] = S.sc[bi];
-          S.sc[bi] = ts;
-          const int tp = S.piv[kk];
-          S.piv[kk] = S.piv[bi];
-          S.piv[bi] = tp;
-        }
-      }
-      __syncwarp();
-      if (lane == 0 && S.K[kk][kk] == 0.0) S.K[kk][kk] = 1.0e-20;
-      __syncwarp();
-      const double inv = 1.0 / S.K[kk][kk];
-      for (int row = kk + 1 + lane; row < 36; row += 32) {
-        const double l = S.K[row][kk] * inv;
-        S.K[row][kk] = l;
-        for (int c = kk + 1; c < 36; ++c) S.K[row][c] -= l * S.K[kk][c];
-      }
-      __syncwarp();
-    }
-    if (kFactorOnly) {
-      const long long blk = t / zb, z = t % zb;
-      for (int e = lane; e < 36 * 36; e += 32) {
-        const int pos = zb == ADP6_ZB ? adp6_stream_pos(e / 36, e % 36) : adp_stream_pos(e / 36, e % 36);
-        // panel-shared factors in the state's type, per-panel ones in FP64
-        if (zb == ADP6_ZB)
-          ((R*)s.adp_lu)[(blk * 1296 + pos) * zb + z] = (R)S.K[e / 36][e % 36];
-        else
-          ((double*)s.adp_lu)[(blk * 1296 + pos) * zb + z] = S.K[e / 36][e % 36];
-      }
-      for (int e = lane; e < 36; e += 32) s.adp_piv[(blk * 36 + e) * zb + z] = (int8_t)S.piv[e];
-      __syncwarp();
-      continue;
-    }
-    // 4. substitution (one lane, reference order)
-    if (lane == 0) {
-      double y[36];
-      for (int a = 0; a < 36; ++a) {
-        double acc = S.rhs[S.piv[a]];
-        for (int b = 0; b < a; ++b) acc -= S.K[a][b] * y[b];
-        y[a] = acc;
-      }
-      for (int a = 35; a >= 0; --a) {
-        double acc = y[a];
-        for (int b = a + 1; b < 36; ++b) acc -= S.K[a][b] * S.sol[b];
-        S.sol[a] = acc / S.K[a][a];
-      }
-    }
-    __syncwarp();
-    // 5. write back the modes, zone B and the energy adjustment
-    if (lane < 30) Vat(s, d, 5 + lane / 10, lane % 10, p, i, j, k) = S.sol[lane];
-    if (lane == 0) {
-      R* U = s.U;
-      const long long o5 = d.at(4, p, i, j, k);
-      const double u6 = U[d.at(5, p, i, j, k)], u7 = U[d.at(6, p, i, j, k)], u8 = U[d.at(7, p, i, j, k)];
-      const double aa = (u6 * u6 + u7 * u7 + u8 * u8) * ph.ob8pi;
-      const double n6 = S.sol[0], n7 = S.sol[10], n8 = S.sol[20];
-      U[d.at(5, p, i, j, k)] = n6;
-      U[d.at(6, p, i, j, k)] = n7;
-      U[d.at(7, p, i, j, k)] = n8;
-      const double bb = (n6 * n6 + n7 * n7 + n8 * n8) * ph.ob8pi;
-      U[o5] = U[o5] - aa + bb;
-    }
-    __syncwarp();
-  }
-}
-
-// STEP 8.d right-hand side with the resident factors: one thread per zone
-// forms the 36 entries (the same sums in the same order as k_adp) and
-// stores them element-major, [36][zones of the ADP range].
-constexpr int ADPR_TPB = 128;
-template <typename R>
-__global__ void __launch_bounds__(ADPR_TPB) k_adp_rhs(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  const long long n = r.count();
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    double* out = (double*)s.adp_rhs + t;
-    if (mask_at(g, d, p, i, j) != 1) {
-#pragma unroll
-      for (int a = 0; a < 36; ++a) out[(long long)a * n] = 0.0;
-      continue;
-    }
-    const double obl0 = 1.0 / fmax(geo(g, d, CS_G_V_SCALE, 0, p, i, j, k), ph.smallnum);
-    const double vc0 = geo(g, d, CS_G_V_CEN, 0, p, i, j, k), vc1 = geo(g, d, CS_G_V_CEN, 1, p, i, j, k),
-                 vc2 = geo(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    double c0[10];
-    coef10(g, d, p, i, j, k, c0);
-    double rhs[30];
-#pragma unroll
-    for (int a = 0; a < 30; ++a) rhs[a] = 0.0;
-#pragma unroll 1
-    for (int f = 0; f < 6; ++f) {
-      const int dir = f / 2;
-      const int fx = (f == 1) ? i - 1 : i, fy = (f == 3) ? j - 1 : j, fz = (f == 5) ? k - 1 : k;
-      const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-      const int BW = dir == 0 ? CS_G_XB_QW : (dir == 1 ? CS_G_YB_QW : CS_G_ZB_QW);
-      const int NF = dir == 0 ? CS_G_XF_N : (dir == 1 ? CS_G_YF_N : CS_G_ZF_N);
-      const int ns = dir == 2 ? 5 : 1;
-      double dacc = 0.0;
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const int nq = dir == 2 ? q : 0;
-        const double nx = geo(g, d, NF, nq, p, fx, fy, fz), ny = geo(g, d, NF, ns + nq, p, fx, fy, fz),
-                     nz = geo(g, d, NF, 2 * ns + nq, p, fx, fy, fz);
-        const double x = (geo(g, d, QP, q, p, fx, fy, fz) - vc0) * obl0;
-        const double y = (geo(g, d, QP, 5 + q, p, fx, fy, fz) - vc1) * obl0;
-        const double z = (geo(g, d, QP, 10 + q, p, fx, fy, fz) - vc2) * obl0;
-        const double bfn[10] = {1.0, x, y, z, x * x - c0[4], y * y - c0[5], z * z - c0[6], x * y - c0[7],
-                                y * z - c0[8], x * z - c0[9]};
-        const double bq = s.Bq[dir][d.at(q, p, fx, fy, fz)];
-#pragma unroll
-        for (int m = 0; m < 10; ++m) {
-          rhs[m] = rhs[m] + (m == 0 ? nx : nx * bfn[m]) * bq;
-          rhs[10 + m] = rhs[10 + m] + (m == 0 ? ny : ny * bfn[m]) * bq;
-          rhs[20 + m] = rhs[20 + m] + (m == 0 ? nz : nz * bfn[m]) * bq;
-        }
-        dacc = dacc + geo(g, d, BW, q, p, fx, fy, fz) * bq;
-      }
-      out[(long long)(30 + f) * n] = dacc;
-    }
-#pragma unroll
-    for (int a = 0; a < 30; ++a) out[(long long)a * n] = rhs[a] + Vat(s, d, 5 + a / 10, a % 10, p, i, j, k);
-  }
-}
-
-// The same right-hand sides for the six panels from panel 1's geometry:
-// one thread per zone position forms r1 = sum_q row_1(q) bq_p(q) with
-// panel 1's quadrature rows and panel p's face values, then rhs_p =
-// T_p r1 + vB_p (the rows of panel p are T_p times panel 1's, see
-// k_adp_solve6), so the geometry is read once for six panels.
-// Four blocks per SM (128 registers) beat three at 168 (measured).
-template <typename R>
-__global__ void __launch_bounds__(ADPR_TPB, 4) k_adp_rhs6(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  const long long n = r.count(), n1 = n / 6;
-  for (long long t1 = blockIdx.x * (long long)blockDim.x + threadIdx.x; t1 < n1;
-       t1 += (long long)gridDim.x * blockDim.x) {
-    int p0, i, j, k;
-    r.decode(t1, p0, i, j, k);
-    const R obl0 = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, 0, i, j, k), R(ph.smallnum));
-    const R vc0 = geoR<R>(g, d, CS_G_V_CEN, 0, 0, i, j, k), vc1 = geoR<R>(g, d, CS_G_V_CEN, 1, 0, i, j, k),
-            vc2 = geoR<R>(g, d, CS_G_V_CEN, 2, 0, i, j, k);
-    R c0[10];
-    coef10(g, d, 0, i, j, k, c0);
-#pragma unroll 1
-    for (int p = 0; p < 6; ++p) {
-      R* out = (R*)s.adp_rhs + p * n1 + t1;
-      if (mask_at(g, d, p, i, j) != 1) {
-#pragma unroll
-        for (int a = 0; a < 36; ++a) out[(long long)a * n] = R(0.0);
-        continue;
-      }
-      R rhs[30];
-#pragma unroll
-      for (int a = 0; a < 30; ++a) rhs[a] = R(0.0);
-#pragma unroll 1
-      for (int f = 0; f < 6; ++f) {
-        const int dir = f / 2;
-        const int fx = (f == 1) ? i - 1 : i, fy = (f == 3) ? j - 1 : j, fz = (f == 5) ? k - 1 : k;
-        const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-        const int BW = dir == 0 ? CS_G_XB_QW : (dir == 1 ? CS_G_YB_QW : CS_G_ZB_QW);
-        const int NF = dir == 0 ? CS_G_XF_N : (dir == 1 ? CS_G_YF_N : CS_G_ZF_N);
-        const int ns = dir == 2 ? 5 : 1;
-        R dacc = R(0.0);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          const int nq = dir == 2 ? q : 0;
-          const R nx = geoR<R>(g, d, NF, nq, 0, fx, fy, fz), ny = geoR<R>(g, d, NF, ns + nq, 0, fx, fy, fz),
-                  nz = geoR<R>(g, d, NF, 2 * ns + nq, 0, fx, fy, fz);
-          const R x = (geoR<R>(g, d, QP, q, 0, fx, fy, fz) - vc0) * obl0;
-          const R y = (geoR<R>(g, d, QP, 5 + q, 0, fx, fy, fz) - vc1) * obl0;
-          const R z = (geoR<R>(g, d, QP, 10 + q, 0, fx, fy, fz) - vc2) * obl0;
-          const R bfn[10] = {R(1.0), x, y, z, x * x - c0[4], y * y - c0[5], z * z - c0[6], x * y - c0[7],
-                             y * z - c0[8], x * z - c0[9]};
-          const R bq = (R)s.Bq[dir][d.at(q, p, fx, fy, fz)];
-#pragma unroll
-          for (int m = 0; m < 10; ++m) {
-            rhs[m] = rhs[m] + (m == 0 ? nx : nx * bfn[m]) * bq;
-            rhs[10 + m] = rhs[10 + m] + (m == 0 ? ny : ny * bfn[m]) * bq;
-            rhs[20 + m] = rhs[20 + m] + (m == 0 ? nz : nz * bfn[m]) * bq;
-          }
-          dacc = dacc + geoR<R>(g, d, BW, q, 0, fx, fy, fz) * bq;
-        }
-        out[(long long)(30 + f) * n] = dacc;
-      }
-      const int8_t* umap = s.adp_pmap + p * 72;
-#pragma unroll
-      for (int v = 0; v < 30; ++v) {
-        const int u = __ldg(umap + v);
-        out[(long long)u * n] = (R)__ldg(umap + 36 + v) * rhs[v] + Vat(s, d, 5 + u / 10, u % 10, p, i, j, k);
-      }
-    }
-  }
-}
-
-// STEP 8.d substitution with the resident factors, one thread per zone.
-// The factor stream of the block's 128 zones (1296 x 1 KB, in consumption
-// order) flows through a ring of ADPS_NS shared-memory stages of ADPS_CH
-// elements (16 KB), filled by bulk asynchronous copies that a producer warp
-// issues as soon as the four consumer warps have released a stage
-// (full / empty mbarrier pairs).  The solution vector lives in shared
-// memory so that the loops stay short; the arithmetic (order included) is
-// that of the reference's forward and back substitution.
-constexpr int ADPS_TPB = ADP_ZB;             // consumer threads (one per zone)
-constexpr int ADPS_THREADS = ADPS_TPB + 32;  // + one producer warp
-constexpr int ADPS_CH = 16;
-constexpr int ADPS_NS = 4;
-constexpr int ADPS_NCH = 1296 / ADPS_CH;
-static_assert(1296 % ADPS_CH == 0, "whole chunks");
-struct AdpsSmem {
-  double stage[ADPS_NS][ADPS_CH][ADPS_TPB];
-  double y[36][ADPS_TPB];
-  uint64_t full[ADPS_NS];
-  uint64_t empty[ADPS_NS];
-};
-
-template <typename R>
-__global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  extern __shared__ __align__(128) unsigned char adps_raw[];
-  AdpsSmem& S = *reinterpret_cast<AdpsSmem*>(adps_raw);
-  const int tid = threadIdx.x;
-  const long long n = r.count();
-  const long long nblk = (n + ADP_ZB - 1) / ADP_ZB;
-  if ((long long)blockIdx.x >= nblk) return;
-  const long long my_iters = (nblk - 1 - blockIdx.x) / gridDim.x + 1;
-  const long long total_chunks = my_iters * ADPS_NCH;
-  if (tid == 0) {
-    for (int q = 0; q < ADPS_NS; ++q) {
-      mbar_init(&S.full[q], 1);
-      mbar_init(&S.empty[q], ADPS_TPB / 32);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid >= ADPS_TPB) {
-    // producer: chunk gch of this CTA is chunk gch % NCH of zone block
-    // blockIdx.x + (gch / NCH) * gridDim.x
-    if (tid == ADPS_TPB) {
-      for (long long gch = 0; gch < total_chunks; ++gch) {
-        const int slot = (int)(gch % ADPS_NS);
-        if (gch >= ADPS_NS) mbar_wait(&S.empty[slot], (uint32_t)(((gch / ADPS_NS) - 1) & 1), s.err_flag);
-        const long long it = gch / ADPS_NCH, c = gch % ADPS_NCH;
-        const long long blk = blockIdx.x + it * gridDim.x;
-        const double* src = (const double*)s.adp_lu + (blk * 1296 + c * ADPS_CH) * (long long)ADP_ZB;
-        mbar_expect_tx(&S.full[slot], ADPS_CH * ADP_ZB * sizeof(double));
-        bulk_g2s(&S.stage[slot][0][0], src, ADPS_CH * ADP_ZB * sizeof(double), &S.full[slot]);
-      }
-    }
-    return;
-  }
-  const int lane = tid & 31;
-  long long gch = 0;  // next chunk to consume
-  int within = ADPS_CH;
-  const double* cur = nullptr;
-  // next factor element of this thread's zone
-  auto next = [&]() -> double {
-    if (within == ADPS_CH) {
-      if (gch > 0) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&S.empty[(int)((gch - 1) % ADPS_NS)]);
-      }
-      const int slot = (int)(gch % ADPS_NS);
-      mbar_wait(&S.full[slot], (uint32_t)((gch / ADPS_NS) & 1), s.err_flag);
-      cur = &S.stage[slot][0][tid];
-      ++gch;
-      within = 0;
-    }
-    return cur[(within++) * ADPS_TPB];
-  };
-  for (long long it = 0; it < my_iters; ++it) {
-    const long long blk = blockIdx.x + it * gridDim.x;
-    const long long t = blk * ADP_ZB + tid;
-    const bool inr = t < n;
-    const int8_t* pv = s.adp_piv + blk * 36 * ADP_ZB + tid;
-    // permuted right-hand side first (36 independent loads), then the
-    // substitution in place
-#pragma unroll
-    for (int a = 0; a < 36; ++a) S.y[a][tid] = inr ? ((const double*)s.adp_rhs)[(long long)pv[a * ADP_ZB] * n + t] : 0.0;
-#pragma unroll 1
-    for (int a = 1; a < 36; ++a) {
-      double acc = S.y[a][tid];
-#pragma unroll 4
-      for (int b = 0; b < a; ++b) acc -= next() * S.y[b][tid];
-      S.y[a][tid] = acc;
-    }
-#pragma unroll 1
-    for (int a = 35; a >= 0; --a) {
-      double acc = S.y[a][tid];
-#pragma unroll 4
-      for (int b = a + 1; b < 36; ++b) acc -= next() * S.y[b][tid];
-      S.y[a][tid] = acc / next();
-    }
-    if (inr) {
-      int p, i, j, k;
-      r.decode(t, p, i, j, k);
-      if (mask_at(g, d, p, i, j) == 1) {
-#pragma unroll
-        for (int a = 0; a < 30; ++a) Vat(s, d, 5 + a / 10, a % 10, p, i, j, k) = S.y[a][tid];
-        R* U = s.U;
-        const long long o5 = d.at(4, p, i, j, k);
-        const double u6 = U[d.at(5, p, i, j, k)], u7 = U[d.at(6, p, i, j, k)], u8 = U[d.at(7, p, i, j, k)];
-        const double aa = (u6 * u6 + u7 * u7 + u8 * u8) * ph.ob8pi;
-        const double n6 = S.y[0][tid], n7 = S.y[10][tid], n8 = S.y[20][tid];
-        U[d.at(5, p, i, j, k)] = n6;
-        U[d.at(6, p, i, j, k)] = n7;
-        U[d.at(7, p, i, j, k)] = n8;
-        const double bb = (n6 * n6 + n7 * n7 + n8 * n8) * ph.ob8pi;
-        U[o5] = U[o5] - aa + bb;
-      }
-    }
-  }
-  // release the last chunk (no producer waits for it; keeps the protocol uniform)
-  __syncwarp();
-  if (lane == 0 && gch > 0) mbar_arrive(&S.empty[(int)((gch - 1) % ADPS_NS)]);
 }
 
 // STEP 9.a (421:6700-6790): zone-centred E = -v x B from the point values.
@@ -1899,182 +1369,7 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
   }
 }
 
-inline Range3 zones_all(const Dims& d) { return {1 - d.G, d.N + d.G, 1 - d.G, d.N + d.G, 1 - d.G, d.nr + d.G}; }
-inline Range3 shrink(const Dims& d, int s) {
-  return {1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.nr + d.G - s};
-}
-
 }  // namespace
-
-// STEP 8.d substitution with factors shared by the six panels.  The six
-// panels of the cubed sphere are rotations of panel 1 by signed
-// permutations R_p (vertex(p, i,j,k) = R_p vertex(1, i,j,k), checked when
-// the mesh is uploaded), so the KKT matrix of zone (i,j,k) of panel p is
-// T_p K_1 T_p^T, T_p being the signed permutation of the 30 B-mode
-// unknowns that R_p induces (identity on the 6 multipliers).  Panel 1's
-// factor stream then serves all six panels: r' = T_p^T r, y' = K_1^-1 r',
-// y = T_p y'.  A CTA takes ADP6_ZB zone positions and all six panels (one
-// consumer warp per panel, one zone per lane, y in registers); a producer
-// warp streams the positions' factors (4 KB stages, in consumption order)
-// through the ring, so each factor byte read from HBM serves six solves.
-// adp_pmap[p][0][v] is the panel-p unknown u fed by panel-1 unknown v,
-// adp_pmap[p][1][v] its sign.
-constexpr int ADP6_CONS = 6 * 32;
-constexpr int ADP6_THREADS = ADP6_CONS + 32;
-constexpr int ADP6_CH = 16;
-constexpr int ADP6_NS = 12;
-constexpr int ADP6_NCH = 1296 / ADP6_CH;
-template <typename F>
-struct Adp6SmemT {
-  F stage[ADP6_NS][ADP6_CH][ADP6_ZB];
-  uint64_t full[ADP6_NS];
-  uint64_t empty[ADP6_NS];
-};
-
-// Element e of the panel-shared factor stream (adp6_stream_pos order):
-// row a, column b; b == a is a diagonal entry of the backward pass.
-struct AdpElem {
-  int a, b;
-};
-__host__ __device__ constexpr AdpElem adp_elem(int e) {
-  if (e < 630) {
-    int b = 0;
-    while (e >= 35 - b) {
-      e -= 35 - b;
-      ++b;
-    }
-    return AdpElem{b + 1 + e, b};
-  }
-  int r = e - 630, a = 35;
-  while (r >= 36 - a) {
-    r -= 36 - a;
-    --a;
-  }
-  return r < 35 - a ? AdpElem{a, a + 1 + r} : AdpElem{a, a};
-}
-static_assert(adp_elem(0).a == 1 && adp_elem(0).b == 0 && adp_elem(34).a == 35 && adp_elem(34).b == 0 &&
-                  adp_elem(35).a == 2 && adp_elem(35).b == 1 && adp_elem(629).a == 35 && adp_elem(629).b == 34,
-              "forward");
-static_assert(adp6_stream_pos(35, 0) == 34 && adp6_stream_pos(2, 1) == 35 && adp6_stream_pos(35, 34) == 629 &&
-                  adp6_stream_pos(35, 35) == 630 && adp6_stream_pos(0, 0) == 1295,
-              "stream positions");
-static_assert(adp_elem(630).a == 35 && adp_elem(630).b == 35 && adp_elem(631).a == 34 && adp_elem(631).b == 35 &&
-                  adp_elem(632).b == 34 && adp_elem(1295).a == 0 && adp_elem(1295).b == 0,
-              "backward");
-
-// One stream element applied to y in registers (every index a compile-time
-// constant): forward and backward eliminations y[a] -= f y[b], the
-// diagonal y[a] /= f -- the substitution order of the reference.
-template <int E, typename F>
-__device__ __forceinline__ void adp6_apply(F (&y)[36], F f) {
-  constexpr AdpElem x = adp_elem(E);
-  if constexpr (x.a == x.b)
-    y[x.a] = y[x.a] / f;
-  else
-    y[x.a] -= f * y[x.b];
-}
-template <int C, typename F, int... W>
-__device__ __forceinline__ void adp6_chunk(F (&y)[36], const F* cur, std::integer_sequence<int, W...>) {
-  (adp6_apply<C * ADP6_CH + W>(y, cur[W * ADP6_ZB]), ...);
-}
-// The whole stream of one zone block, chunk by chunk through the ring:
-// release the previous stage, wait for this one, apply its 16 elements.
-template <typename F, int... C>
-__device__ __forceinline__ void adp6_substitute(F (&y)[36], Adp6SmemT<F>& S, int lane, long long& gch, int* err,
-                                                std::integer_sequence<int, C...>) {
-  auto acquire = [&]() -> const F* {
-    if (gch > 0) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.empty[(int)((gch - 1) % ADP6_NS)]);
-    }
-    const int slot = (int)(gch % ADP6_NS);
-    mbar_wait(&S.full[slot], (uint32_t)((gch / ADP6_NS) & 1), err);
-    ++gch;
-    return &S.stage[slot][0][lane];
-  };
-  (adp6_chunk<C>(y, acquire(), std::make_integer_sequence<int, ADP6_CH>{}), ...);
-}
-
-// The factor stream, the right-hand sides and the substitution are in the
-// state's type R (FP32 in the precision form: half the stream's bytes).
-template <typename R>
-__global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp_solve6(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  extern __shared__ __align__(128) unsigned char adp6_raw[];
-  Adp6SmemT<R>& S = *reinterpret_cast<Adp6SmemT<R>*>(adp6_raw);
-  const int tid = threadIdx.x;
-  const long long n = r.count(), n1 = n / 6;
-  const long long nblk = (n1 + ADP6_ZB - 1) / ADP6_ZB;
-  if ((long long)blockIdx.x >= nblk) return;
-  const long long my_iters = (nblk - 1 - blockIdx.x) / gridDim.x + 1;
-  const long long total_chunks = my_iters * ADP6_NCH;
-  if (tid == 0) {
-    for (int q = 0; q < ADP6_NS; ++q) {
-      mbar_init(&S.full[q], 1);
-      mbar_init(&S.empty[q], ADP6_CONS / 32);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid >= ADP6_CONS) {
-    if (tid == ADP6_CONS) {
-      for (long long gch = 0; gch < total_chunks; ++gch) {
-        const int slot = (int)(gch % ADP6_NS);
-        if (gch >= ADP6_NS) mbar_wait(&S.empty[slot], (uint32_t)(((gch / ADP6_NS) - 1) & 1), s.err_flag);
-        const long long it = gch / ADP6_NCH, c = gch % ADP6_NCH;
-        const long long blk = blockIdx.x + it * gridDim.x;
-        const R* src = (const R*)s.adp_lu + (blk * 1296 + c * ADP6_CH) * (long long)ADP6_ZB;
-        mbar_expect_tx(&S.full[slot], ADP6_CH * ADP6_ZB * sizeof(R));
-        bulk_g2s(&S.stage[slot][0][0], src, ADP6_CH * ADP6_ZB * sizeof(R), &S.full[slot]);
-      }
-    }
-    return;
-  }
-  const int lane = tid & 31, p = tid >> 5;
-  const int8_t* umap = s.adp_pmap + p * 72;
-  const int8_t* smap = umap + 36;
-  long long gch = 0;
-  for (long long it = 0; it < my_iters; ++it) {
-    const long long blk = blockIdx.x + it * gridDim.x;
-    const long long t1 = blk * ADP6_ZB + lane, t = p * n1 + t1;
-    const bool inr = t1 < n1;
-    const int8_t* pv = s.adp_piv + blk * 36 * ADP6_ZB + lane;
-    R y[36];
-#pragma unroll
-    for (int a = 0; a < 36; ++a) {
-      const int v = inr ? pv[a * ADP6_ZB] : 0;
-      const int u = __ldg(umap + v);
-      y[a] = inr ? (R)__ldg(smap + v) * ((const R*)s.adp_rhs)[(long long)u * n + t] : R(0.0);
-    }
-    adp6_substitute(y, S, lane, gch, s.err_flag, std::make_integer_sequence<int, ADP6_NCH>{});
-    if (inr) {
-      int pp, i, j, k;
-      r.decode(t, pp, i, j, k);
-      if (mask_at(g, d, p, i, j) == 1) {
-        double nb[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int v = 0; v < 30; ++v) {
-          const int u = __ldg(umap + v);
-          const double val = (double)__ldg(smap + v) * (double)y[v];
-          Vat(s, d, 5 + u / 10, u % 10, p, i, j, k) = (R)val;
-          if (v % 10 == 0) {
-            if (u == 0) nb[0] = val;
-            if (u == 10) nb[1] = val;
-            if (u == 20) nb[2] = val;
-          }
-        }
-        R* U = s.U;
-        const long long o5 = d.at(4, p, i, j, k);
-        const double u6 = U[d.at(5, p, i, j, k)], u7 = U[d.at(6, p, i, j, k)], u8 = U[d.at(7, p, i, j, k)];
-        const double aa = (u6 * u6 + u7 * u7 + u8 * u8) * ph.ob8pi;
-        U[d.at(5, p, i, j, k)] = nb[0];
-        U[d.at(6, p, i, j, k)] = nb[1];
-        U[d.at(7, p, i, j, k)] = nb[2];
-        const double bb = (nb[0] * nb[0] + nb[1] * nb[1] + nb[2] * nb[2]) * ph.ob8pi;
-        U[o5] = U[o5] - aa + bb;
-      }
-    }
-  }
-}
 
 // STEP 10 (421:9354-9976): min and max over the active interior zones of
 // the 8 primitives (zone values, B from the ADP solve) and of the zone's
@@ -2290,33 +1585,7 @@ void launch_faceB_adp_t(Solve& sv, DStateT<R>& st) {
   mark(sv, "k_faceB");
   k_faceB<R><<<blocks_for(fz.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fz, 2);
   mark(sv, "k_faceB");
-  Range3 a = shrink(d, 1);
-  if (st.adp_lu && st.adp_pmap) {
-    k_adp_rhs6<R><<<blocks_for(a.count() / 6, ADPR_TPB, grid_sms(sv)), ADPR_TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st,
-                                                                                                  a);
-    mark(sv, "k_adp_rhs6");
-    const long long nblk = (a.count() / 6 + ADP6_ZB - 1) / ADP6_ZB;
-    const int grid = (int)std::min<long long>(nblk, (long long)grid_sms(sv) * (sizeof(R) == 4 ? 4 : 2));
-    k_adp_solve6<R><<<grid, ADP6_THREADS, sizeof(Adp6SmemT<R>), sv.stream>>>(d, sv.ph, sv.g, st, a);
-    mark(sv, "k_adp_solve6");
-    return;
-  }
-  if (st.adp_lu) {
-    k_adp_rhs<R><<<blocks_for(a.count(), ADPR_TPB, grid_sms(sv)), ADPR_TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
-    mark(sv, "k_adp_rhs");
-    const long long nblk = (a.count() + ADP_ZB - 1) / ADP_ZB;
-    const int grid = (int)std::min<long long>(nblk, (long long)grid_sms(sv) * 2);
-    k_adp_solve<R><<<grid, ADPS_THREADS, sizeof(AdpsSmem), sv.stream>>>(d, sv.ph, sv.g, st, a);
-    mark(sv, "k_adp_solve");
-    return;
-  }
-  const size_t smem = sizeof(AdpSmem) * ADP_WARPS;
-  long long nwarps = a.count();
-  long long nblk = (nwarps + ADP_WARPS - 1) / ADP_WARPS;
-  long long cap = (long long)grid_sms(sv) * 16;
-  if (nblk > cap) nblk = cap;
-  k_adp<false, R><<<(int)nblk, 32 * ADP_WARPS, smem, sv.stream>>>(d, sv.ph, sv.g, st, a, a.count(), ADP_ZB);
-  mark(sv, "k_adp");
+  launch_adp(sv);
 }
 
 void launch_faceB_adp(Solve& sv) {
@@ -2326,7 +1595,6 @@ void launch_faceB_adp(Solve& sv) {
     launch_faceB_adp_t(sv, sv.st);
 }
 
-long long adp_range_count(const Dims& d) { return shrink(d, 1).count(); }
 long long lsq_range_count(const Dims& d) { return shrink(d, 2).count(); }
 
 template <typename R>
@@ -2352,46 +1620,6 @@ void launch_ops_build(Solve& sv) {
     launch_ops_build_t(sv, sv.stF);
   else
     launch_ops_build_t(sv, sv.st);
-}
-
-long long adp_factor_doubles(const Dims& d, bool shared) {
-  if (shared) return (shrink(d, 1).count() / 6 + ADP6_ZB - 1) / ADP6_ZB * (long long)ADP6_ZB * 1296;
-  return (shrink(d, 1).count() + ADP_ZB - 1) / ADP_ZB * (long long)ADP_ZB * 1296;
-}
-
-void set_adp_smem_limits() {
-  const int smem = (int)(sizeof(AdpSmem) * ADP_WARPS);
-  cudaFuncSetAttribute(k_adp_solve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdpsSmem));
-  cudaFuncSetAttribute(k_adp_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdpsSmem));
-  cudaFuncSetAttribute(k_adp_solve6<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(Adp6SmemT<double>));
-  cudaFuncSetAttribute(k_adp_solve6<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Adp6SmemT<float>));
-  cudaFuncSetAttribute(k_adp<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_adp<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_adp<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_adp<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-}
-
-template <typename R>
-void launch_adp_factor_t(Solve& sv, DStateT<R>& st) {
-  const Dims& d = sv.d;
-  Range3 a = shrink(d, 1);
-  const size_t smem = sizeof(AdpSmem) * ADP_WARPS;
-  // shared factors: panel 1's zones only, in blocks of ADP6_ZB
-  const long long tmax = st.adp_pmap ? a.count() / 6 : a.count();
-  long long nblk = (tmax + ADP_WARPS - 1) / ADP_WARPS;
-  long long cap = (long long)grid_sms(sv) * 16;
-  if (nblk > cap) nblk = cap;
-  k_adp<true, R><<<(int)nblk, 32 * ADP_WARPS, smem, sv.stream>>>(d, sv.ph, sv.g, st, a, tmax,
-                                                                 st.adp_pmap ? ADP6_ZB : ADP_ZB);
-  mark(sv, "k_adp_factor");
-}
-
-void launch_adp_factor(Solve& sv) {
-  if (sv.fp32)
-    launch_adp_factor_t(sv, sv.stF);
-  else
-    launch_adp_factor_t(sv, sv.st);
 }
 
 template <typename R>

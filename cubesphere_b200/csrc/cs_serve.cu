@@ -40,11 +40,8 @@ size_t state_device_bytes(const cs_params& p) {
   // ghost staging values (one per map entry, see mesh_device_bytes)
   bytes += (size_t)6 * 4 * (p.nghost + 1) * (p.ntp + 2 * p.nghost + 1) * (p.nr + 2 * p.nghost + 1) * 12 * 8;
   const size_t na = (size_t)6 * (p.ntp + 2 * p.nghost - 2) * (p.ntp + 2 * p.nghost - 2) * (p.nr + 2 * p.nghost - 2);
-  if (!(p.flags & CS_FLAG_NO_ADP_CACHE)) {
-    // ADP right-hand sides: the state's type with panel-shared factors
-    const size_t esz = (p.flags & CS_FLAG_ADP_PER_PANEL) ? sizeof(double) : rsize;
-    bytes += na * 36 * esz;
-  }
+  // ADP right-hand sides of the per-panel factors
+  if (!(p.flags & CS_FLAG_NO_ADP_CACHE) && (p.flags & CS_FLAG_ADP_PER_PANEL)) bytes += na * 36 * sizeof(double);
   return bytes + ((size_t)64 << 20);
 }
 
@@ -68,12 +65,12 @@ size_t mesh_device_bytes(const cs_params& p) {
     if (p.flags & CS_FLAG_P2) bytes += n10 * (648 + 800) * (f32 ? sizeof(float) : sizeof(double));
   }
   if (!(p.flags & CS_FLAG_NO_ADP_CACHE)) {
-    // factors shared by the six panels (in the state's type) unless
-    // per-panel ones (FP64) are asked for
+    // the inverse's rows shared by the six panels (in the state's type)
+    // unless per-panel factors (FP64) are asked for
     const bool per = (p.flags & CS_FLAG_ADP_PER_PANEL) != 0;
     const size_t nz = per ? na : na / 6;
     const size_t esz = (per || !(p.flags & CS_FLAG_FP32)) ? sizeof(double) : sizeof(float);
-    bytes += (nz + 128) * (1296 * esz + 36);
+    bytes += (nz + 128) * (per ? 1296 * esz + 36 : 645 * esz);
   }
   return bytes + ((size_t)64 << 20);
 }

@@ -66,7 +66,7 @@ struct MeshRes {
   void* op_p2v = nullptr;  // CS_FLAG_P2 one-sided stencil inverses (state's type)
   void* op_p2e = nullptr;
   bool p2_shared = false;  // op_p2v / op_p2e are panel 1's only
-  void* adp_lu = nullptr;   // FP64 per panel; panel-shared ones in the state's type
+  void* adp_lu = nullptr;   // per-panel factors (FP64) or the panel-shared inverse (state's type)
   int8_t* adp_piv = nullptr;
   int8_t* adp_pmap = nullptr;  // ADP factors shared by the panels: per panel [unknown map][sign]
   std::vector<void*> allocs;

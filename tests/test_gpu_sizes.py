@@ -1,0 +1,89 @@
+"""One whole step at sizes where the tiles of the stage kernels end unevenly
+(the smallest meshes, odd extents, a last tile of one zone, more layers than
+a thread's column segment) against the CPU oracle, and batches of FP64 members
+run side by side, which must give each member's own result to the bit.
+
+Tolerances: those of test_gpu_parity (1e-12 of the largest value for the
+state, FP64); the precision form's bounds of test_gpu_precision scaled to one
+step (rounding of FP32 storage, 6e-8, times the two or three stages' few
+operations on it: 5e-6 of the largest value; momentum at rest: of the largest
+sound-speed momentum).
+"""
+import numpy as np
+import pytest
+
+import cubesphere_b200 as cs
+from conftest import has_gpu
+from test_gpu_parity import check_state, face_b_errors, zones
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not has_gpu(), reason="needs a CUDA device")]
+
+SIZES = [(5, 2, 3), (6, 1, 4), (7, 5, 3), (13, 3, 4), (19, 9, 4), (9, 6, 5)]
+
+
+@pytest.mark.parametrize("ntp,nr,ghosts", SIZES)
+@pytest.mark.parametrize("rk", [cs.CS_RK2, cs.CS_SSPRK3, cs.CS_IMEX_RK2])
+def test_one_step_at_uneven_sizes_matches_the_oracle(ntp, nr, ghosts, rk):
+    from oracle import Oracle
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=ntp, nr=nr, nghost=ghosts, rk_scheme=rk)
+    s = cs.Solve(**pr["params"])
+    s.mesh_build()
+    s.init_problem(**pr["init"])
+    st = s.get_state()
+    o = Oracle(s)
+    o.put_state(st)
+    dt, dto = s.evaluate_timestep(1e30), o.evaluate_timestep(1e30)
+    assert abs(dt - dto) <= 1e-12 * dto
+    dt, dto = s.steps(1, dt), o.step(dto)
+    assert abs(dt - dto) <= 1e-12 * dto
+    check_state(s, s.get_state(), o.get_state())
+
+
+@pytest.mark.parametrize("ntp,nr,ghosts", SIZES[::2])
+@pytest.mark.parametrize("p2", [0, cs.CS_FLAG_P2])
+def test_precision_form_at_uneven_sizes(ntp, nr, ghosts, p2):
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=ntp, nr=nr, nghost=ghosts)
+    out = []
+    for form in (0, cs.CS_FLAG_FP32):
+        s = cs.Solve(**pr["params"], flags=form | p2)
+        s.mesh_build()
+        s.init_problem(**pr["init"])
+        s.steps(1, s.evaluate_timestep(1e30))
+        out.append((s, s.get_state()))
+    (s, want), (_, got) = out
+    for q in (0, 4):
+        den = np.abs(zones(s, want["U"][q])).max()
+        assert np.abs(zones(s, got["U"][q]) - zones(s, want["U"][q])).max() <= 5e-6 * den, q
+    mom = np.sqrt(np.abs(zones(s, want["U"][0])).max() * np.abs(zones(s, want["U"][4])).max())
+    for q in (1, 2, 3):
+        assert np.abs(zones(s, got["U"][q]) - zones(s, want["U"][q])).max() <= 5e-6 * mom, q
+    assert max(face_b_errors(s, got, want).values()) <= 5e-6
+
+
+def test_fp64_batches_give_each_members_own_result():
+    """Members of different sizes side by side, many times: every state equals
+    the member's run alone to the bit (a shared-memory stage refilled while a
+    warp still read it showed as a few wrong zones in one member of six)."""
+    members = []
+    for name, over in (("shell32", {}), ("surface32", dict(ntp=48)), ("shell32", dict(ntp=48, nr=24)),
+                       ("shell16", dict(ntp=24, nr=16))):
+        pr = cs.preset(name)
+        pr["params"].update(over)
+        s = cs.Solve(**pr["params"])
+        s.mesh_build()
+        s.init_problem(**pr["init"])
+        st = s.get_state()
+        s.steps(1, s.evaluate_timestep(1e30))
+        members.append((s, st, s.get_state()))
+    b = cs.Batch([m[0] for m in members])
+    for rep in range(40):
+        for s, st, _ in members:
+            s.put_state(st)
+        b.steps(1, [s.evaluate_timestep(1e30) for s, _, _ in members])
+        for n, (s, _, want) in enumerate(members):
+            got = s.get_state()
+            for k in want:
+                assert np.array_equal(got[k], want[k]), (rep, n, k)
+    b.close()
