@@ -559,6 +559,8 @@ int mesh_upload(Solve& sv, MeshRes& m) {
   CS_CUDA(sv, cudaMemcpyAsync(st, m.host.stencil.data(), m.host.stencil.size() * sizeof(int32_t),
                               cudaMemcpyHostToDevice, sv.stream));
   m.g.st = st;
+  m.pos_ext = (float*)mdalloc(sv, m, (size_t)18 * sv.d.S * sizeof(float), e);
+  if (!m.pos_ext) return cuda_fail(sv, e, "cudaMalloc(zone extents)");
   // Ghost-exchange map.
   std::vector<MapEntry> map;
   std::string why = build_fill_map(sv, map);
@@ -869,6 +871,7 @@ int mesh_attach(Solve& sv, const std::shared_ptr<MeshRes>& mp) {
   // State and work arrays.
   sv.fp32 = (sv.p.flags & CS_FLAG_FP32) != 0;
   if (int rc = sv.fp32 ? alloc_state(sv, sv.stF) : alloc_state(sv, sv.st)) return rc;
+  if (fresh) launch_pos_extents(sv, m.pos_ext);
   if (fresh)
     if (int rc = sv.fp32 ? mesh_operators(sv, m, sv.stF) : mesh_operators(sv, m, sv.st)) return rc;
   CS_CUDA(sv, cudaStreamSynchronize(sv.stream));

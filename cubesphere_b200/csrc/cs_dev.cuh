@@ -449,6 +449,7 @@ long long adp_range_count(const Dims& d);
 long long adp_factor_doubles(const Dims& d, bool shared);
 long long lsq_range_count(const Dims& d);
 void launch_ops_build(Solve& s);
+void launch_pos_extents(Solve& s, float* ext);
 void launch_efield(Solve& s);
 // STEP 10 min / max into Solve::step10_keys (no-op without CS_FLAG_STEP10).
 void launch_step10(Solve& s);

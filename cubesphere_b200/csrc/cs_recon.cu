@@ -642,110 +642,183 @@ __device__ __forceinline__ void pos_node(const DGeom& g, const Dims& d, int p, i
   z = (c[2] - vc[2]) * obl0;
 }
 
-// STEP 7.c (440:204-829): shrink the higher modes until the 27 nodal
-// values of density, pressure and entropy lie in the expanded local range.
-// Four blocks per SM (measured).
-template <typename R>
-__global__ void __launch_bounds__(TPB, 4) k_positivity(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+// Half extents of a zone over the 27 positivity nodes, max |x|, |y|, |z| of
+// their scaled offsets (the edge midpoints and the centroid lie within the
+// vertices'), rounded up: geometry only, once per mesh.
+__global__ void k_pos_extents(Dims d, PhysC ph, DGeom g, Range3 r, float* ext) {
+  const long long PS = (long long)NPANEL * d.S;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    const int lo = 2 - d.G, hx = d.N + d.G - 1, hz = d.nr + d.G - 1;
-    if (!(i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz)) {
-      s.giveup[d.at(0, p, i, j, k)] = 0;
-      continue;
-    }
-    const Nbr12 n = load_nbr(g, d, p, i, j);
-    const int px[9] = {i, n.x[0], n.x[1], n.x[2], n.x[3], n.x[8], n.x[9], n.x[10], n.x[11]};
-    const int py[9] = {j, n.y[0], n.y[1], n.y[2], n.y[3], n.y[8], n.y[9], n.y[10], n.y[11]};
-    double mn0 = 1e300, mx0 = -1e300, mn4 = 1e300, mx4 = -1e300, emin = 1e300, emax = -1e300;
-    for (int a = 0; a < 9; ++a)
-      for (int dz = -1; dz <= 1; ++dz) {
-        const long long o = d.idx(px[a], py[a], k + dz);
-        const double v0 = s.V[((long long)0 * NPANEL + p) * d.S + o], v4 = s.V[((long long)4 * NPANEL + p) * d.S + o];
-        const double e = s.ent[(long long)p * d.S + o];
-        mn0 = fmin(mn0, v0);
-        mx0 = fmax(mx0, v0);
-        mn4 = fmin(mn4, v4);
-        mx4 = fmax(mx4, v4);
-        emin = fmin(emin, e);
-        emax = fmax(emax, e);
-      }
-    const double ef = 0.2;
-    const double ff = fmax(fmin((s.flatA[d.at(0, p, i, j, k)] - 0.1) / 0.4, 1.0), 0.0), omff = 1.0 - ff;
-    mn0 = fmax(mn0 * (1.0 - ef * omff), ph.rhofloor);
-    mx0 = fmax(mx0 * (1.0 + ef * omff), ph.rhofloor);
-    mn4 = fmax(mn4 * (1.0 - ef * omff), ph.prsfloor);
-    mx4 = fmax(mx4 * (1.0 + ef * omff), ph.prsfloor);
-    emin = emin * (1.0 - ef * omff);
-    emax = emax * (1.0 + ef * omff);
     const double obl0 = 1.0 / fmax(geo(g, d, CS_G_V_SCALE, 0, p, i, j, k), ph.smallnum);
     const double vc[3] = {geo(g, d, CS_G_V_CEN, 0, p, i, j, k), geo(g, d, CS_G_V_CEN, 1, p, i, j, k),
                           geo(g, d, CS_G_V_CEN, 2, p, i, j, k)};
-    double c0[10];
-    coef10(g, d, p, i, j, k, c0);
-    double vr[10], vp[10], ep[4];
-#pragma unroll
-    for (int m = 0; m < 10; ++m) {
-      vr[m] = Vat(s, d, 0, m, p, i, j, k);
-      vp[m] = Vat(s, d, 4, m, p, i, j, k);
+    double h[3] = {0.0, 0.0, 0.0};
+    for (int a = 0; a < 14; ++a) {
+      double x, y, z;
+      pos_node(g, d, p, i, j, k, a, vc, obl0, x, y, z);
+      h[0] = fmax(h[0], fabs(x));
+      h[1] = fmax(h[1], fabs(y));
+      h[2] = fmax(h[2], fabs(z));
     }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) ep[m] = s.ent[d.at(m, p, i, j, k)];
-    const int niter = 15;
-    const double ratio = pow(0.10, 1.0 / (double)niter);
-    double scale = 1.0;  // cumulative shrink of the higher modes
-    int gave_up = 0;
-    for (int iter = 1; iter <= niter + 1; ++iter) {
-      if (iter == niter + 1) {
-        gave_up = 1;
-        break;
-      }
-      bool pass = true;
-      for (int a = 0; a < 27 && pass; ++a) {
-        double x, y, z;
-        pos_node(g, d, p, i, j, k, a, vc, obl0, x, y, z);
-        const double v1 = d_poly10(vr, c0, x, y, z), v5 = d_poly10(vp, c0, x, y, z);
-        const double en = ep[0] + ep[1] * x + ep[2] * y + ep[3] * z;
-        if (v1 < mn0 || v1 > mx0 || v5 < mn4 || v5 > mx4 || en < emin || en > emax) pass = false;
-      }
-      if (pass) break;
-#pragma unroll
-      for (int m = 1; m < 10; ++m) {
-        vr[m] = ratio * vr[m];
-        vp[m] = ratio * vp[m];
-      }
-#pragma unroll
-      for (int m = 1; m < 4; ++m) ep[m] = ratio * ep[m];
-      scale = scale + 1.0;  // counts the shrinks applied
-    }
-    const int nshrink = (int)(scale - 1.0);
-    if (gave_up || nshrink > 0) {
-      for (int q = 0; q < NVAR; ++q)
-        for (int m = 1; m < 10; ++m) {
-          double v = Vat(s, d, q, m, p, i, j, k);
-          if (gave_up) {
-            v = 0.0;
-          } else {
-            for (int it = 0; it < nshrink; ++it) v = ratio * v;
-          }
-          Vat(s, d, q, m, p, i, j, k) = v;
-        }
-      for (int m = 1; m < 4; ++m) s.ent[d.at(m, p, i, j, k)] = gave_up ? 0.0 : ep[m];
-    }
-    // bit 0: gave up; bits 1-4: shrink passes applied
-    s.giveup[d.at(0, p, i, j, k)] = gave_up | (nshrink << 1);
+    for (int q = 0; q < 3; ++q) ext[q * PS + p * d.S + d.idx(i, j, k)] = __double2float_ru(h[q] * (1.0 + 1e-12));
   }
 }
 
-// A zone that exhausted the shrink passes also zeroes its entropy value
-// (440:569-575); applied after every zone has read its neighbours.
+// The shrink of one zone (440:488-829): the 27 nodal values of density,
+// pressure and entropy against the bounds, at most 15 passes.  Returns the
+// zone's record: bit 0: gave up; bits 1-4: shrink passes applied.
 template <typename R>
-__global__ void k_apply_giveup(Dims d, DStateT<R> s, Range3 r) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    if (s.giveup[d.at(0, p, i, j, k)] & 1) s.ent[d.at(0, p, i, j, k)] = 0.0;
+__device__ __noinline__ int positivity_shrink(const Dims& d, const PhysC& ph, const DGeom& g, const DStateT<R>& s, int p,
+                                              int i, int j, int k, double mn0, double mx0, double mn4, double mx4,
+                                              double emin, double emax) {
+  const double obl0 = 1.0 / fmax(geo(g, d, CS_G_V_SCALE, 0, p, i, j, k), ph.smallnum);
+  const double vc[3] = {geo(g, d, CS_G_V_CEN, 0, p, i, j, k), geo(g, d, CS_G_V_CEN, 1, p, i, j, k),
+                        geo(g, d, CS_G_V_CEN, 2, p, i, j, k)};
+  double c0[10];
+  coef10(g, d, p, i, j, k, c0);
+  double vr[10], vp[10], ep[4];
+#pragma unroll
+  for (int m = 0; m < 10; ++m) {
+    vr[m] = Vat(s, d, 0, m, p, i, j, k);
+    vp[m] = Vat(s, d, 4, m, p, i, j, k);
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) ep[m] = s.ent[d.at(m, p, i, j, k)];
+  const int niter = 15;
+  const double ratio = pow(0.10, 1.0 / (double)niter);
+  int gave_up = 0, nshrink = 0;
+  for (int iter = 1; iter <= niter + 1; ++iter) {
+    if (iter == niter + 1) {
+      gave_up = 1;
+      break;
+    }
+    bool pass = true;
+    for (int a = 0; a < 27 && pass; ++a) {
+      double x, y, z;
+      pos_node(g, d, p, i, j, k, a, vc, obl0, x, y, z);
+      const double v1 = d_poly10(vr, c0, x, y, z), v5 = d_poly10(vp, c0, x, y, z);
+      const double en = ep[0] + ep[1] * x + ep[2] * y + ep[3] * z;
+      if (v1 < mn0 || v1 > mx0 || v5 < mn4 || v5 > mx4 || en < emin || en > emax) pass = false;
+    }
+    if (pass) break;
+#pragma unroll
+    for (int m = 1; m < 10; ++m) {
+      vr[m] = ratio * vr[m];
+      vp[m] = ratio * vp[m];
+    }
+#pragma unroll
+    for (int m = 1; m < 4; ++m) ep[m] = ratio * ep[m];
+    ++nshrink;
+  }
+  if (gave_up || nshrink > 0) {
+    for (int q = 0; q < NVAR; ++q)
+      for (int m = 1; m < 10; ++m) {
+        double v = Vat(s, d, q, m, p, i, j, k);
+        if (gave_up) {
+          v = 0.0;
+        } else {
+          for (int it = 0; it < nshrink; ++it) v = ratio * v;
+        }
+        Vat(s, d, q, m, p, i, j, k) = v;
+      }
+    for (int m = 1; m < 4; ++m) s.ent[d.at(m, p, i, j, k)] = gave_up ? 0.0 : ep[m];
+  }
+  return gave_up | (nshrink << 1);
+}
+
+// STEP 7.c (440:204-829): the 27 nodal values of density, pressure and
+// entropy must lie in the expanded local range, or the zone's higher modes
+// shrink.  In FP64 in every form.
+//
+// Almost every zone passes, so a bound decides first: no node is further
+// from the mean than sum_m |mode m| max |basis m| over the zone's extents,
+// and where the mean plus and minus that stays inside the range (less a
+// margin for the rounding of the nodal sums) the nodes need not be formed.
+// The others run the nodes (positivity_shrink), so every zone ends with the
+// same record as without the bound.  A thread takes kc zones of a radial
+// column and keeps the range of the last three layers: 9 neighbours' loads a
+// zone instead of 27.
+template <typename R>
+__global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g, DStateT<R> s, const float* __restrict__ ext,
+                                                       Range3 r, int kc) {
+  const unsigned ni = r.i1 - r.i0 + 1, nj = r.j1 - r.j0 + 1, ncol = 6 * ni * nj;
+  const unsigned nseg = (r.k1 - r.k0 + kc) / kc, nt = ncol * nseg;
+  const long long PS = (long long)NPANEL * d.S;
+  const int plane = d.NI * d.NJ;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
+    const unsigned seg = t / ncol, col = t - seg * ncol, u = col / ni;
+    const int i = (int)(col - u * ni) + r.i0, j = (int)(u % nj) + r.j0, p = (int)(u / nj);
+    const int ka = r.k0 + (int)seg * kc, kb = min(ka + kc - 1, r.k1);
+    int nbo[9];
+    nbo[0] = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int w = q < 4 ? q : q + 4;
+      nbo[q + 1] = (sten(g, d, p, i, j, w, 1) - j) * d.NI + (sten(g, d, p, i, j, w, 0) - i);
+    }
+    // range of density, pressure and entropy over the nine columns at layer k
+    R lo[3][3], hi[3][3];
+    auto layer = [&](int k, R (&a)[3], R (&b)[3]) {
+      const long long o = (long long)p * d.S + d.idx(i, j, k);
+      const R* f[3] = {s.V + o, s.V + 4 * PS + o, s.ent + o};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        a[c] = b[c] = f[c][0];
+#pragma unroll
+        for (int q = 1; q < 9; ++q) {
+          const R v = f[c][nbo[q]];
+          a[c] = fmin(a[c], v);
+          b[c] = fmax(b[c], v);
+        }
+      }
+    };
+    layer(ka - 1, lo[0], hi[0]);
+    layer(ka, lo[1], hi[1]);
+    for (int k = ka; k <= kb; ++k) {
+      layer(k + 1, lo[2], hi[2]);
+      const long long o = (long long)p * d.S + d.idx(i, j, k);
+      const double ef = 0.2;
+      const double ff = fmax(fmin(((double)s.flatA[o] - 0.1) / 0.4, 1.0), 0.0), omff = 1.0 - ff;
+      double mn[3], mx[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        mn[c] = (double)fmin(lo[0][c], fmin(lo[1][c], lo[2][c])) * (1.0 - ef * omff);
+        mx[c] = (double)fmax(hi[0][c], fmax(hi[1][c], hi[2][c])) * (1.0 + ef * omff);
+      }
+      mn[0] = fmax(mn[0], ph.rhofloor);
+      mx[0] = fmax(mx[0], ph.rhofloor);
+      mn[1] = fmax(mn[1], ph.prsfloor);
+      mx[1] = fmax(mx[1], ph.prsfloor);
+      const double hx = ext[o], hy = ext[PS + o], hz = ext[2 * PS + o];
+      const double* cf = g.f[CS_G_COEF] + o;
+      const double c4 = fabs(__ldg(cf + 4 * PS)), c5 = fabs(__ldg(cf + 5 * PS)), c6 = fabs(__ldg(cf + 6 * PS));
+      // |x x - c| <= max(h h, c); |x y - c| <= h h' + |c|
+      const double bb[9] = {hx, hy, hz, fmax(hx * hx, c4), fmax(hy * hy, c5), fmax(hz * hz, c6),
+                            hx * hy + fabs(__ldg(cf + 7 * PS)), hy * hz + fabs(__ldg(cf + 8 * PS)),
+                            hx * hz + fabs(__ldg(cf + 9 * PS))};
+      bool pass = true;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const R* v = c < 2 ? s.V + 4 * c * PS + o : s.ent + o;
+        const long long ms = c < 2 ? NVAR * PS : PS;
+        const double mean = v[0];
+        double dev = 0.0;
+#pragma unroll
+        for (int m = 1; m < (c < 2 ? 10 : 4); ++m) dev = dev + fabs((double)v[m * ms]) * bb[m - 1];
+        const double room = dev > 0.0 ? dev * (1.0 + 1e-12) + 1e-14 * (fabs(mean) + dev) : 0.0;
+        // written so that a NaN does not pass
+        pass = pass && mean - room >= mn[c] && mean + room <= mx[c];
+      }
+      s.giveup[o] = pass ? 0 : positivity_shrink(d, ph, g, s, p, i, j, k, mn[0], mx[0], mn[1], mx[1], mn[2], mx[2]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        lo[0][c] = lo[1][c];
+        lo[1][c] = lo[2][c];
+        hi[0][c] = hi[1][c];
+        hi[1][c] = hi[2][c];
+      }
+    }
   }
 }
 
@@ -828,6 +901,9 @@ __global__ void k_efield_a(Dims d, DGeom g, DStateT<R> s, Range3 r) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
+    // a zone that exhausted STEP 7.c's shrink passes also zeroes its entropy
+    // value (440:569-575), now that every zone has read its neighbours'
+    if (s.giveup[d.at(0, p, i, j, k)] & 1) s.ent[d.at(0, p, i, j, k)] = 0.0;
     R co[10];
     coef10(g, d, p, i, j, k, co);
     R pv[8];
@@ -1557,12 +1633,14 @@ void launch_weno(Solve& sv) {
 
 template <typename R>
 void launch_positivity_t(Solve& sv, DStateT<R>& st) {
-  const Dims& d = sv.d;
-  Range3 z = zones_all(d);
-  k_positivity<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z);
+  const Range3 z = shrink(sv.d, 1);
+  // a thread takes 8 zones of a column where that leaves four blocks an SM
+  // (fewer loads a zone), 2 otherwise (more threads)
+  const long long per_k = z.count() / (z.k1 - z.k0 + 1);
+  const int kc = z.count() >= (long long)grid_sms(sv) * 4 * TPB * 8 ? 8 : 2;
+  const long long nt = per_k * ((z.k1 - z.k0 + kc) / kc);
+  k_positivity<R><<<blocks_for(nt, TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, sv.mesh->pos_ext, z, kc);
   mark(sv, "k_positivity");
-  k_apply_giveup<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, st, z);
-  mark(sv, "k_apply_giveup");
 }
 
 void launch_positivity(Solve& sv) {
@@ -1596,6 +1674,12 @@ void launch_faceB_adp(Solve& sv) {
 }
 
 long long lsq_range_count(const Dims& d) { return shrink(d, 2).count(); }
+
+void launch_pos_extents(Solve& sv, float* ext) {
+  const Range3 z = shrink(sv.d, 1);
+  k_pos_extents<<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, z, ext);
+  mark(sv, "k_pos_extents");
+}
 
 template <typename R>
 void launch_ops_build_t(Solve& sv, DStateT<R>& st) {

@@ -48,8 +48,8 @@ size_t state_device_bytes(const cs_params& p) {
 size_t mesh_device_bytes(const cs_params& p) {
   const Box b(p.ntp, p.nr, p.nghost);
   const size_t S6 = (size_t)6 * b.size();
-  // geometry 126 words, mask and stencil
-  size_t bytes = 126 * S6 * sizeof(double) + S6 * sizeof(int32_t) + (size_t)6 * 48 * b.NI * b.NJ;
+  // geometry 126 words, zone extents, mask and stencil
+  size_t bytes = 126 * S6 * sizeof(double) + 3 * S6 * sizeof(float) + S6 * sizeof(int32_t) + (size_t)6 * 48 * b.NI * b.NJ;
   // ghost map: per panel 4 strips of G layers, 12 field words per point,
   // 9 bytes per entry (offsets, meta); panel-ownership maps are smaller
   bytes += (size_t)6 * 4 * (p.nghost + 1) * (p.ntp + 2 * p.nghost + 1) * (p.nr + 2 * p.nghost + 1) * 12 * 9 * 2;

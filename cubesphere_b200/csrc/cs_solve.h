@@ -63,6 +63,7 @@ struct MeshRes {
   void* op_m10 = nullptr;
   void* lsq_map = nullptr;  // LsqPanelMap[6] when row weights are panel 1's only
   bool m9_shared = false, m10_shared = false;  // which of op_m9 / op_m10 are panel 1's only
+  float* pos_ext = nullptr;  // half extents of the zones for the positivity bound, [3][6 S]
   void* op_p2v = nullptr;  // CS_FLAG_P2 one-sided stencil inverses (state's type)
   void* op_p2e = nullptr;
   bool p2_shared = false;  // op_p2v / op_p2e are panel 1's only
