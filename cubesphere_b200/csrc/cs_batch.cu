@@ -89,7 +89,10 @@ int run_batch(cs_batch* b, int nsteps, const double* dtcur) {
     const cudaError_t e = cudaGraphLaunch(b->exec, b->stream);
     if (e != cudaSuccess) return bfail(b, CS_ERR_CUDA, std::string("cudaGraphLaunch(batch): ") + cudaGetErrorString(e));
   }
-  for (cs_ctx* m : b->members) m->sv.launches += m->sv.graph_kernels * nsteps;
+  for (cs_ctx* m : b->members) {
+    m->sv.launches += m->sv.graph_kernels * nsteps;
+    m->sv.first_rates = false;
+  }
   return release_members(b);
 }
 

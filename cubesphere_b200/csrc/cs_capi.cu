@@ -903,16 +903,44 @@ void limit_all(Solve& sv) {
   launch_efield(sv);
 }
 
-// The state with the first stage's rates in place of the current ones.
+// While it lives, the rates a stage forms (dU/dt, entropy fluxes, EMFs) go to
+// the first stage's arrays, where the second finds them.
 template <typename R>
-DStateT<R> first_stage_rates(const DStateT<R>& st) {
-  DStateT<R> s1 = st;
-  s1.dUdt = st.K1;
-  for (int q = 0; q < 3; ++q) {
-    s1.EF[q] = st.EF1[q];
-    s1.Ef[q] = st.Ef1[q];
+struct FirstStageRates {
+  DStateT<R>&s, keep;
+  explicit FirstStageRates(DStateT<R>& st) : s(st), keep(st) {
+    s.dUdt = s.K1;
+    for (int q = 0; q < 3; ++q) {
+      s.EF[q] = s.EF1[q];
+      s.Ef[q] = s.Ef1[q];
+    }
   }
-  return s1;
+  ~FirstStageRates() {
+    s.dUdt = keep.dUdt;
+    for (int q = 0; q < 3; ++q) {
+      s.EF[q] = keep.EF[q];
+      s.Ef[q] = keep.Ef[q];
+    }
+  }
+};
+
+// Runs f on the rates the last stage or routine formed.
+template <typename F>
+void with_last_rates(Solve& sv, F f) {
+  if (!sv.first_rates) {
+    f(sv);
+  } else if (sv.fp32) {
+    FirstStageRates<float> from(sv.stF);
+    f(sv);
+  } else {
+    FirstStageRates<double> from(sv.st);
+    f(sv);
+  }
+}
+
+void fluxes_and_edges(Solve& sv) {
+  launch_fluxes(sv);
+  launch_edges(sv);
 }
 
 // IMEX-RK2: ARS(2,2,2) (Ascher, Ruuth & Spiteri 1997) with the fluxes, the
@@ -927,23 +955,10 @@ int run_stage_imex(Solve& sv, int irk) {
   prof_start(sv);
   launch_fill_ghosts(sv);
   limit_all(sv);
-  launch_fluxes(sv);
-  launch_edges(sv);
-  if (irk == 1) {
-    launch_save_stage0(sv);
-    launch_save_stage1_rates(sv);
-    launch_update(sv, gam);
-  } else {
-    launch_add_gravity(sv, (1.0 - gam) / (1.0 - del));
-    launch_restore_stage0(sv);
-    if (sv.fp32)
-      launch_update_with(sv, first_stage_rates(sv.stF), del);
-    else
-      launch_update_with(sv, first_stage_rates(sv.st), del);
-    launch_update(sv, 1.0 - del);
-  }
-  launch_gravity_implicit(sv, gam);
-  launch_cleanup(sv);
+  sv.first_rates = irk == 1;
+  with_last_rates(sv, fluxes_and_edges);
+  launch_update_imex(sv, irk, gam, del);
+  launch_cleanup(sv, false);
   return launch_check(sv, "stage launch");
 }
 
@@ -953,9 +968,7 @@ int run_stage(Solve& sv, int irk) {
   if (irk < 1 || irk > ns) return fail(sv, CS_ERR_ARG, "irk out of range for the RK scheme");
   if (sv.p.rk_scheme == CS_IMEX_RK2) return run_stage_imex(sv, irk);
   double dtmove = 1.0, a0 = 0.0;  // dtmove: fraction of the step
-  int kind = 0;
   if (sv.p.rk_scheme == CS_SSPRK3) {
-    kind = 1;
     if (irk == 2) { a0 = 0.75; dtmove = 0.25; }
     if (irk == 3) { a0 = 1.0 / 3.0; dtmove = 2.0 / 3.0; }
   } else if (irk == 2) {
@@ -967,10 +980,8 @@ int run_stage(Solve& sv, int irk) {
   launch_fluxes(sv);
   launch_edges(sv);
   launch_sources(sv);
-  if (irk == 1) launch_save_stage0(sv);
-  else launch_combine(sv, a0, kind);
-  launch_update(sv, dtmove);
-  launch_cleanup(sv);
+  launch_update_rk(sv, irk, a0, dtmove);
+  launch_cleanup(sv, false);
   return launch_check(sv, "stage launch");
 }
 
@@ -1059,15 +1070,15 @@ cudaError_t debug_copy(Solve& sv, const DStateT<R>& s, int which, size_t nc, dou
     case 0: e = cp(host_out, s.V, nc * S6); break;
     case 1: e = cp(host_out, s.ent, nc * S6); break;
     case 2: e = cp(host_out, s.flatA, S6); break;
-    case 3: e = cp(host_out, s.dUdt, nc * S6); break;
-    case 4: case 5: case 6: e = cpd(host_out, s.Ef[which - 4], S6); break;
+    case 3: e = cp(host_out, sv.first_rates ? s.K1 : s.dUdt, nc * S6); break;
+    case 4: case 5: case 6: e = cpd(host_out, sv.first_rates ? s.Ef1[which - 4] : s.Ef[which - 4], S6); break;
     case 7: case 8: case 9: e = cpd(host_out, s.Bq[which - 7], nc * S6); break;
     case 10: e = cp(host_out, s.E, 3 * S6); break;
     case 11:
       for (int q = 0; q < 6 && e == cudaSuccess; ++q) e = cp(host_out + q * S6, s.S[q], S6);
       break;
     case 12:
-      for (int q = 0; q < 3 && e == cudaSuccess; ++q) e = cp(host_out + q * S6, s.EF[q], S6);
+      for (int q = 0; q < 3 && e == cudaSuccess; ++q) e = cp(host_out + q * S6, sv.first_rates ? s.EF1[q] : s.EF[q], S6);
       break;
     case 13: {
       std::vector<int32_t> flags(S6);
@@ -1449,6 +1460,7 @@ int cs_steps(cs_ctx* ctx, int32_t nsteps, double dtcur, double* dtcurp1) {
     if (int rc = cs::step_graph(sv)) return rc;
     for (int n = 0; n < nsteps; ++n) CS_CUDA(sv, cudaGraphLaunch(sv.graph_exec, sv.stream));
     sv.launches += sv.graph_kernels * nsteps;
+    sv.first_rates = false;
   }
   return cs::read_dt(sv, dtcurp1);
 }
@@ -1526,17 +1538,17 @@ int cs_profile_end(cs_ctx* ctx, int32_t max_kernels, char* names, double* total_
 
 CS_ROUTINE(cs_fill_ghosts, cs::launch_fill_ghosts(sv))
 CS_ROUTINE(cs_limit_all_slopes_p12, cs::limit_all(sv))
-CS_ROUTINE(cs_make_facial_fluxes, cs::launch_fluxes(sv))
-CS_ROUTINE(cs_make_edge_efields_p1, cs::launch_edges(sv))
-CS_ROUTINE(cs_build_non_stiff_sources, cs::launch_sources(sv))
-CS_ROUTINE(cs_cleanup_after_update, cs::launch_cleanup(sv))
+CS_ROUTINE(cs_make_facial_fluxes, sv.first_rates = false; cs::launch_fluxes(sv))
+CS_ROUTINE(cs_make_edge_efields_p1, sv.first_rates = false; cs::launch_edges(sv))
+CS_ROUTINE(cs_build_non_stiff_sources, cs::with_last_rates(sv, cs::launch_sources))
+CS_ROUTINE(cs_cleanup_after_update, cs::launch_cleanup(sv, true))
 
 int cs_update_imex_rk_step_p1(cs_ctx* ctx, double dtmove) {
   if (!ctx) return CS_ERR_ARG;
   Solve& sv = ctx->sv;
   if (int rc = cs::need(sv, true)) return rc;
   cs::launch_set_dt(sv, dtmove);
-  cs::launch_update(sv, 1.0);
+  cs::with_last_rates(sv, [](Solve& s) { cs::launch_update(s, 1.0); });
   return cs::launch_check(sv, "cs_update_imex_rk_step_p1");
 }
 

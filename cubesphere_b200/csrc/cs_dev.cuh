@@ -456,19 +456,17 @@ void launch_step10(Solve& s);
 void launch_fluxes(Solve& s);
 void launch_edges(Solve& s);
 void launch_sources(Solve& s);
-void launch_save_stage0(Solve& s);
-void launch_combine(Solve& s, double a0, int kind);
 // Update, CT and implicit gravity advance by scale times the device-resident
 // time step (DStateT::dt), which launch_set_dt sets and launch_timestep
-// replaces with the next step.
+// replaces with the next step.  launch_update_rk: stage irk of RK2 (a0 0) or
+// SSP-RK3 with its save (first stage) or combine; launch_update_imex: stage
+// irk of ARS(2,2,2) with the implicit gravity.
 void launch_update(Solve& s, double scale);
-template <typename R>
-void launch_update_with(Solve& s, const DStateT<R>& st, double scale);
-void launch_gravity_implicit(Solve& s, double scale);
-void launch_add_gravity(Solve& s, double c);
-void launch_save_stage1_rates(Solve& s);
-void launch_restore_stage0(Solve& s);
-void launch_cleanup(Solve& s);
+void launch_update_rk(Solve& s, int irk, double a0, double scale);
+void launch_update_imex(Solve& s, int irk, double gam, double del);
+// masks: the masked and cube-corner faces first (a stage has done that
+// before its reconstruction and changed none of them since).
+void launch_cleanup(Solve& s, bool masks);
 void launch_timestep(Solve& s);
 void launch_set_dt(Solve& s, double dt);
 // Mass, energy and max |div B| of the interior into out[0..2] (part: the

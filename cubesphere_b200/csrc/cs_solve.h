@@ -102,6 +102,7 @@ struct Solve {
   int device = 0;
   int sm_count = 148;
   bool has_mesh = false, has_state = false;
+  bool first_rates = false;  // the last stage's rates are in the first stage's arrays (IMEX)
   long long launches = 0;  // kernels launched by this solve
   cudaGraph_t graph = nullptr;           // one step, captured by cs_steps / cs_batch_steps
   cudaGraphExec_t graph_exec = nullptr;  // its executable form

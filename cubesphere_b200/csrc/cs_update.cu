@@ -8,6 +8,8 @@
 // CLEANUP_AFTER_UPDATE (485cleanup_after_update.f:383-1273),
 // EVALUATE_TIMESTEP (490evaluate_timestep.f:121-286) and the RK combine of
 // the driver (_I/_1000riemann_geomesh_cs_mhd/1000riemann_geomesh_cs_mhd.f:2661-2773).
+#include <algorithm>
+
 #include "cs_solve.h"
 
 namespace cs {
@@ -104,63 +106,120 @@ __global__ void k_pad_radial(Dims d, DGeom g, DStateT<R> s, int bc_lower, int bc
   }
 }
 
-// RK stage combine on the whole box: kind 0 is the two-stage average
-// (x + x0) / 2, kind 1 the Shu-Osher form a0 x0 + (1 - a0) x.  Segments
-// 0..1 (U, entropy) hold the state's type R, 2..4 (face B) FP64.
-template <typename R>
-struct CombineSeg {
-  R* x[2];
-  const R* x0[2];
-  double* b[3];
-  const double* b0[3];
-  long long n[5];
+// What one pass of the update does besides U += scale dt dU/dt (a stage's
+// save, combine and restore need no passes of their own):
+//   UP_PLAIN  nothing (the routine by itself)
+//   UP_SAVE   first stage: also saves the state
+//   UP_MEAN   (x + x0) / 2 first (RK2's second stage)
+//   UP_MIX    a0 x0 + (1 - a0) x first (SSP-RK3)
+//   UP_IMEX1  UP_SAVE with the first stage's rates, then the implicit gravity
+//   UP_IMEX2  from the saved state: scale0 dt of the first stage's rates, then
+//             scale dt of the current ones with cg S(U) of the current state
+//             added, then the implicit gravity
+enum UpMode { UP_PLAIN, UP_SAVE, UP_MEAN, UP_MIX, UP_IMEX1, UP_IMEX2 };
+struct UpArgs {
+  double scale;   // of the time step, for the current rates
+  double scale0;  // for the first stage's
+  double a0;      // UP_MIX
+  double cg;      // UP_IMEX2
+  double gam;     // implicit gravity
+  bool gravity;
 };
+
+// RK combine of a value with the saved one, in FP64.
+template <int M>
+__device__ __forceinline__ double up_combine(double x, double x0, double a0) {
+  return M == UP_MIX ? a0 * x0 + (1.0 - a0) * x : (x + x0) * 0.5;
+}
+
+// The entropy update (484:330-372) of interior zone (i,j,k) and the
+// conserved->primitive repair.
 template <typename R>
-__global__ void k_combine(CombineSeg<R> sg, long long total, double a0, int kind) {
-  const double a1 = 1.0 - a0;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    long long u = t;
-    int q = 0;
-    while (q < 4 && u >= sg.n[q]) {
-      u -= sg.n[q];
-      ++q;
-    }
-    if (q < 2) {
-      const double x = sg.x[q][u], x0 = sg.x0[q][u];
-      sg.x[q][u] = (R)(kind == 1 ? a0 * x0 + a1 * x : (x + x0) * 0.5);
-    } else {
-      const double x = sg.b[q - 2][u], x0 = sg.b0[q - 2][u];
-      sg.b[q - 2][u] = kind == 1 ? a0 * x0 + a1 * x : (x + x0) * 0.5;
-    }
-  }
+__device__ __forceinline__ void up_entropy(const Dims& d, const PhysC& ph, const DGeom& g, R* const* EF, long long o,
+                                           long long dk, R dt, R& en, R* U) {
+  const double *xa = g.f[CS_G_XF_AREA] + o, *ya = g.f[CS_G_YF_AREA] + o, *za = g.f[CS_G_ZF_AREA] + o;
+  const R div = (R)__ldg(xa) * EF[0][o] - (R)__ldg(xa - 1) * EF[0][o - 1] + (R)__ldg(ya) * EF[1][o] -
+                (R)__ldg(ya - d.NI) * EF[1][o - d.NI] + (R)__ldg(za) * EF[2][o] - (R)__ldg(za - dk) * EF[2][o - dk];
+  R V[8];
+  en = en - dt * div / (R)__ldg(g.f[CS_G_V_VOL] + o);
+  d_cons_to_prim(ph, en, U, V);
 }
 
 // Zone update (484:212-372): U += dt dU/dt on every zone, then on the
-// interior the entropy update and the conserved->primitive repair.  The
-// time step is scale times the device-resident step of the solve.
-template <typename R>
-__global__ void k_update_zones(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, double scale) {
-  const R dt = (R)(scale * *s.dt);
+// interior the entropy update and the conserved->primitive repair, with the
+// stage's combine and the IMEX gravity in the same pass.  The time step is
+// scale times the device-resident step of the solve.
+//
+// Gravity S(U) = (0, -rho g, -m . g), g = GM x / r^3, on the active zones
+// 0..N+1 (the zones of BUILD_NON_STIFF_SOURCES).  rho is unchanged by it, so
+// the implicit stage U = U* + a S(U) has the closed form m = m* - a rho g,
+// E = E* - a m . g.
+template <int M, typename R>
+__global__ void __launch_bounds__(TPB) k_update_zones(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, UpArgs a) {
+  const long long PS = (long long)NPANEL * d.S, dk = (long long)d.NI * d.NJ;
+  const R dt = (R)(a.scale * *s.dt), dt0 = (R)(a.scale0 * *s.dt), ag = (R)(a.gam * *s.dt);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    R U[8];
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
+    const bool inside = i >= 1 && i <= d.N && j >= 1 && j <= d.N && k >= 1 && k <= d.nr;
+    const bool heavy = (M == UP_IMEX1 || M == UP_IMEX2) && a.gravity && i >= 0 && i <= d.N + 1 && j >= 0 && j <= d.N + 1 &&
+                       k >= 0 && k <= d.nr + 1 && mask_at(g, d, p, i, j) == 1;
+    R gx = R(0.0), gy = R(0.0), gz = R(0.0);
+    if (heavy) {
+      const double* cen = g.f[CS_G_V_CEN] + o;
+      const R x = (R)__ldg(cen), y = (R)__ldg(cen + PS), z = (R)__ldg(cen + 2 * PS);
+      const R rad = sqrt(x * x + y * y + z * z);
+      const R gmb = R(ph.gm) * (R(1.0) / (rad * rad * rad));
+      gx = gmb * x;
+      gy = gmb * y;
+      gz = gmb * z;
+    }
+    const R* K = (M == UP_IMEX1 ? s.K1 : s.dUdt) + o;
+    R* const* EF = M == UP_IMEX1 ? s.EF1 : s.EF;
+    R U[8], en = R(0.0);
+    if (M == UP_IMEX2) {
+      R dU[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) U[q] = s.U[d.at(q, p, i, j, k)] + dt * s.dUdt[d.at(q, p, i, j, k)];
-    if (i >= 1 && i <= d.N && j >= 1 && j <= d.N && k >= 1 && k <= d.nr) {
-      const R div = geoR<R>(g, d, CS_G_XF_AREA, 0, p, i, j, k) * s.EF[0][d.at(0, p, i, j, k)] -
-                         geoR<R>(g, d, CS_G_XF_AREA, 0, p, i - 1, j, k) * s.EF[0][d.at(0, p, i - 1, j, k)] +
-                         geoR<R>(g, d, CS_G_YF_AREA, 0, p, i, j, k) * s.EF[1][d.at(0, p, i, j, k)] -
-                         geoR<R>(g, d, CS_G_YF_AREA, 0, p, i, j - 1, k) * s.EF[1][d.at(0, p, i, j - 1, k)] +
-                         geoR<R>(g, d, CS_G_ZF_AREA, 0, p, i, j, k) * s.EF[2][d.at(0, p, i, j, k)] -
-                         geoR<R>(g, d, CS_G_ZF_AREA, 0, p, i, j, k - 1) * s.EF[2][d.at(0, p, i, j, k - 1)];
-      R en = s.ent[d.at(0, p, i, j, k)] - dt * div / geoR<R>(g, d, CS_G_V_VOL, 0, p, i, j, k);
-      R V[8];
-      d_cons_to_prim(ph, en, U, V);
-      s.ent[d.at(0, p, i, j, k)] = en;
+      for (int q = 0; q < 8; ++q) dU[q] = K[q * PS];
+      if (heavy) {
+        const R c = (R)a.cg, rho = s.U[o], m1 = s.U[PS + o], m2 = s.U[2 * PS + o], m3 = s.U[3 * PS + o];
+        dU[1] += c * (-(gx * rho));
+        dU[2] += c * (-(gy * rho));
+        dU[3] += c * (-(gz * rho));
+        dU[4] += c * (-(gx * m1 + gy * m2 + gz * m3));
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) U[q] = s.U0[q * PS + o] + dt0 * s.K1[q * PS + o];
+      if (inside) {
+        en = s.ent0[o];
+        up_entropy(d, ph, g, s.EF1, o, dk, dt0, en, U);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) U[q] = U[q] + dt * dU[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        U[q] = s.U[q * PS + o];
+        if (M == UP_SAVE || M == UP_IMEX1) s.U0[q * PS + o] = U[q];
+        if (M == UP_MEAN || M == UP_MIX) U[q] = (R)up_combine<M>((double)U[q], (double)s.U0[q * PS + o], a.a0);
+        U[q] = U[q] + dt * K[q * PS];
+      }
+      en = s.ent[o];
+      if (M == UP_SAVE || M == UP_IMEX1) s.ent0[o] = en;
+      if (M == UP_MEAN || M == UP_MIX) en = (R)up_combine<M>((double)en, (double)s.ent0[o], a.a0);
+    }
+    if (inside) up_entropy(d, ph, g, EF, o, dk, dt, en, U);
+    else if (M == UP_IMEX2) en = s.ent0[o];
+    if (M != UP_PLAIN || inside) s.ent[o] = en;
+    if (heavy) {
+      U[1] = U[1] - ag * (gx * U[0]);
+      U[2] = U[2] - ag * (gy * U[0]);
+      U[3] = U[3] - ag * (gz * U[0]);
+      U[4] = U[4] - ag * (gx * U[1] + gy * U[2] + gz * U[3]);
     }
 #pragma unroll
-    for (int q = 0; q < 8; ++q) s.U[d.at(q, p, i, j, k)] = U[q];
+    for (int q = 0; q < 8; ++q) s.U[q * PS + o] = U[q];
   }
 }
 
@@ -179,43 +238,80 @@ __device__ __forceinline__ double vang(const DGeom& g, const Dims& d, int p, int
 }
 
 // Constrained-transport face update (484:376-906): Stokes circulation of
-// the edge EMFs with spherical arc lengths for the angular edges.
-template <typename R>
-__global__ void k_ct(Dims d, DGeom g, DStateT<R> s, Range3 r, int dir, double scale) {
-  const double dt = scale * *s.dt;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
+// the edge EMFs with spherical arc lengths for the angular edges, with the
+// stage's save, combine or restore of face B in the same pass.  One launch
+// for the three face directions over every face of the box; only the
+// interior zones' faces have a circulation.
+template <int M, typename R>
+__global__ void __launch_bounds__(TPB) k_ct(Dims d, DGeom g, DStateT<R> s, Range3 r, UpArgs a) {
+  const double dt = a.scale * *s.dt, dt0 = a.scale0 * *s.dt;
+  const long long dk = (long long)d.NI * d.NJ;
+  const unsigned nb = (unsigned)((r.count() + TPB - 1) / TPB);
+  for (unsigned T = blockIdx.x; T < 3 * nb; T += gridDim.x) {
+    const int dir = T % 3;
+    const long long t = (long long)(T / 3) * TPB + threadIdx.x;
+    if (t >= r.count()) continue;
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    const double* Ex = s.Ef[0];
-    const double* Ey = s.Ef[1];
-    const double* Ez = s.Ef[2];
-    if (dir == 0) {
-      const double rout = vrad(g, d, p, i, j, k), rin = vrad(g, d, p, i, j, k - 1), dr = rout - rin;
-      const double th = vang(g, d, p, i, j, i, j - 1, k, 1.0 / rout);
-      const double lin = rin * th, lout = rout * th;
-      const double c = dr * Ez[d.at(0, p, i, j, k)] - dr * Ez[d.at(0, p, i, j - 1, k)] - lout * Ey[d.at(0, p, i, j, k)] +
-                       lin * Ey[d.at(0, p, i, j, k - 1)];
-      double& b = s.Bxf[d.at(0, p, i, j, k)];
-      b = b - dt * c / geo(g, d, CS_G_XF_AREA, 0, p, i, j, k);
-    } else if (dir == 1) {
-      const double rout = vrad(g, d, p, i, j, k), rin = vrad(g, d, p, i, j, k - 1), dr = rout - rin;
-      const double th = vang(g, d, p, i, j, i - 1, j, k, 1.0 / rout);
-      const double lin = rin * th, lout = rout * th;
-      const double c = -dr * Ez[d.at(0, p, i, j, k)] + dr * Ez[d.at(0, p, i - 1, j, k)] + lout * Ex[d.at(0, p, i, j, k)] -
-                       lin * Ex[d.at(0, p, i, j, k - 1)];
-      double& b = s.Byf[d.at(0, p, i, j, k)];
-      b = b - dt * c / geo(g, d, CS_G_YF_AREA, 0, p, i, j, k);
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
+    double* B = dir == 0 ? s.Bxf : (dir == 1 ? s.Byf : s.Bzf);
+    double* B0 = dir == 0 ? s.B0[0] : (dir == 1 ? s.B0[1] : s.B0[2]);
+    const bool inside = i >= (dir != 0) && i <= d.N && j >= (dir != 1) && j <= d.N && k >= (dir != 2) && k <= d.nr;
+    if (M == UP_PLAIN && !inside) continue;
+    double b;
+    if (M == UP_IMEX2) {
+      b = B0[o];
     } else {
-      const double rout = vrad(g, d, p, i, j, k), inv = 1.0 / rout;
-      const double lxp = rout * vang(g, d, p, i, j, i - 1, j, k, inv);
-      const double lxm = rout * vang(g, d, p, i, j - 1, i - 1, j - 1, k, inv);
-      const double lyp = rout * vang(g, d, p, i, j, i, j - 1, k, inv);
-      const double lym = rout * vang(g, d, p, i - 1, j, i - 1, j - 1, k, inv);
-      const double c = lyp * Ey[d.at(0, p, i, j, k)] - lym * Ey[d.at(0, p, i - 1, j, k)] - lxp * Ex[d.at(0, p, i, j, k)] +
-                       lxm * Ex[d.at(0, p, i, j - 1, k)];
-      double& b = s.Bzf[d.at(0, p, i, j, k)];
-      b = b - dt * c / geo(g, d, CS_G_ZF_AREA, 0, p, i, j, k);
+      b = B[o];
+      if (M == UP_SAVE || M == UP_IMEX1) B0[o] = b;
+      if (M == UP_MEAN || M == UP_MIX) b = up_combine<M>(b, B0[o], a.a0);
     }
+    if (inside) {
+      // circulation: the lengths of the four edges once, then the EMFs of the
+      // current rates (and of the first stage's)
+      double w[4];
+      long long e[4];
+      const double area = __ldg((dir == 0 ? g.f[CS_G_XF_AREA] : (dir == 1 ? g.f[CS_G_YF_AREA] : g.f[CS_G_ZF_AREA])) + o);
+      const double rout = vrad(g, d, p, i, j, k);
+      int c0, c2;  // EMF components of edges 0, 1 and 2, 3
+      if (dir == 2) {
+        const double inv = 1.0 / rout;
+        w[0] = rout * vang(g, d, p, i, j, i, j - 1, k, inv);
+        w[1] = -rout * vang(g, d, p, i - 1, j, i - 1, j - 1, k, inv);
+        w[2] = -rout * vang(g, d, p, i, j, i - 1, j, k, inv);
+        w[3] = rout * vang(g, d, p, i, j - 1, i - 1, j - 1, k, inv);
+        c0 = 1;
+        c2 = 0;
+        e[0] = o;
+        e[1] = o - 1;
+        e[2] = o;
+        e[3] = o - d.NI;
+      } else {
+        const double rin = vrad(g, d, p, i, j, k - 1), dr = rout - rin;
+        const double th = dir == 0 ? vang(g, d, p, i, j, i, j - 1, k, 1.0 / rout) : vang(g, d, p, i, j, i - 1, j, k, 1.0 / rout);
+        const double sg = dir == 0 ? 1.0 : -1.0;
+        w[0] = sg * dr;
+        w[1] = -sg * dr;
+        w[2] = -sg * (rout * th);
+        w[3] = sg * (rin * th);
+        c0 = 2;
+        c2 = dir == 0 ? 1 : 0;
+        e[0] = o;
+        e[1] = o - (dir == 0 ? d.NI : 1);
+        e[2] = o;
+        e[3] = o - dk;
+      }
+      if (M == UP_IMEX2) {
+        const double* Ea = c0 == 2 ? s.Ef1[2] : s.Ef1[1];
+        const double* Eb = c2 == 1 ? s.Ef1[1] : s.Ef1[0];
+        b = b - dt0 * (w[0] * Ea[e[0]] + w[1] * Ea[e[1]] + w[2] * Eb[e[2]] + w[3] * Eb[e[3]]) / area;
+      }
+      double* const* Ef = M == UP_IMEX1 ? s.Ef1 : s.Ef;
+      const double* Ea = c0 == 2 ? Ef[2] : Ef[1];
+      const double* Eb = c2 == 1 ? Ef[1] : Ef[0];
+      b = b - dt * (w[0] * Ea[e[0]] + w[1] * Ea[e[1]] + w[2] * Eb[e[2]] + w[3] * Eb[e[3]]) / area;
+    }
+    B[o] = b;
   }
 }
 
@@ -359,182 +455,45 @@ void launch_fill_ghosts(Solve& sv) {
     launch_fill_ghosts_t(sv, sv.st);
 }
 
-template <typename R>
-void launch_save_stage0_t(Solve& sv, const DStateT<R>& st) {
-  const size_t S6 = (size_t)6 * sv.d.S;
-  cudaMemcpyAsync(st.U0, st.U, NVAR * S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.ent0, st.ent, S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.B0[0], st.Bxf, S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.B0[1], st.Byf, S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.B0[2], st.Bzf, S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  mark(sv, "copy_stage0", false);
-}
-void launch_save_stage0(Solve& sv) {
-  if (sv.fp32)
-    launch_save_stage0_t(sv, sv.stF);
-  else
-    launch_save_stage0_t(sv, sv.st);
-}
-
-template <typename R>
-void launch_combine_t(Solve& sv, const DStateT<R>& st, double a0, int kind) {
-  const long long S6 = 6LL * sv.d.S;
-  CombineSeg<R> sg;
-  sg.x[0] = st.U;     sg.x0[0] = st.U0;    sg.n[0] = NVAR * S6;
-  sg.x[1] = st.ent;   sg.x0[1] = st.ent0;  sg.n[1] = S6;
-  sg.b[0] = st.Bxf;   sg.b0[0] = st.B0[0]; sg.n[2] = S6;
-  sg.b[1] = st.Byf;   sg.b0[1] = st.B0[1]; sg.n[3] = S6;
-  sg.b[2] = st.Bzf;   sg.b0[2] = st.B0[2]; sg.n[4] = S6;
-  const long long total = (NVAR + 4) * S6;
-  k_combine<R><<<blocks_for(total, 256, grid_sms(sv)), 256, 0, sv.stream>>>(sg, total, a0, kind);
-  mark(sv, "k_combine");
-}
-void launch_combine(Solve& sv, double a0, int kind) {
-  if (sv.fp32)
-    launch_combine_t(sv, sv.stF, a0, kind);
-  else
-    launch_combine_t(sv, sv.st, a0, kind);
-}
-
-template <typename R>
-void launch_update_with(Solve& sv, const DStateT<R>& st, double scale) {
+template <int M, typename R>
+void launch_update_mode(Solve& sv, const DStateT<R>& st, const UpArgs& a) {
   const Dims& d = sv.d;
-  Range3 z = zones_all(d);
-  k_update_zones<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z, scale);
+  const Range3 z = zones_all(d);
+  k_update_zones<M, R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z, a);
   mark(sv, "k_update_zones");
-  const int N = d.N, nr = d.nr;
-  Range3 fx = {0, N, 1, N, 1, nr}, fy = {1, N, 0, N, 1, nr}, fz = {1, N, 1, N, 0, nr};
-  k_ct<R><<<blocks_for(fx.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, fx, 0, scale);
-  mark(sv, "k_ct");
-  k_ct<R><<<blocks_for(fy.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, fy, 1, scale);
-  mark(sv, "k_ct");
-  k_ct<R><<<blocks_for(fz.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, fz, 2, scale);
+  // UP_PLAIN touches the interior zones' faces only
+  const Range3 f = M == UP_PLAIN ? Range3{0, d.N, 0, d.N, 0, d.nr} : Range3{-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G};
+  const long long nb = 3 * ((f.count() + TPB - 1) / TPB);
+  k_ct<M, R><<<(int)std::min<long long>(nb, (long long)grid_sms(sv) * 64), TPB, 0, sv.stream>>>(d, sv.g, st, f, a);
   mark(sv, "k_ct");
 }
-template void launch_update_with<double>(Solve&, const DStateT<double>&, double);
-template void launch_update_with<float>(Solve&, const DStateT<float>&, double);
-
-void launch_update(Solve& sv, double scale) {
-  if (sv.fp32)
-    launch_update_with(sv, sv.stF, scale);
-  else
-    launch_update_with(sv, sv.st, scale);
-}
-
-// ---- IMEX-RK2: ARS(2,2,2) with the point-mass gravity implicit ----
-// Gravity S(U) = (0, -rho g, -m . g), g = GM x / r^3, on the active zones
-// 0..N+1 (the zones of BUILD_NON_STIFF_SOURCES).  rho is unchanged by it,
-// so the implicit stage U = U* + a S(U) has the closed form
-// m = m* - a rho g, E = E* - a m . g.
 template <typename R>
-__global__ void k_gravity_implicit(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, double scale) {
-  const R a = (R)(scale * *s.dt);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    if (mask_at(g, d, p, i, j) != 1) continue;
-    const R x = geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k), y = geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k),
-                 z = geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    const R rad = sqrt(x * x + y * y + z * z);
-    const R gmb = R(ph.gm) * (R(1.0) / (rad * rad * rad));
-    const R gx = gmb * x, gy = gmb * y, gz = gmb * z;
-    const R rho = s.U[d.at(0, p, i, j, k)];
-    R& m1 = s.U[d.at(1, p, i, j, k)];
-    R& m2 = s.U[d.at(2, p, i, j, k)];
-    R& m3 = s.U[d.at(3, p, i, j, k)];
-    m1 = m1 - a * (gx * rho);
-    m2 = m2 - a * (gy * rho);
-    m3 = m3 - a * (gz * rho);
-    R& e = s.U[d.at(4, p, i, j, k)];
-    e = e - a * (gx * m1 + gy * m2 + gz * m3);
+void launch_update_t(Solve& sv, const DStateT<R>& st, int mode, const UpArgs& a) {
+  switch (mode) {
+    case UP_PLAIN: launch_update_mode<UP_PLAIN>(sv, st, a); break;
+    case UP_SAVE: launch_update_mode<UP_SAVE>(sv, st, a); break;
+    case UP_MEAN: launch_update_mode<UP_MEAN>(sv, st, a); break;
+    case UP_MIX: launch_update_mode<UP_MIX>(sv, st, a); break;
+    case UP_IMEX1: launch_update_mode<UP_IMEX1>(sv, st, a); break;
+    default: launch_update_mode<UP_IMEX2>(sv, st, a);
   }
 }
-
-// dUdt += c S(U) with the gravity of the current state (explicit use of
-// the previous stage's source).
-template <typename R>
-__global__ void k_add_gravity(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, R c) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    if (mask_at(g, d, p, i, j) != 1) continue;
-    const R x = geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k), y = geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k),
-                 z = geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    const R rad = sqrt(x * x + y * y + z * z);
-    const R gmb = R(ph.gm) * (R(1.0) / (rad * rad * rad));
-    const R gx = gmb * x, gy = gmb * y, gz = gmb * z;
-    const R rho = s.U[d.at(0, p, i, j, k)];
-    const R m1 = s.U[d.at(1, p, i, j, k)], m2 = s.U[d.at(2, p, i, j, k)], m3 = s.U[d.at(3, p, i, j, k)];
-    s.dUdt[d.at(1, p, i, j, k)] += c * (-(gx * rho));
-    s.dUdt[d.at(2, p, i, j, k)] += c * (-(gy * rho));
-    s.dUdt[d.at(3, p, i, j, k)] += c * (-(gz * rho));
-    s.dUdt[d.at(4, p, i, j, k)] += c * (-(gx * m1 + gy * m2 + gz * m3));
-  }
-}
-
-template <typename R>
-void launch_gravity_implicit_t(Solve& sv, const DStateT<R>& st, double scale) {
-  Range3 z = {0, sv.d.N + 1, 0, sv.d.N + 1, 0, sv.d.nr + 1};
-  k_gravity_implicit<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, z,
-                                                                                        scale);
-  mark(sv, "k_gravity_implicit");
-}
-void launch_gravity_implicit(Solve& sv, double scale) {
-  if (!(sv.ph.gm > sv.p.smallnum)) return;
+static void launch_update_args(Solve& sv, int mode, UpArgs a) {
+  a.gravity = sv.ph.gm > sv.p.smallnum;
   if (sv.fp32)
-    launch_gravity_implicit_t(sv, sv.stF, scale);
+    launch_update_t(sv, sv.stF, mode, a);
   else
-    launch_gravity_implicit_t(sv, sv.st, scale);
+    launch_update_t(sv, sv.st, mode, a);
 }
-
-template <typename R>
-void launch_add_gravity_t(Solve& sv, const DStateT<R>& st, double c) {
-  Range3 z = {0, sv.d.N + 1, 0, sv.d.N + 1, 0, sv.d.nr + 1};
-  k_add_gravity<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, z, c);
-  mark(sv, "k_add_gravity");
+void launch_update(Solve& sv, double scale) { launch_update_args(sv, UP_PLAIN, {scale, 0.0, 0.0, 0.0, 0.0, false}); }
+void launch_update_rk(Solve& sv, int irk, double a0, double scale) {
+  launch_update_args(sv, irk == 1 ? UP_SAVE : (a0 > 0.0 ? UP_MIX : UP_MEAN), {scale, 0.0, a0, 0.0, 0.0, false});
 }
-void launch_add_gravity(Solve& sv, double c) {
-  if (!(sv.ph.gm > sv.p.smallnum)) return;
-  if (sv.fp32)
-    launch_add_gravity_t(sv, sv.stF, c);
+void launch_update_imex(Solve& sv, int irk, double gam, double del) {
+  if (irk == 1)
+    launch_update_args(sv, UP_IMEX1, {gam, 0.0, 0.0, 0.0, gam, false});
   else
-    launch_add_gravity_t(sv, sv.st, c);
-}
-
-// Copies of the first stage's flux divergence, entropy fluxes and EMFs,
-// and the restore of the step's initial state.
-template <typename R>
-void launch_save_stage1_rates_t(Solve& sv, const DStateT<R>& st) {
-  const size_t S6 = (size_t)6 * sv.d.S;
-  cudaMemcpyAsync(st.K1, st.dUdt, NVAR * S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-  for (int q = 0; q < 3; ++q) {
-    cudaMemcpyAsync(st.EF1[q], st.EF[q], S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-    cudaMemcpyAsync(st.Ef1[q], st.Ef[q], S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  }
-  mark(sv, "copy_stage1_rates", false);
-}
-void launch_save_stage1_rates(Solve& sv) {
-  if (sv.fp32)
-    launch_save_stage1_rates_t(sv, sv.stF);
-  else
-    launch_save_stage1_rates_t(sv, sv.st);
-}
-
-template <typename R>
-void launch_restore_stage0_t(Solve& sv, const DStateT<R>& st) {
-  const size_t S6 = (size_t)6 * sv.d.S;
-  cudaMemcpyAsync(st.U, st.U0, NVAR * S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.ent, st.ent0, S6 * sizeof(R), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.Bxf, st.B0[0], S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.Byf, st.B0[1], S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  cudaMemcpyAsync(st.Bzf, st.B0[2], S6 * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream);
-  mark(sv, "copy_restore", false);
-}
-void launch_restore_stage0(Solve& sv) {
-  if (sv.fp32)
-    launch_restore_stage0_t(sv, sv.stF);
-  else
-    launch_restore_stage0_t(sv, sv.st);
+    launch_update_args(sv, UP_IMEX2, {1.0 - del, del, 0.0, (1.0 - gam) / (1.0 - del), gam, false});
 }
 
 template <typename R>
@@ -543,8 +502,8 @@ void launch_cleanup_t(Solve& sv, const DStateT<R>& st) {
   k_cleanup_zones<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, z);
   mark(sv, "k_cleanup_zones");
 }
-void launch_cleanup(Solve& sv) {
-  launch_face_masks(sv);
+void launch_cleanup(Solve& sv, bool masks) {
+  if (masks) launch_face_masks(sv);
   if (sv.fp32)
     launch_cleanup_t(sv, sv.stF);
   else
