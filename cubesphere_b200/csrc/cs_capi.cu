@@ -1035,9 +1035,9 @@ void drop_graph(Solve& sv) {
 int read_dt(Solve& sv, double* out) {
   unsigned long long bits = 0;
   int flag = 0;
-  const unsigned long long* dtmin = sv.fp32 ? sv.stF.dtmin : sv.st.dtmin;
+  const double* dt = sv.fp32 ? sv.stF.dt : sv.st.dt;
   const int* err_flag = sv.fp32 ? sv.stF.err_flag : sv.st.err_flag;
-  CS_CUDA(sv, cudaMemcpyAsync(&bits, dtmin, sizeof(bits), cudaMemcpyDeviceToHost, sv.stream));
+  CS_CUDA(sv, cudaMemcpyAsync(&bits, dt, sizeof(bits), cudaMemcpyDeviceToHost, sv.stream));
   CS_CUDA(sv, cudaMemcpyAsync(&flag, err_flag, sizeof(flag), cudaMemcpyDeviceToHost, sv.stream));
   CS_CUDA(sv, cudaStreamSynchronize(sv.stream));
   if (flag) return fail(sv, CS_ERR_CUDA, "a bounded device wait gave up (bulk copy did not complete)");

@@ -80,7 +80,8 @@ struct DStateT {
   const int8_t* adp_pmap;                // inverse shared by the panels: per panel [unknown map 36][sign 36], or null
   int* err_flag;                         // device-side error bits (bounded waits that gave up)
   int32_t* giveup;                       // positivity give-up flags per zone
-  unsigned long long* dtmin;             // CFL reduction target (bit pattern of a positive double)
+  unsigned long long* dtmin;             // CFL reduction target (bit pattern of a positive double), then the count of
+                                         // blocks that are done
   double* dt;                            // the solve's current time step (device scalar)
 };
 using DState = DStateT<double>;
@@ -100,20 +101,23 @@ __device__ __forceinline__ R geoR(const DGeom& g, const Dims& d, int f, int c, i
   return (R)__ldg(g.f[f] + d.at(c, p, i, j, k));
 }
 
-// Decode a flat thread index over panels x a 3-D index range.
+// Decode a flat thread index over panels x a 3-D index range, in 32 bits (a
+// solve has fewer than 2^28 points): 64-bit divisions by run-time extents
+// took most of the instructions of the small kernels.
 struct Range3 {
   int i0, i1, j0, j1, k0, k1;
   __host__ __device__ long long count() const {
     return 6LL * (long long)(i1 - i0 + 1) * (j1 - j0 + 1) * (k1 - k0 + 1);
   }
   __device__ void decode(long long t, int& p, int& i, int& j, int& k) const {
-    const long long ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
-    i = (int)(t % ni) + i0;
-    t /= ni;
-    j = (int)(t % nj) + j0;
-    t /= nj;
-    k = (int)(t % nk) + k0;
-    p = (int)(t / nk);
+    const unsigned ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
+    unsigned u = (unsigned)t, v = u / ni;
+    i = (int)(u - v * ni) + i0;
+    u = v / nj;
+    j = (int)(v - u * nj) + j0;
+    v = u / nk;
+    k = (int)(u - v * nk) + k0;
+    p = (int)v;
   }
 };
 

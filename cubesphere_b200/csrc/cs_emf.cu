@@ -7,6 +7,8 @@
 // (pkg/inc/cubesphere/400riemann_integrate/460make_edge_fields_p1.f:335-7037),
 // Two_D_RS_Ez_4State_HLL (620riemann_2d/630...:10-372) and
 // Two_D_RS_Ez_3State_HLL (620riemann_2d/631...:9-338).  One thread per edge.
+#include <algorithm>
+
 #include "cs_solve.h"
 
 namespace cs {
@@ -28,202 +30,181 @@ __device__ __forceinline__ double Bqa(const DStateT<R>& s, const Dims& d, int di
   return s.Bq[dir][d.at(q, p, i, j, k)];
 }
 
-// Simpson point jq on the edge between vertices a and b.
-__device__ __forceinline__ void edge_point(const DGeom& g, const Dims& d, int p, int jq, int ax, int ay, int az, int bx,
-                                           int by, int bz, bool rescale, double* e) {
-  if (jq == 0) {
-    double va[3];
+// E along the tangent of the edge between the vertices va and vb (one sphere)
+// by Simpson's rule: at each point P (the two ends and the middle) the tangent
+// t = va - vb is made orthogonal to the radial direction and normalised,
+//   E . n = (t.E - (t.P)(P.E) / P.P) / sqrt(t.t - (t.P)^2 / P.P).
+__device__ __forceinline__ double along_edge(const double* va, const double* vb, const double* E) {
+  double t[3], m[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      va[q] = geo(g, d, CS_G_VERT, q, p, ax, ay, az);
-      e[q] = 0.5 * (va[q] + geo(g, d, CS_G_VERT, q, p, bx, by, bz));
-    }
-    if (rescale) {
-      const double t = sqrt(va[0] * va[0] + va[1] * va[1] + va[2] * va[2]) / sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) e[q] = e[q] * t;
-    }
-  } else if (jq == 1) {
-#pragma unroll
-    for (int q = 0; q < 3; ++q) e[q] = geo(g, d, CS_G_VERT, q, p, ax, ay, az);
-  } else {
-#pragma unroll
-    for (int q = 0; q < 3; ++q) e[q] = geo(g, d, CS_G_VERT, q, p, bx, by, bz);
+  for (int q = 0; q < 3; ++q) {
+    t[q] = va[q] - vb[q];
+    m[q] = va[q] + vb[q];
   }
+  const double tt = t[0] * t[0] + t[1] * t[1] + t[2] * t[2], tE = t[0] * E[0] + t[1] * E[1] + t[2] * E[2];
+  auto at = [&](const double* P) {
+    const double tP = t[0] * P[0] + t[1] * P[1] + t[2] * P[2];
+    const double f = tP / (P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
+    return (tE - f * (P[0] * E[0] + P[1] * E[1] + P[2] * E[2])) / sqrt(tt - f * tP);
+  };
+  return (4.0 / 6.0) * at(m) + (1.0 / 6.0) * (at(va) + at(vb));
 }
-__device__ __forceinline__ void unit3(double* v) {
-  const double t = 1.0 / sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  v[0] = v[0] * t;
-  v[1] = v[1] * t;
-  v[2] = v[2] * t;
+__device__ __forceinline__ double llf_speed(double a, double b, double c, double e) {
+  return fmax(fmax(fabs(a), fabs(b)), fmax(fabs(c), fabs(e)));
 }
-__device__ __forceinline__ void orth3(double* v, const double* n) {
-  const double t = v[0] * n[0] + v[1] * n[1] + v[2] * n[2];
-  v[0] = v[0] - t * n[0];
-  v[1] = v[1] - t * n[1];
-  v[2] = v[2] - t * n[2];
-  unit3(v);
-}
-__device__ __forceinline__ void llf4(double& SR, double& SL, double& SU, double& SD) {
-  const double t = fmax(fmax(fabs(SR), fabs(SL)), fmax(fabs(SU), fabs(SD)));
-  SR = t;
-  SL = -t;
-  SU = t;
-  SD = -t;
+
+// The symmetrised (LLF) speeds and one E for the four states, USE_2D_LLF_RS_FOR_EZ:
+// with S_R = S_U = -S_L = -S_D = s the four-state solver (d_rs4, 630:10-372)
+// has its interaction region's centroid at the origin, and its two averages
+// agree and reduce to
+//   E + s / (2 sin) ((B_y,R - B_y,L) - (B_n,U - B_n,D)).
+__device__ __forceinline__ double llf_emf(double s, double sin_t, double E, double BnU, double BnD, double ByR, double ByL) {
+  return E + 0.5 * s * ((ByR - ByL) - (BnU - BnD)) / sin_t;
 }
 
 // x-edges (460:393-1493): i in 1..N, j in 0..N, k in 0..nr.
 template <typename R>
-__global__ void k_edges_x(Dims d, DGeom g, DStateT<R> s, Range3 r) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    const double Ex = (E1(s, d, 0, p, i, j, k) + E1(s, d, 0, p, i, j + 1, k) + E1(s, d, 0, p, i, j + 1, k + 1) + E1(s, d, 0, p, i, j, k + 1)) * 0.25;
-    const double Ey = (E1(s, d, 1, p, i, j, k) + E1(s, d, 1, p, i, j + 1, k) + E1(s, d, 1, p, i, j + 1, k + 1) + E1(s, d, 1, p, i, j, k + 1)) * 0.25;
-    const double Ez = (E1(s, d, 2, p, i, j, k) + E1(s, d, 2, p, i, j + 1, k) + E1(s, d, 2, p, i, j + 1, k + 1) + E1(s, d, 2, p, i, j, k + 1)) * 0.25;
-    const double ByR = Bqa(s, d, 2, 4, p, i, j + 1, k), ByL = Bqa(s, d, 2, 3, p, i, j, k);
-    const double BnU = Bqa(s, d, 1, 2, p, i, j, k + 1), BnD = Bqa(s, d, 1, 1, p, i, j, k);
-    double SR = fmax(Sg(s.S[3], d, p, i, j, k + 1), Sg(s.S[3], d, p, i, j, k));
-    double SL = fmin(Sg(s.S[2], d, p, i, j, k + 1), Sg(s.S[2], d, p, i, j, k));
-    double SU = fmax(Sg(s.S[5], d, p, i, j + 1, k), Sg(s.S[5], d, p, i, j, k));
-    double SD = fmin(Sg(s.S[4], d, p, i, j + 1, k), Sg(s.S[4], d, p, i, j, k));
-    llf4(SR, SL, SU, SD);
-    double acc = 0.0;
-    for (int jq = 0; jq < 3; ++jq) {
-      const double wt = jq == 0 ? 4.0 / 6.0 : 1.0 / 6.0;
-      double n2[3], n3[3];
-      edge_point(g, d, p, jq, i, j, k, i - 1, j, k, true, n2);
-      unit3(n2);
+__device__ __forceinline__ void edge_x(const Dims& d, const DGeom& g, const DStateT<R>& s, int p, int i, int j, int k) {
+  const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
+  const int dj = d.NI, dk = d.NI * d.NJ;
+  double E[3], va[3], vb[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) n3[q] = geo(g, d, CS_G_VERT, q, p, i, j, k) - geo(g, d, CS_G_VERT, q, p, i - 1, j, k);
-      orth3(n3, n2);
-      const double Ezl = Ex * n3[0] + Ey * n3[1] + Ez * n3[2];
-      acc = acc + wt * d_rs4(SR, SL, SU, SD, 0.0, 1.0, Ezl, BnU, BnD, ByR, ByL);
-    }
-    s.Ef[0][d.at(0, p, i, j, k)] = acc;
+  for (int q = 0; q < 3; ++q) {
+    const R* e = s.E + q * PS + o;
+    E[q] = ((double)e[0] + (double)e[dj] + (double)e[dj + dk] + (double)e[dk]) * 0.25;
+    va[q] = __ldg(g.f[CS_G_VERT] + q * PS + o);
+    vb[q] = __ldg(g.f[CS_G_VERT] + q * PS + o - 1);
   }
+  const double sp = fmax(llf_speed(s.S[3][o + dk], s.S[3][o], s.S[2][o + dk], s.S[2][o]),
+                         llf_speed(s.S[5][o + dj], s.S[5][o], s.S[4][o + dj], s.S[4][o]));
+  s.Ef[0][o] = llf_emf(sp, 1.0, along_edge(va, vb, E), s.Bq[1][2 * PS + o + dk], s.Bq[1][PS + o], s.Bq[2][4 * PS + o + dj],
+                       s.Bq[2][3 * PS + o]);
 }
 
 // y-edges (460:1497-2587): i in 0..N, j in 1..N, k in 0..nr.
 template <typename R>
-__global__ void k_edges_y(Dims d, DGeom g, DStateT<R> s, Range3 r) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
-    int p, i, j, k;
-    r.decode(t, p, i, j, k);
-    const double Ex = (E1(s, d, 0, p, i, j, k) + E1(s, d, 0, p, i, j, k + 1) + E1(s, d, 0, p, i + 1, j, k + 1) + E1(s, d, 0, p, i + 1, j, k)) * 0.25;
-    const double Ey = (E1(s, d, 1, p, i, j, k) + E1(s, d, 1, p, i, j, k + 1) + E1(s, d, 1, p, i + 1, j, k + 1) + E1(s, d, 1, p, i + 1, j, k)) * 0.25;
-    const double Ez = (E1(s, d, 2, p, i, j, k) + E1(s, d, 2, p, i, j, k + 1) + E1(s, d, 2, p, i + 1, j, k + 1) + E1(s, d, 2, p, i + 1, j, k)) * 0.25;
-    const double ByR = Bqa(s, d, 0, 4, p, i, j, k + 1), ByL = Bqa(s, d, 0, 3, p, i, j, k);
-    const double BnU = Bqa(s, d, 2, 2, p, i + 1, j, k), BnD = Bqa(s, d, 2, 1, p, i, j, k);
-    double SR = fmax(Sg(s.S[5], d, p, i + 1, j, k), Sg(s.S[5], d, p, i, j, k));
-    double SL = fmin(Sg(s.S[4], d, p, i + 1, j, k), Sg(s.S[4], d, p, i, j, k));
-    double SU = fmax(Sg(s.S[1], d, p, i, j, k), Sg(s.S[1], d, p, i, j, k + 1));
-    double SD = fmin(Sg(s.S[0], d, p, i, j, k), Sg(s.S[0], d, p, i, j, k + 1));
-    llf4(SR, SL, SU, SD);
-    double acc = 0.0;
-    for (int jq = 0; jq < 3; ++jq) {
-      const double wt = jq == 0 ? 4.0 / 6.0 : 1.0 / 6.0;
-      double n1[3], n3[3];
-      edge_point(g, d, p, jq, i, j, k, i, j - 1, k, true, n1);
-      unit3(n1);
+__device__ __forceinline__ void edge_y(const Dims& d, const DGeom& g, const DStateT<R>& s, int p, int i, int j, int k) {
+  const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
+  const int dk = d.NI * d.NJ;
+  double E[3], va[3], vb[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) n3[q] = geo(g, d, CS_G_VERT, q, p, i, j, k) - geo(g, d, CS_G_VERT, q, p, i, j - 1, k);
-      orth3(n3, n1);
-      const double Ezl = Ex * n3[0] + Ey * n3[1] + Ez * n3[2];
-      acc = acc + wt * d_rs4(SR, SL, SU, SD, 0.0, 1.0, Ezl, BnU, BnD, ByR, ByL);
+  for (int q = 0; q < 3; ++q) {
+    const R* e = s.E + q * PS + o;
+    E[q] = ((double)e[0] + (double)e[dk] + (double)e[dk + 1] + (double)e[1]) * 0.25;
+    va[q] = __ldg(g.f[CS_G_VERT] + q * PS + o);
+    vb[q] = __ldg(g.f[CS_G_VERT] + q * PS + o - d.NI);
+  }
+  const double sp = fmax(llf_speed(s.S[5][o + 1], s.S[5][o], s.S[4][o + 1], s.S[4][o]),
+                         llf_speed(s.S[1][o + dk], s.S[1][o], s.S[0][o + dk], s.S[0][o]));
+  s.Ef[1][o] = llf_emf(sp, 1.0, along_edge(va, vb, E), s.Bq[2][2 * PS + o + 1], s.Bq[2][PS + o], s.Bq[0][4 * PS + o + dk],
+                       s.Bq[0][3 * PS + o]);
+}
+
+// z-edges (460:2591-3721): i, j in 0..N, k in 1..nr, zero where a neighbour
+// is masked; the four cube corners (460:3725-7037) use the three-state
+// solver.  The vertices of a radial edge are radii times one unit vector, so
+// the three points of the rule share one frame.
+template <typename R>
+__device__ __forceinline__ void edge_z(const Dims& d, const DGeom& g, const DStateT<R>& s, int p, int i, int j, int k) {
+  const int N = d.N, dj = d.NI;
+  const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
+  double e[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) e[q] = __ldg(g.f[CS_G_VERT] + q * PS + o);
+  const double en = 1.0 / sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
+#pragma unroll
+  for (int q = 0; q < 3; ++q) e[q] = e[q] * en;
+  const bool corner = (i == 0 || i == N) && (j == 0 || j == N);
+  if (!corner) {
+    if (mask_at(g, d, p, i, j) == 0 || mask_at(g, d, p, i + 1, j) == 0 || mask_at(g, d, p, i + 1, j + 1) == 0 ||
+        mask_at(g, d, p, i, j + 1) == 0) {
+      s.Ef[2][o] = 0.0;
+      return;
     }
-    s.Ef[1][d.at(0, p, i, j, k)] = acc;
+    double E = 0.0, n1[3], ta[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const R* z = s.E + q * PS + o;
+      E = E + ((double)z[0] + (double)z[1] + (double)z[1 + dj] + (double)z[dj]) * 0.25 * e[q];
+      const double* v = g.f[CS_G_VERT] + q * PS + o;
+      n1[q] = __ldg(v + 1) - __ldg(v - 1);
+      ta[q] = __ldg(v + dj) - __ldg(v - dj);
+    }
+    // cosine of the angle between the two families' normals, made orthogonal
+    // to the edge
+    const double ne = n1[0] * e[0] + n1[1] * e[1] + n1[2] * e[2], te = ta[0] * e[0] + ta[1] * e[1] + ta[2] * e[2];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      n1[q] = n1[q] - ne * e[q];
+      ta[q] = ta[q] - te * e[q];
+    }
+    const double nn = n1[0] * n1[0] + n1[1] * n1[1] + n1[2] * n1[2], tt = ta[0] * ta[0] + ta[1] * ta[1] + ta[2] * ta[2];
+    const double cos_t = (ta[0] * n1[0] + ta[1] * n1[1] + ta[2] * n1[2]) / sqrt(nn * tt);
+    const double sp = fmax(llf_speed(s.S[1][o + dj], s.S[1][o], s.S[0][o + dj], s.S[0][o]),
+                           llf_speed(s.S[3][o + 1], s.S[3][o], s.S[2][o + 1], s.S[2][o]));
+    s.Ef[2][o] = llf_emf(sp, sqrt(1.0 - cos_t * cos_t), E, s.Bq[0][2 * PS + o + dj], s.Bq[0][PS + o], s.Bq[1][4 * PS + o + 1],
+                         s.Bq[1][3 * PS + o]);
+  } else {
+    const int c = (i == 0 && j == 0) ? 0 : (i == N && j == 0) ? 1 : (i == N && j == N) ? 2 : 3;
+    int z1x, z1y, z2x, z2y, z3x, z3y;
+    if (c == 0) { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j + 1; z3x = i + 1; z3y = j; }
+    else if (c == 1) { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j + 1; z3x = i; z3y = j; }
+    else if (c == 2) { z1x = i; z1y = j + 1; z2x = i; z2y = j; z3x = i + 1; z3y = j; }
+    else { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j; z3x = i + 1; z3y = j; }
+    const double ob3 = 1.0 / 3.0;
+    const double Ex = (E1(s, d, 0, p, z1x, z1y, k) + E1(s, d, 0, p, z2x, z2y, k) + E1(s, d, 0, p, z3x, z3y, k)) * ob3;
+    const double Ey = (E1(s, d, 1, p, z1x, z1y, k) + E1(s, d, 1, p, z2x, z2y, k) + E1(s, d, 1, p, z3x, z3y, k)) * ob3;
+    const double Ez = (E1(s, d, 2, p, z1x, z1y, k) + E1(s, d, 2, p, z2x, z2y, k) + E1(s, d, 2, p, z3x, z3y, k)) * ob3;
+    double Bn1, Bn2, Bn3, SR1, SL1, SR2, SL2, SR3, SL3;
+    if (c == 0) {
+      Bn1 = -Bqa(s, d, 1, 4, p, z3x, z3y, k); Bn2 = Bqa(s, d, 0, 2, p, z2x, z2y, k); Bn3 = Bqa(s, d, 1, 3, p, z2x, z2y - 1, k);
+      SR1 = -Sg(s.S[2], d, p, z3x, z3y, k); SL1 = -Sg(s.S[3], d, p, z3x, z3y, k);
+      SR2 = Sg(s.S[1], d, p, z2x, z2y, k); SL2 = Sg(s.S[0], d, p, z2x, z2y, k);
+      SR3 = Sg(s.S[3], d, p, z2x, z2y - 1, k); SL3 = Sg(s.S[2], d, p, z2x, z2y - 1, k);
+    } else if (c == 1) {
+      Bn1 = -Bqa(s, d, 1, 4, p, z1x, z1y - 1, k); Bn2 = Bqa(s, d, 0, 2, p, z2x, z2y, k); Bn3 = Bqa(s, d, 1, 3, p, z3x, z3y, k);
+      SR1 = -Sg(s.S[0], d, p, z3x, z3y, k); SL1 = -Sg(s.S[1], d, p, z3x, z3y, k);
+      SR2 = Sg(s.S[1], d, p, z2x, z2y, k); SL2 = Sg(s.S[0], d, p, z2x, z2y, k);
+      SR3 = Sg(s.S[3], d, p, z3x, z3y, k); SL3 = Sg(s.S[2], d, p, z3x, z3y, k);
+    } else if (c == 2) {
+      Bn1 = Bqa(s, d, 0, 2, p, z1x, z1y, k); Bn2 = Bqa(s, d, 1, 3, p, z2x, z2y, k); Bn3 = -Bqa(s, d, 0, 1, p, z2x, z2y, k);
+      SR1 = Sg(s.S[1], d, p, z1x, z1y, k); SL1 = Sg(s.S[0], d, p, z1x, z1y, k);
+      SR2 = Sg(s.S[3], d, p, z2x, z2y, k); SL2 = Sg(s.S[2], d, p, z2x, z2y, k);
+      SR3 = -Sg(s.S[0], d, p, z2x, z2y, k); SL3 = -Sg(s.S[1], d, p, z2x, z2y, k);
+    } else {
+      Bn1 = -Bqa(s, d, 1, 4, p, z3x, z3y, k); Bn2 = Bqa(s, d, 1, 3, p, z2x, z2y, k); Bn3 = -Bqa(s, d, 0, 1, p, z2x, z2y, k);
+      SR1 = -Sg(s.S[2], d, p, z3x, z3y, k); SL1 = -Sg(s.S[3], d, p, z3x, z3y, k);
+      SR2 = Sg(s.S[3], d, p, z2x, z2y, k); SL2 = Sg(s.S[2], d, p, z2x, z2y, k);
+      SR3 = -Sg(s.S[0], d, p, z2x, z2y, k); SL3 = -Sg(s.S[1], d, p, z2x, z2y, k);
+    }
+    const double tm = fmax(fmax(fmax(fabs(SR1), fabs(SL1)), fmax(fabs(SR2), fabs(SL2))), fmax(fabs(SR3), fabs(SL3)));
+    // one direction along the edge, so the rule's three points agree
+    s.Ef[2][o] = d_rs3(tm, -tm, tm, -tm, tm, -tm, Ex * e[0] + Ey * e[1] + Ez * e[2], Bn1, Bn2, Bn3);
   }
 }
 
-// z-edges (460:2591-3721): i, j in 0..N, k in 1..nr, skipped where a
-// neighbour is masked; the four cube corners (460:3725-7037) use the
-// three-state solver.
+// The three edge directions in one launch: block T is tile T / 3 of
+// direction T % 3.
+//
+// What bounds it: latency of about 30 loads an edge.  Solving the four-state
+// problem in its general form at each of the rule's three points took 136
+// registers and most of the time in FP64 divisions.
 template <typename R>
-__global__ void k_edges_z(Dims d, DGeom g, DStateT<R> s, Range3 r) {
-  const int N = d.N;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(TPB, 6) k_edges(Dims d, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
+  const unsigned nb = (unsigned)((max(r0.count(), max(r1.count(), r2.count())) + TPB - 1) / TPB);
+  for (unsigned T = blockIdx.x; T < 3 * nb; T += gridDim.x) {
+    const int dir = T % 3;
+    const Range3 r = dir == 0 ? r0 : (dir == 1 ? r1 : r2);
+    const long long t = (long long)(T / 3) * TPB + threadIdx.x;
+    if (t >= r.count()) continue;
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    const bool corner = (i == 0 || i == N) && (j == 0 || j == N);
-    double acc = 0.0;
-    if (!corner) {
-      if (mask_at(g, d, p, i, j) == 0 || mask_at(g, d, p, i + 1, j) == 0 || mask_at(g, d, p, i + 1, j + 1) == 0 ||
-          mask_at(g, d, p, i, j + 1) == 0) {
-        s.Ef[2][d.at(0, p, i, j, k)] = 0.0;
-        continue;
-      }
-      const double Ex = (E1(s, d, 0, p, i, j, k) + E1(s, d, 0, p, i + 1, j, k) + E1(s, d, 0, p, i + 1, j + 1, k) + E1(s, d, 0, p, i, j + 1, k)) * 0.25;
-      const double Ey = (E1(s, d, 1, p, i, j, k) + E1(s, d, 1, p, i + 1, j, k) + E1(s, d, 1, p, i + 1, j + 1, k) + E1(s, d, 1, p, i, j + 1, k)) * 0.25;
-      const double Ez = (E1(s, d, 2, p, i, j, k) + E1(s, d, 2, p, i + 1, j, k) + E1(s, d, 2, p, i + 1, j + 1, k) + E1(s, d, 2, p, i, j + 1, k)) * 0.25;
-      const double ByR = Bqa(s, d, 1, 4, p, i + 1, j, k), ByL = Bqa(s, d, 1, 3, p, i, j, k);
-      const double BnU = Bqa(s, d, 0, 2, p, i, j + 1, k), BnD = Bqa(s, d, 0, 1, p, i, j, k);
-      double SR = fmax(Sg(s.S[1], d, p, i, j + 1, k), Sg(s.S[1], d, p, i, j, k));
-      double SL = fmin(Sg(s.S[0], d, p, i, j + 1, k), Sg(s.S[0], d, p, i, j, k));
-      double SU = fmax(Sg(s.S[3], d, p, i + 1, j, k), Sg(s.S[3], d, p, i, j, k));
-      double SD = fmin(Sg(s.S[2], d, p, i + 1, j, k), Sg(s.S[2], d, p, i, j, k));
-      llf4(SR, SL, SU, SD);
-      for (int jq = 0; jq < 3; ++jq) {
-        const double wt = jq == 0 ? 4.0 / 6.0 : 1.0 / 6.0;
-        double n3[3], n1[3], tau[3];
-        edge_point(g, d, p, jq, i, j, k, i, j, k - 1, false, n3);
-        unit3(n3);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          n1[q] = geo(g, d, CS_G_VERT, q, p, i + 1, j, k) - geo(g, d, CS_G_VERT, q, p, i - 1, j, k);
-          tau[q] = geo(g, d, CS_G_VERT, q, p, i, j + 1, k) - geo(g, d, CS_G_VERT, q, p, i, j - 1, k);
-        }
-        orth3(n1, n3);
-        orth3(tau, n3);
-        const double cos_t = tau[0] * n1[0] + tau[1] * n1[1] + tau[2] * n1[2];
-        const double sin_t = sqrt(1.0 - cos_t * cos_t);
-        const double Ezl = Ex * n3[0] + Ey * n3[1] + Ez * n3[2];
-        acc = acc + wt * d_rs4(SR, SL, SU, SD, cos_t, sin_t, Ezl, BnU, BnD, ByR, ByL);
-      }
-    } else {
-      const int c = (i == 0 && j == 0) ? 0 : (i == N && j == 0) ? 1 : (i == N && j == N) ? 2 : 3;
-      int z1x, z1y, z2x, z2y, z3x, z3y;
-      if (c == 0) { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j + 1; z3x = i + 1; z3y = j; }
-      else if (c == 1) { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j + 1; z3x = i; z3y = j; }
-      else if (c == 2) { z1x = i; z1y = j + 1; z2x = i; z2y = j; z3x = i + 1; z3y = j; }
-      else { z1x = i + 1; z1y = j + 1; z2x = i; z2y = j; z3x = i + 1; z3y = j; }
-      const double ob3 = 1.0 / 3.0;
-      const double Ex = (E1(s, d, 0, p, z1x, z1y, k) + E1(s, d, 0, p, z2x, z2y, k) + E1(s, d, 0, p, z3x, z3y, k)) * ob3;
-      const double Ey = (E1(s, d, 1, p, z1x, z1y, k) + E1(s, d, 1, p, z2x, z2y, k) + E1(s, d, 1, p, z3x, z3y, k)) * ob3;
-      const double Ez = (E1(s, d, 2, p, z1x, z1y, k) + E1(s, d, 2, p, z2x, z2y, k) + E1(s, d, 2, p, z3x, z3y, k)) * ob3;
-      double Bn1, Bn2, Bn3, SR1, SL1, SR2, SL2, SR3, SL3;
-      if (c == 0) {
-        Bn1 = -Bqa(s, d, 1, 4, p, z3x, z3y, k); Bn2 = Bqa(s, d, 0, 2, p, z2x, z2y, k); Bn3 = Bqa(s, d, 1, 3, p, z2x, z2y - 1, k);
-        SR1 = -Sg(s.S[2], d, p, z3x, z3y, k); SL1 = -Sg(s.S[3], d, p, z3x, z3y, k);
-        SR2 = Sg(s.S[1], d, p, z2x, z2y, k); SL2 = Sg(s.S[0], d, p, z2x, z2y, k);
-        SR3 = Sg(s.S[3], d, p, z2x, z2y - 1, k); SL3 = Sg(s.S[2], d, p, z2x, z2y - 1, k);
-      } else if (c == 1) {
-        Bn1 = -Bqa(s, d, 1, 4, p, z1x, z1y - 1, k); Bn2 = Bqa(s, d, 0, 2, p, z2x, z2y, k); Bn3 = Bqa(s, d, 1, 3, p, z3x, z3y, k);
-        SR1 = -Sg(s.S[0], d, p, z3x, z3y, k); SL1 = -Sg(s.S[1], d, p, z3x, z3y, k);
-        SR2 = Sg(s.S[1], d, p, z2x, z2y, k); SL2 = Sg(s.S[0], d, p, z2x, z2y, k);
-        SR3 = Sg(s.S[3], d, p, z3x, z3y, k); SL3 = Sg(s.S[2], d, p, z3x, z3y, k);
-      } else if (c == 2) {
-        Bn1 = Bqa(s, d, 0, 2, p, z1x, z1y, k); Bn2 = Bqa(s, d, 1, 3, p, z2x, z2y, k); Bn3 = -Bqa(s, d, 0, 1, p, z2x, z2y, k);
-        SR1 = Sg(s.S[1], d, p, z1x, z1y, k); SL1 = Sg(s.S[0], d, p, z1x, z1y, k);
-        SR2 = Sg(s.S[3], d, p, z2x, z2y, k); SL2 = Sg(s.S[2], d, p, z2x, z2y, k);
-        SR3 = -Sg(s.S[0], d, p, z2x, z2y, k); SL3 = -Sg(s.S[1], d, p, z2x, z2y, k);
-      } else {
-        Bn1 = -Bqa(s, d, 1, 4, p, z3x, z3y, k); Bn2 = Bqa(s, d, 1, 3, p, z2x, z2y, k); Bn3 = -Bqa(s, d, 0, 1, p, z2x, z2y, k);
-        SR1 = -Sg(s.S[2], d, p, z3x, z3y, k); SL1 = -Sg(s.S[3], d, p, z3x, z3y, k);
-        SR2 = Sg(s.S[3], d, p, z2x, z2y, k); SL2 = Sg(s.S[2], d, p, z2x, z2y, k);
-        SR3 = -Sg(s.S[0], d, p, z2x, z2y, k); SL3 = -Sg(s.S[1], d, p, z2x, z2y, k);
-      }
-      const double tm = fmax(fmax(fmax(fabs(SR1), fabs(SL1)), fmax(fabs(SR2), fabs(SL2))), fmax(fabs(SR3), fabs(SL3)));
-      for (int jq = 0; jq < 3; ++jq) {
-        const double wt = jq == 0 ? 4.0 / 6.0 : 1.0 / 6.0;
-        double n3[3];
-        edge_point(g, d, p, jq, i, j, k, i, j, k - 1, false, n3);
-        unit3(n3);
-        const double Ezl = Ex * n3[0] + Ey * n3[1] + Ez * n3[2];
-        acc = acc + wt * d_rs3(tm, -tm, tm, -tm, tm, -tm, Ezl, Bn1, Bn2, Bn3);
-      }
-    }
-    s.Ef[2][d.at(0, p, i, j, k)] = acc;
+    if (dir == 0)
+      edge_x(d, g, s, p, i, j, k);
+    else if (dir == 1)
+      edge_y(d, g, s, p, i, j, k);
+    else
+      edge_z(d, g, s, p, i, j, k);
   }
 }
 
@@ -264,12 +245,9 @@ void launch_edges_t(Solve& sv, DStateT<R>& st) {
   Range3 ex = {1, N, 0, N, 0, nr};
   Range3 ey = {0, N, 1, N, 0, nr};
   Range3 ez = {0, N, 0, N, 1, nr};
-  k_edges_x<R><<<blocks_for(ex.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, ex);
-  mark(sv, "k_edges_x");
-  k_edges_y<R><<<blocks_for(ey.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, ey);
-  mark(sv, "k_edges_y");
-  k_edges_z<R><<<blocks_for(ez.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, ez);
-  mark(sv, "k_edges_z");
+  const long long nb = 3 * ((std::max(ex.count(), std::max(ey.count(), ez.count())) + TPB - 1) / TPB);
+  k_edges<R><<<(int)std::min<long long>(nb, (long long)grid_sms(sv) * 64), TPB, 0, sv.stream>>>(d, sv.g, st, ex, ey, ez);
+  mark(sv, "k_edges");
   if (sv.psync.ncls > 0 && (sv.p.flags & CS_FLAG_PANEL_AVERAGE)) {
     k_avg_emf<R><<<blocks_for(sv.psync.ncls, 128, grid_sms(sv)), 128, 0, sv.stream>>>(st, sv.psync);
     mark(sv, "k_avg_emf");

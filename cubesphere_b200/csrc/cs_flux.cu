@@ -286,19 +286,19 @@ __global__ void __launch_bounds__(FLUX_FACES * 5, sizeof(R) == 4 ? 7 : 4) k_flux
 // exchanged (their normals are opposite) and the negated entropy flux.
 template <typename R>
 __global__ void k_sync_flux(Dims d, DStateT<R> s, PanelSync ps) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ps.nf; t += (long long)gridDim.x * blockDim.x) {
-    const long long dst = ps.f_dst[t], src = ps.f_src[t];
-    const int dd = ps.f_ddir[t], sd = ps.f_sdir[t];
-    const int dp = (int)(dst / d.S), sp = (int)(src / d.S);
-    const long long dof = dst % d.S, sof = src % d.S;
-    R* Fd = s.fcon[dd];
-    const R* Fs = s.fcon[sd];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      Fd[((long long)c * NPANEL + dp) * d.S + dof] = Fs[((long long)(8 + c) * NPANEL + sp) * d.S + sof];
-      Fd[((long long)(8 + c) * NPANEL + dp) * d.S + dof] = Fs[((long long)c * NPANEL + sp) * d.S + sof];
-    }
-    s.EF[dd][dst] = -s.EF[sd][src];
+  const unsigned n = (unsigned)ps.nf;
+  const long long PS = (long long)NPANEL * d.S;
+  // one thread an entry and value: 16 contributions, then the entropy flux
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 17 * n; t += gridDim.x * blockDim.x) {
+    const unsigned c = t / n, e = t - c * n;
+    const unsigned dst = ps.f_dst[e], src = ps.f_src[e];
+    const int dd = ps.f_ddir[e], sd = ps.f_sdir[e];
+    R* Fd = dd == 0 ? s.fcon[0] : s.fcon[1];  // panel edges have x- and y-faces only
+    const R* Fs = sd == 0 ? s.fcon[0] : s.fcon[1];
+    if (c < 16)
+      Fd[c * PS + dst] = Fs[(c ^ 8) * PS + src];
+    else
+      (dd == 0 ? s.EF[0] : s.EF[1])[dst] = -(sd == 0 ? s.EF[0] : s.EF[1])[src];
   }
 }
 
@@ -404,7 +404,7 @@ void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
     k_avg_flux<R><<<blocks_for(sv.psync.nf, 128, grid_sms(sv)), 128, 0, sv.stream>>>(d, st, sv.psync);
     mark(sv, "k_avg_flux");
   } else if (sv.psync.nf > 0) {
-    k_sync_flux<R><<<blocks_for(sv.psync.nf, 128, grid_sms(sv)), 128, 0, sv.stream>>>(d, st, sv.psync);
+    k_sync_flux<R><<<blocks_for(17 * sv.psync.nf, 128, grid_sms(sv)), 128, 0, sv.stream>>>(d, st, sv.psync);
     mark(sv, "k_sync_flux");
   }
   Range3 z = {0, N + 1, 0, N + 1, 0, nr + 1};

@@ -15,55 +15,79 @@ namespace cs {
 
 namespace {
 
-// STEP 2 (zone part, 421:597-635) and STEP 5 (421:1497-1628).
+// STEP 2 (zone part, 421:597-635) and STEP 5 (421:1497-1628) of one zone.
 template <typename R>
-__global__ void k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+__device__ __forceinline__ void prim_zone(const Dims& d, const PhysC& ph, const DGeom& g, const DStateT<R>& s, int p, int i,
+                                          int j, int k) {
+  const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
+  const int m = mask_at(g, d, p, i, j);
+  R U[8], V[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) U[c] = s.U[c * PS + o];
+  if (m == 0) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) U[c] = R(0.0);
+    U[0] = R(ph.rhofloor);
+    U[4] = R(ph.prsfloor) / (R(ph.gamma) - R(1.0));
+  }
+  R en = s.ent[o];
+  d_cons_to_prim(ph, en, U, V);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    s.U[c * PS + o] = U[c];
+    s.V[c * PS + o] = V[c];
+  }
+  s.ent[o] = en;
+  s.ent[PS + o] = R(0.0);
+  s.ent[2 * PS + o] = R(0.0);
+  s.ent[3 * PS + o] = R(0.0);
+  // The higher modes are zero from the start wherever no step writes them.
+  // STEP 8.d writes the B modes of every active zone of its range, STEP 7.b
+  // all of them on the full zones only: between the two (three ghost layers)
+  // the B modes of the last stage go.
+  const int lo = 3 - d.G, hx = d.N + d.G - 2, hz = d.nr + d.G - 2;
+  const bool full = m == 1 && i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz;
+  const bool adp = m == 1 && i >= lo - 1 && i <= hx + 1 && j >= lo - 1 && j <= hx + 1 && k >= lo - 1 && k <= hz + 1;
+  if (adp && !full)
+#pragma unroll
+    for (int q = 0; q < 27; ++q) s.V[((q / 3 + 1) * NVAR + 5 + q % 3) * PS + o] = R(0.0);
+  const R a12 = (V[5] * V[5] + V[6] * V[6] + V[7] * V[7]) * R(ph.ob4pi);
+  s.msonic[o] = sqrt((R(ph.gamma) * V[4] + a12) / V[0]);
+}
+
+// Masked-face zeroing (421:658-759; 485:383-484) of the faces at one index.
+template <typename R>
+__device__ __forceinline__ void mask_faces(const Dims& d, const DGeom& g, const DStateT<R>& s, int p, int i, int j, int k) {
+  const int lo = 1 - d.G, hi = d.N + d.G;
+  // zones are masked at the panel corners only
+  const bool ci = i <= 1 || i >= d.N, cj = j <= 1 || j >= d.N;
+  if (!(ci && cj)) return;
+  if (k >= lo && j >= lo && mask_at(g, d, p, max(i, lo), j) == 0 && mask_at(g, d, p, min(i + 1, hi), j) == 0)
+    s.Bxf[d.at(0, p, i, j, k)] = 0.0;
+  if (k >= lo && i >= lo && mask_at(g, d, p, i, max(j, lo)) == 0 && mask_at(g, d, p, i, min(j + 1, hi)) == 0)
+    s.Byf[d.at(0, p, i, j, k)] = 0.0;
+  if (i >= lo && j >= lo && mask_at(g, d, p, i, j) == 0) s.Bzf[d.at(0, p, i, j, k)] = 0.0;
+}
+
+// The primitives of every zone and the masked faces, one thread an index
+// (the box has one more face than zones along each axis).
+template <typename R>
+__global__ void __launch_bounds__(TPB) k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+  const int lo = 1 - d.G;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    const int m = mask_at(g, d, p, i, j);
-    R U[8], V[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) U[c] = s.U[d.at(c, p, i, j, k)];
-    if (m == 0) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) U[c] = R(0.0);
-      U[0] = R(ph.rhofloor);
-      U[4] = R(ph.prsfloor) / (R(ph.gamma) - R(1.0));
-    }
-    R en = s.ent[d.at(0, p, i, j, k)];
-    d_cons_to_prim(ph, en, U, V);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      s.U[d.at(c, p, i, j, k)] = U[c];
-      s.V[d.at(c, p, i, j, k)] = V[c];
-    }
-    s.ent[d.at(0, p, i, j, k)] = en;
-    s.ent[d.at(1, p, i, j, k)] = R(0.0);
-    s.ent[d.at(2, p, i, j, k)] = R(0.0);
-    s.ent[d.at(3, p, i, j, k)] = R(0.0);
-    // Modes 2..10 stay zero wherever the P12 steps do not write them.
-    const int lo = 3 - d.G, hx = d.N + d.G - 2, hz = d.nr + d.G - 2;
-    const bool full = m == 1 && i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz;
-    if (!full)
-      for (int q = NVAR; q < NVAR * NMODE; ++q) s.V[d.at(q, p, i, j, k)] = R(0.0);
-    const R a12 = (V[5] * V[5] + V[6] * V[6] + V[7] * V[7]) * R(ph.ob4pi);
-    s.msonic[d.at(0, p, i, j, k)] = sqrt((R(ph.gamma) * V[4] + a12) / V[0]);
+    mask_faces(d, g, s, p, i, j, k);
+    if (i >= lo && j >= lo && k >= lo) prim_zone(d, ph, g, s, p, i, j, k);
   }
 }
 
-// Masked-face zeroing (421:658-759; 485:383-484).
 template <typename R>
 __global__ void k_zero_masked_faces(Dims d, DGeom g, DStateT<R> s, Range3 r) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    const int lo = 1 - d.G, hi = d.N + d.G;
-    if (k >= lo && j >= lo && mask_at(g, d, p, max(i, lo), j) == 0 && mask_at(g, d, p, min(i + 1, hi), j) == 0)
-      s.Bxf[d.at(0, p, i, j, k)] = 0.0;
-    if (k >= lo && i >= lo && mask_at(g, d, p, i, max(j, lo)) == 0 && mask_at(g, d, p, i, min(j + 1, hi)) == 0)
-      s.Byf[d.at(0, p, i, j, k)] = 0.0;
-    if (i >= lo && j >= lo && mask_at(g, d, p, i, j) == 0) s.Bzf[d.at(0, p, i, j, k)] = 0.0;
+    mask_faces(d, g, s, p, i, j, k);
   }
 }
 
@@ -1529,13 +1553,19 @@ void launch_step10(Solve& sv) {
     launch_step10_t(sv, sv.st);
 }
 
+inline Range3 faces_all(const Dims& d) { return {-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G}; }
+template <typename R>
+void launch_tricorner_t(Solve& sv, const DStateT<R>& st) {
+  k_tricorner<R><<<blocks_for(6LL * 4 * sv.d.G * (sv.d.NK - 1), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.g, st);
+  mark(sv, "k_tricorner");
+}
+
 template <typename R>
 void launch_prim_and_masks_t(Solve& sv, DStateT<R>& st) {
-  const Dims& d = sv.d;
-  Range3 z = zones_all(d);
-  k_prim<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z);
+  const Range3 f = faces_all(sv.d);
+  k_prim<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, f);
   mark(sv, "k_prim");
-  launch_face_masks(sv);
+  launch_tricorner_t(sv, st);
 }
 
 void launch_prim_and_masks(Solve& sv) {
@@ -1547,12 +1577,10 @@ void launch_prim_and_masks(Solve& sv) {
 
 template <typename R>
 void launch_face_masks_t(Solve& sv, DStateT<R>& st) {
-  const Dims& d = sv.d;
-  Range3 f = {-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G};
-  k_zero_masked_faces<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, f);
+  const Range3 f = faces_all(sv.d);
+  k_zero_masked_faces<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.g, st, f);
   mark(sv, "k_zero_masked_faces");
-  k_tricorner<R><<<blocks_for(6LL * 4 * d.G * (d.NK - 1), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st);
-  mark(sv, "k_tricorner");
+  launch_tricorner_t(sv, st);
 }
 
 void launch_face_masks(Solve& sv) {

@@ -63,45 +63,43 @@ __global__ void k_fill_scatter(DStateT<R> s, const int32_t* __restrict__ dst, co
     fill_store(s, meta[t] & 7, dst[t], tmp[t]);
 }
 
-// Radial outflow padding below k = 1 and above k = nr (826:190-420).  Two
-// columns that share an x- or y-face copy the same value into it.
+// Radial outflow padding below k = 1 and above k = nr (826:190-420), one
+// thread a column and ghost layer.  Two columns that share an x- or y-face
+// copy the same value into it.
 template <typename R>
 __global__ void k_pad_radial(Dims d, DGeom g, DStateT<R> s, int bc_lower, int bc_upper) {
-  const int n1 = d.N + 2 * d.G;
-  const long long n = 6LL * n1 * n1;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % n1) + 1 - d.G;
-    const int j = (int)((t / n1) % n1) + 1 - d.G;
-    const int p = (int)(t / ((long long)n1 * n1));
+  const unsigned n1 = d.N + 2 * d.G, ncol = 6 * n1 * n1;
+  const long long PS = (long long)NPANEL * d.S;
+  const int dj = d.NI;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * d.G * ncol; t += gridDim.x * blockDim.x) {
+    const unsigned layer = t / ncol, col = t - layer * ncol, u = col / n1;
+    const int i = (int)(col - u * n1) + 1 - d.G, j = (int)(u % n1) + 1 - d.G, p = (int)(u / n1);
     if (mask_at(g, d, p, i, j) != 1) continue;
-    if (bc_lower == 2) {
-      for (int kk = 1; kk <= d.G; ++kk) {
-        const int l = 1 - kk, r = 1;
-        for (int q = 0; q < NVAR; ++q) s.U[d.at(q, p, i, j, l)] = s.U[d.at(q, p, i, j, r)];
-        s.Bxf[d.at(0, p, i, j, l)] = s.Bxf[d.at(0, p, i, j, r)];
-        s.Bxf[d.at(0, p, i - 1, j, l)] = s.Bxf[d.at(0, p, i - 1, j, r)];
-        s.Byf[d.at(0, p, i, j, l)] = s.Byf[d.at(0, p, i, j, r)];
-        s.Byf[d.at(0, p, i, j - 1, l)] = s.Byf[d.at(0, p, i, j - 1, r)];
-        s.Bzf[d.at(0, p, i, j, l - 1)] = s.Bzf[d.at(0, p, i, j, r - 1)];
-      }
-    }
-    if (bc_upper == 2) {
-      const int r = d.nr;
-      for (int kk = 1; kk <= d.G; ++kk) {
-        const int l = d.nr + kk;
-        const double vr = geo(g, d, CS_G_V_VOL, 0, p, i, j, r), vl = geo(g, d, CS_G_V_VOL, 0, p, i, j, l);
-        for (int q = 0; q < NVAR; ++q) s.U[d.at(q, p, i, j, l)] = s.U[d.at(q, p, i, j, r)] * vr / vl;
-        s.Bzf[d.at(0, p, i, j, l)] =
-            s.Bzf[d.at(0, p, i, j, r)] * geo(g, d, CS_G_ZF_AREA, 0, p, i, j, r) / geo(g, d, CS_G_ZF_AREA, 0, p, i, j, l);
-        s.Bxf[d.at(0, p, i, j, l)] =
-            s.Bxf[d.at(0, p, i, j, r)] * geo(g, d, CS_G_XF_AREA, 0, p, i, j, r) / geo(g, d, CS_G_XF_AREA, 0, p, i, j, l);
-        s.Byf[d.at(0, p, i, j, l)] =
-            s.Byf[d.at(0, p, i, j, r)] * geo(g, d, CS_G_YF_AREA, 0, p, i, j, r) / geo(g, d, CS_G_YF_AREA, 0, p, i, j, l);
-        s.Bxf[d.at(0, p, i - 1, j, l)] = s.Bxf[d.at(0, p, i - 1, j, r)] * geo(g, d, CS_G_XF_AREA, 0, p, i - 1, j, r) /
-                                          geo(g, d, CS_G_XF_AREA, 0, p, i - 1, j, l);
-        s.Byf[d.at(0, p, i, j - 1, l)] = s.Byf[d.at(0, p, i, j - 1, r)] * geo(g, d, CS_G_YF_AREA, 0, p, i, j - 1, r) /
-                                          geo(g, d, CS_G_YF_AREA, 0, p, i, j - 1, l);
-      }
+    const bool upper = (int)layer >= d.G;
+    const int kk = (int)layer - (upper ? d.G : 0) + 1;
+    const long long b = (long long)p * d.S;
+    if (!upper) {
+      if (bc_lower != 2) continue;
+      const long long l = b + d.idx(i, j, 1 - kk), r = b + d.idx(i, j, 1), dk = (long long)d.NI * d.NJ;
+#pragma unroll
+      for (int q = 0; q < NVAR; ++q) s.U[q * PS + l] = s.U[q * PS + r];
+      s.Bxf[l] = s.Bxf[r];
+      s.Bxf[l - 1] = s.Bxf[r - 1];
+      s.Byf[l] = s.Byf[r];
+      s.Byf[l - dj] = s.Byf[r - dj];
+      s.Bzf[l - dk] = s.Bzf[r - dk];
+    } else {
+      if (bc_upper != 2) continue;
+      const long long l = b + d.idx(i, j, d.nr + kk), r = b + d.idx(i, j, d.nr);
+      const double *vol = g.f[CS_G_V_VOL], *xa = g.f[CS_G_XF_AREA], *ya = g.f[CS_G_YF_AREA], *za = g.f[CS_G_ZF_AREA];
+      const double vr = __ldg(vol + r), vl = __ldg(vol + l);
+#pragma unroll
+      for (int q = 0; q < NVAR; ++q) s.U[q * PS + l] = s.U[q * PS + r] * vr / vl;
+      s.Bzf[l] = s.Bzf[r] * __ldg(za + r) / __ldg(za + l);
+      s.Bxf[l] = s.Bxf[r] * __ldg(xa + r) / __ldg(xa + l);
+      s.Byf[l] = s.Byf[r] * __ldg(ya + r) / __ldg(ya + l);
+      s.Bxf[l - 1] = s.Bxf[r - 1] * __ldg(xa + r - 1) / __ldg(xa + l - 1);
+      s.Byf[l - dj] = s.Byf[r - dj] * __ldg(ya + r - dj) / __ldg(ya + l - dj);
     }
   }
 }
@@ -387,18 +385,17 @@ __global__ void k_cleanup_zones(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 
   }
 }
 
-__global__ void k_set_f64(double* p, double v) { *p = v; }
-
-// The CFL reduction starts from 1.1 times the current step (490:121-286);
-// its result becomes the solve's next step.
-__global__ void k_dt_start(const double* dt, unsigned long long* dtmin) {
-  *dtmin = (unsigned long long)__double_as_longlong(1.1 * *dt);
+// The solve's time step, and the start of the next CFL reduction: 1.1 times
+// it (490:121-286).
+__global__ void k_set_dt(double* dt, unsigned long long* dtmin, double v) {
+  *dt = v;
+  *dtmin = (unsigned long long)__double_as_longlong(1.1 * v);
 }
-__global__ void k_dt_commit(const unsigned long long* dtmin, double* dt) { *dt = __longlong_as_double((long long)*dtmin); }
 
 // CFL limit over the active interior zones; the minimum positive double is
 // found with an integer atomicMin on its bit pattern (positive IEEE doubles
-// order like their bit patterns).
+// order like their bit patterns).  The last block to finish makes the result
+// the solve's next step and starts the reduction after it.
 template <typename R>
 __global__ void k_timestep(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   double dtl = 1.0e300;
@@ -427,6 +424,17 @@ __global__ void k_timestep(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   for (int o = 16; o > 0; o >>= 1) dtl = fmin(dtl, __shfl_down_sync(0xffffffffu, dtl, o));
   if ((threadIdx.x & 31) == 0 && dtl < 1.0e300 && dtl > 0.0)
     atomicMin(s.dtmin, (unsigned long long)__double_as_longlong(dtl));
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned* done = reinterpret_cast<unsigned*>(s.dtmin + 1);
+    __threadfence();
+    if (atomicAdd(done, 1u) == gridDim.x - 1) {
+      *done = 0;
+      const double dt = __longlong_as_double((long long)atomicAdd(s.dtmin, 0ULL));
+      *s.dt = dt;
+      *s.dtmin = (unsigned long long)__double_as_longlong(1.1 * dt);
+    }
+  }
 }
 
 inline Range3 zones_all(const Dims& d) { return {1 - d.G, d.N + d.G, 1 - d.G, d.N + d.G, 1 - d.G, d.nr + d.G}; }
@@ -444,7 +452,7 @@ void launch_fill_ghosts_t(Solve& sv, const DStateT<R>& st) {
     mark(sv, "k_fill_scatter");
   }
   const int n1 = sv.d.N + 2 * sv.d.G;
-  k_pad_radial<R><<<blocks_for(6LL * n1 * n1, TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.g, st, sv.p.bc_lower,
+  k_pad_radial<R><<<blocks_for(12LL * sv.d.G * n1 * n1, TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.g, st, sv.p.bc_lower,
                                                                                       sv.p.bc_upper);
   mark(sv, "k_pad_radial");
 }
@@ -512,13 +520,9 @@ void launch_cleanup(Solve& sv, bool masks) {
 
 template <typename R>
 void launch_timestep_t(Solve& sv, const DStateT<R>& st) {
-  k_dt_start<<<1, 1, 0, sv.stream>>>(st.dt, st.dtmin);
-  mark(sv, "k_dt_start");
   Range3 r = {1, sv.d.N, 1, sv.d.N, 1, sv.d.nr};
   k_timestep<R><<<blocks_for(r.count(), 256, grid_sms(sv)), 256, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, r);
   mark(sv, "k_timestep");
-  k_dt_commit<<<1, 1, 0, sv.stream>>>(st.dtmin, st.dt);
-  mark(sv, "k_dt_commit");
 }
 void launch_timestep(Solve& sv) {
   if (sv.fp32)
@@ -607,7 +611,7 @@ void launch_diag(Solve& sv, double* part, double* out) {
 size_t diag_scratch_doubles() { return 3 * DIAG_BLOCKS + 4; }
 
 void launch_set_dt(Solve& sv, double dt) {
-  k_set_f64<<<1, 1, 0, sv.stream>>>(sv.fp32 ? sv.stF.dt : sv.st.dt, dt);
+  k_set_dt<<<1, 1, 0, sv.stream>>>(sv.fp32 ? sv.stF.dt : sv.st.dt, sv.fp32 ? sv.stF.dtmin : sv.st.dtmin, dt);
   mark(sv, "k_set_dt");
 }
 
