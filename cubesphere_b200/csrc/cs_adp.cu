@@ -152,9 +152,11 @@ __global__ void __launch_bounds__(32 * ADP_WARPS) k_adp(Dims d, PhysC ph, DGeom 
     }
     __syncwarp();
     // 3. elimination with scaled partial pivoting
+    double kmax = 0.0;  // largest entry this lane has seen
     for (int row = lane; row < 36; row += 32) {
       double m = 0.0;
       for (int c = 0; c < 36; ++c) m = fmax(m, fabs(S.K[row][c]));
+      kmax = fmax(kmax, m);
       S.sc[row] = (m == 0.0) ? 0.0 : 1.0 / m;
       S.piv[row] = row;
     }
@@ -221,6 +223,17 @@ __global__ void __launch_bounds__(32 * ADP_WARPS) k_adp(Dims d, PhysC ph, DGeom 
         for (int b = a + 1; b < 36; ++b) acc -= S.K[a][b] * y[b];
         y[a] = acc / S.K[a][a];
       }
+      // the size of K times that of its inverse, for the mesh build's choice
+      double ymax = 0.0;
+#pragma unroll
+      for (int u = 0; u < 30; ++u) ymax = fmax(ymax, lane < 30 ? fabs(y[u]) : 0.0);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        kmax = fmax(kmax, __shfl_xor_sync(0xffffffffu, kmax, off));
+        ymax = fmax(ymax, __shfl_xor_sync(0xffffffffu, ymax, off));
+      }
+      if (lane == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(s.err_flag) + 1, (unsigned long long)__double_as_longlong(kmax * ymax));
       if (lane < 30) {
         R* out = (R*)s.adp_lu + t / ADP6_ZB * (long long)(ADP6_WORDS * ADP6_ZB) + t % ADP6_ZB;
         const int g = lane / 10, j = lane % 10;
@@ -607,8 +620,7 @@ __device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, Rin
     adp6_unit<2 * c>(acc, xr, w, wp, xm, x, xn, xp);
     if constexpr (2 * c + 1 < ADP6_WORDS / ADP6_UNIT)
       adp6_unit<2 * c + 1>(acc, xr, w + ADP6_UNIT * ADP6_ZB, wp + ADP6_UNIT * ADP6_ZB, xm, x, xn, xp);
-    // this warp's reads are done before the copy engine may write the stage
-    // again (arriving alone let a refill overtake reads still in flight)
+    // this warp's reads are done before the copy engine may write the stage again
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.empty[ring.slot]);

@@ -787,9 +787,7 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
       if (!m.op_p2v || !m.op_p2e) return cuda_fail(sv, e, "cudaMalloc(P2 stencil inverses)");
     }
   }
-  if (!(sv.p.flags & CS_FLAG_NO_ADP_CACHE)) {
-    int8_t pmap[6 * 72];
-    const bool shared = !(sv.p.flags & CS_FLAG_ADP_PER_PANEL) && adp_panel_maps(m.host, pmap);
+  auto adp_operators = [&](bool shared, const int8_t* pmap) -> int {
     // panel-shared inverses in the state's type (the precision form applies
     // them in FP32), per-panel factors and their right-hand sides in FP64
     const size_t esz = shared ? sizeof(R) : sizeof(double);
@@ -809,10 +807,40 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
         if (!m.adp_piv || !s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP factors)");
       }
       if (shared) {
-        m.adp_pmap = (int8_t*)mdalloc(sv, m, sizeof pmap, e);
+        m.adp_pmap = (int8_t*)mdalloc(sv, m, 6 * 72, e);
         if (!m.adp_pmap) return cuda_fail(sv, e, "cudaMalloc(ADP panel maps)");
-        CS_CUDA(sv, cudaMemcpyAsync(m.adp_pmap, pmap, sizeof pmap, cudaMemcpyHostToDevice, sv.stream));
+        CS_CUDA(sv, cudaMemcpyAsync(m.adp_pmap, pmap, 6 * 72, cudaMemcpyHostToDevice, sv.stream));
         CS_CUDA(sv, cudaStreamSynchronize(sv.stream));  // pmap is a stack array
+      }
+    }
+    s.adp_pmap = m.adp_pmap;
+    s.adp_lu = m.adp_lu;
+    s.adp_piv = m.adp_piv;
+    if (m.adp_lu) launch_adp_factor(sv);
+    return CS_OK;
+  };
+  if (!(sv.p.flags & CS_FLAG_NO_ADP_CACHE)) {
+    int8_t pmap[6 * 72];
+    const bool shared = !(sv.p.flags & CS_FLAG_ADP_PER_PANEL) && adp_panel_maps(m.host, pmap);
+    if (int rc = adp_operators(shared, pmap)) return rc;
+    // The inverse is as good as the factors while the matrices are well
+    // conditioned: max |K| max |K^-1| is 10 to 1000 on shells and surfaces of
+    // ordinary aspect, and rounding enlarged that much is below 1e-12.  Beyond
+    // (a radial extrapolation through r = 0, say) the factors serve.
+    if (shared && m.adp_lu) {
+      double cond = 0.0;
+      CS_CUDA(sv, cudaMemcpyAsync(&cond, s.err_flag + 2, sizeof cond, cudaMemcpyDeviceToHost, sv.stream));
+      CS_CUDA(sv, cudaStreamSynchronize(sv.stream));
+      if (!(cond <= 1.0e4)) {
+        const size_t held = (size_t)adp_factor_doubles(d, true) * sizeof(R) + 6 * 72;
+        for (void* q : {m.adp_lu, (void*)m.adp_pmap}) {
+          m.allocs.erase(std::find(m.allocs.begin(), m.allocs.end(), q));
+          CS_CUDA(sv, cudaFree(q));
+        }
+        m.bytes -= held;
+        m.adp_lu = nullptr;
+        m.adp_pmap = nullptr;
+        if (int rc = adp_operators(false, pmap)) return rc;
       }
     }
   }
@@ -827,7 +855,6 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
   s.adp_lu = m.adp_lu;
   s.adp_piv = m.adp_piv;
   launch_ops_build(sv);
-  if (m.adp_lu) launch_adp_factor(sv);
   CS_CUDA(sv, cudaGetLastError());
   return CS_OK;
 }

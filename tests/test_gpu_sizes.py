@@ -1,6 +1,8 @@
 """One whole step at sizes where the tiles of the stage kernels end unevenly
 (the smallest meshes, odd extents, a last tile of one zone, more layers than
-a thread's column segment) against the CPU oracle, and batches of FP64 members
+a thread's column segment; with one radial zone and four ghost layers the
+padding runs through r = 0, where the ADP matrices are too ill conditioned for
+their inverses and the mesh keeps the factors) against the CPU oracle, and batches of FP64 members
 run side by side, which must give each member's own result to the bit.
 
 Tolerances: those of test_gpu_parity (1e-12 of the largest value for the
@@ -64,8 +66,8 @@ def test_precision_form_at_uneven_sizes(ntp, nr, ghosts, p2):
 
 def test_fp64_batches_give_each_members_own_result():
     """Members of different sizes side by side, many times: every state equals
-    the member's run alone to the bit (a shared-memory stage refilled while a
-    warp still read it showed as a few wrong zones in one member of six)."""
+    the member's run alone to the bit (an earlier pair of ADP kernels
+    left a few wrong zones in one member run of thirty)."""
     members = []
     for name, over in (("shell32", {}), ("surface32", dict(ntp=48)), ("shell32", dict(ntp=48, nr=24)),
                        ("shell16", dict(ntp=24, nr=16))):
