@@ -20,261 +20,275 @@ namespace {
 
 constexpr int TPB = 128;
 
-template <typename R>
-__device__ __forceinline__ R Vm(const DStateT<R>& s, const Dims& d, int comp, int mode, int p, long long o) {
-  return s.V[((long long)(mode * NVAR + comp) * NPANEL + p) * d.S + o];
-}
-
-// A block takes 32 faces, in two phases.  Face states (450:545-2931): the
-// first two warps put each side's five quadrature points, in the side
-// zone's scaled coordinates, and its basis moments in shared memory; then
-// the five warps evaluate the 18 (side, primitive or entropy) polynomials
-// of each face at the five points, each reading that variable's modes once,
-// into shared memory, so no face state goes through HBM.  Fluxes: one face
-// quadrature point per thread (warp = point) rotates
-// the two states to the face frame, solves the HLL problem and rotates the
+// A block takes 32 faces with five warps, in three phases.  Basis: warp q
+// forms, for both sides, the nine centred monomials of quadrature point q in
+// the side zone's scaled coordinates.  Face states (450:545-2931): the 18
+// (side, primitive or entropy) polynomials of each face at the five points,
+// two variables of a side at a time, so that a variable's modes are read once
+// and a basis value once for two variables; the warp without a second pair
+// forms the frame of the x- and y-faces and the two area / volume ratios, once
+// a face.  Fluxes: one quadrature point per thread (warp = point) rotates the
+// two states to the face frame, solves the HLL problem and rotates the
 // contributions back; they meet in shared memory and are summed in point
-// order (the order of the reference's quadrature loop).  One launch covers
-// the three face directions: tile T is tile T / 3 of direction T % 3, so the
-// x, y and z faces of about the same zone rows run side by side and L2
-// serves a zone's modes to all three.
+// order (the order of the reference's quadrature loop).  No face state goes
+// through HBM.  One launch covers the three face directions: tile T is tile
+// T / 3 of direction T % 3, so the x, y and z faces of about the same zone
+// rows run side by side and L2 serves a zone's modes to all three.
+//
+// What bounds it: FP64 latency at the 20 warps its registers and shared memory
+// allow, so what counts is the FP64 instructions of a point.
 constexpr int FLUX_FACES = 32;
 // Registers / occupancy: 4 blocks per SM suit the FP64 instantiation, 7 the
 // FP32 one (measured on the 6 x 128^2 x 64 shell).
 template <typename R>
 __global__ void __launch_bounds__(FLUX_FACES * 5, sizeof(R) == 4 ? 7 : 4) k_flux(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
-  // the point coordinates and moments are dead once the face states are
-  // formed, so they share their space with the flux contributions
+  // the basis is dead once the face states are formed, so it shares its space
+  // with the flux contributions
   union Scratch {
     R red[5][16][FLUX_FACES];
-    struct {
-      R pc[2][5][3][FLUX_FACES];  // [side][point][x y z][face]
-      R cf[2][6][FLUX_FACES];     // [side][moments 4-9][face]
-    } g;
+    R bs[2][5][9][FLUX_FACES];  // [side][point][x y z xx yy zz xy yz xz][face]
   };
   __shared__ Scratch sc;
-  R(&red)[5][16][FLUX_FACES] = sc.red;
   __shared__ R fs[2][9][5][FLUX_FACES];  // [side][primitive 0-7, entropy][point][face]
-  __shared__ long long zo[2][FLUX_FACES];  // box offset of each side's zone
+  __shared__ R fr[9][FLUX_FACES];        // frame of an x- or y-face: A, B, C
+  __shared__ R av[2][FLUX_FACES];        // area / volume of each side
   const int lane = threadIdx.x % FLUX_FACES, jq = threadIdx.x / FLUX_FACES;
-  const long long nt0 = (r0.count() + FLUX_FACES - 1) / FLUX_FACES, nt1 = (r1.count() + FLUX_FACES - 1) / FLUX_FACES,
-                  nt2 = (r2.count() + FLUX_FACES - 1) / FLUX_FACES;
-  const long long ntile = 3 * max(nt0, max(nt1, nt2));
-  for (long long T = blockIdx.x; T < ntile; T += gridDim.x) {
-    const int dir = (int)(T % 3);
-    const long long tile = T / 3;
+  const long long PS = (long long)NPANEL * d.S;
+  const unsigned nt0 = (unsigned)((r0.count() + FLUX_FACES - 1) / FLUX_FACES),
+                 nt1 = (unsigned)((r1.count() + FLUX_FACES - 1) / FLUX_FACES),
+                 nt2 = (unsigned)((r2.count() + FLUX_FACES - 1) / FLUX_FACES);
+  const unsigned ntile = 3 * max(nt0, max(nt1, nt2));
+  for (unsigned T = blockIdx.x; T < ntile; T += gridDim.x) {
+    const int dir = T % 3;
+    const unsigned tile = T / 3;
     const Range3 r = dir == 0 ? r0 : (dir == 1 ? r1 : r2);
     if (tile >= (dir == 0 ? nt0 : (dir == 1 ? nt1 : nt2))) continue;  // uniform over the block
-    const long long nf = r.count();
-    const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-    const int QW = dir == 0 ? CS_G_XF_QW : (dir == 1 ? CS_G_YF_QW : CS_G_ZF_QW);
-    const int AR = dir == 0 ? CS_G_XF_AREA : (dir == 1 ? CS_G_YF_AREA : CS_G_ZF_AREA);
-    R* F = s.fcon[dir];
-    R* SLo = s.S[2 * dir];
-    R* SHi = s.S[2 * dir + 1];
-    R* EF = s.EF[dir];
-    const long long t = tile * FLUX_FACES + lane;
-    const bool valid = t < nf;
+    const double* qp = dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP]);
+    const double* qw = dir == 0 ? g.f[CS_G_XF_QW] : (dir == 1 ? g.f[CS_G_YF_QW] : g.f[CS_G_ZF_QW]);
+    const double* ar = dir == 0 ? g.f[CS_G_XF_AREA] : (dir == 1 ? g.f[CS_G_YF_AREA] : g.f[CS_G_ZF_AREA]);
+    R* F = dir == 0 ? s.fcon[0] : (dir == 1 ? s.fcon[1] : s.fcon[2]);
+    const unsigned t = tile * FLUX_FACES + lane;
+    const bool valid = t < (unsigned)r.count();
     int p = 0, i = 0, j = 0, k = 0;
     if (valid) r.decode(t, p, i, j, k);
-    int lx = i, ly = j, lz = k, rx = i, ry = j, rz = k;
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
+    // the two side zones; one remapped through istencil at a panel corner
+    long long zo0 = o, zo1 = o;
     bool skip = !valid;
     if (valid) {
-      if (dir == 0) {
-        const int mL = mask_at(g, d, p, i, j), mR = mask_at(g, d, p, i + 1, j);
-        rx = i + 1;
-        if (mL == 0 && mR == 1) { lx = sten(g, d, p, rx, ry, 1, 0); ly = sten(g, d, p, rx, ry, 1, 1); }
-        else if (mL == 1 && mR == 0) { rx = sten(g, d, p, lx, ly, 0, 0); ry = sten(g, d, p, lx, ly, 0, 1); }
-        else if (mL == 0 && mR == 0) skip = true;
-      } else if (dir == 1) {
-        const int mL = mask_at(g, d, p, i, j), mR = mask_at(g, d, p, i, j + 1);
-        ry = j + 1;
-        if (mL == 0 && mR == 1) { lx = sten(g, d, p, rx, ry, 3, 0); ly = sten(g, d, p, rx, ry, 3, 1); }
-        else if (mL == 1 && mR == 0) { rx = sten(g, d, p, lx, ly, 2, 0); ry = sten(g, d, p, lx, ly, 2, 1); }
-        else if (mL == 0 && mR == 0) skip = true;
-      } else {
+      int lx = i, ly = j, rx = i, ry = j, rz = k;
+      if (dir == 2) {
         if (mask_at(g, d, p, i, j) == 0) skip = true;
         rz = k + 1;
+      } else {
+        const int w = 2 * dir;  // istencil entry of the upper neighbour, w + 1 of the lower
+        rx += dir == 0;
+        ry += dir == 1;
+        const int mL = mask_at(g, d, p, i, j), mR = mask_at(g, d, p, rx, ry);
+        if (mL == 0 && mR == 1) {
+          lx = sten(g, d, p, rx, ry, w + 1, 0);
+          ly = sten(g, d, p, rx, ry, w + 1, 1);
+        } else if (mL == 1 && mR == 0) {
+          rx = sten(g, d, p, lx, ly, w, 0);
+          ry = sten(g, d, p, lx, ly, w, 1);
+        } else if (mL == 0 && mR == 0) {
+          skip = true;
+        }
       }
+      zo0 = (long long)p * d.S + d.idx(lx, ly, k);
+      zo1 = (long long)p * d.S + d.idx(rx, ry, rz);
     }
-    // phase 1a: each side's points and moments (a side remapped through
-    // istencil at a panel corner is the remapped zone)
-    if (jq < 2 && !skip) {
-      const int side = jq;
-      const int zx = side ? rx : lx, zy = side ? ry : ly, zz = side ? rz : lz;
-      zo[side][lane] = d.idx(zx, zy, zz);
-      const R obl = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, p, zx, zy, zz), R(ph.smallnum));
-      const R cx = geoR<R>(g, d, CS_G_V_CEN, 0, p, zx, zy, zz), cy = geoR<R>(g, d, CS_G_V_CEN, 1, p, zx, zy, zz),
-              cz = geoR<R>(g, d, CS_G_V_CEN, 2, p, zx, zy, zz);
+    if (!skip) {
+      const R qx = (R)__ldg(qp + jq * PS + o), qy = (R)__ldg(qp + (5 + jq) * PS + o), qz = (R)__ldg(qp + (10 + jq) * PS + o);
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        sc.g.pc[side][q][0][lane] = (geoR<R>(g, d, QP, q, p, i, j, k) - cx) * obl;
-        sc.g.pc[side][q][1][lane] = (geoR<R>(g, d, QP, 5 + q, p, i, j, k) - cy) * obl;
-        sc.g.pc[side][q][2][lane] = (geoR<R>(g, d, QP, 10 + q, p, i, j, k) - cz) * obl;
+      for (int side = 0; side < 2; ++side) {
+        const long long z = side ? zo1 : zo0;
+        const double* cen = g.f[CS_G_V_CEN] + z;
+        const double* cf = g.f[CS_G_COEF] + z;
+        const R obl = rcp_newton(fmax((R)__ldg(g.f[CS_G_V_SCALE] + z), R(ph.smallnum)));
+        const R x = (qx - (R)__ldg(cen)) * obl, y = (qy - (R)__ldg(cen + PS)) * obl, zz = (qz - (R)__ldg(cen + 2 * PS)) * obl;
+        R(&b)[9][FLUX_FACES] = sc.bs[side][jq];
+        b[0][lane] = x;
+        b[1][lane] = y;
+        b[2][lane] = zz;
+        b[3][lane] = x * x - (R)__ldg(cf + 4 * PS);
+        b[4][lane] = y * y - (R)__ldg(cf + 5 * PS);
+        b[5][lane] = zz * zz - (R)__ldg(cf + 6 * PS);
+        b[6][lane] = x * y - (R)__ldg(cf + 7 * PS);
+        b[7][lane] = y * zz - (R)__ldg(cf + 8 * PS);
+        b[8][lane] = x * zz - (R)__ldg(cf + 9 * PS);
       }
-#pragma unroll
-      for (int m = 4; m < 10; ++m) sc.g.cf[side][m - 4][lane] = geoR<R>(g, d, CS_G_COEF, m, p, zx, zy, zz);
     }
     __syncthreads();
-    // phase 1b: task v = 0..17 (side v / 9, variable v % 9) of this face;
-    // warp jq takes tasks jq, jq + 5, jq + 10, jq + 15
     if (!skip) {
-#pragma unroll 1
-      for (int v = jq; v < 18; v += 5) {
-        const int side = v / 9, var = v % 9;
-        const long long oz = zo[side][lane];
-        R cc[10];
-        cc[0] = cc[1] = cc[2] = cc[3] = R(0.0);
+      // pairs 0-3 of side 0 and 4-7 of side 1: primitives 2 n, 2 n + 1
+      auto pair = [&](int pr) {
+        const int side = pr >> 2, c = 2 * (pr & 3);
+        const R* v = s.V + c * PS + (side ? zo1 : zo0);
+        R m[2][10];
 #pragma unroll
-        for (int m = 4; m < 10; ++m) cc[m] = sc.g.cf[side][m - 4][lane];
-        if (var < 8) {
-          R w[10];
+        for (int a = 0; a < 10; ++a) {
+          m[0][a] = v[a * NVAR * PS];
+          m[1][a] = v[(a * NVAR + 1) * PS];
+        }
 #pragma unroll
-          for (int m = 0; m < 10; ++m) w[m] = Vm(s, d, var, m, p, oz);
+        for (int q = 0; q < 5; ++q) {
+          R u0 = m[0][0], u1 = m[1][0];
 #pragma unroll
-          for (int q = 0; q < 5; ++q)
-            fs[side][var][q][lane] =
-                d_poly10(w, cc, sc.g.pc[side][q][0][lane], sc.g.pc[side][q][1][lane], sc.g.pc[side][q][2][lane]);
-        } else {
-          const R* E = s.ent;
-          const R e0 = E[((long long)0 * NPANEL + p) * d.S + oz], e1 = E[((long long)1 * NPANEL + p) * d.S + oz],
-                  e2 = E[((long long)2 * NPANEL + p) * d.S + oz], e3 = E[((long long)3 * NPANEL + p) * d.S + oz];
+          for (int a = 1; a < 10; ++a) {
+            const R b = sc.bs[side][q][a - 1][lane];
+            u0 = u0 + m[0][a] * b;
+            u1 = u1 + m[1][a] * b;
+          }
+          fs[side][c][q][lane] = u0;
+          fs[side][c + 1][q][lane] = u1;
+        }
+      };
+      pair(jq);
+      if (jq < 3) {
+        pair(jq + 5);
+      } else if (jq == 3) {
 #pragma unroll
-          for (int q = 0; q < 5; ++q)
-            fs[side][8][q][lane] = e0 + e1 * sc.g.pc[side][q][0][lane] + e2 * sc.g.pc[side][q][1][lane] +
-                                   e3 * sc.g.pc[side][q][2][lane];
+        for (int side = 0; side < 2; ++side) {
+          const R* e = s.ent + (side ? zo1 : zo0);
+          const R e0 = e[0], e1 = e[PS], e2 = e[2 * PS], e3 = e[3 * PS];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const R(&b)[9][FLUX_FACES] = sc.bs[side][q];
+            fs[side][8][q][lane] = e0 + e1 * b[0][lane] + e2 * b[1][lane] + e3 * b[2][lane];
+          }
+        }
+      } else {
+        const R area = (R)__ldg(ar + o);
+        av[0][lane] = area * rcp_newton((R)__ldg(g.f[CS_G_V_VOL] + zo0));
+        av[1][lane] = area * rcp_newton((R)__ldg(g.f[CS_G_V_VOL] + zo1));
+        if (dir < 2) {
+          const double* nv = (dir == 0 ? g.f[CS_G_XF_N] : g.f[CS_G_YF_N]) + o;
+          const double* fc = (dir == 0 ? g.f[CS_G_XF_CEN] : g.f[CS_G_YF_CEN]) + o;
+          const R Ax = (R)__ldg(nv), Ay = (R)__ldg(nv + PS), Az = (R)__ldg(nv + 2 * PS);
+          R ex = (R)__ldg(fc), ey = (R)__ldg(fc + PS), ez = (R)__ldg(fc + 2 * PS);
+          const R tt = rcp_newton(fmax(sqrt(ex * ex + ey * ey + ez * ez), R(ph.smallnum)));
+          ex = ex * tt;
+          ey = ey * tt;
+          ez = ez * tt;
+          // the radial direction and its product with the normal: C and
+          // B = C x A on x-faces; B and C = A x B on y-faces
+          const R sx = ey * Az - ez * Ay, sy = ez * Ax - ex * Az, sz = ex * Ay - ey * Ax;
+          const bool xf = dir == 0;
+          fr[0][lane] = Ax;
+          fr[1][lane] = Ay;
+          fr[2][lane] = Az;
+          fr[3][lane] = xf ? sx : ex;
+          fr[4][lane] = xf ? sy : ey;
+          fr[5][lane] = xf ? sz : ez;
+          fr[6][lane] = xf ? ex : -sx;
+          fr[7][lane] = xf ? ey : -sy;
+          fr[8][lane] = xf ? ez : -sz;
         }
       }
     }
     __syncthreads();
-    // phase 2: the flux at point jq of face lane
+    // the flux at point jq of face lane
     if (skip) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) red[jq][c][lane] = R(0.0);
+      for (int c = 0; c < 16; ++c) sc.red[jq][c][lane] = R(0.0);
     } else {
       R Ax, Ay, Az, Bx, By, Bz, Cx, Cy, Cz;
-      if (dir == 0) {
-        Ax = geoR<R>(g, d, CS_G_XF_N, 0, p, i, j, k);
-        Ay = geoR<R>(g, d, CS_G_XF_N, 1, p, i, j, k);
-        Az = geoR<R>(g, d, CS_G_XF_N, 2, p, i, j, k);
-        Cx = geoR<R>(g, d, CS_G_XF_CEN, 0, p, i, j, k);
-        Cy = geoR<R>(g, d, CS_G_XF_CEN, 1, p, i, j, k);
-        Cz = geoR<R>(g, d, CS_G_XF_CEN, 2, p, i, j, k);
-        const R tt = R(1.0) / fmax(sqrt(Cx * Cx + Cy * Cy + Cz * Cz), R(ph.smallnum));
-        Cx = Cx * tt;
-        Cy = Cy * tt;
-        Cz = Cz * tt;
-        Bx = Cy * Az - Cz * Ay;
-        By = Cz * Ax - Cx * Az;
-        Bz = Cx * Ay - Cy * Ax;
-      } else if (dir == 1) {
-        Ax = geoR<R>(g, d, CS_G_YF_N, 0, p, i, j, k);
-        Ay = geoR<R>(g, d, CS_G_YF_N, 1, p, i, j, k);
-        Az = geoR<R>(g, d, CS_G_YF_N, 2, p, i, j, k);
-        Bx = geoR<R>(g, d, CS_G_YF_CEN, 0, p, i, j, k);
-        By = geoR<R>(g, d, CS_G_YF_CEN, 1, p, i, j, k);
-        Bz = geoR<R>(g, d, CS_G_YF_CEN, 2, p, i, j, k);
-        const R tt = R(1.0) / fmax(sqrt(Bx * Bx + By * By + Bz * Bz), R(ph.smallnum));
-        Bx = Bx * tt;
-        By = By * tt;
-        Bz = Bz * tt;
-        Cx = Ay * Bz - Az * By;
-        Cy = Az * Bx - Ax * Bz;
-        Cz = Ax * By - Ay * Bx;
+      if (dir < 2) {
+        Ax = fr[0][lane];
+        Ay = fr[1][lane];
+        Az = fr[2][lane];
+        Bx = fr[3][lane];
+        By = fr[4][lane];
+        Bz = fr[5][lane];
+        Cx = fr[6][lane];
+        Cy = fr[7][lane];
+        Cz = fr[8][lane];
       } else {
-        auto vt = [&](int q, int x, int y) { return geoR<R>(g, d, CS_G_VERT, q, p, x, y, k); };
-        Ax = geoR<R>(g, d, CS_G_ZF_N, jq, p, i, j, k);
-        Ay = geoR<R>(g, d, CS_G_ZF_N, 5 + jq, p, i, j, k);
-        Az = geoR<R>(g, d, CS_G_ZF_N, 10 + jq, p, i, j, k);
-        R tt = R(1.0) / fmax(sqrt(Ax * Ax + Ay * Ay + Az * Az), R(ph.smallnum));
+        const double* nv = g.f[CS_G_ZF_N] + o;
+        const double* vt = g.f[CS_G_VERT] + o;
+        const int dj = d.NI;
+        Ax = (R)__ldg(nv + jq * PS);
+        Ay = (R)__ldg(nv + (5 + jq) * PS);
+        Az = (R)__ldg(nv + (10 + jq) * PS);
+        R tt = rcp_newton(fmax(sqrt(Ax * Ax + Ay * Ay + Az * Az), R(ph.smallnum)));
         Ax = Ax * tt;
         Ay = Ay * tt;
         Az = Az * tt;
-        Bx = vt(0, i, j) + vt(0, i, j - 1) - vt(0, i - 1, j) - vt(0, i - 1, j - 1);
-        By = vt(1, i, j) + vt(1, i, j - 1) - vt(1, i - 1, j) - vt(1, i - 1, j - 1);
-        Bz = vt(2, i, j) + vt(2, i, j - 1) - vt(2, i - 1, j) - vt(2, i - 1, j - 1);
+        auto across = [&](const double* v) {
+          return (R)__ldg(v) + (R)__ldg(v - dj) - (R)__ldg(v - 1) - (R)__ldg(v - 1 - dj);
+        };
+        Bx = across(vt);
+        By = across(vt + PS);
+        Bz = across(vt + 2 * PS);
         tt = Bx * Ax + By * Ay + Bz * Az;
         Bx = Bx - tt * Ax;
         By = By - tt * Ay;
         Bz = Bz - tt * Az;
-        tt = R(1.0) / fmax(sqrt(Bx * Bx + By * By + Bz * Bz), R(ph.smallnum));
+        tt = rcp_newton(fmax(sqrt(Bx * Bx + By * By + Bz * Bz), R(ph.smallnum)));
         Bx = Bx * tt;
         By = By * tt;
         Bz = Bz * tt;
         Cx = Ay * Bz - Az * By;
         Cy = Az * Bx - Ax * Bz;
         Cz = Ax * By - Ay * Bx;
-        tt = R(1.0) / fmax(sqrt(Cx * Cx + Cy * Cy + Cz * Cz), R(ph.smallnum));
+        tt = rcp_newton(fmax(sqrt(Cx * Cx + Cy * Cy + Cz * Cz), R(ph.smallnum)));
         Cx = Cx * tt;
         Cy = Cy * tt;
         Cz = Cz * tt;
       }
-      R VL[8], VR[8];
+      R V[2][8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        VL[c] = fs[0][c][jq][lane];
-        VR[c] = fs[1][c][jq][lane];
-      }
-      const R entL = fs[0][8][jq][lane], entR = fs[1][8][jq][lane];
+      for (int side = 0; side < 2; ++side) {
+        V[side][0] = fs[side][0][jq][lane];
+        V[side][4] = fs[side][4][jq][lane];
 #pragma unroll
-      for (int o = 1; o <= 5; o += 4) {
-        R a1 = Ax * VL[o] + Ay * VL[o + 1] + Az * VL[o + 2];
-        R b1 = Bx * VL[o] + By * VL[o + 1] + Bz * VL[o + 2];
-        R c1 = Cx * VL[o] + Cy * VL[o + 1] + Cz * VL[o + 2];
-        VL[o] = a1;
-        VL[o + 1] = b1;
-        VL[o + 2] = c1;
-        a1 = Ax * VR[o] + Ay * VR[o + 1] + Az * VR[o + 2];
-        b1 = Bx * VR[o] + By * VR[o + 1] + Bz * VR[o + 2];
-        c1 = Cx * VR[o] + Cy * VR[o + 1] + Cz * VR[o + 2];
-        VR[o] = a1;
-        VR[o + 1] = b1;
-        VR[o + 2] = c1;
+        for (int u = 1; u <= 5; u += 4) {
+          const R w0 = fs[side][u][jq][lane], w1 = fs[side][u + 1][jq][lane], w2 = fs[side][u + 2][jq][lane];
+          V[side][u] = Ax * w0 + Ay * w1 + Az * w2;
+          V[side][u + 1] = Bx * w0 + By * w1 + Bz * w2;
+          V[side][u + 2] = Cx * w0 + Cy * w1 + Cz * w2;
+        }
       }
       R FlL[8], FlR[8], FL[8], FR[8], SL, SR, entF;
-      d_hll(ph, VL, VR, entL, entR, FlL, FlR, FL, FR, SL, SR, entF);
-      const long long fo = d.idx(i, j, k);
+      d_hll(ph, V[0], V[1], fs[0][8][jq][lane], fs[1][8][jq][lane], FlL, FlR, FL, FR, SL, SR, entF);
       if (jq == 0) {
-        SLo[((long long)p) * d.S + fo] = SL;
-        SHi[((long long)p) * d.S + fo] = SR;
-        EF[((long long)p) * d.S + fo] = entF;
+        (dir == 0 ? s.S[0] : (dir == 1 ? s.S[2] : s.S[4]))[o] = SL;
+        (dir == 0 ? s.S[1] : (dir == 1 ? s.S[3] : s.S[5]))[o] = SR;
+        (dir == 0 ? s.EF[0] : (dir == 1 ? s.EF[1] : s.EF[2]))[o] = entF;
       }
-      const R wt = geoR<R>(g, d, QW, jq, p, i, j, k);
-      const R area = geoR<R>(g, d, AR, 0, p, i, j, k);
-      const R volL = geoR<R>(g, d, CS_G_V_VOL, 0, p, lx, ly, lz), volR = geoR<R>(g, d, CS_G_V_VOL, 0, p, rx, ry, rz);
-      // rotate back to global components: fluctuation + flux on each side
-      auto back = [&](const R* W, int c) {
-        if (c == 0 || c == 4) return W[c];
-        const int o = c < 4 ? 1 : 5, a = c - o;
-        const R ea = a == 0 ? Ax : (a == 1 ? Ay : Az), eb = a == 0 ? Bx : (a == 1 ? By : Bz),
-                     ec = a == 0 ? Cx : (a == 1 ? Cy : Cz);
-        return ea * W[o] + eb * W[o + 1] + ec * W[o + 2];
-      };
+      const R wt = (R)__ldg(qw + jq * PS + o);
       // the two sides' net contributions (fluctuation + flux) summed in the
       // face frame and rotated back once, and area / volume once per side
       // (the reference rotates each term and divides every term; the
       // results differ from it in the last bits only)
-      R GL[8], GR[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        GL[c] = FlL[c] + FL[c];
-        GR[c] = FlR[c] - FR[c];
+        FlL[c] = FlL[c] + FL[c];
+        FlR[c] = FlR[c] - FR[c];
       }
-      const R aL = area / volL, aR = area / volR;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        red[jq][c][lane] = wt * back(GL, c) * aL;
-        red[jq][8 + c][lane] = wt * back(GR, c) * aR;
+      for (int side = 0; side < 2; ++side) {
+        const R* G = side ? FlR : FlL;
+        const R a = av[side][lane];
+        R(*out)[FLUX_FACES] = sc.red[jq] + 8 * side;
+        out[0][lane] = wt * G[0] * a;
+        out[4][lane] = wt * G[4] * a;
+#pragma unroll
+        for (int u = 1; u <= 5; u += 4) {
+          out[u][lane] = wt * (Ax * G[u] + Bx * G[u + 1] + Cx * G[u + 2]) * a;
+          out[u + 1][lane] = wt * (Ay * G[u] + By * G[u + 1] + Cy * G[u + 2]) * a;
+          out[u + 2][lane] = wt * (Az * G[u] + Bz * G[u + 1] + Cz * G[u + 2]) * a;
+        }
       }
     }
     __syncthreads();
     if (valid) {
-      const long long fo = d.idx(i, j, k);
       for (int c = jq; c < 16; c += 5) {
         R acc = R(0.0);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) acc = acc + red[q][c][lane];
-        F[((long long)c * NPANEL + p) * d.S + fo] = acc;
+        for (int q = 0; q < 5; ++q) acc = acc + sc.red[q][c][lane];
+        F[c * PS + o] = acc;
       }
     }
     __syncthreads();
