@@ -505,7 +505,7 @@ int alloc_state(Solve& sv, DStateT<R>& s) {
   s.adp_pmap = m.adp_pmap;
   s.adp_rhs = nullptr;
   if (m.adp_lu && !m.adp_pmap) {  // k_adp6 keeps its right-hand sides in shared memory
-    s.adp_rhs = dalloc(sv, (size_t)adp_range_count(d) * 36 * sizeof(double), e);
+    s.adp_rhs = dalloc(sv, (size_t)adp_range_count(sv) * 36 * sizeof(double), e);
     if (!s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP right-hand sides)");
   }
   s.giveup = (int32_t*)dalloc(sv, S6 * sizeof(int32_t), e);
@@ -791,9 +791,9 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
     // panel-shared inverses in the state's type (the precision form applies
     // them in FP32), per-panel factors and their right-hand sides in FP64
     const size_t esz = shared ? sizeof(R) : sizeof(double);
-    const long long nf = adp_factor_doubles(d, shared);
+    const long long nf = adp_factor_doubles(sv, shared);
     const size_t lu_bytes = (size_t)nf * esz, pv_bytes = shared ? 0 : (size_t)nf / 36;
-    const size_t rhs_bytes = shared ? 0 : (size_t)adp_range_count(d) * 36 * esz;
+    const size_t rhs_bytes = shared ? 0 : (size_t)adp_range_count(sv) * 36 * esz;
     size_t fr = 0, tot = 0;
     // room left after them and their right-hand sides: the FP32 form's state
     // staging (one FP64 word per point, cs_state_put / cs_state_get) and 2 GB
@@ -832,7 +832,7 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
       CS_CUDA(sv, cudaMemcpyAsync(&cond, s.err_flag + 2, sizeof cond, cudaMemcpyDeviceToHost, sv.stream));
       CS_CUDA(sv, cudaStreamSynchronize(sv.stream));
       if (!(cond <= 1.0e4)) {
-        const size_t held = (size_t)adp_factor_doubles(d, true) * sizeof(R) + 6 * 72;
+        const size_t held = (size_t)adp_factor_doubles(sv, true) * sizeof(R) + 6 * 72;
         for (void* q : {m.adp_lu, (void*)m.adp_pmap}) {
           m.allocs.erase(std::find(m.allocs.begin(), m.allocs.end(), q));
           CS_CUDA(sv, cudaFree(q));

@@ -451,8 +451,8 @@ void launch_faceB_adp(Solve& s);
 void launch_adp(Solve& s);
 void launch_adp_factor(Solve& s);
 void set_adp_smem_limits();
-long long adp_range_count(const Dims& d);
-long long adp_factor_doubles(const Dims& d, bool shared);
+long long adp_range_count(const Solve& sv);
+long long adp_factor_doubles(const Solve& sv, bool shared);
 long long lsq_range_count(const Dims& d);
 void launch_ops_build(Solve& s);
 void launch_pos_extents(Solve& s, float* ext);

@@ -18,7 +18,7 @@ namespace {
 // STEP 2 (zone part, 421:597-635) and STEP 5 (421:1497-1628) of one zone.
 template <typename R>
 __device__ __forceinline__ void prim_zone(const Dims& d, const PhysC& ph, const DGeom& g, const DStateT<R>& s, int p, int i,
-                                          int j, int k) {
+                                          int j, int k, int al) {
   const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
   const int m = mask_at(g, d, p, i, j);
   R U[8], V[8];
@@ -42,12 +42,12 @@ __device__ __forceinline__ void prim_zone(const Dims& d, const PhysC& ph, const 
   s.ent[2 * PS + o] = R(0.0);
   s.ent[3 * PS + o] = R(0.0);
   // The higher modes are zero from the start wherever no step writes them.
-  // STEP 8.d writes the B modes of every active zone of its range, STEP 7.b
-  // all of them on the full zones only: between the two (three ghost layers)
-  // the B modes of the last stage go.
+  // STEP 8.d writes the B modes of the active zones al layers around the
+  // interior, STEP 7.b all of them on its own zones, which may be a layer
+  // less: there the B modes of the last stage go.
   const int lo = 3 - d.G, hx = d.N + d.G - 2, hz = d.nr + d.G - 2;
-  const bool full = m == 1 && i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz;
-  const bool adp = m == 1 && i >= lo - 1 && i <= hx + 1 && j >= lo - 1 && j <= hx + 1 && k >= lo - 1 && k <= hz + 1;
+  const bool full = i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz;
+  const bool adp = m == 1 && i > -al && i <= d.N + al && j > -al && j <= d.N + al && k > -al && k <= d.nr + al;
   if (adp && !full)
 #pragma unroll
     for (int q = 0; q < 27; ++q) s.V[((q / 3 + 1) * NVAR + 5 + q % 3) * PS + o] = R(0.0);
@@ -72,13 +72,13 @@ __device__ __forceinline__ void mask_faces(const Dims& d, const DGeom& g, const 
 // The primitives of every zone and the masked faces, one thread an index
 // (the box has one more face than zones along each axis).
 template <typename R>
-__global__ void __launch_bounds__(TPB) k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+__global__ void __launch_bounds__(TPB) k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, int al) {
   const int lo = 1 - d.G;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
     mask_faces(d, g, s, p, i, j, k);
-    if (i >= lo && j >= lo && k >= lo) prim_zone(d, ph, g, s, p, i, j, k);
+    if (i >= lo && j >= lo && k >= lo) prim_zone(d, ph, g, s, p, i, j, k, al);
   }
 }
 
@@ -1013,7 +1013,7 @@ __device__ __forceinline__ void e9c_minv(const Dims& d, const DGeom& g, int p, i
 // nothing else.  kCached: the inverse normal matrix comes from the
 // operator cache.  Blocks per SM: 4 for FP64, 6 for FP32 (measured).
 template <bool kCached, bool kShared, typename R>
-__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, Range3 rs) {
   const R ob12 = R(1.0) / R(12.0), ob180 = R(1.0) / R(180.0), ob144 = R(1.0) / R(144.0);
   const LsqOrder<kShared> ord(r);
   for (long long it = ord.begin(); it < ord.nit; it += ord.stride()) {
@@ -1041,7 +1041,10 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
 #pragma unroll
       for (int e = 0; e < 100; ++e) Minv[e] = (R)Md[e];
     }
-    const R* wc = s.op_m10 + tw;
+    // the zone's place in the weights' range rs
+    const long long nsp = rs.count() / 6, nw = kShared ? nsp : 6 * nsp;
+    const long long ts = ((long long)(k - rs.k0) * (rs.j1 - rs.j0 + 1) + (j - rs.j0)) * (rs.i1 - rs.i0 + 1) + (i - rs.i0);
+    const R* wc = s.op_m10 + (kShared ? ts : ts + p * nsp);
     auto MI = [&](int e) { return Minv[kCached ? 0 : e]; };
     R Y[3][10];
 #pragma unroll
@@ -1060,7 +1063,7 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
           off = d.idx(w < 0 ? i : n.x[w], w < 0 ? j : n.y[w], k + c_n18[rr - 1][1]);
         }
 #pragma unroll
-        for (int a = 0; a < 10; ++a) A[a] = __ldg(wc + (long long)(rr * 10 + a) * ord.nw);
+        for (int a = 0; a < 10; ++a) A[a] = __ldg(wc + (long long)(rr * 10 + a) * nw);
       } else {
         e9c_row(d, g, p, i, j, k, n, rr, cx, cy, cz, obl0, c0, A, off);
       }
@@ -1563,7 +1566,8 @@ void launch_tricorner_t(Solve& sv, const DStateT<R>& st) {
 template <typename R>
 void launch_prim_and_masks_t(Solve& sv, DStateT<R>& st) {
   const Range3 f = faces_all(sv.d);
-  k_prim<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, f);
+  k_prim<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, f,
+                                                                                    adp_layers(sv));
   mark(sv, "k_prim");
   launch_tricorner_t(sv, st);
 }
@@ -1681,10 +1685,11 @@ void launch_positivity(Solve& sv) {
 template <typename R>
 void launch_faceB_adp_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
-  const int G = d.G, N = d.N, nr = d.nr;
-  Range3 fx = {1 - G, N + G - 1, 2 - G, N + G - 1, 2 - G, nr + G - 1};
-  Range3 fy = {2 - G, N + G - 1, 1 - G, N + G - 1, 2 - G, nr + G - 1};
-  Range3 fz = {2 - G, N + G - 1, 2 - G, N + G - 1, 1 - G, nr + G - 1};
+  // the faces of the zones STEP 8.d solves
+  Range3 fx = around(d, adp_layers(sv)), fy = fx, fz = fx;
+  fx.i0 -= 1;
+  fy.j0 -= 1;
+  fz.k0 -= 1;
   k_faceB<R><<<blocks_for(fx.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, 0);
   mark(sv, "k_faceB");
   k_faceB<R><<<blocks_for(fy.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fy, 1);
@@ -1737,7 +1742,9 @@ void launch_ops_build(Solve& sv) {
 template <typename R>
 void launch_efield_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
-  Range3 z = zones_all(d), a = shrink(d, 1), b = shrink(d, 2);
+  Range3 a = around(d, 1), b = shrink(d, 2);
+  // P2's stencils reach two zones beyond theirs
+  const Range3 z = (sv.p.flags & CS_FLAG_P2) ? zones_all(d) : around(d, 2);
   k_efield_a<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, z);
   mark(sv, "k_efield_a");
   if (sv.p.flags & CS_FLAG_P2) {  // LIMIT_ALL_SLOPES_P2's STEP 9.b
@@ -1756,11 +1763,11 @@ void launch_efield_t(Solve& sv, DStateT<R>& st) {
   }
   if (st.op_m10)
     if (st.lsq_map10)
-      k_efield_c<true, true, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_efield_c<true, true, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
     else
-      k_efield_c<true, false, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_efield_c<true, false, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
   else
-    k_efield_c<false, false, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+    k_efield_c<false, false, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
   mark(sv, "k_efield_c");
 }
 
