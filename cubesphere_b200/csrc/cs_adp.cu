@@ -589,22 +589,10 @@ __device__ __forceinline__ void adp6_unit(F (&acc)[3][10], F (&xr)[3][10], const
   }
 }
 
-// Position in the ring: slot and the parity of its current phase.
-struct RingPos {
-  int slot = 0;
-  uint32_t par = 0;
-  __device__ __forceinline__ void next() {
-    if (++slot == ADP6_NS) {
-      slot = 0;
-      par ^= 1;
-    }
-  }
-};
-
 // The whole stream of one zone block: wait for a stage, apply its two units,
 // release it.
 template <typename F, int... C>
-__device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, RingPos& ring, int lane, int a, int h,
+__device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, RingPos<ADP6_NS>& ring, int lane, int a, int h,
                                            int* err, std::integer_sequence<int, C...>) {
   const F* xm = &S.x[30][3 * h][lane];
   const F* x = &S.x[10 * a][3 * h][lane];
@@ -652,7 +640,7 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
   __syncthreads();
   if (tid >= ADP6_CONS) {
     if (tid == ADP6_CONS) {
-      RingPos ring;
+      RingPos<ADP6_NS> ring;
       bool first = true;  // the ring's first round finds every stage free
       for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
         const R* src = (const R*)s.adp_lu + blk * (long long)(ADP6_WORDS * ADP6_ZB);
@@ -670,7 +658,7 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
     return;
   }
   const int lane = tid & 31, w = tid >> 5;
-  RingPos ring;
+  RingPos<ADP6_NS> ring;
   for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     const long long t1 = blk * ADP6_ZB + lane;
     const bool inr = t1 < n1;

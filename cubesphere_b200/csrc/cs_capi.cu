@@ -886,6 +886,7 @@ int mesh_attach(Solve& sv, const std::shared_ptr<MeshRes>& mp) {
   CS_CUDA(sv, cudaStreamCreateWithFlags(&sv.stream, cudaStreamNonBlocking));
   CS_CUDA(sv, pool_acquire(sv));
   set_adp_smem_limits();
+  set_weno_smem_limits();
   const bool fresh = !m.on_device;
   if (fresh)
     if (int rc = mesh_upload(sv, m)) return rc;

@@ -435,9 +435,8 @@ __device__ __forceinline__ void d_matinv(const R* A, R* Ainv) {
   }
 }
 
-// Row stride of STEP 7.b's resident row weights [162][stride]: the zone
-// count rounded up to 4 elements, so each row starts on a 16-byte (FP32) or
-// 32-byte (FP64) boundary.
+// Zones the resident row weights of STEP 7.b hold words for: rounded up to 4,
+// so that every row of a block is a multiple of 16 bytes.
 __host__ __device__ constexpr long long m9_stride(long long n) { return (n + 3) / 4 * 4; }
 
 // Host-side launch helpers implemented in the .cu files.
@@ -446,11 +445,14 @@ void launch_prim_and_masks(Solve& s);
 void launch_face_masks(Solve& s);
 void launch_flattener(Solve& s);
 void launch_weno(Solve& s);
+// STEP 7.b on zones r from the resident row weights.
+void launch_weno7b(Solve& s, const Range3& r);
 void launch_positivity(Solve& s);
 void launch_faceB_adp(Solve& s);
 void launch_adp(Solve& s);
 void launch_adp_factor(Solve& s);
 void set_adp_smem_limits();
+void set_weno_smem_limits();
 long long adp_range_count(const Solve& sv);
 long long adp_factor_doubles(const Solve& sv, bool shared);
 long long lsq_range_count(const Dims& d);

@@ -451,36 +451,14 @@ struct LsqOrder {
   }
 };
 
-// Mode mm of panel p's least-squares solution from the sums Y over panel
-// 1's row weights: sign x Y at panel 1's mode (src >> 4mm) & 15, which lies
-// in mm's group (the constant, x y z, xx yy zz, xy yz xz), so the choice is
-// a select among three registers.  Y holds modes M0.. (M0 = 0 with the
-// constant, 1 without).
-template <int M0, typename R>
-__device__ __forceinline__ R lsq_rotated(const R* Y, int mm, unsigned long long src, unsigned int neg) {
-  const int mu = (int)((src >> (4 * mm)) & 15);
-  R v;
-  if (mm == 0) {
-    v = Y[0 - M0];
-  } else {
-    const int g0 = 1 + 3 * ((mm - 1) / 3);
-    v = mu == g0 ? Y[g0 - M0] : (mu == g0 + 1 ? Y[g0 + 1 - M0] : Y[g0 + 2 - M0]);
-  }
-  return ((neg >> mm) & 1u) ? -v : v;
-}
-
-// STEP 7.b (421:3869-4551): 18-zone quadratic least squares hybridised
-// with the linear WENO slopes (MRWENO weights, flattener damping).  With
-// kCached the inverse normal matrix (geometry only) comes from the
-// operator cache built at mesh build; the result is the same either way.
-constexpr int W7B_QG = NVAR;
-template <bool kCached, bool kShared, typename R>
-__global__ void __launch_bounds__(TPB) k_weno7b(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  const R ob12 = R(1.0) / R(12.0), ob180 = R(1.0) / R(180.0), ob144 = R(1.0) / R(144.0);
-  const LsqOrder<kShared> ord(r);
-  for (long long it = ord.begin(); it < ord.nit; it += ord.stride()) {
-    long long t, tw;
-    if (!ord.zone(it, t, tw)) continue;
+// STEP 7.b (421:3869-4551) without resident row weights
+// (CS_FLAG_NO_OP_CACHE): 18-zone quadratic least squares hybridised with the
+// linear WENO slopes (MRWENO weights, flattener damping), the rows rebuilt
+// and the normal matrix inverted in every stage.  With the weights:
+// k_weno7b.
+template <typename R>
+__global__ void __launch_bounds__(TPB) k_weno7b_rebuild(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
     if (mask_at(g, d, p, i, j) != 1) continue;
@@ -490,15 +468,10 @@ __global__ void __launch_bounds__(TPB) k_weno7b(Dims d, PhysC ph, DGeom g, DStat
     coef10(g, d, p, i, j, k, c0);
     const R cx = geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k), cy = geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k),
                  cz = geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    // kCached: the least-squares solution operator comes from the cache as
-    // W_rr = Minv A_rr^T, one 9-vector per stencil row (geometry only), so
-    // the slopes are X = sum_rr W_rr (V_rr - V_0) with no row rebuild and
-    // no neighbour geometry; without the cache the rows are rebuilt and the
-    // inverse applied to their sums.
-    R Minv[kCached ? 1 : 81];
-    if (!kCached) {
-      // formed in FP64 in every form, like the cached row weights; the
-      // precision form rounds the inverse once
+    // formed in FP64 in every form, like the resident row weights; the
+    // precision form rounds the inverse once
+    R Minv[81];
+    {
       double c0d[10], Md[81];
       coef10(g, d, p, i, j, k, c0d);
       const double l0d = fmax(geo(g, d, CS_G_V_SCALE, 0, p, i, j, k), ph.smallnum);
@@ -507,86 +480,41 @@ __global__ void __launch_bounds__(TPB) k_weno7b(Dims d, PhysC ph, DGeom g, DStat
 #pragma unroll
       for (int e = 0; e < 81; ++e) Minv[e] = (R)Md[e];
     }
-    // kShared: panel 1's row weights; the sums are rotated at the end
-    const R* wc = s.op_m9 + tw;
-    auto MI = [&](int e) { return Minv[kCached ? 0 : e]; };
     const R f = s.flatA[d.at(0, p, i, j, k)];
-    const R betalo = f + (R(1.0) - f) * R(2.0);
-    const R ghi = f * R(0.6) + (R(1.0) - f) * R(0.95), glo = R(1.0) - ghi, obghi = R(1.0) / ghi, grat = glo / ghi;
-    // The primitives go in groups of W7B_QG, each group rebuilding the
-    // matrix rows; on B200 one group of all eight is faster than smaller
-    // groups (the row rebuild costs more than the extra live sums).  Every
-    // component's sums run over the rows in the same order either way.
+    R v0[NVAR], Y[NVAR][9];
+#pragma unroll
+    for (int q = 0; q < NVAR; ++q) {
+      v0[q] = s.V[((long long)q * NPANEL + p) * d.S + d.idx(i, j, k)];
+#pragma unroll
+      for (int a = 0; a < 9; ++a) Y[q][a] = R(0.0);
+    }
 #pragma unroll 1
-    for (int q0 = 0; q0 < NVAR; q0 += W7B_QG) {
-      R v0[W7B_QG];
+    for (int rr = 0; rr < 18; ++rr) {
+      R A[9];
+      long long off;
+      w7b_row(d, ph, g, p, i, j, k, n, rr, cx, cy, cz, l0, obl0, c0, A, off);
 #pragma unroll
-      for (int qq = 0; qq < W7B_QG; ++qq) v0[qq] = s.V[((long long)(q0 + qq) * NPANEL + p) * d.S + d.idx(i, j, k)];
-      R Y[W7B_QG][9];
+      for (int q = 0; q < NVAR; ++q) {
+        const R Rv = s.V[((long long)q * NPANEL + p) * d.S + off] - v0[q];
 #pragma unroll
-      for (int qq = 0; qq < W7B_QG; ++qq)
-#pragma unroll
-        for (int a = 0; a < 9; ++a) Y[qq][a] = R(0.0);
-#pragma unroll 1
-      for (int rr = 0; rr < 18; ++rr) {
-        R A[9];
-        long long off;
-        if (kCached) {
-          const int w = c_n18[rr][0];
-          off = d.idx(w < 0 ? i : n.x[w], w < 0 ? j : n.y[w], k + c_n18[rr][1]);
-#pragma unroll
-          for (int a = 0; a < 9; ++a) A[a] = __ldg(wc + (long long)(rr * 9 + a) * m9_stride(ord.nw));
-        } else {
-          w7b_row(d, ph, g, p, i, j, k, n, rr, cx, cy, cz, l0, obl0, c0, A, off);
-        }
-#pragma unroll
-        for (int qq = 0; qq < W7B_QG; ++qq) {
-          const R Rv = s.V[((long long)(q0 + qq) * NPANEL + p) * d.S + off] - v0[qq];
-#pragma unroll
-          for (int a = 0; a < 9; ++a) Y[qq][a] = Y[qq][a] + A[a] * Rv;
-        }
+        for (int a = 0; a < 9; ++a) Y[q][a] = Y[q][a] + A[a] * Rv;
       }
-      const unsigned long long qsrc = kShared ? s.lsq_map9[p].src : LSQ_IDENTITY_SRC;
-      const unsigned int qneg = kShared ? s.lsq_map9[p].neg : 0u;
+    }
 #pragma unroll
-      for (int qq = 0; qq < W7B_QG; ++qq) {
-        const int q = q0 + qq;
-        R X[9];
+    for (int q = 0; q < NVAR; ++q) {
+      R X[9];
 #pragma unroll
-        for (int a = 0; a < 9; ++a) {
-          if (kCached) {
-            X[a] = kShared ? lsq_rotated<1>(Y[qq], a + 1, qsrc, qneg) : Y[qq][a];
-          } else {
-            R sacc = R(0.0);
+      for (int a = 0; a < 9; ++a) {
+        R sacc = R(0.0);
 #pragma unroll
-            for (int b = 0; b < 9; ++b) sacc = sacc + MI(a * 9 + b) * Y[qq][b];
-            X[a] = sacc;
-          }
-        }
-        const R v2 = Vat(s, d, q, 1, p, i, j, k), v3 = Vat(s, d, q, 2, p, i, j, k), v4 = Vat(s, d, q, 3, p, i, j, k);
-        const R ISlo = betalo * (v2 * v2 + v3 * v3 + v4 * v4) * ob12;
-        R Phi[9];
-        Phi[0] = X[0] * obghi - v2 * grat;
-        Phi[1] = X[1] * obghi - v3 * grat;
-        Phi[2] = X[2] * obghi - v4 * grat;
-#pragma unroll
-        for (int a = 3; a < 9; ++a) Phi[a] = X[a] * obghi;
-        const R IShi = (Phi[0] * Phi[0] + Phi[1] * Phi[1] + Phi[2] * Phi[2]) * ob12 +
-                            (Phi[3] * Phi[3]) * (sqr(c0[4] - ob12) + ob180) + (Phi[4] * Phi[4]) * (sqr(c0[5] - ob12) + ob180) +
-                            (Phi[5] * Phi[5]) * (sqr(c0[6] - ob12) + ob180) + (Phi[6] * Phi[6]) * (c0[7] * c0[7] + ob144) +
-                            (Phi[7] * Phi[7]) * (c0[8] * c0[8] + ob144) + (Phi[8] * Phi[8]) * (c0[9] * c0[9] + ob144);
-        const R tau = fabs(IShi - ISlo);
-        R Wlo = glo * (R(1.0) + tau / (ISlo + R(ph.smallnum))), Whi = ghi * (R(1.0) + tau / (IShi + R(ph.smallnum)));
-        const R aa = R(1.0) / (Wlo + Whi);
-        Wlo = Wlo * aa;
-        Whi = Whi * aa;
-        const R x = R(1.0) - f;
-        Vat(s, d, q, 1, p, i, j, k) = (Whi * Phi[0] + Wlo * v2) * x;
-        Vat(s, d, q, 2, p, i, j, k) = (Whi * Phi[1] + Wlo * v3) * x;
-        Vat(s, d, q, 3, p, i, j, k) = (Whi * Phi[2] + Wlo * v4) * x;
-#pragma unroll
-        for (int m = 4; m < 10; ++m) Vat(s, d, q, m, p, i, j, k) = (Whi * Phi[m - 1]) * x;
+        for (int b = 0; b < 9; ++b) sacc = sacc + Minv[a * 9 + b] * Y[q][b];
+        X[a] = sacc;
       }
+      const R lin[3] = {Vat(s, d, q, 1, p, i, j, k), Vat(s, d, q, 2, p, i, j, k), Vat(s, d, q, 3, p, i, j, k)};
+      R out[9];
+      mrweno_hybrid(X, lin, c0, f, R(ph.smallnum), out);
+#pragma unroll
+      for (int m = 1; m < 10; ++m) Vat(s, d, q, m, p, i, j, k) = out[m - 1];
     }
   }
 }
@@ -615,7 +543,7 @@ __global__ void k_ops_m9(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
       for (int a = 0; a < 9; ++a) {
         double w = 0.0;
         for (int b = 0; b < 9; ++b) w = w + Minv[a * 9 + b] * A[b];
-        s.op_m9[(long long)(rr * 9 + a) * m9_stride(nr_) + t] = (R)w;
+        s.op_m9[m9_at(t, rr * 9 + a, nr_)] = (R)w;
       }
     }
   }
@@ -1378,8 +1306,9 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
         for (int m = 0; m < NM; ++m) Y[c][m] = R(0.0);
       const LsqPanelMap* cmap = kE ? s.lsq_map10 : s.lsq_map9;
       const long long tc = cmap ? t - (long long)p * npp : t, ncw = cmap ? npp : nz;
-      const R* wc = (kE ? s.op_m10 : s.op_m9) + tc;
-      const long long cstride = kE ? ncw : m9_stride(ncw);
+      const M9Block cb = m9_block(tc / 32, ncw);
+      const R* wc = kE ? s.op_m10 + tc : s.op_m9 + cb.off + tc % 32;
+      const long long cstride = kE ? ncw : cb.wid;
 #pragma unroll
       for (int rr = 0; rr < NR + 9; ++rr) {
         const int ro = kE ? rr - 1 : rr;  // E: the zone itself first
@@ -1647,12 +1576,11 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
     k_weno_ao_split<false, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_weno7a");
   }
-  if (st.op_m9 && st.lsq_map9)
-    k_weno7b<true, true, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
-  else if (st.op_m9)
-    k_weno7b<true, false, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
-  else
-    k_weno7b<false, false, R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+  if (st.op_m9) {
+    launch_weno7b(sv, b);
+    return;
+  }
+  k_weno7b_rebuild<R><<<blocks_for(b.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
   mark(sv, "k_weno7b");
 }
 

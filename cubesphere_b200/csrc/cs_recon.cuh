@@ -55,6 +55,93 @@ static __device__ __noinline__ void mbar_wait(uint64_t* bar, uint32_t parity, in
   atomicOr(err, 1);
 }
 
+// Position in a ring of NS shared-memory stages: slot and the parity of its
+// current phase.
+template <int NS>
+struct RingPos {
+  int slot = 0;
+  uint32_t par = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == NS) {
+      slot = 0;
+      par ^= 1;
+    }
+  }
+};
+
+// Mode mm of panel p's least-squares solution from the sums Y over panel
+// 1's row weights: sign x Y at panel 1's mode (src >> 4mm) & 15, which lies
+// in mm's group (the constant, x y z, xx yy zz, xy yz xz), so the choice is
+// a select among three registers.  Y holds modes M0.. (M0 = 0 with the
+// constant, 1 without).
+template <int M0, typename R>
+__device__ __forceinline__ R lsq_rotated(const R* Y, int mm, unsigned long long src, unsigned int neg) {
+  const int mu = (int)((src >> (4 * mm)) & 15);
+  R v;
+  if (mm == 0) {
+    v = Y[0 - M0];
+  } else {
+    const int g0 = 1 + 3 * ((mm - 1) / 3);
+    v = mu == g0 ? Y[g0 - M0] : (mu == g0 + 1 ? Y[g0 + 1 - M0] : Y[g0 + 2 - M0]);
+  }
+  return ((neg >> mm) & 1u) ? -v : v;
+}
+
+// MRWENO weights of a quadratic least-squares solution X (modes x .. xz)
+// against the linear WENO slopes lin (421:4440-4551 for the primitives,
+// 421:8700-9350 for E): the quadratic polynomial's modes Phi with the linear
+// part taken out, and the normalised weights of the two.
+template <typename R>
+__device__ __forceinline__ void mrweno_weights(const R* X, const R* lin, const R* c0, R f, R ghi, R glo, R obghi, R grat,
+                                               R smallnum, R* Phi, R& Wlo, R& Whi) {
+  const R ob12 = R(1.0) / R(12.0), ob180 = R(1.0) / R(180.0), ob144 = R(1.0) / R(144.0);
+  const R betalo = f + (R(1.0) - f) * R(2.0);
+  const R ISlo = betalo * (lin[0] * lin[0] + lin[1] * lin[1] + lin[2] * lin[2]) * ob12;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) Phi[a] = X[a] * obghi - lin[a] * grat;
+#pragma unroll
+  for (int a = 3; a < 9; ++a) Phi[a] = X[a] * obghi;
+  const R IShi = (Phi[0] * Phi[0] + Phi[1] * Phi[1] + Phi[2] * Phi[2]) * ob12 +
+                 (Phi[3] * Phi[3]) * (sqr(c0[4] - ob12) + ob180) + (Phi[4] * Phi[4]) * (sqr(c0[5] - ob12) + ob180) +
+                 (Phi[5] * Phi[5]) * (sqr(c0[6] - ob12) + ob180) + (Phi[6] * Phi[6]) * (c0[7] * c0[7] + ob144) +
+                 (Phi[7] * Phi[7]) * (c0[8] * c0[8] + ob144) + (Phi[8] * Phi[8]) * (c0[9] * c0[9] + ob144);
+  const R tau = fabs(IShi - ISlo);
+  Wlo = glo * (R(1.0) + tau / (ISlo + smallnum));
+  Whi = ghi * (R(1.0) + tau / (IShi + smallnum));
+  const R aa = R(1.0) / (Wlo + Whi);
+  Wlo = Wlo * aa;
+  Whi = Whi * aa;
+}
+
+// The hybrid's modes x .. xz, damped by the flattener f.
+template <typename R>
+__device__ __forceinline__ void mrweno_hybrid(const R* X, const R* lin, const R* c0, R f, R smallnum, R* out) {
+  const R ghi = f * R(0.6) + (R(1.0) - f) * R(0.95), glo = R(1.0) - ghi, obghi = R(1.0) / ghi, grat = glo / ghi;
+  R Phi[9], Wlo, Whi;
+  mrweno_weights(X, lin, c0, f, ghi, glo, obghi, grat, smallnum, Phi, Wlo, Whi);
+  const R x = R(1.0) - f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) out[a] = (Whi * Phi[a] + Wlo * lin[a]) * x;
+#pragma unroll
+  for (int a = 3; a < 9; ++a) out[a] = (Whi * Phi[a]) * x;
+}
+
+// STEP 7.b's resident row weights of n zones: blocks of 32 zones [162][32],
+// the last one [162][m9_stride(n) - 32 (blocks - 1)], so that a block is one
+// contiguous run for the bulk copies.
+struct M9Block {
+  long long off;  // of the block's first word
+  int wid;        // zones in a row
+};
+__device__ __forceinline__ M9Block m9_block(long long blk, long long n) {
+  return {blk * 162 * 32, (int)min(32LL, m9_stride(n) - blk * 32)};
+}
+// Word e of zone t.
+__device__ __forceinline__ long long m9_at(long long t, int e, long long n) {
+  const M9Block b = m9_block(t / 32, n);
+  return b.off + (long long)e * b.wid + t % 32;
+}
+
 // The interior zones and w layers around them.
 inline Range3 around(const Dims& d, int w) { return {1 - w, d.N + w, 1 - w, d.N + w, 1 - w, d.nr + w}; }
 // Layers around the interior on which STEP 8.d solves the B modes.  The stage
