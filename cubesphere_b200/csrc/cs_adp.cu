@@ -482,12 +482,13 @@ __global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph,
 // adp_pmap[p][0][v] is the panel-p unknown u fed by panel-1 unknown v,
 // adp_pmap[p][1][v] its sign.
 //
-// A CTA takes ADP6_ZB zone positions and the six panels.  First a warp forms
-// the 36 right-hand sides of one panel (panel 1's quadrature rows times the
-// panel's face values, plus its present modes) into shared memory; then warp
-// w applies the inverse to three panels, rows of component w % 3 (10 modes x
-// 3 panels of sums in registers), while a producer warp streams the packed
-// inverse through a ring of bulk copies that runs ahead across both phases.
+// A CTA takes ADP6_ZB zone positions and the six panels; a warp the rows of
+// component w % 3 for three of them (10 modes x 3 panels of sums in
+// registers).  First the 36 right-hand sides (panel 1's quadrature rows times
+// the panels' face values, plus their present modes) go to shared memory;
+// then the warp applies the inverse's rows to them, while a producer warp
+// streams the packed inverse through a ring of bulk copies that runs ahead
+// across both phases.
 //
 // What bounds it: the 645-word stream (5.2 KB a position in FP64) and the
 // modes, about 1.8 KB a zone of HBM traffic.  Each streamed word is read from
@@ -496,13 +497,16 @@ __global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph,
 constexpr int ADP6_CONS = 6 * 32;
 constexpr int ADP6_THREADS = ADP6_CONS + 32;
 constexpr int ADP6_CH = 2 * ADP6_UNIT;  // words a ring stage
-constexpr int ADP6_NS = 6;
+constexpr int ADP6_NS = 4;
 constexpr int ADP6_NCH = (ADP6_WORDS + ADP6_CH - 1) / ADP6_CH;  // the last one holds one unit
 template <typename F>
 struct Adp6SmemT {
   F stage[ADP6_NS][ADP6_CH][ADP6_ZB];
   F x[36][6][ADP6_ZB];  // right-hand sides in panel 1's unknowns
-  F nb[6][3][ADP6_ZB];  // the panels' new zone B
+  F bas[2][5][9][ADP6_ZB];  // monomials of a face's points, alternating over the faces
+  // the panels' new zone B [panel][component]: in the second half of bas, which
+  // the next block's faces reach after a barrier
+  __device__ __forceinline__ F* nb(int p, int c) { return &bas[1][0][0][0] + (p * 3 + c) * ADP6_ZB; }
   uint64_t full[ADP6_NS];
   uint64_t empty[ADP6_NS];
 };
@@ -658,66 +662,96 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
     return;
   }
   const int lane = tid & 31, w = tid >> 5;
+  const long long PS = (long long)NPANEL * d.S;
   RingPos<ADP6_NS> ring;
   for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     const long long t1 = blk * ADP6_ZB + lane;
     const bool inr = t1 < n1;
-    int p0 = 0, i = 0, j = 0, k = 0;
+    // lanes past the range work on its first position and store nothing
+    int p0 = 0, i = r.i0, j = r.j0, k = r.k0;
     if (inr) r.decode(t1, p0, i, j, k);
-    // panel w's right-hand sides: r1 = sum_q row_1(q) bq_w(q) + T_w^T vB_w
-    if (inr && mask_at(g, d, w, i, j) == 1) {
-      const R obl0 = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, 0, i, j, k), R(ph.smallnum));
-      const R vc0 = geoR<R>(g, d, CS_G_V_CEN, 0, 0, i, j, k), vc1 = geoR<R>(g, d, CS_G_V_CEN, 1, 0, i, j, k),
-              vc2 = geoR<R>(g, d, CS_G_V_CEN, 2, 0, i, j, k);
-      R c0[10];
-      coef10(g, d, 0, i, j, k, c0);
-      R rhs[30];
-#pragma unroll
-      for (int a = 0; a < 30; ++a) rhs[a] = R(0.0);
-#pragma unroll 1
-      for (int f = 0; f < 6; ++f) {
-        const int dir = f / 2;
-        const int fx = (f == 1) ? i - 1 : i, fy = (f == 3) ? j - 1 : j, fz = (f == 5) ? k - 1 : k;
-        const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-        const int BW = dir == 0 ? CS_G_XB_QW : (dir == 1 ? CS_G_YB_QW : CS_G_ZB_QW);
-        const int NF = dir == 0 ? CS_G_XF_N : (dir == 1 ? CS_G_YF_N : CS_G_ZF_N);
-        const int ns = dir == 2 ? 5 : 1;
-        const double* Bq = dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2]);
-        R dacc = R(0.0);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          const int nq = dir == 2 ? q : 0;
-          const R nx = geoR<R>(g, d, NF, nq, 0, fx, fy, fz), ny = geoR<R>(g, d, NF, ns + nq, 0, fx, fy, fz),
-                  nz = geoR<R>(g, d, NF, 2 * ns + nq, 0, fx, fy, fz);
-          const R x = (geoR<R>(g, d, QP, q, 0, fx, fy, fz) - vc0) * obl0;
-          const R y = (geoR<R>(g, d, QP, 5 + q, 0, fx, fy, fz) - vc1) * obl0;
-          const R z = (geoR<R>(g, d, QP, 10 + q, 0, fx, fy, fz) - vc2) * obl0;
-          const R bq = (R)Bq[d.at(q, w, fx, fy, fz)];
-          const R bfn[10] = {R(1.0), x, y, z, x * x - c0[4], y * y - c0[5], z * z - c0[6], x * y - c0[7],
-                             y * z - c0[8], x * z - c0[9]};
-#pragma unroll
-          for (int m = 0; m < 10; ++m) {
-            rhs[m] = rhs[m] + (m == 0 ? nx : nx * bfn[m]) * bq;
-            rhs[10 + m] = rhs[10 + m] + (m == 0 ? ny : ny * bfn[m]) * bq;
-            rhs[20 + m] = rhs[20 + m] + (m == 0 ? nz : nz * bfn[m]) * bq;
-          }
-          dacc = dacc + geoR<R>(g, d, BW, q, 0, fx, fy, fz) * bq;
-        }
-        S.x[30 + f][w][lane] = dacc;
-      }
-      const int8_t* umap = s.adp_pmap + w * 72;
-#pragma unroll
-      for (int v = 0; v < 30; ++v) {
-        const int u = __ldg(umap + v);
-        S.x[v][w][lane] = rhs[v] + (R)__ldg(umap + 36 + v) * Vat(s, d, 5 + u / 10, u % 10, w, i, j, k);
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 36; ++v) S.x[v][w][lane] = R(0.0);
-    }
-    adp6_sync();
+    // right-hand sides r1 = sum_q row_1(q) bq_p(q) + T_p^T vB_p, rows of
+    // component a for panels 3 h .. 3 h + 2: panel 1's quadrature points one
+    // face at a time, their monomials formed once by a warp a point
     const int a = w % 3, h = w / 3;
     R acc[3][10];
+    {
+      const unsigned zo = (unsigned)d.idx(i, j, k);  // box offset of the position
+      const double* cen = g.f[CS_G_V_CEN] + zo;
+      const double* cf = g.f[CS_G_COEF] + zo;
+      const R obl0 = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + zo), R(ph.smallnum));
+      const R vc0 = (R)__ldg(cen), vc1 = (R)__ldg(cen + PS), vc2 = (R)__ldg(cen + 2 * PS);
+      R c0[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m) c0[m] = (R)__ldg(cf + (4 + m) * PS);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int8_t* umap = s.adp_pmap + (3 * h + q) * 72 + 10 * a;
+#pragma unroll
+        for (int m = 0; m < 10; ++m) {
+          const int u = __ldg(umap + m);
+          acc[q][m] = (R)__ldg(umap + 36 + m) * s.V[(u % 10 * NVAR + 5 + u / 10) * PS + (3 * h + q) * d.S + zo];
+        }
+      }
+#pragma unroll 1
+      for (int f = 0; f < 6; ++f) {
+        const int dir = f >> 1;
+        const unsigned fo = zo - ((f & 1) ? (dir == 0 ? 1 : (dir == 1 ? d.NI : d.NI * d.NJ)) : 0);
+        R(&bas)[5][9][ADP6_ZB] = S.bas[f & 1];
+        if (w < 5) {
+          const double* qp = (dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP])) + fo;
+          const R x = ((R)__ldg(qp + w * PS) - vc0) * obl0, y = ((R)__ldg(qp + (5 + w) * PS) - vc1) * obl0,
+                  z = ((R)__ldg(qp + (10 + w) * PS) - vc2) * obl0;
+          bas[w][0][lane] = x;
+          bas[w][1][lane] = y;
+          bas[w][2][lane] = z;
+          bas[w][3][lane] = x * x - c0[0];
+          bas[w][4][lane] = y * y - c0[1];
+          bas[w][5][lane] = z * z - c0[2];
+          bas[w][6][lane] = x * y - c0[3];
+          bas[w][7][lane] = y * z - c0[4];
+          bas[w][8][lane] = x * z - c0[5];
+        }
+        const double* Bq = (dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2])) + 3 * h * d.S + fo;
+        const double* nf = (dir == 0 ? g.f[CS_G_XF_N] : (dir == 1 ? g.f[CS_G_YF_N] : g.f[CS_G_ZF_N])) + fo;
+        R bq[3][5], nn[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+          nn[c] = (R)__ldg(nf + (dir == 2 ? 5 * a + c : a) * PS);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) bq[q][c] = (R)Bq[c * PS + q * d.S];
+        }
+        if (a == 0) {
+          const double* bw = (dir == 0 ? g.f[CS_G_XB_QW] : (dir == 1 ? g.f[CS_G_YB_QW] : g.f[CS_G_ZB_QW])) + fo;
+          R dacc[3] = {R(0.0), R(0.0), R(0.0)};
+#pragma unroll
+          for (int c = 0; c < 5; ++c) {
+            const R wt = (R)__ldg(bw + c * PS);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) dacc[q] = dacc[q] + wt * bq[q][c];
+          }
+#pragma unroll
+          for (int q = 0; q < 3; ++q) S.x[30 + f][3 * h + q][lane] = dacc[q];
+        }
+        adp6_sync();
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) acc[q][0] = acc[q][0] + nn[c] * bq[q][c];
+#pragma unroll
+          for (int m = 0; m < 9; ++m) {
+            const R e = nn[c] * bas[c][m][lane];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) acc[q][1 + m] = acc[q][1 + m] + e * bq[q][c];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int m = 0; m < 10; ++m) S.x[10 * a + m][3 * h + q][lane] = acc[q][m];
+    }
+    adp6_sync();
 #pragma unroll
     for (int q = 0; q < 3; ++q)
 #pragma unroll
@@ -733,7 +767,7 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
           const int u = __ldg(umap + m);
           const R val = (R)__ldg(umap + 36 + m) * acc[q][m];
           Vat(s, d, 5 + u / 10, u % 10, p, i, j, k) = val;
-          if (m == 0) S.nb[p][u / 10][lane] = val;
+          if (m == 0) S.nb(p, u / 10)[lane] = val;
         }
       }
     }
@@ -741,7 +775,7 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
     if (inr && mask_at(g, d, w, i, j) == 1) {
       R* U = s.U;
       const long long o5 = d.at(4, w, i, j, k);
-      const double nb0 = S.nb[w][0][lane], nb1 = S.nb[w][1][lane], nb2 = S.nb[w][2][lane];
+      const double nb0 = S.nb(w, 0)[lane], nb1 = S.nb(w, 1)[lane], nb2 = S.nb(w, 2)[lane];
       const double u6 = U[d.at(5, w, i, j, k)], u7 = U[d.at(6, w, i, j, k)], u8 = U[d.at(7, w, i, j, k)];
       const double aa = (u6 * u6 + u7 * u7 + u8 * u8) * ph.ob8pi;
       U[d.at(5, w, i, j, k)] = nb0;
