@@ -775,18 +775,32 @@ __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g
 }
 
 // STEP 8.a-c (421:4686-5567): B at the five quadrature points of each face,
-// averaged from both sides and shifted to the facial mean.
+// averaged from both sides and shifted to the facial mean.  One thread a
+// face, the three directions in one launch (block T is tile T / 3 of
+// direction T % 3, so that L2 serves a zone's modes to all three).
+//
+// What bounds it: the loads of 30 modes a side.  Evaluating all three
+// components of both sides at once took 252 registers, 8 warps an SM.  The
+// face normal is one vector on x- and y-faces, so there each side's modes are
+// first contracted with it (10 values, one polynomial); on z-faces, where it
+// varies over the points, the components are taken one after another.
 template <typename R>
-__global__ void __launch_bounds__(TPB) k_faceB(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, int dir) {
-  const int QP = dir == 0 ? CS_G_XF_QP : (dir == 1 ? CS_G_YF_QP : CS_G_ZF_QP);
-  const int BW = dir == 0 ? CS_G_XB_QW : (dir == 1 ? CS_G_YB_QW : CS_G_ZB_QW);
-  const int NF = dir == 0 ? CS_G_XF_N : (dir == 1 ? CS_G_YF_N : CS_G_ZF_N);
-  double* Bq = s.Bq[dir];
-  const double* Bf = dir == 0 ? s.Bxf : (dir == 1 ? s.Byf : s.Bzf);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_faceB(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
+  const unsigned nt0 = (unsigned)((r0.count() + TPB - 1) / TPB), nt1 = (unsigned)((r1.count() + TPB - 1) / TPB),
+                 nt2 = (unsigned)((r2.count() + TPB - 1) / TPB);
+  for (unsigned T = blockIdx.x; T < 3 * max(nt0, max(nt1, nt2)); T += gridDim.x) {
+    // opaque to the compiler, which would otherwise form the addresses of all
+    // planes before the loop and spill them
+    long long PS = (long long)NPANEL * d.S;
+    asm volatile("" : "+l"(PS));
+    const int dir = T % 3;
+    const Range3 r = dir == 0 ? r0 : (dir == 1 ? r1 : r2);
+    const long long t = (long long)(T / 3) * TPB + threadIdx.x;
+    if (t >= r.count()) continue;
     int p, i, j, k;
     r.decode(t, p, i, j, k);
-    int lx = i, ly = j, lz = k, rx = i, ry = j, rz = k;
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
+    int lx = i, ly = j, rx = i, ry = j, rz = k;
     bool skip = false;
     if (dir == 0) {
       const int mL = mask_at(g, d, p, i, j), mR = mask_at(g, d, p, i + 1, j);
@@ -804,46 +818,60 @@ __global__ void __launch_bounds__(TPB) k_faceB(Dims d, PhysC ph, DGeom g, DState
       if (mask_at(g, d, p, i, j) == 0) skip = true;
       rz = k + 1;
     }
+    const double* qp = (dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP])) + o;
+    const double* qw = (dir == 0 ? g.f[CS_G_XB_QW] : (dir == 1 ? g.f[CS_G_YB_QW] : g.f[CS_G_ZB_QW])) + o;
+    const double* nf = (dir == 0 ? g.f[CS_G_XF_N] : (dir == 1 ? g.f[CS_G_YF_N] : g.f[CS_G_ZF_N])) + o;
     // the two sides' values in the state's type; the shift to the facial
     // mean in FP64, so the values average to the FP64 face B exactly
     R bq[5] = {R(0), R(0), R(0), R(0), R(0)};
     if (!skip) {
-      const R obl0 = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, p, lx, ly, lz), R(ph.smallnum));
-      const R obl02 = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, p, rx, ry, rz), R(ph.smallnum));
-      R cL[10], cR[10], vL[3][10], vR[3][10];
-      coef10(g, d, p, lx, ly, lz, cL);
-      coef10(g, d, p, rx, ry, rz, cR);
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        const long long z = (long long)p * d.S + (side ? d.idx(rx, ry, rz) : d.idx(lx, ly, k));
+        const R obl = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + z), R(ph.smallnum));
+        const double* cen = g.f[CS_G_V_CEN] + z;
+        const R cx = (R)__ldg(cen), cy = (R)__ldg(cen + PS), cz = (R)__ldg(cen + 2 * PS);
+        R c[10];
 #pragma unroll
-      for (int b = 0; b < 3; ++b)
+        for (int m = 4; m < 10; ++m) c[m] = (R)__ldg(g.f[CS_G_COEF] + m * PS + z);
+        R px[5], py[5], pz[5];
 #pragma unroll
-        for (int m = 0; m < 10; ++m) {
-          vL[b][m] = Vat(s, d, 5 + b, m, p, lx, ly, lz);
-          vR[b][m] = Vat(s, d, 5 + b, m, p, rx, ry, rz);
+        for (int q = 0; q < 5; ++q) {
+          px[q] = ((R)__ldg(qp + q * PS) - cx) * obl;
+          py[q] = ((R)__ldg(qp + (5 + q) * PS) - cy) * obl;
+          pz[q] = ((R)__ldg(qp + (10 + q) * PS) - cz) * obl;
         }
-      const R lcx = geoR<R>(g, d, CS_G_V_CEN, 0, p, lx, ly, lz), lcy = geoR<R>(g, d, CS_G_V_CEN, 1, p, lx, ly, lz),
-              lcz = geoR<R>(g, d, CS_G_V_CEN, 2, p, lx, ly, lz);
-      const R rcx = geoR<R>(g, d, CS_G_V_CEN, 0, p, rx, ry, rz), rcy = geoR<R>(g, d, CS_G_V_CEN, 1, p, rx, ry, rz),
-              rcz = geoR<R>(g, d, CS_G_V_CEN, 2, p, rx, ry, rz);
+        const R* v = s.V + 5 * PS + z;
+        if (dir < 2) {
+          const R n0 = (R)__ldg(nf), n1 = (R)__ldg(nf + PS), n2 = (R)__ldg(nf + 2 * PS);
+          R m[10];
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const int nq = dir == 2 ? q : 0, ns = dir == 2 ? 5 : 1;
-        const R nx = geoR<R>(g, d, NF, 0 * ns + nq, p, i, j, k), ny = geoR<R>(g, d, NF, 1 * ns + nq, p, i, j, k),
-                nz = geoR<R>(g, d, NF, 2 * ns + nq, p, i, j, k);
-        const R px = geoR<R>(g, d, QP, q, p, i, j, k), py = geoR<R>(g, d, QP, 5 + q, p, i, j, k),
-                pz = geoR<R>(g, d, QP, 10 + q, p, i, j, k);
-        const R x = (px - lcx) * obl0, y = (py - lcy) * obl0, z = (pz - lcz) * obl0;
-        const R x2 = (px - rcx) * obl02, y2 = (py - rcy) * obl02, z2 = (pz - rcz) * obl02;
-        const R bx = d_poly10(vL[0], cL, x, y, z), by = d_poly10(vL[1], cL, x, y, z), bz = d_poly10(vL[2], cL, x, y, z);
-        const R bx2 = d_poly10(vR[0], cR, x2, y2, z2), by2 = d_poly10(vR[1], cR, x2, y2, z2),
-                bz2 = d_poly10(vR[2], cR, x2, y2, z2);
-        bq[q] = R(0.5) * (nx * (bx + bx2) + ny * (by + by2) + nz * (bz + bz2));
+          for (int a = 0; a < 10; ++a)
+            m[a] = n0 * v[a * NVAR * PS] + n1 * v[(a * NVAR + 1) * PS] + n2 * v[(a * NVAR + 2) * PS];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) bq[q] = bq[q] + d_poly10(m, c, px[q], py[q], pz[q]);
+        } else {
+#pragma unroll 1
+          for (int b = 0; b < 3; ++b) {
+            R m[10];
+#pragma unroll
+            for (int a = 0; a < 10; ++a) m[a] = v[(a * NVAR + b) * PS];
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+              bq[q] = bq[q] + (R)__ldg(nf + (5 * b + q) * PS) * d_poly10(m, c, px[q], py[q], pz[q]);
+          }
+        }
       }
     }
-    double bd = Bf[d.at(0, p, i, j, k)];
+    double bd = (dir == 0 ? s.Bxf : (dir == 1 ? s.Byf : s.Bzf))[o];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) bd = bd - geo(g, d, BW, q, p, i, j, k) * (double)bq[q];
+    for (int q = 0; q < 5; ++q) {
+      bq[q] = R(0.5) * bq[q];
+      bd = bd - __ldg(qw + q * PS) * (double)bq[q];
+    }
+    double* Bq = (dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2])) + o;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) Bq[d.at(q, p, i, j, k)] = (double)bq[q] + bd;
+    for (int q = 0; q < 5; ++q) Bq[q * PS] = (double)bq[q] + bd;
   }
 }
 
@@ -1618,11 +1646,9 @@ void launch_faceB_adp_t(Solve& sv, DStateT<R>& st) {
   fx.i0 -= 1;
   fy.j0 -= 1;
   fz.k0 -= 1;
-  k_faceB<R><<<blocks_for(fx.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, 0);
-  mark(sv, "k_faceB");
-  k_faceB<R><<<blocks_for(fy.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fy, 1);
-  mark(sv, "k_faceB");
-  k_faceB<R><<<blocks_for(fz.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fz, 2);
+  const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + TPB - 1) / TPB);
+  const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 64);
+  k_faceB<R><<<nb, TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
   mark(sv, "k_faceB");
   launch_adp(sv);
 }
