@@ -228,8 +228,6 @@ __global__ void k_flat_bc(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, con
   }
 }
 
-// Stencils of STEP 7.a: (neighbour in plane, neighbour in plane, dz).
-__constant__ int c_st8[8][3] = {{0, 2, 1}, {0, 2, -1}, {1, 2, 1}, {1, 2, -1}, {0, 3, 1}, {0, 3, -1}, {1, 3, 1}, {1, 3, -1}};
 // Central 18-zone stencil of STEP 7.b / 9.c: (neighbour w or -1 for self, dz).
 __constant__ int c_n18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {-1, 1}, {-1, -1}, {8, 0}, {9, 0},  {10, 0},
                                  {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
@@ -247,54 +245,75 @@ __device__ __forceinline__ Nbr12 load_nbr(const DGeom& g, const Dims& d, int p, 
   return n;
 }
 
-// STEP 7.a (kE false) and STEP 9.b (kE true, the WENO-AO slopes of the
-// three E components, 421:6840-8400) with the work of a zone spread over
-// three threads: a block takes 32 zones; warp w first forms stencils w,
-// w + 3, w + 6 of each zone's eight one-sided 3x3 stencils (two in-plane
-// neighbours and one radial, 421:2561-3110) as closed-form inverses of the
-// scaled centroid offsets into shared memory; then, for variables w, w + 3,
-// w + 6 (STEP 7.a: primitives 0-7, 8 = entropy; STEP 9.b: E component w),
-// it forms the eight stencil gradients and their mean and combines them
-// with the WENO weights (IS + eps)^-4, central weight 100 (421:3116-3432),
-// so no thread keeps the 72 inverse entries in registers.  kEnt: the
-// entropy only (LIMIT_ALL_SLOPES_P2's STEP 7.a limits the entropy this way,
-// 420:5396-6306, and the primitives with k_p2).
+// STEP 7.a and STEP 9.b: the WENO-AO slopes (421:2465-3807, 421:6840-8400)
+// with the work of a zone spread over three threads.  A block takes 32 zones;
+// warp w first forms stencils w, w + 3, w + 6 of each zone's eight one-sided
+// 3x3 stencils (two in-plane neighbours and one radial, 421:2561-3110) as
+// closed-form inverses of the scaled centroid offsets into shared memory;
+// then, for its variables, the eight stencil gradients and their mean and
+// combines them with the WENO weights (IS + eps)^-4, central weight 100
+// (421:3116-3432), so no thread keeps the 72 inverse entries in registers.
+//   W7_PRIM  primitives 0-7 and (8) the entropy, variables w, w + 3, w + 6
+//   W7_E     E component w
+//   W7_ENT   the entropy only, by the last warp (LIMIT_ALL_SLOPES_P2's STEP
+//            7.a, 420:5396-6306; k_p2 does its primitives)
+//
+// What bounds it: FP64 instructions (the weights are FP64 in every form) and
+// latency at 18 (FP32: 24) warps an SM.  The neighbours are box offsets in
+// shared memory (tables indexed at run time lived in local memory), a
+// variable's values are loaded while the one before is worked on, and the nine
+// weights take Newton reciprocals.
+enum W7Kind { W7_PRIM, W7_E, W7_ENT };
 constexpr int W7A_ZT = 32;
-template <bool kE, typename R, bool kEnt = false>
-__global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_ao_split(Dims d, PhysC ph, DGeom g,
-                                                                                        DStateT<R> s, Range3 r) {
+template <W7Kind kK, typename R>
+__global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_slopes(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   __shared__ R ai[72][W7A_ZT];  // [stencil * 9 + entry][zone]
-  // c_st8 as a compile-time table, so that the unrolled stencil loop
-  // indexes the neighbour list with constants (registers, not local memory)
-  constexpr int st8[8][3] = {{0, 2, 1}, {0, 2, -1}, {1, 2, 1}, {1, 2, -1}, {0, 3, 1}, {0, 3, -1}, {1, 3, 1}, {1, 3, -1}};
+  __shared__ int nbo[4][W7A_ZT];  // box offsets of the R, L, U, D neighbours
   const int zl = threadIdx.x % W7A_ZT, w = threadIdx.x / W7A_ZT;
-  const long long nz = r.count(), ntile = (nz + W7A_ZT - 1) / W7A_ZT;
-  for (long long T = blockIdx.x; T < ntile; T += gridDim.x) {
-    const long long t = T * W7A_ZT + zl;
+  const unsigned nz = (unsigned)r.count(), ntile = (nz + W7A_ZT - 1) / W7A_ZT;
+  const int plane = d.NI * d.NJ;
+  const long long PS = (long long)NPANEL * d.S;
+  constexpr int nv = kK == W7_PRIM ? 9 : 3;
+  for (unsigned T = blockIdx.x; T < ntile; T += gridDim.x) {
+    const unsigned t = T * W7A_ZT + zl;
     int p = 0, i = 0, j = 0, k = 0;
     bool act = t < nz;
     if (act) {
       r.decode(t, p, i, j, k);
       act = mask_at(g, d, p, i, j) == 1;
     }
-    Nbr12 n;
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
     if (act) {
-      n = load_nbr(g, d, p, i, j);
-      const R obl0 = R(1.0) / fmax(geoR<R>(g, d, CS_G_V_SCALE, 0, p, i, j, k), R(ph.smallnum));
-      const R cx = geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k), cy = geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k),
-              cz = geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k);
+      nbo[w][zl] = (sten(g, d, p, i, j, w, 1) - j) * d.NI + (sten(g, d, p, i, j, w, 0) - i);
+      if (w == 0) nbo[3][zl] = (sten(g, d, p, i, j, 3, 1) - j) * d.NI + (sten(g, d, p, i, j, 3, 0) - i);
+    }
+    __syncthreads();
+    // variable q's value and its differences to R, L, U, D, up, down
+    auto load = [&](int q, R& f0, R (&D)[6]) {
+      const R* f = (kK == W7_E ? s.Esnap + q * PS : (kK == W7_PRIM && q < 8 ? s.V + q * PS : s.ent)) + o;
+      f0 = f[0];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) D[a] = f[nbo[a][zl]];
+      D[4] = f[plane];
+      D[5] = f[-plane];
+    };
+    const bool mine = act && (kK != W7_ENT || w == 2);
+    R f0 = R(0.0), D[6];
+    if (mine) load(w, f0, D);
+    if (act) {
+      const double* cen = g.f[CS_G_V_CEN] + o;
+      const R obl0 = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + o), R(ph.smallnum));
+      const R cx = (R)__ldg(cen), cy = (R)__ldg(cen + PS), cz = (R)__ldg(cen + 2 * PS);
+      // stencil st: neighbour (st >> 1) & 1 (R, L), 2 + (st >> 2) (U, D), dz +1 (even) or -1
 #pragma unroll 1
       for (int st = w; st < 8; st += 3) {
-        const int w1 = c_st8[st][0], w2 = c_st8[st][1], dz = c_st8[st][2];
-        const R a11 = (geoR<R>(g, d, CS_G_V_CEN, 0, p, n.x[w1], n.y[w1], k) - cx) * obl0;
-        const R a12 = (geoR<R>(g, d, CS_G_V_CEN, 1, p, n.x[w1], n.y[w1], k) - cy) * obl0;
-        const R a13 = (geoR<R>(g, d, CS_G_V_CEN, 2, p, n.x[w1], n.y[w1], k) - cz) * obl0;
-        const R a21 = (geoR<R>(g, d, CS_G_V_CEN, 0, p, n.x[w2], n.y[w2], k) - cx) * obl0;
-        const R a22 = (geoR<R>(g, d, CS_G_V_CEN, 1, p, n.x[w2], n.y[w2], k) - cy) * obl0;
-        const R a23 = (geoR<R>(g, d, CS_G_V_CEN, 2, p, n.x[w2], n.y[w2], k) - cz) * obl0;
-        const R a31 = (geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k + dz) - cx) * obl0;
-        const R a32 = (geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k + dz) - cy) * obl0;
-        const R a33 = (geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k + dz) - cz) * obl0;
+        const int o1 = nbo[(st >> 1) & 1][zl], o2 = nbo[2 + (st >> 2)][zl], o3 = (st & 1) ? -plane : plane;
+        const R a11 = ((R)__ldg(cen + o1) - cx) * obl0, a12 = ((R)__ldg(cen + PS + o1) - cy) * obl0,
+                a13 = ((R)__ldg(cen + 2 * PS + o1) - cz) * obl0;
+        const R a21 = ((R)__ldg(cen + o2) - cx) * obl0, a22 = ((R)__ldg(cen + PS + o2) - cy) * obl0,
+                a23 = ((R)__ldg(cen + 2 * PS + o2) - cz) * obl0;
+        const R a31 = ((R)__ldg(cen + o3) - cx) * obl0, a32 = ((R)__ldg(cen + PS + o3) - cy) * obl0,
+                a33 = ((R)__ldg(cen + 2 * PS + o3) - cz) * obl0;
         R ob = (-a13 * a22 * a31 + a12 * a23 * a31 + a13 * a21 * a32 - a11 * a23 * a32 - a12 * a21 * a33 + a11 * a22 * a33);
         ob = copysign(R(1.0), ob) / fmax(R(1.0e-32), fabs(ob));
         ai[st * 9 + 0][zl] = (-a23 * a32 + a22 * a33) * ob;
@@ -309,19 +328,17 @@ __global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_ao_
       }
     }
     __syncthreads();
-    if (act) {
+    if (mine) {
 #pragma unroll 1
-      for (int q = kEnt ? (w == 2 ? 8 : 9) : w; q < (kE ? 3 : 9); q += 3) {
-        const R* f = kE ? s.Esnap + ((long long)q * NPANEL + p) * d.S
-                        : (q < 8 ? s.V + ((long long)q * NPANEL + p) * d.S : s.ent + (long long)p * d.S);
-        const R f0 = f[d.idx(i, j, k)];
+      for (int q = kK == W7_ENT ? 8 : w; q < (kK == W7_ENT ? 9 : nv); q += 3) {
+        R g0 = R(0.0), Dn[6];
+        if (q + 3 < nv) load(q + 3, g0, Dn);
+#pragma unroll
+        for (int a = 0; a < 6; ++a) D[a] = D[a] - f0;
         R X[3][9];
 #pragma unroll
         for (int st = 0; st < 8; ++st) {
-          const int w1 = st8[st][0], w2 = st8[st][1], dz = st8[st][2];
-          const R R0 = f[d.idx(n.x[w1], n.y[w1], k)] - f0;
-          const R R1 = f[d.idx(n.x[w2], n.y[w2], k)] - f0;
-          const R R2 = f[d.idx(i, j, k + dz)] - f0;
+          const R R0 = D[(st >> 1) & 1], R1 = D[2 + (st >> 2)], R2 = D[4 + (st & 1)];
 #pragma unroll
           for (int rr = 0; rr < 3; ++rr)
             X[rr][st] = ai[st * 9 + rr * 3 + 0][zl] * R0 + ai[st * 9 + rr * 3 + 1][zl] * R1 + ai[st * 9 + rr * 3 + 2][zl] * R2;
@@ -330,41 +347,35 @@ __global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_ao_
         for (int rr = 0; rr < 3; ++rr)
           X[rr][8] = R(0.125) * (X[rr][0] + X[rr][1] + X[rr][2] + X[rr][3] + X[rr][4] + X[rr][5] + X[rr][6] + X[rr][7]);
         // The nonlinear weights (IS + eps)^-4 span far more than the FP32
-        // range, so they are formed in FP64 in every form.
-        double W[9];
+        // range, so they are formed in FP64 in every form; accumulated
+        // stencil by stencil and normalised at the end.
+        double sw = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
 #pragma unroll
         for (int st = 0; st < 9; ++st) {
           const double x0 = X[0][st], x1 = X[1][st], x2 = X[2][st];
-          const double IS = x0 * x0 + x1 * x1 + x2 * x2;
-          const double tt = IS + ph.smallnum;
-          const double t2 = tt * tt;
-          W[st] = (st < 8 ? 1.0 : 100.0) / (t2 * t2);
+          const double v = rcp_newton(x0 * x0 + x1 * x1 + x2 * x2 + ph.smallnum), v2 = v * v;
+          const double W = st < 8 ? v2 * v2 : 100.0 * (v2 * v2);
+          sw = sw + W;
+          t0 = t0 + W * x0;
+          t1 = t1 + W * x1;
+          t2 = t2 + W * x2;
         }
-        const double a11 = 1.0 / (W[0] + W[1] + W[2] + W[3] + W[4] + W[5] + W[6] + W[7] + W[8]);
+        const double a11 = 1.0 / sw;
+        const R gr[3] = {(R)(t0 * a11), (R)(t1 * a11), (R)(t2 * a11)};
+        if (kK == W7_E) {
 #pragma unroll
-        for (int st = 0; st < 9; ++st) W[st] = W[st] * a11;
-        R gr[3];
+          for (int m = 0; m < 3; ++m) s.E[(3 * (m + 1) + q) * PS + o] = gr[m];
+        } else if (kK == W7_PRIM && q < 8) {
 #pragma unroll
-        for (int rr = 0; rr < 3; ++rr) {
-          double tt = W[0] * (double)X[rr][0];
-#pragma unroll
-          for (int st = 1; st < 9; ++st) tt = tt + W[st] * (double)X[rr][st];
-          gr[rr] = (R)tt;
-        }
-        if (kE) {
-          s.E[d.at(3 + q, p, i, j, k)] = gr[0];
-          s.E[d.at(6 + q, p, i, j, k)] = gr[1];
-          s.E[d.at(9 + q, p, i, j, k)] = gr[2];
-        } else if (q < 8) {
-          Vat(s, d, q, 1, p, i, j, k) = gr[0];
-          Vat(s, d, q, 2, p, i, j, k) = gr[1];
-          Vat(s, d, q, 3, p, i, j, k) = gr[2];
+          for (int m = 0; m < 3; ++m) s.V[((m + 1) * NVAR + q) * PS + o] = gr[m];
         } else {
-          const R om = R(1.0) - s.flatA[d.at(0, p, i, j, k)];
-          s.ent[d.at(1, p, i, j, k)] = gr[0] * om;
-          s.ent[d.at(2, p, i, j, k)] = gr[1] * om;
-          s.ent[d.at(3, p, i, j, k)] = gr[2] * om;
+          const R om = R(1.0) - s.flatA[o];
+#pragma unroll
+          for (int m = 0; m < 3; ++m) s.ent[(m + 1) * PS + o] = gr[m] * om;
         }
+        f0 = g0;
+#pragma unroll
+        for (int a = 0; a < 6; ++a) D[a] = Dn[a];
       }
     }
     __syncthreads();
@@ -1589,7 +1600,7 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
   if (sv.p.flags & CS_FLAG_P2) {  // LIMIT_ALL_SLOPES_P2's STEP 7.a
     const long long nt = (b.count() + W7A_ZT - 1) / W7A_ZT;
     const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
-    k_weno_ao_split<false, R, true><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+    k_weno_slopes<W7_ENT, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
     mark(sv, "k_p2_entropy");
     if (st.p2_map)
       k_p2<false, true, P2_CPT, R><<<p2_blocks(sv, b, true), 256 / P2_CPT, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
@@ -1601,7 +1612,7 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
   {
     const long long nt = (a.count() + W7A_ZT - 1) / W7A_ZT;
     const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
-    k_weno_ao_split<false, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
+    k_weno_slopes<W7_PRIM, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_weno7a");
   }
   if (st.op_m9) {
@@ -1712,7 +1723,7 @@ void launch_efield_t(Solve& sv, DStateT<R>& st) {
   {
     const long long nt = (a.count() + W7A_ZT - 1) / W7A_ZT;
     const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
-    k_weno_ao_split<true, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
+    k_weno_slopes<W7_E, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_efield_b");
   }
   if (st.op_m10)
