@@ -24,9 +24,9 @@ constexpr int TPB = 128;
 // forms, for both sides, the nine centred monomials of quadrature point q in
 // the side zone's scaled coordinates.  Face states (450:545-2931): the 18
 // (side, primitive or entropy) polynomials of each face at the five points,
-// two variables of a side at a time, so that a variable's modes are read once
-// and a basis value once for two variables; the warp without a second pair
-// forms the frame of the x- and y-faces and the two area / volume ratios, once
+// four primitives of a side a warp, so that a mode is read once and a basis
+// value once for four primitives; the fifth warp takes the entropies, the frame
+// of the x- and y-faces and the two area / volume ratios, once
 // a face.  Fluxes: one quadrature point per thread (warp = point) rotates the
 // two states to the face frame, solves the HLL problem and rotates the
 // contributions back; they meet in shared memory and are summed in point
@@ -35,8 +35,11 @@ constexpr int TPB = 128;
 // T / 3 of direction T % 3, so the x, y and z faces of about the same zone
 // rows run side by side and L2 serves a zone's modes to all three.
 //
-// What bounds it: FP64 latency at the 20 warps its registers and shared memory
-// allow, so what counts is the FP64 instructions of a point.
+// What bounds it: L1 (73 % busy, mostly shared-memory words) and FP64 latency
+// at the 20 warps its registers and shared memory allow.  ms of a 6 x 128^2 x
+// 64 step, FP64 / FP32: 29.5 / 19.8 with every thread forming its point's basis
+// per variable, 22.3 / 14.6 with the basis kept and two primitives a warp at a
+// time, 21.3 / 14.1 with four.
 constexpr int FLUX_FACES = 32;
 // Registers / occupancy: 4 blocks per SM suit the FP64 instantiation, 7 the
 // FP32 one (measured on the 6 x 128^2 x 64 shell).
@@ -121,33 +124,33 @@ __global__ void __launch_bounds__(FLUX_FACES * 5, sizeof(R) == 4 ? 7 : 4) k_flux
     }
     __syncthreads();
     if (!skip) {
-      // pairs 0-3 of side 0 and 4-7 of side 1: primitives 2 n, 2 n + 1
-      auto pair = [&](int pr) {
-        const int side = pr >> 2, c = 2 * (pr & 3);
+      if (jq < 4) {  // primitives 4 (jq & 1) .. + 3 of side jq >> 1
+        const int side = jq >> 1, c = 4 * (jq & 1);
         const R* v = s.V + c * PS + (side ? zo1 : zo0);
-        R m[2][10];
+        R u[5][4];
 #pragma unroll
-        for (int a = 0; a < 10; ++a) {
-          m[0][a] = v[a * NVAR * PS];
-          m[1][a] = v[(a * NVAR + 1) * PS];
+        for (int n = 0; n < 4; ++n) {
+          const R m = v[n * PS];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) u[q][n] = m;
         }
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          R u0 = m[0][0], u1 = m[1][0];
+        for (int a = 1; a < 10; ++a) {
+          R m[4];
 #pragma unroll
-          for (int a = 1; a < 10; ++a) {
-            const R b = sc.bs[side][q][a - 1][lane];
-            u0 = u0 + m[0][a] * b;
-            u1 = u1 + m[1][a] * b;
+          for (int n = 0; n < 4; ++n) m[n] = v[(a * NVAR + n) * PS];
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const R bv = sc.bs[side][q][a - 1][lane];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) u[q][n] = u[q][n] + m[n] * bv;
           }
-          fs[side][c][q][lane] = u0;
-          fs[side][c + 1][q][lane] = u1;
         }
-      };
-      pair(jq);
-      if (jq < 3) {
-        pair(jq + 5);
-      } else if (jq == 3) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+          for (int n = 0; n < 4; ++n) fs[side][c + n][q][lane] = u[q][n];
+      } else {
 #pragma unroll
         for (int side = 0; side < 2; ++side) {
           const R* e = s.ent + (side ? zo1 : zo0);
@@ -158,7 +161,6 @@ __global__ void __launch_bounds__(FLUX_FACES * 5, sizeof(R) == 4 ? 7 : 4) k_flux
             fs[side][8][q][lane] = e0 + e1 * b[0][lane] + e2 * b[1][lane] + e3 * b[2][lane];
           }
         }
-      } else {
         const R area = (R)__ldg(ar + o);
         av[0][lane] = area * rcp_newton((R)__ldg(g.f[CS_G_V_VOL] + zo0));
         av[1][lane] = area * rcp_newton((R)__ldg(g.f[CS_G_V_VOL] + zo1));
