@@ -779,10 +779,10 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
       if (!m.op_m10) return fail(sv, CS_ERR_NOMEM, "no device room for the least-squares operators CS_FLAG_P2 needs");
       m.p2_shared = shared;
       const long long np = shared ? nl / 6 : nl;
-      const size_t pb = (size_t)np * (648 + 800) * sizeof(R);
+      const size_t pb = ((size_t)(np + 31) / 32 * 32 * 648 + (size_t)np * 800) * sizeof(R);
       if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || pb + (size_t)8 * S6 + ((size_t)2 << 30) >= fr)
         return fail(sv, CS_ERR_NOMEM, "no device room for the CS_FLAG_P2 stencil inverses");
-      m.op_p2v = mdalloc(sv, m, (size_t)np * 648 * sizeof(R), e);
+      m.op_p2v = mdalloc(sv, m, (size_t)((np + 31) / 32 * 32) * 648 * sizeof(R), e);  // whole blocks
       m.op_p2e = m.op_p2v ? mdalloc(sv, m, (size_t)np * 800 * sizeof(R), e) : nullptr;
       if (!m.op_p2v || !m.op_p2e) return cuda_fail(sv, e, "cudaMalloc(P2 stencil inverses)");
     }
@@ -886,6 +886,7 @@ int mesh_attach(Solve& sv, const std::shared_ptr<MeshRes>& mp) {
   CS_CUDA(sv, cudaStreamCreateWithFlags(&sv.stream, cudaStreamNonBlocking));
   CS_CUDA(sv, pool_acquire(sv));
   set_adp_smem_limits();
+  set_p2_smem_limits();
   set_weno_smem_limits();
   const bool fresh = !m.on_device;
   if (fresh)

@@ -70,7 +70,7 @@ struct DStateT {
   R* op_m10;                             // STEP 9.c row weights Minv A_rr^T, [19 x 10][zones of shrink(2)], or null
   const LsqPanelMap* lsq_map9;           // op_m9 shared by the panels (panel 1's zones only), or null
   const LsqPanelMap* lsq_map10;          // op_m10 likewise
-  R* op_p2v;                             // CS_FLAG_P2 STEP 7.a stencil inverses, [8 x 9 x 9][zones of shrink(2)], or null
+  R* op_p2v;                             // CS_FLAG_P2 STEP 7.a stencil inverses of the zones of shrink(2), [32-zone block][8 x 9 x 9][32], or null
   R* op_p2e;                             // CS_FLAG_P2 STEP 9.b stencil inverses, [8 x 10 x 10][zones of shrink(2)], or null
   const LsqPanelMap* p2_map;             // op_p2v / op_p2e shared by the panels, or null
   void* adp_lu;                          // ADP operators per block of zones, or null: the KKT factors (FP64, [1296 in use
@@ -452,6 +452,7 @@ void launch_faceB_adp(Solve& s);
 void launch_adp(Solve& s);
 void launch_adp_factor(Solve& s);
 void set_adp_smem_limits();
+void set_p2_smem_limits();
 void set_weno_smem_limits();
 long long adp_range_count(const Solve& sv);
 long long adp_factor_doubles(const Solve& sv, bool shared);

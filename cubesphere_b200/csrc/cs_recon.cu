@@ -256,7 +256,7 @@ __device__ __forceinline__ Nbr12 load_nbr(const DGeom& g, const Dims& d, int p, 
 //   W7_PRIM  primitives 0-7 and (8) the entropy, variables w, w + 3, w + 6
 //   W7_E     E component w
 //   W7_ENT   the entropy only, by the last warp (LIMIT_ALL_SLOPES_P2's STEP
-//            7.a, 420:5396-6306; k_p2 does its primitives)
+//            7.a, 420:5396-6306; k_p2_prim does its primitives)
 //
 // What bounds it: FP64 instructions (the weights are FP64 in every form) and
 // latency at 18 (FP32: 24) warps an SM.  The neighbours are box offsets in
@@ -1164,7 +1164,8 @@ __device__ __forceinline__ void p2_zone(const Nbr12& n, int st, int rr, int i, i
 // The inverses of every zone's eight one-sided stencil matrices (geometry
 // only), built once per mesh: STEP 7.a's 9 x 9 RECONSTRUCTION_COEFS systems
 // (the modes x .. xz from the zone-average differences) into
-// op_p2v[(st * 9 + m) * 9 + rr][zone] and STEP 9.b's 10 x 10
+// op_p2v (word (st * 9 + m) * 9 + rr of blocks of 32 zones,
+// [block][648][32]: a stencil is one bulk copy) and STEP 9.b's 10 x 10
 // INTERPOLATION_COEFS systems (the zone itself first, modes 1 .. xz from
 // the point values) into op_p2e[(st * 10 + m) * 10 + rr][zone], inverted by
 // MATINV's LU (121matinv.f:8).  Shared by the panels: panel 1's zones only.
@@ -1207,35 +1208,263 @@ __global__ void k_ops_p2(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
       }
       d_matinv<9>(A, Ai);
       d_matinv<10>(B, Bi);
-      for (int e = 0; e < 81; ++e) s.op_p2v[(long long)(st * 81 + e) * nr_ + t] = (R)Ai[e];
+      for (int e = 0; e < 81; ++e) s.op_p2v[(t / 32 * 648 + st * 81 + e) * 32 + t % 32] = (R)Ai[e];
       for (int e = 0; e < 100; ++e) s.op_p2e[(long long)(st * 100 + e) * nr_ + t] = (R)Bi[e];
     }
   }
 }
 
-// STEP 7.a (kE false) / STEP 9.b (kE true) of LIMIT_ALL_SLOPES_P2.  A block
-// takes 32 zones and all the variables (the 8 primitives / the 3 E
-// components), a thread one zone and CPT variables: the nine stencils'
-// modes (eight one-sided from the resident inverses, the central one from
-// P12's resident row weights: STEP 7.b's 18-zone least squares, STEP 9.c's
-// 19-zone one), their smoothness indicators over the zone's unit cube
-// (420:5245-5257) and WENO weights 1 and 100 over (IS + smallnum)^4 (in
-// FP64 in every form), then the weighted modes, summed stencil by stencil
-// in the reference's order (the one-sided stencils' modes formed again
-// rather than kept: 72 values a variable).  Each operator word is loaded
-// once for the CPT variables of the thread (the sums are the same for any
-// CPT).  STEP 7.a writes modes 2..10 damped by the flattener; STEP 9.b only
-// the point value, flattened toward the unlimited one (the edge solver
-// consumes nothing else).  With kShared the inverses are panel 1's, rotated
-// per panel like the row weights, and iteration T covers tile T / 6 of
-// panel T % 6 so that the six blocks reading one tile's inverses run
-// together.
-template <bool kE, bool kShared, int CPT, typename R>
-__global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
-  constexpr int NM = kE ? 10 : 9, NR = kE ? 10 : 9, M0 = kE ? 0 : 1, NO = kE ? 1 : 9;
+// Central 18-zone stencil: (neighbour or 12 for the zone itself, dz).
+__constant__ int c_n18s[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {12, 1}, {12, -1}, {8, 0}, {9, 0},  {10, 0},
+                                  {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
+
+// STEP 7.a of LIMIT_ALL_SLOPES_P2.  A block takes 32 zones, a warp two of the 8
+// primitives.  For each of the eight one-sided stencils a thread forms its
+// primitives' modes from the resident inverse, their smoothness indicator over
+// the zone's unit cube (420:5245-5257) and the WENO weight 1 / (IS +
+// smallnum)^4 (in FP64 in every form), and adds the weighted modes; then the
+// central stencil (STEP 7.b's resident row weights) with weight 100, and the
+// sum is normalised, so that no stencil is formed twice.  Modes 2..10 are
+// stored damped by the flattener.
+//
+// A producer warp brings the inverses, a stencil a stage, through a ring of
+// bulk copies; a stencil's neighbour values are loaded while the one before is
+// worked on.  With kShared the inverses are panel 1's, rotated per panel like
+// the row weights, and tile T is tile T / 6 of panel T % 6, so that L2 serves
+// them to six blocks.
+//
+// What bounds it: shared-memory reads of the inverses, one per two
+// multiply-adds, at the 12 to 16 warps its registers allow.  Two warps that
+// read every word from L2 themselves, twice (once for the indicators, once for
+// the modes), with four primitives a thread in 255 registers, took 13.4 ms of a
+// 6 x 64^2 x 32 step in FP64; this takes 7.6.
+constexpr int P2_NW = 4;  // warps of a block but the producer
+constexpr int P2_CONS = 32 * P2_NW;
+constexpr int P2_THREADS = P2_CONS + 32;
+// blocks an SM: three in FP64, with some of the sums in local memory, measured
+// 7.6 ms a step, two without that 8.2
+constexpr int p2_blocks(size_t word) { return word == 4 ? 4 : 3; }
+template <typename R>
+struct P2Smem {
+  static constexpr int NS = sizeof(R) == 4 ? 3 : 2;
+  R stage[NS][81][32];
+  int nbo[2][13][32];  // in-plane neighbours as box offsets (12: the zone), alternating over the tiles
+  uint64_t full[NS];
+  uint64_t empty[NS];
+};
+template <bool kShared, typename R>
+__global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+  using Smem = P2Smem<R>;
+  extern __shared__ __align__(128) unsigned char p2_raw[];
+  Smem& S = *reinterpret_cast<Smem*>(p2_raw);
+  const int tid = threadIdx.x;
+  const long long nz = r.count(), npp = nz / 6;
+  const unsigned nw = (unsigned)(kShared ? npp : nz), ntile = kShared ? 6 * ((nw + 31) / 32) : (nw + 31) / 32;
+  if (tid == 0) {
+    for (int q = 0; q < Smem::NS; ++q) {
+      mbar_init(&S.full[q], 1);
+      mbar_init(&S.empty[q], P2_NW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  RingPos<Smem::NS> ring;
+  if (tid >= P2_CONS) {
+    if (tid == P2_CONS) {
+      const R* op = s.op_p2v;
+      constexpr uint32_t bytes = 81 * 32 * sizeof(R);
+      bool first = true;  // the ring's first round finds every stage free
+      for (unsigned T = blockIdx.x; T < ntile; T += gridDim.x) {
+        const R* src = op + (long long)(kShared ? T / 6 : T) * (8 * 81 * 32);
+        for (int st = 0; st < 8; ++st) {
+          if (!first) mbar_wait(&S.empty[ring.slot], ring.par ^ 1, s.err_flag);
+          mbar_expect_tx(&S.full[ring.slot], bytes);
+          bulk_g2s(&S.stage[ring.slot][0][0], src + st * (81 * 32), bytes, &S.full[ring.slot]);
+          ring.next();
+          if (ring.slot == 0) first = false;
+        }
+      }
+    }
+    return;
+  }
+  const int lane = tid & 31, w = tid >> 5;
+  const int plane = d.NI * d.NJ;
+  const long long PS = (long long)NPANEL * d.S;
+  int buf = 0;
+  for (unsigned T = blockIdx.x; T < ntile; T += gridDim.x, buf ^= 1) {
+    const unsigned tw = (kShared ? T / 6 : T) * 32 + lane;
+    bool act = tw < nw;
+    const long long t = kShared ? (T % 6) * npp + tw : tw;
+    int p = 0, i = r.i0, j = r.j0, k = r.k0;
+    if (act) {
+      r.decode(t, p, i, j, k);
+      act = mask_at(g, d, p, i, j) == 1;
+    }
+    int(&nbo)[13][32] = S.nbo[buf];
+    if (act) {
+      for (int n = w; n < 12; n += P2_NW) {
+        nbo[n][lane] = (sten(g, d, p, i, j, n, 1) - j) * d.NI + (sten(g, d, p, i, j, n, 0) - i);
+      }
+    }
+    if (w == 0) nbo[12][lane] = 0;
+    // the offsets are complete; the other copy is no longer read
+    asm volatile("bar.sync 1, %0;" ::"n"(P2_CONS) : "memory");
+    const long long o = (long long)p * d.S + d.idx(i, j, k);
+    const R* f = s.V + 2 * w * PS + o;
+    // smoothness weight of the modes xx .. xz over the unit cube (x y z: 1 /
+    // 12).  The one-sided stencils' modes stay in panel 1's frame (with
+    // kShared) and so take panel 1's moments; their sum is rotated once.
+    double wis[6];
+    auto cube_weights = [&](long long z) {
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const double c = act ? __ldg(g.f[CS_G_COEF] + (4 + m) * PS + z) : 0.0;
+        wis[m] = m < 3 ? sqr(c - 1.0 / 12.0) + 1.0 / 180.0 : sqr(c) + 1.0 / 144.0;
+      }
+    };
+    cube_weights(kShared ? d.idx(i, j, k) : o);
+    auto smooth = [&](const R* X) {  // X: modes x .. xz
+      return ((double)X[0] * X[0] + (double)X[1] * X[1] + (double)X[2] * X[2]) * (1.0 / 12.0) +
+             ((double)X[3] * X[3]) * wis[0] + ((double)X[4] * X[4]) * wis[1] + ((double)X[5] * X[5]) * wis[2] +
+             ((double)X[6] * X[6]) * wis[3] + ((double)X[7] * X[7]) * wis[4] + ((double)X[8] * X[8]) * wis[5];
+    };
+    R f0[2];
+    double sw[2], acc[2][9];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      f0[c] = act ? f[c * PS] : R(0.0);
+      sw[c] = 0.0;
+#pragma unroll
+      for (int m = 0; m < 9; ++m) acc[c][m] = 0.0;
+    }
+    auto add = [&](int c, const R* X, double w0) {  // weighted modes of one stencil
+      const double v = rcp_newton(smooth(X) + ph.smallnum), v2 = v * v, W = w0 * (v2 * v2);
+      sw[c] = sw[c] + W;
+#pragma unroll
+      for (int m = 0; m < 9; ++m) acc[c][m] = acc[c][m] + W * (double)X[m];
+    };
+    // the nine zones of stencil st (p2_zone's order)
+    auto load = [&](int st, R (&D)[2][9]) {
+      const int q = st & 3, dz = st < 4 ? plane : -plane, right = q == 0 || q == 3 ? 0 : 1, up = q < 2 ? 0 : 1;
+      const int oa = nbo[right][lane], ob = nbo[2 + up][lane];
+      const int off[9] = {oa, ob, dz, nbo[4 + right][lane], nbo[6 + up][lane], 2 * dz, nbo[8 + q][lane], oa + dz, ob + dz};
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int rr = 0; rr < 9; ++rr) D[c][rr] = act ? f[c * PS + off[rr]] : R(0.0);
+    };
+    R D[2][9];
+    load(0, D);
+#pragma unroll 1
+    for (int st = 0; st < 8; ++st) {
+      R Dn[2][9];
+      if (st < 7) load(st + 1, Dn);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int rr = 0; rr < 9; ++rr) D[c][rr] = D[c][rr] - f0[c];
+      if (!mbar_try_wait(&S.full[ring.slot], ring.par)) mbar_wait(&S.full[ring.slot], ring.par, s.err_flag);
+      const R(&A)[81][32] = S.stage[ring.slot];
+      R Y[2][9];
+#pragma unroll
+      for (int m = 0; m < 9; ++m) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) Y[c][m] = R(0.0);
+#pragma unroll
+        for (int rr = 0; rr < 9; ++rr) {
+          const R a = A[m * 9 + rr][lane];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) Y[c][m] = Y[c][m] + a * D[c][rr];
+        }
+      }
+      // this warp's reads are done before the copy engine may write the stage again
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.empty[ring.slot]);
+      ring.next();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        add(c, Y[c], 1.0);
+#pragma unroll
+        for (int rr = 0; rr < 9; ++rr) D[c][rr] = Dn[c][rr];
+      }
+    }
+    if (!act) continue;
+    if (kShared) {
+      cube_weights(o);
+      const unsigned long long qsrc = s.p2_map[p].src;
+      const unsigned int qneg = s.p2_map[p].neg;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        double a1[9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) a1[m] = acc[c][m];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) acc[c][m] = lsq_rotated<1>(a1, m + 1, qsrc, qneg);
+      }
+    }
+    {  // central stencil from the resident row weights
+      R Y[2][9];
+      const LsqPanelMap* cmap = s.lsq_map9;
+      const long long tc = cmap ? t - (long long)p * npp : t, ncw = cmap ? npp : nz;
+      const M9Block cb = m9_block(tc / 32, ncw);
+      const R* wc = s.op_m9 + cb.off + tc % 32;
+      const long long cstride = cb.wid;
+#pragma unroll
+      for (int m = 0; m < 9; ++m)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) Y[c][m] = R(0.0);
+#pragma unroll 3
+      for (int rr = 0; rr < 18; ++rr) {
+        const int off = nbo[c_n18s[rr][0]][lane] + c_n18s[rr][1] * plane;
+        R v[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) v[c] = f[c * PS + off] - f0[c];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+          const R a = __ldg(wc + (long long)(rr * 9 + m) * cstride);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) Y[c][m] = Y[c][m] + a * v[c];
+        }
+      }
+      const unsigned long long csrc = cmap ? cmap[p].src : LSQ_IDENTITY_SRC;
+      const unsigned int cneg = cmap ? cmap[p].neg : 0u;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        R X[9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) X[m] = cmap ? lsq_rotated<1>(Y[c], m + 1, csrc, cneg) : Y[c][m];
+        add(c, X, 100.0);
+      }
+    }
+    const R fl = s.flatA[o], x = R(1.0) - fl;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const double wn = 1.0 / sw[c];
+#pragma unroll
+      for (int m = 0; m < 9; ++m) s.V[((m + 1) * NVAR + 2 * w + c) * PS + o] = (R)(acc[c][m] * wn) * x;
+    }
+  }
+}
+
+// STEP 9.b of LIMIT_ALL_SLOPES_P2, a thread one zone and the three E components:
+// the nine stencils' modes (eight one-sided from the resident inverses, the
+// zone itself first; the central one STEP 9.c's 19-zone row weights), their
+// smoothness indicators and weights as in k_p2_prim, then the weighted point
+// values, summed stencil by stencil (the one-sided stencils' constants formed
+// again rather than kept).  Each operator word is loaded once for the three
+// components, from L2: a ring of the stencils' inverses, with a warp a
+// component, measured 3.6 ms of a 6 x 64^2 x 32 step against 2.8, since its
+// reads of shared memory serve one multiply-add each and its stages leave
+// room for four blocks an SM.  Only the point value is stored, flattened toward
+// the unlimited one (the edge solver consumes nothing else).  Panel order as
+// in k_p2_prim.
+template <bool kShared, typename R>
+__global__ void __launch_bounds__(32) k_p2_efield(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+  constexpr int NM = 10, NR = 10;
   constexpr int n18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {-1, 1}, {-1, -1}, {8, 0}, {9, 0},  {10, 0},
                               {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
-  const int lane = threadIdx.x & 31, q0 = (threadIdx.x >> 5) * CPT;
+  const int lane = threadIdx.x;
   const long long nz = r.count(), npp = nz / 6, nw = kShared ? npp : nz;
   const long long ntile = kShared ? 6 * ((npp + 31) / 32) : (nz + 31) / 32;
   const long long cstr = (long long)NPANEL * d.S;  // stride between variables
@@ -1270,47 +1499,46 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
              ((double)X[3] * X[3]) * wis[3] + ((double)X[4] * X[4]) * wis[4] + ((double)X[5] * X[5]) * wis[5] +
              ((double)X[6] * X[6]) * wis[6] + ((double)X[7] * X[7]) * wis[7] + ((double)X[8] * X[8]) * wis[8];
     };
-    const R* fb = (kE ? s.Esnap : s.V) + ((long long)q0 * NPANEL + p) * d.S;
+    const R* fb = s.Esnap + (long long)p * d.S;
     const long long o0 = d.idx(i, j, k);
-    R f0[CPT];
+    R f0[3];
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) f0[c] = fb[c * cstr + o0];
+    for (int c = 0; c < 3; ++c) f0[c] = fb[c * cstr + o0];
     const unsigned long long qsrc = kShared ? s.p2_map[p].src : LSQ_IDENTITY_SRC;
     const unsigned int qneg = kShared ? s.p2_map[p].neg : 0u;
-    const R* op = (kE ? s.op_p2e : s.op_p2v) + tw;
+    const R* op = s.op_p2e + tw;
     // The modes of one-sided stencil st for the thread's variables, group
     // by group -- the groups the panel rotations permute within (for E the
     // constant first, then x y z, the squares, the cross terms) -- rotated
     // to this panel and handed to visit(group, X[variable][0..2]); groups
     // g0 .. g1 - 1 only.  Three modes a variable are live at a time.
-    constexpr int NG = kE ? 4 : 3;
+    constexpr int NG = 4;
     auto stencil = [&](int st, int g0, int g1, auto&& visit) {
-      R Rv[CPT][NR];
+      R Rv[3][NR];
 #pragma unroll
       for (int rr = 0; rr < NR; ++rr) {
         int zx = i, zy = j, zz = k;
-        if (!kE || rr > 0) p2_zone(n, st, rr - (kE ? 1 : 0), i, j, k, zx, zy, zz);
+        if (rr > 0) p2_zone(n, st, rr - 1, i, j, k, zx, zy, zz);
         const long long off = d.idx(zx, zy, zz);
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          const R v = fb[c * cstr + off];
-          Rv[c][rr] = kE ? v : v - f0[c];
+        for (int c = 0; c < 3; ++c) {
+          Rv[c][rr] = fb[c * cstr + off];
         }
       }
 #pragma unroll
       for (int gi = 0; gi < NG; ++gi) {
         if (gi < g0 || gi >= g1) continue;
-        const int mb = kE ? (gi == 0 ? 0 : 3 * gi - 2) : 3 * gi + 1;  // first mode of the group
-        const int gs = (kE && gi == 0) ? 1 : 3;
-        R Y[CPT][3];
+        const int mb = gi == 0 ? 0 : 3 * gi - 2;  // first mode of the group
+        const int gs = gi == 0 ? 1 : 3;
+        R Y[3][3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
           if (q < gs) {
             R w[NR];
 #pragma unroll
-            for (int rr = 0; rr < NR; ++rr) w[rr] = __ldg(op + (long long)((st * NM + mb - M0 + q) * NR + rr) * nw);
+            for (int rr = 0; rr < NR; ++rr) w[rr] = __ldg(op + (long long)((st * NM + mb + q) * NR + rr) * nw);
 #pragma unroll
-            for (int c = 0; c < CPT; ++c) {
+            for (int c = 0; c < 3; ++c) {
               R acc = R(0.0);
 #pragma unroll
               for (int rr = 0; rr < NR; ++rr) acc = acc + w[rr] * Rv[c][rr];
@@ -1318,7 +1546,7 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
             }
           }
         }
-        R X[CPT][3];
+        R X[3][3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
           if (q < gs) {
@@ -1326,7 +1554,7 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
             const int mu = kShared ? (int)((qsrc >> (4 * mm)) & 15) - mb : q;
             const bool ng = kShared && ((qneg >> mm) & 1u);
 #pragma unroll
-            for (int c = 0; c < CPT; ++c) {
+            for (int c = 0; c < 3; ++c) {
               const R v = mu == 0 ? Y[c][0] : (mu == 1 ? Y[c][1] : Y[c][2]);
               X[c][q] = ng ? -v : v;
             }
@@ -1335,54 +1563,51 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
         visit(gi, X);
       }
     };
-    double IS[CPT][9];
-    R X8[CPT][NM];
+    double IS[3][9];
+    R X8[3][NM];
     {  // central stencil from the resident row weights
-      R Y[CPT][NM];
+      R Y[3][NM];
 #pragma unroll
-      for (int c = 0; c < CPT; ++c)
+      for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int m = 0; m < NM; ++m) Y[c][m] = R(0.0);
-      const LsqPanelMap* cmap = kE ? s.lsq_map10 : s.lsq_map9;
+      const LsqPanelMap* cmap = s.lsq_map10;
       const long long tc = cmap ? t - (long long)p * npp : t, ncw = cmap ? npp : nz;
-      const M9Block cb = m9_block(tc / 32, ncw);
-      const R* wc = kE ? s.op_m10 + tc : s.op_m9 + cb.off + tc % 32;
-      const long long cstride = kE ? ncw : cb.wid;
+      const R* wc = s.op_m10 + tc;
 #pragma unroll
       for (int rr = 0; rr < NR + 9; ++rr) {
-        const int ro = kE ? rr - 1 : rr;  // E: the zone itself first
+        const int ro = rr - 1;  // the zone itself first
         const int w = ro < 0 ? -1 : n18[ro][0], dz = ro < 0 ? 0 : n18[ro][1];
         const long long off = d.idx(w < 0 ? i : n.x[w], w < 0 ? j : n.y[w], k + dz);
-        R Rv[CPT];
+        R Rv[3];
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          const R v = fb[c * cstr + off];
-          Rv[c] = kE ? v : v - f0[c];
+        for (int c = 0; c < 3; ++c) {
+          Rv[c] = fb[c * cstr + off];
         }
 #pragma unroll
         for (int m = 0; m < NM; ++m) {
-          const R wv = __ldg(wc + (long long)(rr * NM + m) * cstride);
+          const R wv = __ldg(wc + (long long)(rr * NM + m) * ncw);
 #pragma unroll
-          for (int c = 0; c < CPT; ++c) Y[c][m] = Y[c][m] + wv * Rv[c];
+          for (int c = 0; c < 3; ++c) Y[c][m] = Y[c][m] + wv * Rv[c];
         }
       }
       const unsigned long long csrc = cmap ? cmap[p].src : LSQ_IDENTITY_SRC;
       const unsigned int cneg = cmap ? cmap[p].neg : 0u;
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) {
+      for (int c = 0; c < 3; ++c) {
 #pragma unroll
-        for (int m = 0; m < NM; ++m) X8[c][m] = cmap ? lsq_rotated<M0>(Y[c], m + M0, csrc, cneg) : Y[c][m];
-        IS[c][8] = smooth(X8[c] + (kE ? 1 : 0));
+        for (int m = 0; m < NM; ++m) X8[c][m] = cmap ? lsq_rotated<0>(Y[c], m, csrc, cneg) : Y[c][m];
+        IS[c][8] = smooth(X8[c] + 1);
       }
     }
 #pragma unroll 1
     for (int st = 0; st < 8; ++st) {
-      double sm[CPT];
+      double sm[3];
       stencil(st, 0, NG, [&](int gi, R (*X)[3]) {
-        const int gg = kE ? gi - 1 : gi;  // 0: x y z, 1: the squares, 2: the cross terms
-        if (gg < 0) return;               // E's constant has no indicator term
+        const int gg = gi - 1;  // 0: x y z, 1: the squares, 2: the cross terms
+        if (gg < 0) return;     // the constant has no indicator term
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
+        for (int c = 0; c < 3; ++c) {
           const double a0 = X[c][0], a1 = X[c][1], a2 = X[c][2];
           if (gg == 0)
             sm[c] = (a0 * a0 + a1 * a1 + a2 * a2) * wis[0];
@@ -1391,11 +1616,11 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
         }
       });
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) IS[c][st] = sm[c];
+      for (int c = 0; c < 3; ++c) IS[c][st] = sm[c];
     }
-    double W[CPT][9];
+    double W[3][9];
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) {
+    for (int c = 0; c < 3; ++c) {
 #pragma unroll
       for (int st = 0; st < 9; ++st) {
         const double tt = IS[c][st] + ph.smallnum, t2 = tt * tt;
@@ -1406,36 +1631,19 @@ __global__ void __launch_bounds__(32 * (kE ? 3 : 8) / CPT) k_p2(Dims d, PhysC ph
 #pragma unroll
       for (int st = 0; st < 9; ++st) W[c][st] = W[c][st] * wn;
     }
-    double acc[CPT][NO];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c)
-#pragma unroll
-      for (int m = 0; m < NO; ++m) acc[c][m] = 0.0;
+    double acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
     for (int st = 0; st < 8; ++st) {
-      stencil(st, 0, kE ? 1 : NG, [&](int gi, R (*X)[3]) {
+      stencil(st, 0, 1, [&](int, R (*X)[3]) {
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          const double ws = W[c][st];
-#pragma unroll
-          for (int q = 0; q < (kE ? 1 : 3); ++q) {
-            const int m = kE ? 0 : 3 * gi + q;
-            acc[c][m] = st == 0 ? ws * (double)X[c][q] : acc[c][m] + ws * (double)X[c][q];
-          }
-        }
+        for (int c = 0; c < 3; ++c) acc[c] = acc[c] + W[c][st] * (double)X[c][0];
       });
     }
     const R fl = s.flatA[d.at(0, p, i, j, k)], x = R(1.0) - fl;
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-#pragma unroll
-      for (int m = 0; m < NO; ++m) acc[c][m] = acc[c][m] + W[c][8] * (double)X8[c][m];
-      if (kE) {
-        s.E[d.at(q0 + c, p, i, j, k)] = fl * f0[c] + x * (R)acc[c][0];
-      } else {
-#pragma unroll
-        for (int m = 0; m < NO; ++m) Vat(s, d, q0 + c, 1 + m, p, i, j, k) = (R)acc[c][m] * x;
-      }
+    for (int c = 0; c < 3; ++c) {
+      acc[c] = acc[c] + W[c][8] * (double)X8[c][0];
+      s.E[d.at(c, p, i, j, k)] = fl * f0[c] + x * (R)acc[c];
     }
   }
 }
@@ -1582,15 +1790,16 @@ void launch_flattener(Solve& sv) {
     launch_flattener_t(sv, sv.st);
 }
 
-// Primitives a thread of STEP 7.a's k_p2 takes (each operator word loaded
-// once for all of them; 1 / 2 / 4 measured 233 / 153 / 113 ms per shell128
-// step).  STEP 9.b's takes the three E components.
-constexpr int P2_CPT = 4;
-// Grid of k_p2 over range b: 32-zone tiles (panel-interleaved when shared).
-inline int p2_blocks(Solve& sv, const Range3& b, bool shared) {
-  const long long npp = b.count() / 6;
-  const long long nt = shared ? 6 * ((npp + 31) / 32) : (b.count() + 31) / 32;
-  return (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
+// 32-zone tiles of range b, panel-interleaved when the inverses are shared.
+inline long long p2_tiles(const Range3& b, bool shared) {
+  return shared ? 6 * ((b.count() / 6 + 31) / 32) : (b.count() + 31) / 32;
+}
+
+void set_p2_smem_limits() {
+  cudaFuncSetAttribute(k_p2_prim<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P2Smem<double>));
+  cudaFuncSetAttribute(k_p2_prim<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P2Smem<double>));
+  cudaFuncSetAttribute(k_p2_prim<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P2Smem<float>));
+  cudaFuncSetAttribute(k_p2_prim<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P2Smem<float>));
 }
 
 template <typename R>
@@ -1602,10 +1811,11 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
     const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
     k_weno_slopes<W7_ENT, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
     mark(sv, "k_p2_entropy");
+    const int np = (int)std::min<long long>(p2_tiles(b, st.p2_map), (long long)grid_sms(sv) * p2_blocks(sizeof(R)));
     if (st.p2_map)
-      k_p2<false, true, P2_CPT, R><<<p2_blocks(sv, b, true), 256 / P2_CPT, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_p2_prim<true, R><<<np, P2_THREADS, sizeof(P2Smem<R>), sv.stream>>>(d, sv.ph, sv.g, st, b);
     else
-      k_p2<false, false, P2_CPT, R><<<p2_blocks(sv, b, false), 256 / P2_CPT, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_p2_prim<false, R><<<np, P2_THREADS, sizeof(P2Smem<R>), sv.stream>>>(d, sv.ph, sv.g, st, b);
     mark(sv, "k_p2_prim");
     return;
   }
@@ -1713,10 +1923,11 @@ void launch_efield_t(Solve& sv, DStateT<R>& st) {
   k_efield_a<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, z);
   mark(sv, "k_efield_a");
   if (sv.p.flags & CS_FLAG_P2) {  // LIMIT_ALL_SLOPES_P2's STEP 9.b
+    const int nb = (int)std::min<long long>(p2_tiles(b, st.p2_map), (long long)grid_sms(sv) * 16);
     if (st.p2_map)
-      k_p2<true, true, 3, R><<<p2_blocks(sv, b, true), 32, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_p2_efield<true, R><<<nb, 32, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
     else
-      k_p2<true, false, 3, R><<<p2_blocks(sv, b, false), 32, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
+      k_p2_efield<false, R><<<nb, 32, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
     mark(sv, "k_p2_efield");
     return;
   }
