@@ -49,13 +49,12 @@ ALGO_WORDS_PER_UNIT = {
     # resident KKT factors (1296) + pivots (36 bytes) + the 36 right-hand
     # sides in, 30 B modes and U(5:8) out (U read and written: 8)
     "k_adp_solve": 1296 + 4.5 + 36 + 30 + 8,
-    # the same with the factors shared by the six panels (1/6 per zone)
-    "k_adp_solve6": (1296 + 4.5) / 6 + 36 + 30 + 8,
     # face-B quadrature values (30), B modes (30), geometry of the 6 faces
     # (normals 42, points 90, weights 30) and of the zone (14), 36 out
     "k_adp_rhs": 30 + 30 + 162 + 14 + 36,
-    # the same with panel 1's geometry serving the six panels (1/6 per zone)
-    "k_adp_rhs6": 30 + 30 + (162 + 14) / 6 + 36,
+    # both in one kernel where the panels share panel 1's geometry and packed
+    # inverse (645 words; 1/6 per zone each)
+    "k_adp6": 30 + 30 + (162 + 14 + 645) / 6 + 30 + 8,
     # one launch per stage, the three face directions (units = zones): the
     # zone's 80 modes, 4 entropy modes, 10 moments, centroid and scale in;
     # per direction the face geometry (15 points, 5 weights, normals /

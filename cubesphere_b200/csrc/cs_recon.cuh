@@ -126,6 +126,9 @@ __device__ __forceinline__ void mrweno_hybrid(const R* X, const R* lin, const R*
   for (int a = 3; a < 9; ++a) out[a] = (Whi * Phi[a]) * x;
 }
 
+// The line of p to L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // STEP 7.b's resident row weights of n zones: blocks of 32 zones [162][32],
 // the last one [162][m9_stride(n) - 32 (blocks - 1)], so that a block is one
 // contiguous run for the bulk copies.
