@@ -763,7 +763,7 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
     // room left after them as for the ADP factors below
     if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && bytes + (size_t)8 * S6 + ((size_t)2 << 30) < fr) {
       m.op_m9 = mdalloc(sv, m, (size_t)m9_stride(n9) * 162 * sizeof(R), e);
-      m.op_m10 = m.op_m9 ? mdalloc(sv, m, (size_t)n10 * 190 * sizeof(R), e) : nullptr;
+      m.op_m10 = m.op_m9 ? mdalloc(sv, m, (size_t)n10 * 190 * sizeof(R) + 16, e) : nullptr;  // copies are whole 16 bytes
       if (!m.op_m9 || !m.op_m10) return cuda_fail(sv, e, "cudaMalloc(least-squares operators)");
       if (shared) {
         m.lsq_map = mdalloc(sv, m, sizeof qmap, e);

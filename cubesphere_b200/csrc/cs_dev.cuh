@@ -447,6 +447,8 @@ void launch_flattener(Solve& s);
 void launch_weno(Solve& s);
 // STEP 7.b on zones r from the resident row weights.
 void launch_weno7b(Solve& s, const Range3& r);
+// STEP 9.c on zones r from the resident row weights, stored over zones rs.
+void launch_efield_c(Solve& s, const Range3& r, const Range3& rs);
 void launch_positivity(Solve& s);
 void launch_faceB_adp(Solve& s);
 void launch_adp(Solve& s);

@@ -432,36 +432,6 @@ __device__ __forceinline__ void w7b_minv(const Dims& d, const PhysC& ph, const D
   d_matinv<9>(M, Minv);
 }
 
-// Zones of a least-squares range in the order a stage visits them.  With
-// the row weights shared by the panels (kShared), iteration it covers tile
-// it / 6 of panel it % 6, so the six blocks that read one tile's weights run
-// side by side and five of them find the weights in L2; otherwise the plain
-// grid-stride order.  t indexes the range, tw the stored weights (panel 1's
-// zone when shared); nw is their stride.
-template <bool kShared>
-struct LsqOrder {
-  long long nr, npp, nw, nit;
-  __device__ explicit LsqOrder(const Range3& r) {
-    nr = r.count();
-    npp = nr / 6;
-    nw = kShared ? npp : nr;
-    nit = kShared ? 6 * ((npp + blockDim.x - 1) / blockDim.x) : nr;
-  }
-  __device__ long long begin() const {
-    return kShared ? (long long)blockIdx.x : blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  }
-  __device__ long long stride() const { return kShared ? (long long)gridDim.x : (long long)gridDim.x * blockDim.x; }
-  __device__ bool zone(long long it, long long& t, long long& tw) const {
-    if (!kShared) {
-      t = tw = it;
-      return true;
-    }
-    tw = (it / 6) * blockDim.x + threadIdx.x;
-    t = (it % 6) * npp + tw;
-    return tw < npp;
-  }
-};
-
 // STEP 7.b (421:3869-4551) without resident row weights
 // (CS_FLAG_NO_OP_CACHE): 18-zone quadratic least squares hybridised with the
 // linear WENO slopes (MRWENO weights, flattener damping), the rows rebuilt
@@ -554,7 +524,7 @@ __global__ void k_ops_m9(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
       for (int a = 0; a < 9; ++a) {
         double w = 0.0;
         for (int b = 0; b < 9; ++b) w = w + Minv[a * 9 + b] * A[b];
-        s.op_m9[m9_at(t, rr * 9 + a, nr_)] = (R)w;
+        s.op_m9[w_at<162>(t, rr * 9 + a, nr_)] = (R)w;
       }
     }
   }
@@ -974,18 +944,14 @@ __device__ __forceinline__ void e9c_minv(const Dims& d, const DGeom& g, int p, i
   d_matinv<10>(M, Minv);
 }
 
-// STEP 9.c (421:8464-9350): 19-point interpolation least squares
-// hybridised with the slopes; the point value is flattened toward E_pt.
-// Only the point value (mode 1) is stored: the LLF edge solver consumes
-// nothing else.  kCached: the inverse normal matrix comes from the
-// operator cache.  Blocks per SM: 4 for FP64, 6 for FP32 (measured).
-template <bool kCached, bool kShared, typename R>
-__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, Range3 rs) {
-  const R ob12 = R(1.0) / R(12.0), ob180 = R(1.0) / R(180.0), ob144 = R(1.0) / R(144.0);
-  const LsqOrder<kShared> ord(r);
-  for (long long it = ord.begin(); it < ord.nit; it += ord.stride()) {
-    long long t, tw;
-    if (!ord.zone(it, t, tw)) continue;
+// STEP 9.c (421:8464-9350) without resident row weights
+// (CS_FLAG_NO_OP_CACHE): 19-point interpolation least squares hybridised with
+// the slopes, the rows rebuilt and the normal matrix inverted in every stage;
+// the point value is flattened toward E_pt.  Only the point value (mode 1) is
+// stored: the LLF edge solver consumes nothing else.
+template <typename R>
+__global__ void __launch_bounds__(TPB) k_efield_c_rebuild(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
     if (mask_at(g, d, p, i, j) != 1) continue;
@@ -995,11 +961,9 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
     coef10(g, d, p, i, j, k, c0);
     const R cx = geoR<R>(g, d, CS_G_V_CEN, 0, p, i, j, k), cy = geoR<R>(g, d, CS_G_V_CEN, 1, p, i, j, k),
                  cz = geoR<R>(g, d, CS_G_V_CEN, 2, p, i, j, k);
-    // kCached: the solution operator comes from the cache as the row weights
-    // W_rr = Minv A_rr^T (geometry only), so X = sum_rr W_rr E_rr directly.
-    R Minv[kCached ? 1 : 100];
-    if (!kCached) {
-      // formed in FP64 in every form, like the cached row weights
+    // formed in FP64 in every form, like the resident row weights
+    R Minv[100];
+    {
       double c0d[10], Md[100];
       coef10(g, d, p, i, j, k, c0d);
       e9c_minv<double>(d, g, p, i, j, k, n, geo(g, d, CS_G_V_CEN, 0, p, i, j, k), geo(g, d, CS_G_V_CEN, 1, p, i, j, k),
@@ -1008,11 +972,6 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
 #pragma unroll
       for (int e = 0; e < 100; ++e) Minv[e] = (R)Md[e];
     }
-    // the zone's place in the weights' range rs
-    const long long nsp = rs.count() / 6, nw = kShared ? nsp : 6 * nsp;
-    const long long ts = ((long long)(k - rs.k0) * (rs.j1 - rs.j0 + 1) + (j - rs.j0)) * (rs.i1 - rs.i0 + 1) + (i - rs.i0);
-    const R* wc = s.op_m10 + (kShared ? ts : ts + p * nsp);
-    auto MI = [&](int e) { return Minv[kCached ? 0 : e]; };
     R Y[3][10];
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -1022,18 +981,7 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
     for (int rr = 0; rr < 19; ++rr) {
       R A[10];
       long long off;
-      if (kCached) {
-        if (rr == 0) {
-          off = d.idx(i, j, k);
-        } else {
-          const int w = c_n18[rr - 1][0];
-          off = d.idx(w < 0 ? i : n.x[w], w < 0 ? j : n.y[w], k + c_n18[rr - 1][1]);
-        }
-#pragma unroll
-        for (int a = 0; a < 10; ++a) A[a] = __ldg(wc + (long long)(rr * 10 + a) * nw);
-      } else {
-        e9c_row(d, g, p, i, j, k, n, rr, cx, cy, cz, obl0, c0, A, off);
-      }
+      e9c_row(d, g, p, i, j, k, n, rr, cx, cy, cz, obl0, c0, A, off);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const R Rv = s.Esnap[((long long)q * NPANEL + p) * d.S + off];
@@ -1042,46 +990,23 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_efield_c(Dims d
       }
     }
     const R f = s.flatA[d.at(0, p, i, j, k)];
-    const R betalo = f + (R(1.0) - f) * R(2.0);
     const R ghi = f * R(0.6) + (R(1.0) - f) * R(0.95), glo = R(1.0) - ghi, obghi = R(1.0) / ghi, grat = glo / ghi;
-    const unsigned long long qsrc = kShared ? s.lsq_map10[p].src : LSQ_IDENTITY_SRC;
-    const unsigned int qneg = kShared ? s.lsq_map10[p].neg : 0u;
 #pragma unroll 1
     for (int q = 0; q < 3; ++q) {
       R X[10];
 #pragma unroll
       for (int a = 0; a < 10; ++a) {
-        if (kCached) {
-          X[a] = kShared ? lsq_rotated<0>(Y[q], a, qsrc, qneg) : Y[q][a];
-        } else {
-          R acc = R(0.0);
+        R acc = R(0.0);
 #pragma unroll
-          for (int b = 0; b < 10; ++b) acc = acc + MI(a * 10 + b) * Y[q][b];
-          X[a] = acc;
-        }
+        for (int b = 0; b < 10; ++b) acc = acc + Minv[a * 10 + b] * Y[q][b];
+        X[a] = acc;
       }
-      R e[4];
-      e[0] = s.Esnap[((long long)q * NPANEL + p) * d.S + d.idx(i, j, k)];
-#pragma unroll
-      for (int m = 1; m < 4; ++m) e[m] = s.E[d.at(m * 3 + q, p, i, j, k)];
-      const R ISlo = betalo * (e[1] * e[1] + e[2] * e[2] + e[3] * e[3]) * ob12;
-      R Phi[10];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) Phi[m] = X[m] * obghi - e[m] * grat;
-#pragma unroll
-      for (int m = 4; m < 10; ++m) Phi[m] = X[m] * obghi;
-      const R IShi = (Phi[1] * Phi[1] + Phi[2] * Phi[2] + Phi[3] * Phi[3]) * ob12 +
-                          (Phi[4] * Phi[4]) * (sqr(c0[4] - ob12) + ob180) + (Phi[5] * Phi[5]) * (sqr(c0[5] - ob12) + ob180) +
-                          (Phi[6] * Phi[6]) * (sqr(c0[6] - ob12) + ob180) + (Phi[7] * Phi[7]) * (c0[7] * c0[7] + ob144) +
-                          (Phi[8] * Phi[8]) * (c0[8] * c0[8] + ob144) + (Phi[9] * Phi[9]) * (c0[9] * c0[9] + ob144);
-      const R tau = fabs(IShi - ISlo);
-      R Wlo = glo * (R(1.0) + tau / (ISlo + R(ph.smallnum))), Whi = ghi * (R(1.0) + tau / (IShi + R(ph.smallnum)));
-      const R aa = R(1.0) / (Wlo + Whi);
-      Wlo = Wlo * aa;
-      Whi = Whi * aa;
-      const R x = R(1.0) - f;
-      const R e0 = Whi * Phi[0] + Wlo * e[0];
-      s.E[d.at(q, p, i, j, k)] = e[0] * f + e0 * x;
+      const R e0 = s.Esnap[((long long)q * NPANEL + p) * d.S + d.idx(i, j, k)];
+      const R e[3] = {s.E[d.at(3 + q, p, i, j, k)], s.E[d.at(6 + q, p, i, j, k)], s.E[d.at(9 + q, p, i, j, k)]};
+      R Wlo, Whi, Phi[9];
+      mrweno_weights(X + 1, e, c0, f, ghi, glo, obghi, grat, R(ph.smallnum), Phi, Wlo, Whi);
+      const R eh = Whi * (X[0] * obghi - e0 * grat) + Wlo * e0;
+      s.E[d.at(q, p, i, j, k)] = e0 * f + eh * (R(1.0) - f);
     }
   }
 }
@@ -1109,7 +1034,7 @@ __global__ void k_ops_m10(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
       for (int a = 0; a < 10; ++a) {
         double w = 0.0;
         for (int b = 0; b < 10; ++b) w = w + Minv[a * 10 + b] * A[b];
-        s.op_m10[(long long)(rr * 10 + a) * nr_ + t] = (R)w;
+        s.op_m10[w_at<190>(t, rr * 10 + a, nr_)] = (R)w;
       }
     }
   }
@@ -1407,7 +1332,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
       R Y[2][9];
       const LsqPanelMap* cmap = s.lsq_map9;
       const long long tc = cmap ? t - (long long)p * npp : t, ncw = cmap ? npp : nz;
-      const M9Block cb = m9_block(tc / 32, ncw);
+      const WBlock cb = w_block<162>(tc / 32, ncw);
       const R* wc = s.op_m9 + cb.off + tc % 32;
       const long long cstride = cb.wid;
 #pragma unroll
@@ -1573,7 +1498,8 @@ __global__ void __launch_bounds__(32) k_p2_efield(Dims d, PhysC ph, DGeom g, DSt
         for (int m = 0; m < NM; ++m) Y[c][m] = R(0.0);
       const LsqPanelMap* cmap = s.lsq_map10;
       const long long tc = cmap ? t - (long long)p * npp : t, ncw = cmap ? npp : nz;
-      const R* wc = s.op_m10 + tc;
+      const WBlock cb = w_block<190>(tc / 32, ncw);
+      const R* wc = s.op_m10 + cb.off + tc % 32;
 #pragma unroll
       for (int rr = 0; rr < NR + 9; ++rr) {
         const int ro = rr - 1;  // the zone itself first
@@ -1586,7 +1512,7 @@ __global__ void __launch_bounds__(32) k_p2_efield(Dims d, PhysC ph, DGeom g, DSt
         }
 #pragma unroll
         for (int m = 0; m < NM; ++m) {
-          const R wv = __ldg(wc + (long long)(rr * NM + m) * ncw);
+          const R wv = __ldg(wc + (rr * NM + m) * cb.wid);
 #pragma unroll
           for (int c = 0; c < 3; ++c) Y[c][m] = Y[c][m] + wv * Rv[c];
         }
@@ -1937,13 +1863,11 @@ void launch_efield_t(Solve& sv, DStateT<R>& st) {
     k_weno_slopes<W7_E, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_efield_b");
   }
-  if (st.op_m10)
-    if (st.lsq_map10)
-      k_efield_c<true, true, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
-    else
-      k_efield_c<true, false, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
-  else
-    k_efield_c<false, false, R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a, b);
+  if (st.op_m10) {
+    launch_efield_c(sv, a, b);
+    return;
+  }
+  k_efield_c_rebuild<R><<<blocks_for(a.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
   mark(sv, "k_efield_c");
 }
 

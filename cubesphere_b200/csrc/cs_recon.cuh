@@ -129,19 +129,22 @@ __device__ __forceinline__ void mrweno_hybrid(const R* X, const R* lin, const R*
 // The line of p to L2.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// STEP 7.b's resident row weights of n zones: blocks of 32 zones [162][32],
-// the last one [162][m9_stride(n) - 32 (blocks - 1)], so that a block is one
-// contiguous run for the bulk copies.
-struct M9Block {
+// The resident row weights of n zones, W words a zone (STEP 7.b's 162, STEP
+// 9.c's 190): blocks of 32 zones [W][32], the last one [W][what is left], so
+// that a block is one contiguous run for the bulk copies.  STEP 7.b's zones
+// are rounded up to 4 and STEP 9.c's copies are of whole 16 bytes.
+struct WBlock {
   long long off;  // of the block's first word
   int wid;        // zones in a row
 };
-__device__ __forceinline__ M9Block m9_block(long long blk, long long n) {
-  return {blk * 162 * 32, (int)min(32LL, m9_stride(n) - blk * 32)};
+template <int W>
+__device__ __forceinline__ WBlock w_block(long long blk, long long n) {
+  return {blk * W * 32, (int)min(32LL, (W == 162 ? m9_stride(n) : n) - blk * 32)};
 }
 // Word e of zone t.
-__device__ __forceinline__ long long m9_at(long long t, int e, long long n) {
-  const M9Block b = m9_block(t / 32, n);
+template <int W>
+__device__ __forceinline__ long long w_at(long long t, int e, long long n) {
+  const WBlock b = w_block<W>(t / 32, n);
   return b.off + (long long)e * b.wid + t % 32;
 }
 
