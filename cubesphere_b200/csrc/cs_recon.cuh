@@ -150,11 +150,8 @@ __device__ __forceinline__ long long w_at(long long t, int e, long long n) {
 
 // The interior zones and w layers around them.
 inline Range3 around(const Dims& d, int w) { return {1 - w, d.N + w, 1 - w, d.N + w, 1 - w, d.nr + w}; }
-// Layers around the interior on which STEP 8.d solves the B modes.  The stage
-// reads E in one layer (the edge EMFs); P12's STEPS 9.b / 9.c run on it and
-// read point values of E, made of the ADP modes, one layer further, P2's
-// stencils, run on one layer more where there are four, two.  The layers beyond hold primitives and slopes for those only.
-inline int adp_layers(const Solve& sv) { return (sv.p.flags & CS_FLAG_P2) ? sv.p.nghost - 1 : 2; }
+// Layers around the interior on which STEP 8.d solves the B modes.
+inline int adp_layers(const Solve& sv) { return sv.adp_w; }
 inline Range3 zones_all(const Dims& d) { return {1 - d.G, d.N + d.G, 1 - d.G, d.N + d.G, 1 - d.G, d.nr + d.G}; }
 inline Range3 shrink(const Dims& d, int s) {
   return {1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.nr + d.G - s};

@@ -67,6 +67,7 @@ struct MeshRes {
   void* op_p2v = nullptr;  // CS_FLAG_P2 one-sided stencil inverses (state's type)
   void* op_p2e = nullptr;
   bool p2_shared = false;  // op_p2v / op_p2e are panel 1's only
+  int adp_w = 0;            // layers around the interior the ADP operators cover
   void* adp_lu = nullptr;   // per-panel factors (FP64) or the panel-shared inverse (state's type)
   int8_t* adp_piv = nullptr;
   int8_t* adp_pmap = nullptr;  // ADP factors shared by the panels: per panel [unknown map][sign]
@@ -107,6 +108,7 @@ struct Solve {
   cudaGraph_t graph = nullptr;           // one step, captured by cs_steps / cs_batch_steps
   cudaGraphExec_t graph_exec = nullptr;  // its executable form
   long long graph_kernels = 0;           // kernels in that graph
+  int adp_w = 0;                         // layers around the interior STEP 8.d solves
   double grid_frac = 1.0;                // share of the SMs a launch's grid is sized for (autotuned in batches)
   Prof prof;
   std::string err;
@@ -130,6 +132,18 @@ int cuda_fail(Solve& sv, cudaError_t e, const char* what);
 void* solve_alloc(Solve& sv, size_t bytes, cudaError_t& e);
 // The seeded initial state built on the device (cs_init_problem).
 int init_problem_device(Solve& sv, const cs_init_desc& desc);
+// Whether the fill that starts a stage gives every ghost its value.  With a
+// radial boundary code other than outflow the radial ghosts are the caller's,
+// and what a stage does to them reaches the next one.
+inline bool ghosts_filled(const cs_params& p) { return p.bc_lower == 2 && p.bc_upper == 2; }
+// Layers around the interior that STEP 8.d has to solve.  The stage reads E in
+// one layer (the edge EMFs); P12's STEPS 9.b / 9.c run on it and read point
+// values of E, made of the ADP modes, one layer further, P2's stencils, run on
+// one layer more where there are four, two.  The layers beyond hold primitives
+// and slopes for those only, but a caller's ghosts take their zone B too.
+inline int adp_layers_needed(const cs_params& p) {
+  return (p.flags & CS_FLAG_P2) || !ghosts_filled(p) ? p.nghost - 1 : 2;
+}
 // Identity of the mesh a parameter set needs (solves with equal keys can
 // share one MeshRes).
 std::string mesh_key(const cs_params& p);

@@ -89,3 +89,41 @@ def test_fp64_batches_give_each_members_own_result():
             for k in want:
                 assert np.array_equal(got[k], want[k]), (rep, n, k)
     b.close()
+
+
+@pytest.mark.parametrize("lower,upper", [(0, 0), (2, 0), (0, 2)])
+@pytest.mark.parametrize("rk", [cs.CS_RK2, cs.CS_SSPRK3, cs.CS_IMEX_RK2])
+def test_ghosts_of_the_callers_match_the_oracle(lower, upper, rk):
+    """A radial boundary code other than outflow leaves the radial ghosts to the
+    caller: the stages carry them along, and the next stage reads them."""
+    from oracle import Oracle
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=10, nr=5, rk_scheme=rk, bc_lower=lower, bc_upper=upper)
+    s = cs.Solve(**pr["params"])
+    s.mesh_build()
+    s.init_problem(**pr["init"])
+    o = Oracle(s)
+    o.put_state(s.get_state())
+    dt, dto = s.evaluate_timestep(1e30), o.evaluate_timestep(1e30)
+    for _ in range(3):
+        dt, dto = s.steps(1, dt), o.step(dto)
+        assert abs(dt - dto) <= 1e-12 * dto
+        check_state(s, s.get_state(), o.get_state())
+
+
+def test_a_shared_mesh_serves_solves_of_other_boundary_codes():
+    """Solves that share a mesh may differ in their boundary codes; each gives
+    what it gives on its own mesh (up to the ADP operators' rounding, 1e-12)."""
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=10, nr=5)
+    for first, second in (((2, 2), (0, 0)), ((0, 0), (2, 2))):
+        a = cs.Solve(**{**pr["params"], "bc_lower": first[0], "bc_upper": first[1]})
+        a.mesh_build()
+        out = []
+        for share in (False, True):
+            s = cs.Solve(**{**pr["params"], "bc_lower": second[0], "bc_upper": second[1]})
+            s.mesh_share(a) if share else s.mesh_build()
+            s.init_problem(**pr["init"])
+            s.steps(2, s.evaluate_timestep(1e30))
+            out.append(s.get_state())
+        check_state(s, out[1], out[0])
