@@ -379,7 +379,7 @@ __global__ void k_gather(Dims d, DGeom g, DStateT<R> s, Range3 r) {
   }
 }
 
-// Point-mass gravity on zones 0..N+1 (470:147-244).
+// Point-mass gravity (470:147-244).
 template <typename R>
 __global__ void k_sources(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
@@ -407,9 +407,12 @@ template <typename R>
 void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
   const int N = d.N, nr = d.nr;
-  Range3 fx = {-1, N + 1, 0, N + 1, 0, nr + 1};
-  Range3 fy = {0, N + 1, -1, N + 1, 0, nr + 1};
-  Range3 fz = {0, N + 1, 0, N + 1, -1, nr + 1};
+  // the faces of the zones to gather, and the layer across the interior's whose
+  // speeds and fluxes its edges read
+  const Range3 z = stage_zones(sv, 1);
+  Range3 fx = {z.i0 - 1, z.i1, 0, N + 1, 0, nr + 1};
+  Range3 fy = {0, N + 1, z.j0 - 1, z.j1, 0, nr + 1};
+  Range3 fz = {0, N + 1, 0, N + 1, z.k0 - 1, z.k1};
   {
     const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + FLUX_FACES - 1) / FLUX_FACES);
     const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 32);
@@ -423,7 +426,6 @@ void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
     k_sync_flux<R><<<blocks_for(17 * sv.psync.nf, 128, grid_sms(sv)), 128, 0, sv.stream>>>(d, st, sv.psync);
     mark(sv, "k_sync_flux");
   }
-  Range3 z = {0, N + 1, 0, N + 1, 0, nr + 1};
   k_gather<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, z);
   mark(sv, "k_gather");
 }
@@ -439,7 +441,7 @@ template <typename R>
 void launch_sources_t(Solve& sv, DStateT<R>& st) {
   if (!(sv.ph.gm > sv.p.smallnum)) return;
   const Dims& d = sv.d;
-  Range3 z = {0, d.N + 1, 0, d.N + 1, 0, d.nr + 1};
+  const Range3 z = stage_zones(sv, 1);
   k_sources<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z);
   mark(sv, "k_sources");
 }

@@ -169,6 +169,14 @@ inline int blocks_for(long long n, int threads, int sm_count) {
   return (int)b;
 }
 
+// The zones whose state a stage moves: w layers around the interior where the
+// ghosts are the caller's (w < 0: all of them).
+inline Range3 stage_zones(const Solve& sv, int w) {
+  const Dims& d = sv.d;
+  const int l = ghosts_filled(sv.p) ? 0 : (w < 0 ? d.G : w);
+  return {1 - l, d.N + l, 1 - l, d.N + l, 1 - l, d.nr + l};
+}
+
 }  // namespace cs
 
 // The opaque context of the C ABI: one resident solve.

@@ -143,7 +143,7 @@ __device__ __forceinline__ void up_entropy(const Dims& d, const PhysC& ph, const
   d_cons_to_prim(ph, en, U, V);
 }
 
-// Zone update (484:212-372): U += dt dU/dt on every zone, then on the
+// Zone update (484:212-372): U += dt dU/dt on the zones r, then on the
 // interior the entropy update and the conserved->primitive repair, with the
 // stage's combine and the IMEX gravity in the same pass.  The time step is
 // scale times the device-resident step of the solve.
@@ -238,8 +238,8 @@ __device__ __forceinline__ double vang(const DGeom& g, const Dims& d, int p, int
 // Constrained-transport face update (484:376-906): Stokes circulation of
 // the edge EMFs with spherical arc lengths for the angular edges, with the
 // stage's save, combine or restore of face B in the same pass.  One launch
-// for the three face directions over every face of the box; only the
-// interior zones' faces have a circulation.
+// for the three face directions over the faces r; only the interior zones'
+// faces have a circulation.
 template <int M, typename R>
 __global__ void __launch_bounds__(TPB) k_ct(Dims d, DGeom g, DStateT<R> s, Range3 r, UpArgs a) {
   const double dt = a.scale * *s.dt, dt0 = a.scale0 * *s.dt;
@@ -466,11 +466,11 @@ void launch_fill_ghosts(Solve& sv) {
 template <int M, typename R>
 void launch_update_mode(Solve& sv, const DStateT<R>& st, const UpArgs& a) {
   const Dims& d = sv.d;
-  const Range3 z = zones_all(d);
+  const Range3 z = stage_zones(sv, -1);
   k_update_zones<M, R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z, a);
   mark(sv, "k_update_zones");
   // UP_PLAIN touches the interior zones' faces only
-  const Range3 f = M == UP_PLAIN ? Range3{0, d.N, 0, d.N, 0, d.nr} : Range3{-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G};
+  const Range3 f = M == UP_PLAIN || ghosts_filled(sv.p) ? Range3{0, d.N, 0, d.N, 0, d.nr} : Range3{-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G};
   const long long nb = 3 * ((f.count() + TPB - 1) / TPB);
   k_ct<M, R><<<(int)std::min<long long>(nb, (long long)grid_sms(sv) * 64), TPB, 0, sv.stream>>>(d, sv.g, st, f, a);
   mark(sv, "k_ct");
@@ -505,17 +505,17 @@ void launch_update_imex(Solve& sv, int irk, double gam, double del) {
 }
 
 template <typename R>
-void launch_cleanup_t(Solve& sv, const DStateT<R>& st) {
-  Range3 z = zones_all(sv.d);
+void launch_cleanup_t(Solve& sv, const DStateT<R>& st, const Range3& z) {
   k_cleanup_zones<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, z);
   mark(sv, "k_cleanup_zones");
 }
 void launch_cleanup(Solve& sv, bool masks) {
   if (masks) launch_face_masks(sv);
+  const Range3 z = masks ? zones_all(sv.d) : stage_zones(sv, -1);
   if (sv.fp32)
-    launch_cleanup_t(sv, sv.stF);
+    launch_cleanup_t(sv, sv.stF, z);
   else
-    launch_cleanup_t(sv, sv.st);
+    launch_cleanup_t(sv, sv.st, z);
 }
 
 template <typename R>
