@@ -127,3 +127,24 @@ def test_a_shared_mesh_serves_solves_of_other_boundary_codes():
             s.steps(2, s.evaluate_timestep(1e30))
             out.append(s.get_state())
         check_state(s, out[1], out[0])
+
+
+def test_reciprocals_by_newton_steps_are_within_two_units():
+    """The stage kernels form 1 / rho by Newton steps.  Two gases at rest without
+    field, rho over 22 decades: the fast speed is sqrt(gamma p / rho), where two
+    units of the reciprocal, the two products' roundings and the two roots' add
+    up to less than 4 units (eps each) of the speed."""
+    rng = np.random.default_rng(7)
+    rho = 10.0 ** rng.uniform(-11.0, 11.0, 4096)
+    prs = rng.uniform(0.5, 2.0, rho.size)
+    c = np.zeros((rho.size, 18))
+    for side in (0, 8):
+        c[:, side] = rho
+        c[:, side + 4] = prs
+    c[:, 16:] = 1.0
+    gamma = 5.0 / 3.0
+    out = cs.pointwise(2, c, gamma=gamma)
+    want = np.sqrt(np.longdouble(gamma) * prs.astype(np.longdouble) / rho.astype(np.longdouble))
+    for sign, got in ((-1.0, out[:, 32]), (1.0, out[:, 33])):
+        err = np.abs(sign * got - want) / want
+        assert err.max() <= 4 * np.finfo(float).eps, float(err.max())
