@@ -498,6 +498,8 @@ constexpr int ADP6_CONS = 6 * 32;
 constexpr int ADP6_THREADS = ADP6_CONS + 32;
 constexpr int ADP6_CH = 2 * ADP6_UNIT;  // words a ring stage
 constexpr int ADP6_NS = 4;
+constexpr int ADP6_FB = 4;           // faces held by the copies ahead
+constexpr int ADP6_FROWS = 15 + 30;  // rows of a face
 constexpr int ADP6_NCH = (ADP6_WORDS + ADP6_CH - 1) / ADP6_CH;  // the last one holds one unit
 template <typename F>
 struct Adp6SmemT {
@@ -507,6 +509,13 @@ struct Adp6SmemT {
   // the panels' new zone B [panel][component]: in the second half of bas, which
   // the next block's faces reach after a barrier
   __device__ __forceinline__ F* nb(int p, int c) { return &bas[1][0][0][0] + (p * 3 + c) * ADP6_ZB; }
+  // copies ahead: a face's points (rows 0-14) and its B at them (row 15 + 5
+  // panel + point), in the rows of x that hold right-hand sides later
+  __device__ __forceinline__ double (*face(int f))[ADP6_ZB] {
+    static_assert(sizeof(F) == 4 || ADP6_FB * ADP6_FROWS * sizeof(double) <= 30 * 6 * sizeof(F), "face rows in x");
+    return reinterpret_cast<double(*)[ADP6_ZB]>(&x[0][0][0]) + f % ADP6_FB * ADP6_FROWS;
+  }
+  F geo[sizeof(F) == 8 ? 10 : 1][ADP6_ZB];  // copies ahead: the position's centroid, 1 / scale and moments
   uint64_t full[ADP6_NS];
   uint64_t empty[ADP6_NS];
 };
@@ -624,8 +633,147 @@ __device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, Rin
 // Barrier of the six consumer warps (the producer is not part of it).
 __device__ __forceinline__ void adp6_sync() { asm volatile("bar.sync 1, %0;" ::"n"(ADP6_CONS) : "memory"); }
 
+// Copy of one word a lane to shared memory, in the background.
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// Box offset of face f of position zo.
+__device__ __forceinline__ unsigned adp6_face(const Dims& d, int f, unsigned zo) {
+  const int dir = f >> 1;
+  return zo - ((f & 1) ? (dir == 0 ? 1 : (dir == 1 ? d.NI : d.NI * d.NJ)) : 0);
+}
+
+// Start the copies of face f: warp w the point w (the rows it reads itself
+// before the barrier) and panel w.  A group of copies a face.
+template <typename R>
+__device__ __forceinline__ void adp6_fetch(Adp6SmemT<R>& S, const Dims& d, const DGeom& g, const DStateT<R>& s, int f, unsigned zo,
+                                           int lane, int w) {
+  const long long PS = (long long)NPANEL * d.S;
+  const int dir = f >> 1;
+  const unsigned fo = adp6_face(d, f, zo);
+  double(*fr)[ADP6_ZB] = S.face(f);
+  if (w < 5) {
+    const double* qp = (dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP])) + fo + w * PS;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) copy8(&fr[5 * c + w][lane], qp + 5 * c * PS);
+  }
+  const double* Bq = (dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2])) + w * d.S + fo;
+#pragma unroll
+  for (int c = 0; c < 5; ++c) copy8(&fr[15 + 5 * w + c][lane], Bq + c * PS);
+}
+template <typename R>
+__device__ __forceinline__ void adp6_fetch_first(Adp6SmemT<R>& S, const Dims& d, const DGeom& g, const DStateT<R>& s, unsigned zo,
+                                                 int lane, int w) {
+#pragma unroll 1
+  for (int f = 0; f < ADP6_FB - 1; ++f) {
+    adp6_fetch(S, d, g, s, f, zo, lane, w);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+}
+
+// The right-hand sides (see k_adp6) from copies that run three faces ahead; the
+// first three are on their way.  Leaves x free.
+template <typename R>
+__device__ __forceinline__ void adp6_rhs_ahead(R (&acc)[3][10], Adp6SmemT<R>& S, const Dims& d, const PhysC& ph, const DGeom& g,
+                                               const DStateT<R>& s, unsigned zo, int lane, int w, int a, int h) {
+  const long long PS = (long long)NPANEL * d.S;
+  if (w == 5) {
+    const double* cen = g.f[CS_G_V_CEN] + zo;
+    const double* cf = g.f[CS_G_COEF] + 4 * PS + zo;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) S.geo[c][lane] = (R)__ldg(cen + c * PS);
+    S.geo[3][lane] = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + zo), R(ph.smallnum));
+#pragma unroll
+    for (int m = 0; m < 6; ++m) S.geo[4 + m][lane] = (R)__ldg(cf + m * PS);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int8_t* umap = s.adp_pmap + (3 * h + q) * 72 + 10 * a;
+#pragma unroll
+    for (int m = 0; m < 10; ++m) {
+      const int u = __ldg(umap + m);
+      acc[q][m] = (R)__ldg(umap + 36 + m) * s.V[(u % 10 * NVAR + 5 + u / 10) * PS + (3 * h + q) * d.S + zo];
+    }
+  }
+  // normals and (component 0's warps) face weights, a face ahead
+  R nn[5], wt[5];
+  auto scalars = [&](int f) {
+    const int dir = f >> 1;
+    const unsigned fo = adp6_face(d, f, zo);
+    const double* nf = (dir == 0 ? g.f[CS_G_XF_N] : (dir == 1 ? g.f[CS_G_YF_N] : g.f[CS_G_ZF_N])) + fo;
+    const double* bw = (dir == 0 ? g.f[CS_G_XB_QW] : (dir == 1 ? g.f[CS_G_YB_QW] : g.f[CS_G_ZB_QW])) + fo;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      nn[c] = (R)__ldg(nf + (dir == 2 ? 5 * a + c : a) * PS);
+      if (a == 0) wt[c] = (R)__ldg(bw + c * PS);
+    }
+  };
+  scalars(0);
+  adp6_sync();  // geo
+#pragma unroll 1
+  for (int f = 0; f < 6; ++f) {
+    R(&bas)[5][9][ADP6_ZB] = S.bas[f & 1];
+    const double(*fr)[ADP6_ZB] = S.face(f);
+    asm volatile("cp.async.wait_group %0;" ::"n"(ADP6_FB - 2) : "memory");
+    if (w < 5) {
+      const R ob = S.geo[3][lane], x = ((R)fr[w][lane] - S.geo[0][lane]) * ob, y = ((R)fr[5 + w][lane] - S.geo[1][lane]) * ob,
+              z = ((R)fr[10 + w][lane] - S.geo[2][lane]) * ob;
+      bas[w][0][lane] = x;
+      bas[w][1][lane] = y;
+      bas[w][2][lane] = z;
+      bas[w][3][lane] = x * x - S.geo[4][lane];
+      bas[w][4][lane] = y * y - S.geo[5][lane];
+      bas[w][5][lane] = z * z - S.geo[6][lane];
+      bas[w][6][lane] = x * y - S.geo[7][lane];
+      bas[w][7][lane] = y * z - S.geo[8][lane];
+      bas[w][8][lane] = x * z - S.geo[9][lane];
+    }
+    // this face's rows and monomials are complete, the face before's no longer
+    // read
+    adp6_sync();
+    if (a == 0) {
+      R dacc[3] = {R(0.0), R(0.0), R(0.0)};
+#pragma unroll
+      for (int c = 0; c < 5; ++c)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) dacc[q] = dacc[q] + wt[c] * (R)fr[15 + 5 * (3 * h + q) + c][lane];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) S.x[30 + f][3 * h + q][lane] = dacc[q];
+    }
+    R n5[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) n5[c] = nn[c];
+    if (f + ADP6_FB - 1 < 6) adp6_fetch(S, d, g, s, f + ADP6_FB - 1, zo, lane, w);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (f < 5) scalars(f + 1);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      R bq[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) bq[q] = (R)fr[15 + 5 * (3 * h + q) + c][lane];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) acc[q][0] = acc[q][0] + n5[c] * bq[q];
+#pragma unroll
+      for (int m = 0; m < 9; ++m) {
+        const R e = n5[c] * bas[c][m][lane];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) acc[q][1 + m] = acc[q][1 + m] + e * bq[q];
+      }
+    }
+  }
+  adp6_sync();  // the last face's rows have been read
+}
+
 // The stream, the right-hand sides and the sums are in the state's type R
 // (FP32 in the precision form: half the stream's bytes).
+//
+// In FP64 a face's points and values come through copies that run three faces
+// ahead, into the next block's too: 13.1 -> 10.2 ms of a 6 x 128^2 x 64 step,
+// 0.300 -> 0.279 of a 6 x 32^2 x 16 one, the same on the smallest.  The FP32
+// form's right-hand sides leave room for two faces only, with which it was
+// slower (8.7 -> 9.0 ms, 0.57 -> 0.66 ms on 6 x 50^2 x 13): its threads load
+// their own.
 template <typename R>
 __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   extern __shared__ __align__(128) unsigned char adp6_raw[];
@@ -663,7 +811,15 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
   }
   const int lane = tid & 31, w = tid >> 5;
   const long long PS = (long long)NPANEL * d.S;
+  constexpr bool kAhead = sizeof(R) == 8;
   RingPos<ADP6_NS> ring;
+  auto fetch_first = [&](long long blk) {  // of a block's position
+    const long long t1 = blk * ADP6_ZB + lane;
+    int p0 = 0, i = r.i0, j = r.j0, k = r.k0;
+    if (t1 < n1) r.decode(t1, p0, i, j, k);
+    adp6_fetch_first(S, d, g, s, (unsigned)d.idx(i, j, k), lane, w);
+  };
+  if constexpr (kAhead) fetch_first(blockIdx.x);
   for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     const long long t1 = blk * ADP6_ZB + lane;
     const bool inr = t1 < n1;
@@ -677,72 +833,76 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
     R acc[3][10];
     {
       const unsigned zo = (unsigned)d.idx(i, j, k);  // box offset of the position
-      const double* cen = g.f[CS_G_V_CEN] + zo;
-      const double* cf = g.f[CS_G_COEF] + zo;
-      const R obl0 = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + zo), R(ph.smallnum));
-      const R vc0 = (R)__ldg(cen), vc1 = (R)__ldg(cen + PS), vc2 = (R)__ldg(cen + 2 * PS);
-      R c0[6];
+      if constexpr (kAhead) {
+        adp6_rhs_ahead(acc, S, d, ph, g, s, zo, lane, w, a, h);
+      } else {
+        const double* cen = g.f[CS_G_V_CEN] + zo;
+        const double* cf = g.f[CS_G_COEF] + zo;
+        const R obl0 = R(1.0) / fmax((R)__ldg(g.f[CS_G_V_SCALE] + zo), R(ph.smallnum));
+        const R vc0 = (R)__ldg(cen), vc1 = (R)__ldg(cen + PS), vc2 = (R)__ldg(cen + 2 * PS);
+        R c0[6];
 #pragma unroll
-      for (int m = 0; m < 6; ++m) c0[m] = (R)__ldg(cf + (4 + m) * PS);
+        for (int m = 0; m < 6; ++m) c0[m] = (R)__ldg(cf + (4 + m) * PS);
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const int8_t* umap = s.adp_pmap + (3 * h + q) * 72 + 10 * a;
+        for (int q = 0; q < 3; ++q) {
+          const int8_t* umap = s.adp_pmap + (3 * h + q) * 72 + 10 * a;
 #pragma unroll
-        for (int m = 0; m < 10; ++m) {
-          const int u = __ldg(umap + m);
-          acc[q][m] = (R)__ldg(umap + 36 + m) * s.V[(u % 10 * NVAR + 5 + u / 10) * PS + (3 * h + q) * d.S + zo];
+          for (int m = 0; m < 10; ++m) {
+            const int u = __ldg(umap + m);
+            acc[q][m] = (R)__ldg(umap + 36 + m) * s.V[(u % 10 * NVAR + 5 + u / 10) * PS + (3 * h + q) * d.S + zo];
+          }
         }
-      }
 #pragma unroll 1
-      for (int f = 0; f < 6; ++f) {
-        const int dir = f >> 1;
-        const unsigned fo = zo - ((f & 1) ? (dir == 0 ? 1 : (dir == 1 ? d.NI : d.NI * d.NJ)) : 0);
-        R(&bas)[5][9][ADP6_ZB] = S.bas[f & 1];
-        if (w < 5) {
-          const double* qp = (dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP])) + fo;
-          const R x = ((R)__ldg(qp + w * PS) - vc0) * obl0, y = ((R)__ldg(qp + (5 + w) * PS) - vc1) * obl0,
-                  z = ((R)__ldg(qp + (10 + w) * PS) - vc2) * obl0;
-          bas[w][0][lane] = x;
-          bas[w][1][lane] = y;
-          bas[w][2][lane] = z;
-          bas[w][3][lane] = x * x - c0[0];
-          bas[w][4][lane] = y * y - c0[1];
-          bas[w][5][lane] = z * z - c0[2];
-          bas[w][6][lane] = x * y - c0[3];
-          bas[w][7][lane] = y * z - c0[4];
-          bas[w][8][lane] = x * z - c0[5];
-        }
-        const double* Bq = (dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2])) + 3 * h * d.S + fo;
-        const double* nf = (dir == 0 ? g.f[CS_G_XF_N] : (dir == 1 ? g.f[CS_G_YF_N] : g.f[CS_G_ZF_N])) + fo;
-        R bq[3][5], nn[5];
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-          nn[c] = (R)__ldg(nf + (dir == 2 ? 5 * a + c : a) * PS);
-#pragma unroll
-          for (int q = 0; q < 3; ++q) bq[q][c] = (R)Bq[c * PS + q * d.S];
-        }
-        if (a == 0) {
-          const double* bw = (dir == 0 ? g.f[CS_G_XB_QW] : (dir == 1 ? g.f[CS_G_YB_QW] : g.f[CS_G_ZB_QW])) + fo;
-          R dacc[3] = {R(0.0), R(0.0), R(0.0)};
+        for (int f = 0; f < 6; ++f) {
+          const int dir = f >> 1;
+          const unsigned fo = zo - ((f & 1) ? (dir == 0 ? 1 : (dir == 1 ? d.NI : d.NI * d.NJ)) : 0);
+          R(&bas)[5][9][ADP6_ZB] = S.bas[f & 1];
+          if (w < 5) {
+            const double* qp = (dir == 0 ? g.f[CS_G_XF_QP] : (dir == 1 ? g.f[CS_G_YF_QP] : g.f[CS_G_ZF_QP])) + fo;
+            const R x = ((R)__ldg(qp + w * PS) - vc0) * obl0, y = ((R)__ldg(qp + (5 + w) * PS) - vc1) * obl0,
+                    z = ((R)__ldg(qp + (10 + w) * PS) - vc2) * obl0;
+            bas[w][0][lane] = x;
+            bas[w][1][lane] = y;
+            bas[w][2][lane] = z;
+            bas[w][3][lane] = x * x - c0[0];
+            bas[w][4][lane] = y * y - c0[1];
+            bas[w][5][lane] = z * z - c0[2];
+            bas[w][6][lane] = x * y - c0[3];
+            bas[w][7][lane] = y * z - c0[4];
+            bas[w][8][lane] = x * z - c0[5];
+          }
+          const double* Bq = (dir == 0 ? s.Bq[0] : (dir == 1 ? s.Bq[1] : s.Bq[2])) + 3 * h * d.S + fo;
+          const double* nf = (dir == 0 ? g.f[CS_G_XF_N] : (dir == 1 ? g.f[CS_G_YF_N] : g.f[CS_G_ZF_N])) + fo;
+          R bq[3][5], nn[5];
 #pragma unroll
           for (int c = 0; c < 5; ++c) {
-            const R wt = (R)__ldg(bw + c * PS);
+            nn[c] = (R)__ldg(nf + (dir == 2 ? 5 * a + c : a) * PS);
 #pragma unroll
-            for (int q = 0; q < 3; ++q) dacc[q] = dacc[q] + wt * bq[q][c];
+            for (int q = 0; q < 3; ++q) bq[q][c] = (R)Bq[c * PS + q * d.S];
           }
+          if (a == 0) {
+            const double* bw = (dir == 0 ? g.f[CS_G_XB_QW] : (dir == 1 ? g.f[CS_G_YB_QW] : g.f[CS_G_ZB_QW])) + fo;
+            R dacc[3] = {R(0.0), R(0.0), R(0.0)};
 #pragma unroll
-          for (int q = 0; q < 3; ++q) S.x[30 + f][3 * h + q][lane] = dacc[q];
-        }
-        adp6_sync();
+            for (int c = 0; c < 5; ++c) {
+              const R wt = (R)__ldg(bw + c * PS);
 #pragma unroll
-        for (int c = 0; c < 5; ++c) {
+              for (int q = 0; q < 3; ++q) dacc[q] = dacc[q] + wt * bq[q][c];
+            }
 #pragma unroll
-          for (int q = 0; q < 3; ++q) acc[q][0] = acc[q][0] + nn[c] * bq[q][c];
+            for (int q = 0; q < 3; ++q) S.x[30 + f][3 * h + q][lane] = dacc[q];
+          }
+          adp6_sync();
 #pragma unroll
-          for (int m = 0; m < 9; ++m) {
-            const R e = nn[c] * bas[c][m][lane];
+          for (int c = 0; c < 5; ++c) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) acc[q][1 + m] = acc[q][1 + m] + e * bq[q][c];
+            for (int q = 0; q < 3; ++q) acc[q][0] = acc[q][0] + nn[c] * bq[q][c];
+#pragma unroll
+            for (int m = 0; m < 9; ++m) {
+              const R e = nn[c] * bas[c][m][lane];
+#pragma unroll
+              for (int q = 0; q < 3; ++q) acc[q][1 + m] = acc[q][1 + m] + e * bq[q][c];
+            }
           }
         }
       }
@@ -772,6 +932,9 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
       }
     }
     adp6_sync();
+    if constexpr (kAhead) {  // x has been read
+      if (blk + gridDim.x < nblk) fetch_first(blk + gridDim.x);
+    }
     if (inr && mask_at(g, d, w, i, j) == 1) {
       R* U = s.U;
       const long long o5 = d.at(4, w, i, j, k);
