@@ -415,8 +415,7 @@ void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
   Range3 fz = {0, N + 1, 0, N + 1, z.k0 - 1, z.k1};
   {
     const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + FLUX_FACES - 1) / FLUX_FACES);
-    const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 32);
-    k_flux<R><<<nb, FLUX_FACES * 5, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
+    k_flux<R><<<tile_blocks(sv, nt, 32), FLUX_FACES * 5, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
     mark(sv, "k_flux");
   }
   if (sv.psync.nf > 0 && (sv.p.flags & CS_FLAG_PANEL_AVERAGE)) {

@@ -1734,7 +1734,7 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
   Range3 a = shrink(d, 1), b = shrink(d, 2);
   if (sv.p.flags & CS_FLAG_P2) {  // LIMIT_ALL_SLOPES_P2's STEP 7.a
     const long long nt = (b.count() + W7A_ZT - 1) / W7A_ZT;
-    const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
+    const int nb = tile_blocks(sv, nt, 16);
     k_weno_slopes<W7_ENT, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, b);
     mark(sv, "k_p2_entropy");
     const int np = (int)std::min<long long>(p2_tiles(b, st.p2_map), (long long)grid_sms(sv) * p2_blocks(sizeof(R)));
@@ -1747,7 +1747,7 @@ void launch_weno_t(Solve& sv, DStateT<R>& st) {
   }
   {
     const long long nt = (a.count() + W7A_ZT - 1) / W7A_ZT;
-    const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
+    const int nb = tile_blocks(sv, nt, 16);
     k_weno_slopes<W7_PRIM, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_weno7a");
   }
@@ -1794,8 +1794,7 @@ void launch_faceB_adp_t(Solve& sv, DStateT<R>& st) {
   fy.j0 -= 1;
   fz.k0 -= 1;
   const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + TPB - 1) / TPB);
-  const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 64);
-  k_faceB<R><<<nb, TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
+  k_faceB<R><<<tile_blocks(sv, nt, 64), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
   mark(sv, "k_faceB");
   launch_adp(sv);
 }
@@ -1859,7 +1858,7 @@ void launch_efield_t(Solve& sv, DStateT<R>& st) {
   }
   {
     const long long nt = (a.count() + W7A_ZT - 1) / W7A_ZT;
-    const int nb = (int)std::min<long long>(nt, (long long)grid_sms(sv) * 16);
+    const int nb = tile_blocks(sv, nt, 16);
     k_weno_slopes<W7_E, R><<<nb, W7A_ZT * 3, 0, sv.stream>>>(d, sv.ph, sv.g, st, a);
     mark(sv, "k_efield_b");
   }
