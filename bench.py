@@ -732,11 +732,9 @@ def run_gpu(args):
     dom = max(prof.items(), key=lambda kv: kv[1][0])
     dname, (dms, dcount) = dom
     G, N, nr = s.G, s.N, s.nr
-    units = 6 * (N + 2 * G - 2) ** 2 * (nr + 2 * G - 2)  # zones of the shrink-1 range (7.a / 8.d / 9.b)
-    if dname in ("k_weno7b", "k_efield_c"):
-        units = 6 * (N + 2 * G - 4) ** 2 * (nr + 2 * G - 4)
-    if dname == "k_flux":
-        units = 6 * (N + 4) ** 2 * (nr + 4)
+    # zones of the kernel's range: layers around the interior
+    layers = {"k_weno7a": G - 1, "k_weno7b": G - 2, "k_adp6": 2, "k_faceB": 2, "k_positivity": G - 2}.get(dname, 1)
+    units = 6 * (N + 2 * layers) ** 2 * (nr + 2 * layers)
     launch_s = dms / dcount / 1e3
     per_launch = stage_b * units
     achieved = per_launch / launch_s / 1e9

@@ -188,7 +188,8 @@ __device__ __forceinline__ void edge_z(const Dims& d, const DGeom& g, const DSta
 //
 // What bounds it: latency of about 30 loads an edge.  Solving the four-state
 // problem in its general form at each of the rule's three points took 136
-// registers and most of the time in FP64 divisions.
+// registers and most of the time in FP64 divisions: 2.9 ms of a 6 x 128^2 x 64
+// step against 1.2.
 template <typename R>
 __global__ void __launch_bounds__(TPB, 6) k_edges(Dims d, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
   const unsigned nb = (unsigned)((max(r0.count(), max(r1.count(), r2.count())) + TPB - 1) / TPB);

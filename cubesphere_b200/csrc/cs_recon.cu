@@ -262,7 +262,8 @@ __device__ __forceinline__ Nbr12 load_nbr(const DGeom& g, const Dims& d, int p, 
 // latency at 18 (FP32: 24) warps an SM.  The neighbours are box offsets in
 // shared memory (tables indexed at run time lived in local memory), a
 // variable's values are loaded while the one before is worked on, and the nine
-// weights take Newton reciprocals.
+// weights take Newton reciprocals.  ms of a 6 x 128^2 x 64 step, before / now:
+// STEP 7.a 7.1 / 4.6 (FP32 5.5 / 3.6), STEP 9.b 4.0 / 2.2 (3.1 / 1.8).
 enum W7Kind { W7_PRIM, W7_E, W7_ENT };
 constexpr int W7A_ZT = 32;
 template <W7Kind kK, typename R>
@@ -671,7 +672,8 @@ __device__ __noinline__ int positivity_shrink(const Dims& d, const PhysC& ph, co
 // The others run the nodes (positivity_shrink), so every zone ends with the
 // same record as without the bound.  A thread takes kc zones of a radial
 // column and keeps the range of the last three layers: 9 neighbours' loads a
-// zone instead of 27.
+// zone instead of 27.  ms of a 6 x 128^2 x 64 step: 4.35 (FP32 form 5.0) with the
+// nodes of every zone, 1.66 (1.63) so; what is left is the reads of the modes.
 template <typename R>
 __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g, DStateT<R> s, const float* __restrict__ ext,
                                                        Range3 r, int kc) {
@@ -764,7 +766,8 @@ __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g
 // components of both sides at once took 252 registers, 8 warps an SM.  The
 // face normal is one vector on x- and y-faces, so there each side's modes are
 // first contracted with it (10 values, one polynomial); on z-faces, where it
-// varies over the points, the components are taken one after another.
+// varies over the points, the components are taken one after another.  ms of a
+// 6 x 128^2 x 64 step, that / this: 7.7 / 5.6 (FP32 7.4 / 3.9).
 template <typename R>
 __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_faceB(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
   const unsigned nt0 = (unsigned)((r0.count() + TPB - 1) / TPB), nt1 = (unsigned)((r1.count() + TPB - 1) / TPB),

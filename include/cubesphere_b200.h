@@ -121,7 +121,7 @@ typedef struct cs_params {
  * state, entropy, primitives and their modes, the flattener, face states and
  * fluxes, dU/dt, the stage copies, the resident least-squares inverses, the
  * face-B quadrature evaluations and the ADP constrained least squares:
- * right-hand sides, panel-shared factors, substitution) is stored and
+ * right-hand sides, panel-shared inverses, solution) is stored and
  * computed in FP32; the geometry, face B, the shift of the quadrature
  * values to the FP64 face mean, the ADP factorisation itself (stored
  * rounded), the edge EMFs, the CT update, the positivity fix and the
@@ -131,15 +131,15 @@ typedef struct cs_params {
  * through cs_state_get / cs_state_put stays FP64 at the boundary. */
 #define CS_FLAG_FP32 8
 /* cs_params.flags: keep one set of ADP factors per panel.  By default the
- * resident ADP factors are panel 1's only and serve all six panels: the
+ * resident ADP operators are panel 1's only and serve all six panels: the
  * panels are rotations of panel 1 by signed permutations (checked on the
  * vertices when the mesh is uploaded), under which the KKT matrix of a zone
  * transforms by the induced signed permutation of the unknowns, so one
- * factor read from HBM serves six solves and the cache takes 1/6 of the
- * memory (1.7 KB per zone).  The reference factors every zone's system
+ * packed symmetric inverse read from HBM serves six solves (0.86 KB per zone
+ * against 10.4 KB).  The reference factors every zone's system
  * (420/421 STEP 8.d); its solutions agree with the per-panel factors to
  * round-off.  This flag restores per-panel factors; meshes without the
- * symmetry use them anyway. */
+ * symmetry, or too ill conditioned for an inverse, use them anyway. */
 #define CS_FLAG_ADP_PER_PANEL 16
 /* cs_params.flags: keep one set of least-squares row weights per panel.  By
  * default the resident row weights W_r = Minv A_r^T of STEP 9.c (and of

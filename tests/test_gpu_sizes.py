@@ -144,7 +144,7 @@ def test_reciprocals_by_newton_steps_are_within_two_units():
         c[:, side + 4] = prs
     c[:, 16:] = 1.0
     gamma = 5.0 / 3.0
-    out = cs.pointwise(2, c, ntp=4, nr=1, gamma=gamma)
+    out = cs.pointwise(2, c, ntp=8, nr=4, gamma=gamma)
     want = np.sqrt(np.longdouble(gamma) * prs.astype(np.longdouble) / rho.astype(np.longdouble))
     for sign, got in ((-1.0, out[:, 32]), (1.0, out[:, 33])):
         err = np.abs(sign * got - want) / want
