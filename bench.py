@@ -70,15 +70,15 @@ ALGO_WORDS_PER_UNIT = {
 }
 
 # DRAM bytes per unit and launch (read + write) measured by ncu on the
-# shell32 case (units: 190,608 zones of the ADP range, 155,520 of the flux /
-# least-squares ranges; 14 launches each), FP64 and precision form; the full
+# shell32 case (units: 155,520 zones of the ADP and STEP 7.b ranges, 124,848 of
+# the flux and STEP 9.c ranges; 14 launches each), FP64 and precision form; the full
 # shell128 launches are too large to capture, so roofline.traffic scales
 # these by the units of a full launch.
 MEASURED_TRAFFIC_PER_UNIT = {
-    "k_adp_solve6": 2274.8,
-    "k_flux": 2085.8,
-    "k_weno7b": 2188.9,
-    "k_efield_c": 486.5,
+    "k_adp6": 1710.6,
+    "k_flux": 2251.2,
+    "k_weno7b": 2178.9,
+    "k_efield_c": 487.6,
 }
 MEASURED_TRAFFIC_PER_UNIT_FP32 = {
     "k_adp_solve6": 1117.1,
@@ -92,10 +92,10 @@ MEASURED_TRAFFIC_PER_UNIT_FP32 = {
 # device in the same run (cs_fp64_fma_rate); the nominal rate, 148 SMs x 64
 # FP64 FMA per clock x 2 x 1.965 GHz = 37.2 TFLOP/s, is kept for context.
 FP64_FLOP_PER_UNIT = {
-    "k_adp_solve6": 3154.2,
-    "k_flux": 16485.3,
-    "k_weno7b": 3727.7,
-    "k_efield_c": 1529.2,
+    "k_adp6": 4455.1,
+    "k_flux": 14498.6,
+    "k_weno7b": 3900.7,
+    "k_efield_c": 1780.4,
 }
 FP64_NOMINAL_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12
 
