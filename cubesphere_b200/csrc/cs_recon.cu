@@ -680,7 +680,6 @@ __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g
   const unsigned ni = r.i1 - r.i0 + 1, nj = r.j1 - r.j0 + 1, ncol = 6 * ni * nj;
   const unsigned nseg = (r.k1 - r.k0 + kc) / kc, nt = ncol * nseg;
   const long long PS = (long long)NPANEL * d.S;
-  const int plane = d.NI * d.NJ;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     const unsigned seg = t / ncol, col = t - seg * ncol, u = col / ni;
     const int i = (int)(col - u * ni) + r.i0, j = (int)(u % nj) + r.j0, p = (int)(u / nj);
