@@ -81,10 +81,10 @@ MEASURED_TRAFFIC_PER_UNIT = {
     "k_efield_c": 487.6,
 }
 MEASURED_TRAFFIC_PER_UNIT_FP32 = {
-    "k_adp_solve6": 1117.1,
-    "k_flux": 1489.4,
-    "k_weno7b": 420.0,
-    "k_efield_c": 262.9,
+    "k_adp6": 948.3,
+    "k_flux": 1653.8,
+    "k_weno7b": 441.4,
+    "k_efield_c": 274.1,
 }
 # FP64 operations per unit and launch (2 x DFMA + DADD + DMUL thread
 # instructions), from the same FP64 capture.  The path is FP64-bound, so the
