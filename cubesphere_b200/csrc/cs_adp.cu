@@ -411,10 +411,7 @@ __global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph,
   // next factor element of this thread's zone
   auto next = [&]() -> double {
     if (within == ADPS_CH) {
-      if (gch > 0) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&S.empty[(int)((gch - 1) % ADPS_NS)]);
-      }
+      if (gch > 0) ring_release(&S.empty[(int)((gch - 1) % ADPS_NS)], lane);
       const int slot = (int)(gch % ADPS_NS);
       mbar_wait(&S.full[slot], (uint32_t)((gch / ADPS_NS) & 1), s.err_flag);
       cur = &S.stage[slot][0][tid];
@@ -465,9 +462,6 @@ __global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph,
       }
     }
   }
-  // release the last chunk (no producer waits for it; keeps the protocol uniform)
-  __syncwarp();
-  if (lane == 0 && gch > 0) mbar_arrive(&S.empty[(int)((gch - 1) % ADPS_NS)]);
 }
 
 }  // namespace
@@ -624,10 +618,7 @@ __device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, Rin
     adp6_unit<2 * c>(acc, xr, w, wp, xm, x, xn, xp);
     if constexpr (2 * c + 1 < ADP6_WORDS / ADP6_UNIT)
       adp6_unit<2 * c + 1>(acc, xr, w + ADP6_UNIT * ADP6_ZB, wp + ADP6_UNIT * ADP6_ZB, xm, x, xn, xp);
-    // this warp's reads are done before the copy engine may write the stage again
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&S.empty[ring.slot]);
+    ring_release(&S.empty[ring.slot], lane);
     ring.next();
   };
   (chunk(std::integral_constant<int, C>{}), ...);

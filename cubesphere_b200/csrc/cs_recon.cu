@@ -1304,10 +1304,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
           for (int c = 0; c < 2; ++c) Y[c][m] = Y[c][m] + a * D[c][rr];
         }
       }
-      // this warp's reads are done before the copy engine may write the stage again
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.empty[ring.slot]);
+      ring_release(&S.empty[ring.slot], lane);
       ring.next();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {

@@ -55,6 +55,15 @@ static __device__ __noinline__ void mbar_wait(uint64_t* bar, uint32_t parity, in
   atomicOr(err, 1);
 }
 
+// A consumer warp's release of a ring stage.  Every lane's reads are fenced
+// against the async proxy first: the copy that refills the stage is not ordered
+// behind loads that are still in flight, only behind this fence and the arrive.
+__device__ __forceinline__ void ring_release(uint64_t* empty, int lane) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) mbar_arrive(empty);
+}
+
 // Position in a ring of NS shared-memory stages: slot and the parity of its
 // current phase.
 template <int NS>

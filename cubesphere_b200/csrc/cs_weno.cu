@@ -167,10 +167,7 @@ __global__ void __launch_bounds__(W7_THREADS, sizeof(R) == 4 ? 4 : 3) k_weno7b(D
           Y[1][a] = Y[1][a] + m * d1;
         }
       }
-      // this warp's reads are done before the copy engine may write the stage again
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.empty[ring.slot]);
+      ring_release(&S.empty[ring.slot], lane);
       ring.next();
       if (c < 2)
 #pragma unroll
@@ -315,10 +312,7 @@ __global__ void __launch_bounds__(E9_THREADS, sizeof(R) == 4 ? 8 : 6) k_efield_c
         if (c * E9_ROWS + rr < 19)
 #pragma unroll
           for (int a = 0; a < 10; ++a) Y[a] = Y[a] + A[(rr * 10 + a) * wid] * D[c * E9_ROWS + rr < 19 ? c * E9_ROWS + rr : 0];
-      // this warp's reads are done before the copy engine may write the stage again
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&S.empty[ring.slot]);
+      ring_release(&S.empty[ring.slot], lane);
       ring.next();
     }
     if (act) {

@@ -105,6 +105,37 @@ def test_batch_of_p2_solves_matches_each_solve_alone():
             s.close()
 
 
+def test_batches_on_the_adp_factors_give_each_members_own_result():
+    """Members that substitute with per-panel ADP factors (asked for, in both
+    precision forms, or kept because the mesh is too ill conditioned for the
+    inverse) side by side, many times: every state equals the member's run
+    alone, bit for bit."""
+    members = []
+    for name, over, flags in (("shell32", {}, cs.CS_FLAG_ADP_PER_PANEL), ("shell16", dict(ntp=6, nr=1), 0),
+                              ("surface32", dict(ntp=48), cs.CS_FLAG_ADP_PER_PANEL),
+                              ("shell32", dict(ntp=24), cs.CS_FLAG_ADP_PER_PANEL | cs.CS_FLAG_FP32)):
+        s = make((name, over, {}, flags))
+        st = s.get_state()
+        s.profile_begin()
+        dt = s.evaluate_timestep(1e30)
+        s.step(dt)
+        assert "k_adp_solve" in s.profile_end(), name
+        s.put_state(st)
+        dt = s.steps(2, s.evaluate_timestep(1e30))
+        members.append((s, st, dt, s.get_state()))
+    b = cs.Batch([m[0] for m in members])
+    for rep in range(20):
+        for s, st, _, _ in members:
+            s.put_state(st)
+        dts = b.steps(2, [s.evaluate_timestep(1e30) for s, _, _, _ in members])
+        for q, (s, _, dt, want) in enumerate(members):
+            assert dts[q] == dt, (rep, q)
+            got = s.get_state()
+            for k in want:
+                assert np.array_equal(got[k], want[k]), (rep, q, k)
+    b.close()
+
+
 def test_autotune_changes_no_result():
     want = alone(2)
     sols = [make(m) for m in MEMBERS]
