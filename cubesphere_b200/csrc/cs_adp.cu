@@ -624,8 +624,7 @@ __device__ __forceinline__ void adp6_apply(F (&acc)[3][10], Adp6SmemT<F>& S, Rin
   (chunk(std::integral_constant<int, C>{}), ...);
 }
 
-// Barrier of the six consumer warps (the producer is not part of it).
-__device__ __forceinline__ void adp6_sync() { asm volatile("bar.sync 1, %0;" ::"n"(ADP6_CONS) : "memory"); }
+__device__ __forceinline__ void adp6_sync() { consumer_sync<ADP6_CONS>(); }
 
 // Copy of one word a lane to shared memory, in the background.
 __device__ __forceinline__ void copy8(double* dst, const double* src) {

@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
     }
     if (w == 0) nbo[12][lane] = 0;
     // the offsets are complete; the other copy is no longer read
-    asm volatile("bar.sync 1, %0;" ::"n"(P2_CONS) : "memory");
+    consumer_sync<P2_CONS>();
     const long long o = (long long)p * d.S + d.idx(i, j, k);
     const R* f = s.V + 2 * w * PS + o;
     // smoothness weight of the modes xx .. xz over the unit cube (x y z: 1 /

@@ -64,6 +64,15 @@ __device__ __forceinline__ void ring_release(uint64_t* empty, int lane) {
   if (lane == 0) mbar_arrive(empty);
 }
 
+// Barrier of a ring kernel's N consumer threads (the producer is not part of
+// it).  It is an aligned one: lanes that skipped a masked zone's work come
+// together with their warp first.
+template <int N>
+__device__ __forceinline__ void consumer_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
+}
+
 // Position in a ring of NS shared-memory stages: slot and the parity of its
 // current phase.
 template <int NS>

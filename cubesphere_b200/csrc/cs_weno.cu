@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(W7_THREADS, sizeof(R) == 4 ? 4 : 3) k_weno7b(D
     const int wid = w_block<162>(kShared ? T / 6 : T, nw).wid;
     int(&nbo)[12][32] = S.nbo[buf];
     // the offsets are complete; the other copy is no longer read
-    asm volatile("bar.sync 1, %0;" ::"n"(W7_CONS) : "memory");
+    consumer_sync<W7_CONS>();
     const R* v = s.V + 2 * w * PS + o;  // primitives 2 w and 2 w + 1
     // differences to the neighbours of stencil rows 6 c .. 6 c + 5, loaded one
     // ring stage ahead of their use
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(E9_THREADS, sizeof(R) == 4 ? 8 : 6) k_efield_c
     }
     const int wid = w_block<190>(kShared ? T / 6 : T, nw).wid;
     // the offsets are complete; the other copy is no longer read
-    asm volatile("bar.sync 1, %0;" ::"n"(E9_CONS) : "memory");
+    consumer_sync<E9_CONS>();
     const long long o = (long long)p * d.S + d.idx(i, j, k);
     const R* f = s.Esnap + w * PS + o;
     R D[19];

@@ -63,6 +63,18 @@ def test_p2_whole_steps_match_oracle(name, nsteps, flags, rk):
         check_state(s, s.get_state(), o.get_state())
 
 
+@pytest.mark.parametrize("ntp,nr,ghosts", [(5, 2, 3), (13, 3, 4), (19, 9, 4), (9, 6, 5)])
+@pytest.mark.parametrize("flags", [0, cs.CS_FLAG_LSQ_PER_PANEL])
+def test_p2_step_at_uneven_sizes_matches_oracle(ntp, nr, ghosts, flags):
+    """One step where warps hold masked and active zones side by side and the
+    last tile of a panel is short."""
+    s, o, st = make_pair("shell16", P2 | flags, ntp=ntp, nr=nr, nghost=ghosts)
+    dt_s, dt_o = s.evaluate_timestep(1e30), o.evaluate_timestep(1e30)
+    dt_s, dt_o = s.steps(1, dt_s), o.step(dt_o)
+    assert abs(dt_s - dt_o) <= TOL_STATE * dt_o
+    check_state(s, s.get_state(), o.get_state())
+
+
 def test_p2_differs_from_p12():
     """The flag changes the scheme: after one step the states of P2 and P12
     differ by far more than round-off (the third-order stencils' truncation
