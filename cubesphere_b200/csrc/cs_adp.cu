@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(ADP6_THREADS, sizeof(R) == 4 ? 4 : 2) k_adp6(D
 template <typename R>
 void launch_adp_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
-  Range3 a = around(d, adp_layers(sv));
+  const Range3 a = adp_zones(sv);
   if (st.adp_lu && st.adp_pmap) {
     const long long nblk = (a.count() / 6 + ADP6_ZB - 1) / ADP6_ZB;
     const int grid = (int)std::min<long long>(nblk, (long long)grid_sms(sv) * (sizeof(R) == 4 ? 4 : 2));
@@ -979,7 +979,7 @@ void launch_adp(Solve& sv) {
     launch_adp_t(sv, sv.st);
 }
 
-long long adp_range_count(const Solve& sv) { return around(sv.d, adp_layers(sv)).count(); }
+long long adp_range_count(const Solve& sv) { return adp_zones(sv).count(); }
 long long adp_factor_doubles(const Solve& sv, bool shared) {
   const long long n = adp_range_count(sv);
   if (shared) return (n / 6 + ADP6_ZB - 1) / ADP6_ZB * (long long)ADP6_ZB * ADP6_WORDS;
@@ -1001,7 +1001,7 @@ void set_adp_smem_limits() {
 template <typename R>
 void launch_adp_factor_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
-  Range3 a = around(d, adp_layers(sv));
+  const Range3 a = adp_zones(sv);
   const size_t smem = sizeof(AdpSmem) * ADP_WARPS;
   // shared factors: panel 1's zones only, in blocks of ADP6_ZB
   const long long tmax = st.adp_pmap ? a.count() / 6 : a.count();

@@ -500,12 +500,9 @@ int alloc_state(Solve& sv, DStateT<R>& s) {
   s.op_p2v = (R*)m.op_p2v;
   s.op_p2e = (R*)m.op_p2e;
   s.p2_map = m.p2_shared ? (const LsqPanelMap*)m.lsq_map : nullptr;
-  // a mesh whose operators cover fewer layers than this solve needs serves it
-  // without them
-  const bool adp = m.adp_w == sv.adp_w;
-  s.adp_lu = adp ? m.adp_lu : nullptr;
+  s.adp_lu = m.adp_lu;
   s.adp_piv = m.adp_piv;
-  s.adp_pmap = adp ? m.adp_pmap : nullptr;
+  s.adp_pmap = m.adp_pmap;
   s.adp_rhs = nullptr;
   if (s.adp_lu && !s.adp_pmap) {  // k_adp6 keeps its right-hand sides in shared memory
     s.adp_rhs = dalloc(sv, (size_t)adp_range_count(sv) * 36 * sizeof(double), e);
@@ -892,8 +889,6 @@ int mesh_attach(Solve& sv, const std::shared_ptr<MeshRes>& mp) {
   set_p2_smem_limits();
   set_weno_smem_limits();
   const bool fresh = !m.on_device;
-  if (fresh) m.adp_w = adp_layers_needed(sv.p);
-  sv.adp_w = std::max(m.adp_w, adp_layers_needed(sv.p));
   if (fresh)
     if (int rc = mesh_upload(sv, m)) return rc;
   sv.g = m.g;

@@ -18,7 +18,7 @@ namespace {
 // STEP 2 (zone part, 421:597-635) and STEP 5 (421:1497-1628) of one zone.
 template <typename R>
 __device__ __forceinline__ void prim_zone(const Dims& d, const PhysC& ph, const DGeom& g, const DStateT<R>& s, int p, int i,
-                                          int j, int k, int al) {
+                                          int j, int k, const AdpLayers& al) {
   const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
   const int m = mask_at(g, d, p, i, j);
   R U[8], V[8];
@@ -42,12 +42,13 @@ __device__ __forceinline__ void prim_zone(const Dims& d, const PhysC& ph, const 
   s.ent[2 * PS + o] = R(0.0);
   s.ent[3 * PS + o] = R(0.0);
   // The higher modes are zero from the start wherever no step writes them.
-  // STEP 8.d writes the B modes of the active zones al layers around the
-  // interior, STEP 7.b all of them on its own zones, which may be a layer
-  // less: there the B modes of the last stage go.
+  // STEP 8.d writes the B modes of the active zones of its range, STEP 7.b all of
+  // them on its own zones, which may be a layer less: there the B modes of the
+  // last stage go.
   const int lo = 3 - d.G, hx = d.N + d.G - 2, hz = d.nr + d.G - 2;
   const bool full = i >= lo && i <= hx && j >= lo && j <= hx && k >= lo && k <= hz;
-  const bool adp = m == 1 && i > -al && i <= d.N + al && j > -al && j <= d.N + al && k > -al && k <= d.nr + al;
+  const bool adp = m == 1 && i > -al.side && i <= d.N + al.side && j > -al.side && j <= d.N + al.side && k > -al.radial &&
+                   k <= d.nr + al.radial;
   if (adp && !full)
 #pragma unroll
     for (int q = 0; q < 27; ++q) s.V[((q / 3 + 1) * NVAR + 5 + q % 3) * PS + o] = R(0.0);
@@ -72,7 +73,7 @@ __device__ __forceinline__ void mask_faces(const Dims& d, const DGeom& g, const 
 // The primitives of every zone and the masked faces, one thread an index
 // (the box has one more face than zones along each axis).
 template <typename R>
-__global__ void __launch_bounds__(TPB) k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, int al) {
+__global__ void __launch_bounds__(TPB) k_prim(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, AdpLayers al) {
   const int lo = 1 - d.G;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
@@ -1668,7 +1669,7 @@ template <typename R>
 void launch_prim_and_masks_t(Solve& sv, DStateT<R>& st) {
   const Range3 f = faces_all(sv.d);
   k_prim<R><<<blocks_for(f.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(sv.d, sv.ph, sv.g, st, f,
-                                                                                    adp_layers(sv));
+                                                                                    adp_layers(sv.p));
   mark(sv, "k_prim");
   launch_tricorner_t(sv, st);
 }
@@ -1788,7 +1789,7 @@ template <typename R>
 void launch_faceB_adp_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
   // the faces of the zones STEP 8.d solves
-  Range3 fx = around(d, adp_layers(sv)), fy = fx, fz = fx;
+  Range3 fx = adp_zones(sv), fy = fx, fz = fx;
   fx.i0 -= 1;
   fy.j0 -= 1;
   fz.k0 -= 1;

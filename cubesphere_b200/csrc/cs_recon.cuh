@@ -168,8 +168,12 @@ __device__ __forceinline__ long long w_at(long long t, int e, long long n) {
 
 // The interior zones and w layers around them.
 inline Range3 around(const Dims& d, int w) { return {1 - w, d.N + w, 1 - w, d.N + w, 1 - w, d.nr + w}; }
-// Layers around the interior on which STEP 8.d solves the B modes.
-inline int adp_layers(const Solve& sv) { return sv.adp_w; }
+// The zones STEP 8.d solves the B modes of.
+inline Range3 adp_zones(const Solve& sv) {
+  const Dims& d = sv.d;
+  const AdpLayers l = adp_layers(sv.p);
+  return {1 - l.side, d.N + l.side, 1 - l.side, d.N + l.side, 1 - l.radial, d.nr + l.radial};
+}
 inline Range3 zones_all(const Dims& d) { return {1 - d.G, d.N + d.G, 1 - d.G, d.N + d.G, 1 - d.G, d.nr + d.G}; }
 inline Range3 shrink(const Dims& d, int s) {
   return {1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.N + d.G - s, 1 - d.G + s, d.nr + d.G - s};

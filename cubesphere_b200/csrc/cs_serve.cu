@@ -39,7 +39,7 @@ size_t state_device_bytes(const cs_params& p) {
   size_t bytes = (rwords * rsize + dwords * sizeof(double)) * S6 + S6 * sizeof(int32_t);
   // ghost staging values (one per map entry, see mesh_device_bytes)
   bytes += (size_t)6 * 4 * (p.nghost + 1) * (p.ntp + 2 * p.nghost + 1) * (p.nr + 2 * p.nghost + 1) * 12 * 8;
-  const int al = 2 * (p.nghost - 1);  // two sides of the widest ADP range (P2, callers' ghosts)
+  const int al = 2 * (p.nghost - 1);  // two sides of the widest ADP range (P2's)
   const size_t na = (size_t)6 * (p.ntp + al) * (p.ntp + al) * (p.nr + al);
   // ADP right-hand sides of the per-panel factors
   if (!(p.flags & CS_FLAG_NO_ADP_CACHE) && (p.flags & CS_FLAG_ADP_PER_PANEL)) bytes += na * 36 * sizeof(double);
@@ -55,7 +55,7 @@ size_t mesh_device_bytes(const cs_params& p) {
   // 9 bytes per entry (offsets, meta); panel-ownership maps are smaller
   bytes += (size_t)6 * 4 * (p.nghost + 1) * (p.ntp + 2 * p.nghost + 1) * (p.nr + 2 * p.nghost + 1) * 12 * 9 * 2;
   const size_t nl = (size_t)6 * (p.ntp + 2 * p.nghost - 4) * (p.ntp + 2 * p.nghost - 4) * (p.nr + 2 * p.nghost - 4);
-  const int al = 2 * (p.nghost - 1);  // two sides of the widest ADP range (P2, callers' ghosts)
+  const int al = 2 * (p.nghost - 1);  // two sides of the widest ADP range (P2's)
   const size_t na = (size_t)6 * (p.ntp + al) * (p.ntp + al) * (p.nr + al);
   if (!(p.flags & CS_FLAG_NO_OP_CACHE)) {
     // row weights shared by the six panels unless per-panel ones are asked
@@ -322,8 +322,7 @@ int cs_serve_submit(cs_server* sv, const cs_request* req, int64_t* id) {
   r.req = *req;
   r.t_submit = cs::Clock::now();
   r.bytes = cs::state_device_bytes(req->params);
-  // a mesh built for fewer ADP layers would serve without its operators
-  r.mesh = cs::mesh_key(req->params) + "/" + std::to_string(cs::adp_layers_needed(req->params));
+  r.mesh = cs::mesh_key(req->params);
   {
     std::lock_guard<std::mutex> lk(sv->mu);
     r.id = sv->next_id++;

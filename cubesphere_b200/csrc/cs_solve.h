@@ -68,7 +68,6 @@ struct MeshRes {
   void* op_p2v = nullptr;  // CS_FLAG_P2 one-sided stencil inverses (state's type)
   void* op_p2e = nullptr;
   bool p2_shared = false;  // op_p2v / op_p2e are panel 1's only
-  int adp_w = 0;            // layers around the interior the ADP operators cover
   void* adp_lu = nullptr;   // per-panel factors (FP64) or the panel-shared inverse (state's type)
   int8_t* adp_piv = nullptr;
   int8_t* adp_pmap = nullptr;  // ADP factors shared by the panels: per panel [unknown map][sign]
@@ -109,7 +108,6 @@ struct Solve {
   cudaGraph_t graph = nullptr;           // one step, captured by cs_steps / cs_batch_steps
   cudaGraphExec_t graph_exec = nullptr;  // its executable form
   long long graph_kernels = 0;           // kernels in that graph
-  int adp_w = 0;                         // layers around the interior STEP 8.d solves
   double grid_frac = 1.0;                // share of the SMs a launch's grid is sized for (autotuned in batches)
   Prof prof;
   std::string err;
@@ -137,14 +135,18 @@ int init_problem_device(Solve& sv, const cs_init_desc& desc);
 // radial boundary code other than outflow the radial ghosts are the caller's,
 // and what a stage does to them reaches the next one.
 inline bool ghosts_filled(const cs_params& p) { return p.bc_lower == 2 && p.bc_upper == 2; }
-// Layers around the interior that STEP 8.d has to solve.  The stage reads E in
-// one layer (the edge EMFs); P12's STEPS 9.b / 9.c run on it and read point
-// values of E, made of the ADP modes, one layer further, P2's stencils, run on
-// one layer more where there are four, two.  The layers beyond hold primitives
-// and slopes for those only, but a caller's ghosts take their zone B too.
-inline int adp_layers_needed(const cs_params& p) {
-  return (p.flags & CS_FLAG_P2) || !ghosts_filled(p) ? p.nghost - 1 : 2;
-}
+// Layers beyond the panel's sides and beyond its radial ends that STEP 8.d
+// solves.  The stage reads E in one layer (the edge EMFs); P12's STEPS 9.b / 9.c
+// run on it and read point values of E, made of the ADP modes, one layer
+// further, P2's stencils, run on one layer more where there are four, two.  Past
+// the sides no more is needed, since the next stage's fill sets those zones
+// anew; past the radial ends the zone B that STEP 8.d sets goes into what the
+// ghosts carry to the next stage, so all layers are solved that have faces.
+// Both follow from the mesh parameters and flags that solves on one mesh share.
+struct AdpLayers {
+  int side, radial;
+};
+inline AdpLayers adp_layers(const cs_params& p) { return {(p.flags & CS_FLAG_P2) ? p.nghost - 1 : 2, p.nghost - 1}; }
 // Identity of the mesh a parameter set needs (solves with equal keys can
 // share one MeshRes).
 std::string mesh_key(const cs_params& p);

@@ -130,6 +130,23 @@ def test_a_shared_mesh_serves_solves_of_other_boundary_codes():
         check_state(s, out[1], out[0])
 
 
+@pytest.mark.parametrize("first,second", [((2, 2), (0, 0)), ((0, 0), (2, 2)), ((2, 2), (0, 2))])
+def test_a_shared_mesh_serves_its_adp_operators_whatever_the_boundary_codes(first, second):
+    """Solves on one mesh use its ADP inverses in every stage, whichever
+    boundary codes the mesh was built with."""
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=10, nr=5)
+    a = cs.Solve(**{**pr["params"], "bc_lower": first[0], "bc_upper": first[1]})
+    a.mesh_build()
+    s = cs.Solve(**{**pr["params"], "bc_lower": second[0], "bc_upper": second[1]})
+    s.mesh_share(a)
+    s.init_problem(**pr["init"])
+    s.profile_begin()
+    s.step(s.evaluate_timestep(1e30))
+    kernels = s.profile_end()
+    assert kernels["k_adp6"][1] == 2 and "k_adp" not in kernels, sorted(kernels)
+
+
 def test_reciprocals_by_newton_steps_are_within_two_units():
     """The stage kernels form 1 / rho by Newton steps.  Two gases at rest without
     field, rho over 22 decades: the fast speed is sqrt(gamma p / rho), where two
