@@ -351,7 +351,9 @@ __global__ void k_avg_flux(Dims d, DStateT<R> s, PanelSync ps) {
 }
 
 // dU/dt of each zone from its six faces (x, then y, then z; lower face,
-// upper face) for the zones whose faces were all computed.
+// upper face).  The fluxes end with the radial face at the far side of the
+// first ghost (face -1 and face nr + 1), so the second ghost has that one face
+// only, as in the reference, which adds each face to both its zones.
 template <typename R>
 __global__ void k_gather(Dims d, DGeom g, DStateT<R> s, Range3 r) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
@@ -365,13 +367,15 @@ __global__ void k_gather(Dims d, DGeom g, DStateT<R> s, Range3 r) {
       const long long oy[2] = {d.idx(i, j - 1, k), d.idx(i, j, k)};
       const long long oz[2] = {d.idx(i, j, k - 1), d.idx(i, j, k)};
       const long long* os[3] = {ox, oy, oz};
-      for (int dir = 0; dir < 3; ++dir) {
+      const bool first = k >= 0 && k <= d.nr + 1;  // not a second ghost
+      for (int dir = first ? 0 : 2; dir < 3; ++dir) {
         const R* F = s.fcon[dir];
+        if (k >= 0)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          acc[c] = acc[c] - F[((long long)(8 + c) * NPANEL + p) * d.S + os[dir][0]];
-          acc[c] = acc[c] - F[((long long)c * NPANEL + p) * d.S + os[dir][1]];
-        }
+          for (int c = 0; c < 8; ++c) acc[c] = acc[c] - F[((long long)(8 + c) * NPANEL + p) * d.S + os[dir][0]];
+        if (k <= d.nr + 1)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) acc[c] = acc[c] - F[((long long)c * NPANEL + p) * d.S + os[dir][1]];
       }
     }
 #pragma unroll
@@ -409,10 +413,10 @@ void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
   const int N = d.N, nr = d.nr;
   // the faces of the zones to gather, and the layer across the interior's whose
   // speeds and fluxes its edges read
-  const Range3 z = stage_zones(sv, 1);
-  Range3 fx = {z.i0 - 1, z.i1, 0, N + 1, 0, nr + 1};
-  Range3 fy = {0, N + 1, z.j0 - 1, z.j1, 0, nr + 1};
-  Range3 fz = {0, N + 1, 0, N + 1, z.k0 - 1, z.k1};
+  const Range3 z = stage_zones(sv, 2);
+  Range3 fx = {0, N, 0, N + 1, 0, nr + 1};
+  Range3 fy = {0, N + 1, 0, N, 0, nr + 1};
+  Range3 fz = {0, N + 1, 0, N + 1, std::max(z.k0, 0) - 1, std::min(z.k1, nr + 1)};
   {
     const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + FLUX_FACES - 1) / FLUX_FACES);
     k_flux<R><<<tile_blocks(sv, nt, 32), FLUX_FACES * 5, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);

@@ -183,12 +183,13 @@ inline int tile_blocks(const Solve& sv, long long nt, int per_sm) {
   return (int)(sv.grid_frac < 1.0 ? std::min<long long>(nt, (long long)grid_sms(sv) * per_sm) : std::min<long long>(nt, 1 << 30));
 }
 
-// The zones whose state a stage moves: w layers around the interior where the
-// ghosts are the caller's (w < 0: all of them).
+// The zones whose state a stage moves: the panel's own columns (the fill that
+// starts the next stage sets every ghost beside the panel from such a column),
+// w radial ghosts beyond either end where those are the caller's.
 inline Range3 stage_zones(const Solve& sv, int w) {
   const Dims& d = sv.d;
-  const int l = ghosts_filled(sv.p) ? 0 : (w < 0 ? d.G : w);
-  return {1 - l, d.N + l, 1 - l, d.N + l, 1 - l, d.nr + l};
+  const int l = ghosts_filled(sv.p) ? 0 : w;
+  return {1, d.N, 1, d.N, 1 - l, d.nr + l};
 }
 
 }  // namespace cs

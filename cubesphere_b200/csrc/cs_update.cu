@@ -468,11 +468,11 @@ void launch_fill_ghosts(Solve& sv) {
 template <int M, typename R>
 void launch_update_mode(Solve& sv, const DStateT<R>& st, const UpArgs& a) {
   const Dims& d = sv.d;
-  const Range3 z = stage_zones(sv, -1);
+  const Range3 z = stage_zones(sv, d.G);
   k_update_zones<M, R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z, a);
   mark(sv, "k_update_zones");
   // UP_PLAIN touches the interior zones' faces only
-  const Range3 f = M == UP_PLAIN || ghosts_filled(sv.p) ? Range3{0, d.N, 0, d.N, 0, d.nr} : Range3{-d.G, d.N + d.G, -d.G, d.N + d.G, -d.G, d.nr + d.G};
+  const Range3 f = M == UP_PLAIN ? Range3{0, d.N, 0, d.N, 0, d.nr} : Range3{0, d.N, 0, d.N, z.k0 - 1, z.k1};
   const long long nb = 3 * ((f.count() + TPB - 1) / TPB);
   k_ct<M, R><<<(int)std::min<long long>(nb, (long long)grid_sms(sv) * 64), TPB, 0, sv.stream>>>(d, sv.g, st, f, a);
   mark(sv, "k_ct");
@@ -513,7 +513,7 @@ void launch_cleanup_t(Solve& sv, const DStateT<R>& st, const Range3& z) {
 }
 void launch_cleanup(Solve& sv, bool masks) {
   if (masks) launch_face_masks(sv);
-  const Range3 z = masks ? zones_all(sv.d) : stage_zones(sv, -1);
+  const Range3 z = masks ? zones_all(sv.d) : stage_zones(sv, sv.d.G);
   if (sv.fp32)
     launch_cleanup_t(sv, sv.stF, z);
   else

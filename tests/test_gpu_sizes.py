@@ -112,6 +112,54 @@ def test_callers_ghosts_take_their_zone_b(codes, flags):
             assert np.abs(a - b).max() > 0.0
 
 
+def own_columns(s, a, face=None):
+    """Zones (or faces of direction `face`) of the panels' own columns, through all radial layers."""
+    G, N = s.G, s.N
+    return a[..., 1 - (face == 2):, G + 1 - (face == 1):G + N + 1, G + 1 - (face == 0):G + N + 1]
+
+
+def check_columns(s, got, want, tol=1e-12):
+    """check_state through the radial ghosts."""
+    for q in range(8):
+        a, b = own_columns(s, got["U"][q]), own_columns(s, want["U"][q])
+        assert np.abs(a - b).max() <= tol * np.abs(b).max(), ("U", q, np.abs(a - b).max() / np.abs(b).max())
+    a, b = own_columns(s, got["ent"]), own_columns(s, want["ent"])
+    assert np.abs(a - b).max() <= tol * np.abs(b).max(), ("ent", np.abs(a - b).max() / np.abs(b).max())
+    den = max(np.abs(own_columns(s, want[k], d)).max() for d, k in enumerate(("bxf", "byf", "bzf")))
+    for d, k in enumerate(("bxf", "byf", "bzf")):
+        e = np.abs(own_columns(s, got[k], d) - own_columns(s, want[k], d)).max()
+        assert e <= tol * den, (k, e / den)
+
+
+@pytest.mark.parametrize("codes", [(0, 0), (2, 0), (0, 2)])
+@pytest.mark.parametrize("rk", [cs.CS_RK2, cs.CS_SSPRK3, cs.CS_IMEX_RK2])
+def test_callers_ghosts_match_the_oracle_over_whole_steps(codes, rk):
+    """Radial ghosts of the caller's, which the stages advance like the
+    reference's: three steps, ghosts compared too."""
+    from oracle import Oracle
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=10, nr=5, rk_scheme=rk)
+    filled = cs.Solve(**pr["params"])
+    filled.mesh_build(device=False)
+    o = Oracle(filled)
+    o.put_state(filled.init_problem_host(**pr["init"]))
+    o.fill_ghosts()
+    st = o.get_state()
+    noise = 1.0 + 0.02 * np.random.default_rng(11).uniform(-1.0, 1.0, st["U"].shape[1:])
+    noise[:, filled.G + 1:filled.G + filled.nr + 1] = 1.0
+    st["U"] = st["U"] * noise
+    s = cs.Solve(**{**pr["params"], "bc_lower": codes[0], "bc_upper": codes[1]})
+    s.mesh_build()
+    o = Oracle(s)
+    s.put_state(st)
+    o.put_state(st)
+    dt, dto = s.evaluate_timestep(1e30), o.evaluate_timestep(1e30)
+    for n in range(3):
+        dt, dto = s.step(dt), o.step(dto)
+        assert abs(dt - dto) <= 1e-12 * dto, (n, dt, dto)
+        check_columns(s, s.get_state(), o.get_state())
+
+
 def test_a_shared_mesh_serves_solves_of_other_boundary_codes():
     """Solves that share a mesh may differ in their boundary codes; each gives
     what it gives on its own mesh (up to the ADP operators' rounding, 1e-12)."""
