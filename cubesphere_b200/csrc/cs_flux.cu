@@ -413,10 +413,10 @@ void launch_fluxes_t(Solve& sv, DStateT<R>& st) {
   const int N = d.N, nr = d.nr;
   // the faces of the zones to gather, and the layer across the interior's whose
   // speeds and fluxes its edges read
-  const Range3 z = stage_zones(sv, 2);
+  const Range3 z = own_columns(d, 2);
   Range3 fx = {0, N, 0, N + 1, 0, nr + 1};
   Range3 fy = {0, N + 1, 0, N, 0, nr + 1};
-  Range3 fz = {0, N + 1, 0, N + 1, std::max(z.k0, 0) - 1, std::min(z.k1, nr + 1)};
+  Range3 fz = {0, N + 1, 0, N + 1, -1, nr + 1};
   {
     const long long nt = 3 * ((std::max(fx.count(), std::max(fy.count(), fz.count())) + FLUX_FACES - 1) / FLUX_FACES);
     k_flux<R><<<tile_blocks(sv, nt, 32), FLUX_FACES * 5, 0, sv.stream>>>(d, sv.ph, sv.g, st, fx, fy, fz);
@@ -444,7 +444,7 @@ template <typename R>
 void launch_sources_t(Solve& sv, DStateT<R>& st) {
   if (!(sv.ph.gm > sv.p.smallnum)) return;
   const Dims& d = sv.d;
-  const Range3 z = stage_zones(sv, 1);
+  const Range3 z = own_columns(d, 1);
   k_sources<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z);
   mark(sv, "k_sources");
 }

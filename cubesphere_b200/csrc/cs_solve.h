@@ -131,10 +131,6 @@ int cuda_fail(Solve& sv, cudaError_t e, const char* what);
 void* solve_alloc(Solve& sv, size_t bytes, cudaError_t& e);
 // The seeded initial state built on the device (cs_init_problem).
 int init_problem_device(Solve& sv, const cs_init_desc& desc);
-// Whether the fill that starts a stage gives every ghost its value.  With a
-// radial boundary code other than outflow the radial ghosts are the caller's,
-// and what a stage does to them reaches the next one.
-inline bool ghosts_filled(const cs_params& p) { return p.bc_lower == 2 && p.bc_upper == 2; }
 // Layers beyond the panel's sides and beyond its radial ends that STEP 8.d
 // solves.  The stage reads E in one layer (the edge EMFs); P12's STEPS 9.b / 9.c
 // run on it and read point values of E, made of the ADP modes, one layer
@@ -183,14 +179,12 @@ inline int tile_blocks(const Solve& sv, long long nt, int per_sm) {
   return (int)(sv.grid_frac < 1.0 ? std::min<long long>(nt, (long long)grid_sms(sv) * per_sm) : std::min<long long>(nt, 1 << 30));
 }
 
-// The zones whose state a stage moves: the panel's own columns (the fill that
-// starts the next stage sets every ghost beside the panel from such a column),
-// w radial ghosts beyond either end where those are the caller's.
-inline Range3 stage_zones(const Solve& sv, int w) {
-  const Dims& d = sv.d;
-  const int l = ghosts_filled(sv.p) ? 0 : w;
-  return {1, d.N, 1, d.N, 1 - l, d.nr + l};
-}
+// The panel's own columns with w radial ghosts at either end: what a stage
+// moves.  The fill that starts the next stage sets every ghost beside the panel
+// from such a column.  The radial ghosts carry over: all of their state where it
+// is the caller's, and with outflow the entropy, which the padding leaves alone
+// and which gives a ghost at the pressure floor its pressure.
+inline Range3 own_columns(const Dims& d, int w) { return {1, d.N, 1, d.N, 1 - w, d.nr + w}; }
 
 }  // namespace cs
 

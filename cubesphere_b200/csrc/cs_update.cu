@@ -468,7 +468,7 @@ void launch_fill_ghosts(Solve& sv) {
 template <int M, typename R>
 void launch_update_mode(Solve& sv, const DStateT<R>& st, const UpArgs& a) {
   const Dims& d = sv.d;
-  const Range3 z = stage_zones(sv, d.G);
+  const Range3 z = own_columns(d, d.G);
   k_update_zones<M, R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.ph, sv.g, st, z, a);
   mark(sv, "k_update_zones");
   // UP_PLAIN touches the interior zones' faces only
@@ -513,7 +513,7 @@ void launch_cleanup_t(Solve& sv, const DStateT<R>& st, const Range3& z) {
 }
 void launch_cleanup(Solve& sv, bool masks) {
   if (masks) launch_face_masks(sv);
-  const Range3 z = masks ? zones_all(sv.d) : stage_zones(sv, sv.d.G);
+  const Range3 z = masks ? zones_all(sv.d) : own_columns(sv.d, sv.d.G);
   if (sv.fp32)
     launch_cleanup_t(sv, sv.stF, z);
   else

@@ -319,7 +319,11 @@ int cs_state_put_amr(cs_ctx* ctx, int32_t n_cc_components, const double* U_amr, 
 int cs_state_get_amr(cs_ctx* ctx, int32_t n_cc_components, double* U_amr, double* entropygr_amr, double* Bxf_amr,
                      double* Byf_amr, double* Bzf_amr);
 
-/* Whole-stage and whole-step entry points (device resident, on ctx's stream). */
+/* Whole-stage and whole-step entry points (device resident, on ctx's stream).
+ * A stage starts with the ghost fill and moves the panels' own columns, the
+ * radial ghosts of these columns included; the ghosts beside a panel keep what
+ * the fill gave them until the next one (cs_fill_ghosts brings them up to date
+ * for a caller that reads whole boxes). */
 int cs_stage(cs_ctx* ctx, int32_t irk, double dtcur);
 int cs_step(cs_ctx* ctx, double dtcur, double* dtcurp1);
 /* nsteps steps, each at the time step the previous one chose (the driver's
@@ -334,7 +338,9 @@ int cs_evaluate_timestep(cs_ctx* ctx, double dtcur, double* dtcurp1);
 int cs_synchronize(cs_ctx* ctx);
 
 /* Per-routine entry points with the reference routine names, for
- * step-by-step parity (each runs on the resident state). */
+ * step-by-step parity (each runs on the resident state).  The face fluxes, the
+ * sources and the update form and move the panels' own columns only, as in a
+ * stage. */
 int cs_fill_ghosts(cs_ctx* ctx);
 int cs_limit_all_slopes_p12(cs_ctx* ctx);
 int cs_make_facial_fluxes(cs_ctx* ctx);
