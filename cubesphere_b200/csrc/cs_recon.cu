@@ -859,15 +859,17 @@ __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_faceB(Dims d, P
   }
 }
 
-// STEP 9.a (421:6700-6790): zone-centred E = -v x B from the point values.
+// STEP 9.a (421:6700-6790): zone-centred E = -v x B from the point values, on
+// the zones z of r.
 template <typename R>
-__global__ void k_efield_a(Dims d, DGeom g, DStateT<R> s, Range3 r) {
+__global__ void k_efield_a(Dims d, DGeom g, DStateT<R> s, Range3 r, Range3 z) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < r.count(); t += (long long)gridDim.x * blockDim.x) {
     int p, i, j, k;
     r.decode(t, p, i, j, k);
     // a zone that exhausted STEP 7.c's shrink passes also zeroes its entropy
     // value (440:569-575), now that every zone has read its neighbours'
     if (s.giveup[d.at(0, p, i, j, k)] & 1) s.ent[d.at(0, p, i, j, k)] = 0.0;
+    if (i < z.i0 || i > z.i1 || j < z.j0 || j > z.j1 || k < z.k0 || k > z.k1) continue;
     R co[10];
     coef10(g, d, p, i, j, k, co);
     R pv[8];
@@ -1843,9 +1845,11 @@ template <typename R>
 void launch_efield_t(Solve& sv, DStateT<R>& st) {
   const Dims& d = sv.d;
   Range3 a = around(d, 1), b = shrink(d, 2);
-  // P2's stencils reach two zones beyond theirs
+  // P2's stencils reach two zones beyond theirs; STEP 7.c's zones all zero
+  // their entropy where they gave up
   const Range3 z = (sv.p.flags & CS_FLAG_P2) ? zones_all(d) : around(d, 2);
-  k_efield_a<R><<<blocks_for(z.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, z);
+  const Range3 r = (sv.p.flags & CS_FLAG_P2) ? z : shrink(d, 1);
+  k_efield_a<R><<<blocks_for(r.count(), TPB, grid_sms(sv)), TPB, 0, sv.stream>>>(d, sv.g, st, r, z);
   mark(sv, "k_efield_a");
   if (sv.p.flags & CS_FLAG_P2) {  // LIMIT_ALL_SLOPES_P2's STEP 9.b
     const int nb = (int)std::min<long long>(p2_tiles(b, st.p2_map), (long long)grid_sms(sv) * 16);

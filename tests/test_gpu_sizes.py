@@ -191,6 +191,38 @@ def test_radial_ghosts_at_the_pressure_floor_match_the_oracle(rk, ghosts):
         check_columns(s, s.get_state(), o.get_state())
 
 
+@pytest.mark.parametrize("p2,out_to", [(0, 3), (cs.CS_FLAG_P2, 2)])
+def test_ghosts_that_give_up_zero_their_entropy_like_the_oracle(p2, out_to):
+    """STEP 7.c in ghosts of the caller's that are rough enough to exhaust its
+    shrink passes in every layer that has modes."""
+    from oracle import Oracle
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=10, nr=5)
+    filled = cs.Solve(**pr["params"])
+    filled.mesh_build(device=False)
+    o = Oracle(filled)
+    o.put_state(filled.init_problem_host(**pr["init"]))
+    o.fill_ghosts()
+    st = o.get_state()
+    s = cs.Solve(**pr["params"], bc_lower=0, bc_upper=0, flags=p2)
+    rough = 1.0 - 0.97 * np.random.default_rng(1).uniform(0.0, 1.0, st["U"].shape[1:])
+    rough[:, s.params.nghost:s.params.nghost + s.params.nr + 2] = 1.0  # the interior and the first ghosts
+    st["U"] = st["U"] * rough
+    s.mesh_build()
+    o = Oracle(s)
+    out = []
+    for x in (s, o):
+        x.put_state(st)
+        x.fill_ghosts()
+        x.limit_all_slopes_p12()
+        out.append(own_columns(s, x.get_state()["ent"])[0])
+    got, want = out
+    for layer in (s.G - out_to, s.G + s.nr + out_to - 1):  # the columns start with ghost layer G
+        assert (want[:, layer] == 0.0).any()
+    assert np.array_equal(got == 0.0, want == 0.0)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
 def test_a_shared_mesh_serves_solves_of_other_boundary_codes():
     """Solves that share a mesh may differ in their boundary codes; each gives
     what it gives on its own mesh (up to the ADP operators' rounding, 1e-12)."""
