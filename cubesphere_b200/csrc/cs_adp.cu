@@ -2,6 +2,8 @@
 // zones' B modes (421limit_all_slopes_p12.f:5574-6675,
 // 253, 120matsolve.f), with the panel-shared inverse, the per-panel factors
 // or factored in place.
+#include <math_constants.h>
+
 #include "cs_recon.cuh"
 
 namespace cs {
@@ -51,9 +53,26 @@ struct AdpSmem {
   int piv[36];
 };
 
+// acc + err: the sum of products so far and what rounding left out of it, by
+// Knuth's error-free sum and a product whose error is one fused multiply-add
+// (roundings spelled out, so that none are contracted away).
+__device__ __forceinline__ void add_product(double& acc, double& err, double a, double b) {
+  const double p = __dmul_rn(a, b), e = __fma_rn(a, b, -p), s = __dadd_rn(acc, p), t = __dsub_rn(s, acc);
+  err = __dadd_rn(err, __dadd_rn(__dadd_rn(__dsub_rn(acc, __dsub_rn(s, t)), __dsub_rn(p, t)), e));
+  acc = s;
+}
+
 // kFactorOnly: assemble and factor the geometry-only KKT matrix and store
 // the factors and the row permutation for k_adp_solve, or (zb == ADP6_ZB)
 // the packed rows of the inverse for k_adp6 (once per mesh).
+//
+// The inverse's columns are refined once, with residuals carried to twice the
+// precision, so that what is stored is the rounded inverse.  Without that its
+// application errs up to 20 times as much as a substitution with the factors
+// (thin surfaces of 12^2 x 3 zones: 7e-11 of the largest mode against 3e-12);
+// with it less than half as much on every mesh, in FP32 too, where the
+// substitution itself rounded at every element (12^2 x 3: 1.3e-3 for the
+// factors in FP32, 8.6e-4 for the inverse).
 // tmax: zones of the range handled (all of it, or panel 1's share when the
 // factors are shared by the six panels); zb: zones per factor block.
 template <bool kFactorOnly, typename R>
@@ -140,6 +159,10 @@ __global__ void __launch_bounds__(32 * ADP_WARPS) k_adp(Dims d, PhysC ph, DGeom 
       S.K[m][30 + f] = S.C[f][m];
       S.K[30 + f][m] = S.C[f][m];
     }
+    if (kFactorOnly && zb == ADP6_ZB) {  // the mode block for the residuals, in place of the rows
+      __syncwarp();
+      for (int e = lane; e < 900; e += 32) S.Q[e / 30][e % 30] = S.K[e / 30][e % 30];
+    }
     for (int e = lane; e < 36; e += 32) {
       S.K[30 + e / 6][30 + e % 6] = 0.0;
     }
@@ -223,10 +246,43 @@ __global__ void __launch_bounds__(32 * ADP_WARPS) k_adp(Dims d, PhysC ph, DGeom 
         for (int b = a + 1; b < 36; ++b) acc -= S.K[a][b] * y[b];
         y[a] = acc / S.K[a][a];
       }
-      // the size of K times that of its inverse, for the mesh build's choice
-      double ymax = 0.0;
+      // y += K^-1 (e_c - K y); z is in local memory, so that the loops stay loops
+      double z[36];
+#pragma unroll 1
+      for (int a = 0; a < 36; ++a) {
+        const int row = S.piv[a];
+        double acc = row == lane ? 1.0 : 0.0, err = 0.0;
+        if (row < 30) {
+          const double* k = S.Q[row];
 #pragma unroll
-      for (int u = 0; u < 30; ++u) ymax = fmax(ymax, lane < 30 ? fabs(y[u]) : 0.0);
+          for (int b = 0; b < 30; ++b) add_product(acc, err, -k[b], y[b]);
+#pragma unroll
+          for (int f = 0; f < 6; ++f) add_product(acc, err, -S.C[f][row], y[30 + f]);
+        } else {
+          const double* k = S.C[row - 30];
+#pragma unroll
+          for (int b = 0; b < 30; ++b) add_product(acc, err, -k[b], y[b]);
+        }
+        acc = acc + err;
+#pragma unroll 1
+        for (int b = 0; b < a; ++b) acc -= S.K[a][b] * z[b];
+        z[a] = acc;
+      }
+#pragma unroll 1
+      for (int a = 35; a >= 0; --a) {
+        double acc = z[a];
+#pragma unroll 1
+        for (int b = a + 1; b < 36; ++b) acc -= S.K[a][b] * z[b];
+        z[a] = acc / S.K[a][a];
+      }
+#pragma unroll
+      for (int a = 0; a < 36; ++a) y[a] = y[a] + z[a];
+      // the size of K times that of its inverse, for the mesh build's choice
+      // (infinite where an entry is not finite)
+      double ymax = 0.0;
+      if (lane < 30)
+#pragma unroll
+        for (int u = 0; u < 30; ++u) ymax = isfinite(y[u]) ? fmax(ymax, fabs(y[u])) : CUDART_INF;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
         kmax = fmax(kmax, __shfl_xor_sync(0xffffffffu, kmax, off));

@@ -258,6 +258,36 @@ def test_a_shared_mesh_serves_its_adp_operators_whatever_the_boundary_codes(firs
     assert kernels["k_adp6"][1] == 2 and "k_adp" not in kernels, sorted(kernels)
 
 
+@pytest.mark.parametrize("name,ntp,nr,ghosts", [("surface32", 12, 3, 4), ("shell16", 13, 3, 4), ("shell16", 12, 3, 4)])
+def test_adp_inverses_are_as_accurate_as_the_factors(name, ntp, nr, ghosts):
+    """B modes by the packed inverse against the per-panel factors on meshes whose
+    matrices are the worst conditioned that keep the inverse (max |K| max
+    |K^-1| of 2200, 880 and 640).  Against 80-bit elimination the factors err by
+    up to 5e-14 of a zone's largest mode and a rounded inverse by 1e-14, and the
+    right-hand sides' roundings add 2e-14: 2e-13 leaves them twice that and is
+    below an inverse that keeps the elimination's own errors (2e-13 to 6e-13)."""
+    pr = cs.preset(name)
+    pr["params"].update(ntp=ntp, nr=nr, nghost=ghosts)
+    out = []
+    for flags, kernel in ((0, "k_adp6"), (cs.CS_FLAG_ADP_PER_PANEL, "k_adp_solve")):
+        s = cs.Solve(**pr["params"], flags=flags)
+        s.mesh_build()
+        s.init_problem(**pr["init"])
+        s.fill_ghosts()
+        s.limit_all_slopes_p12()
+        V = s.debug("V")
+        s.profile_begin()
+        s.step(s.evaluate_timestep(1e30))
+        assert kernel in s.profile_end()
+        out.append(np.stack([V[8 * m + c] for m in range(10) for c in (5, 6, 7)]))
+    lay = slice(s.G + 1 - (s.G - 1), s.G + s.nr + s.G)  # layers 2 - G .. nr + G - 1
+    side = slice(s.G - 1, s.G + s.N + 3)                # two beside the panel
+    a, b = (x[:, :, lay, side, side] for x in out)
+    on = (s.mask()[:, lay, side, side] == 1) & (np.abs(b).max(0) > 0.0)
+    err = (np.abs(a - b).max(0)[on] / np.abs(b).max(0)[on]).max()
+    assert err <= 2e-13, err
+
+
 def test_reciprocals_by_newton_steps_are_within_two_units():
     """The stage kernels form 1 / rho by Newton steps.  Two gases at rest without
     field, rho over 22 decades: the fast speed is sqrt(gamma p / rho), where two
