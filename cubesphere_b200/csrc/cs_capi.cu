@@ -505,8 +505,13 @@ int alloc_state(Solve& sv, DStateT<R>& s) {
   s.adp_pmap = m.adp_pmap;
   s.adp_rhs = nullptr;
   if (s.adp_lu && !s.adp_pmap) {  // k_adp6 keeps its right-hand sides in shared memory
-    s.adp_rhs = dalloc(sv, (size_t)adp_range_count(sv) * 36 * sizeof(double), e);
-    if (!s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP right-hand sides)");
+    const size_t rhs_bytes = (size_t)adp_range_count(sv) * 36 * sizeof(double);
+    if (!(sv.p.flags & CS_FLAG_ADP_PER_PANEL) && sv.reserve && !sv.reserve(0, rhs_bytes)) {
+      s.adp_lu = nullptr;  // factor in every stage
+    } else {
+      s.adp_rhs = dalloc(sv, rhs_bytes, e);
+      if (!s.adp_rhs) return cuda_fail(sv, e, "cudaMalloc(ADP right-hand sides)");
+    }
   }
   s.giveup = (int32_t*)dalloc(sv, S6 * sizeof(int32_t), e);
   if (sv.p.flags & CS_FLAG_STEP10) {
@@ -823,10 +828,12 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
     int8_t pmap[6 * 72];
     const bool shared = !(sv.p.flags & CS_FLAG_ADP_PER_PANEL) && adp_panel_maps(m.host, pmap);
     if (int rc = adp_operators(shared, pmap)) return rc;
-    // The inverse is as good as the factors while the matrices are well
-    // conditioned: max |K| max |K^-1| is 10 to 1000 on shells and surfaces of
-    // ordinary aspect, and rounding enlarged that much is below 1e-12.  Beyond
-    // (a radial extrapolation through r = 0, say) the factors serve.
+    // max |K| max |K^-1| is 10 to 40 on shells and surfaces of ordinary aspect
+    // and reaches 2200 on the thinnest; there the inverse is closer to the exact
+    // solution than the factors, in FP64 and in FP32.  Far beyond (1.4e9 with a
+    // radial vertex at r = 0) what the matrix makes of the right-hand sides'
+    // rounding exceeds the agreement asked of a step, whatever is applied to them,
+    // and the factors serve, whose elimination is the reference's.
     if (shared && m.adp_lu) {
       double cond = 0.0;
       CS_CUDA(sv, cudaMemcpyAsync(&cond, s.err_flag + 2, sizeof cond, cudaMemcpyDeviceToHost, sv.stream));
@@ -840,7 +847,9 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
         m.bytes -= held;
         m.adp_lu = nullptr;
         m.adp_pmap = nullptr;
-        if (int rc = adp_operators(false, pmap)) return rc;
+        const size_t nf = (size_t)adp_factor_doubles(sv, false);
+        if (!sv.reserve || sv.reserve(nf * sizeof(double) + nf / 36 - held, (size_t)adp_range_count(sv) * 36 * sizeof(double)))
+          if (int rc = adp_operators(false, pmap)) return rc;
       }
     }
   }

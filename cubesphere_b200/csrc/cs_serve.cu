@@ -133,6 +133,20 @@ struct cs_server {
 namespace cs {
 namespace {
 
+// Frees cached meshes that no running solve uses, oldest key first, until
+// `need` more bytes fit in the budget; returns whether they do.
+bool make_room(cs_server* sv, size_t need) {
+  for (auto it = sv->meshes.begin(); sv->reserved + need > sv->budget && it != sv->meshes.end();) {
+    if (it->second.mesh && it->second.mesh.use_count() == 1) {
+      sv->reserved -= it->second.bytes;
+      it = sv->meshes.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  return sv->reserved + need <= sv->budget;
+}
+
 void run_request(cs_server* sv, int64_t id) {
   cudaSetDevice(sv->device);
   Request* r;
@@ -143,6 +157,15 @@ void run_request(cs_server* sv, int64_t id) {
   }
   cs_ctx* ctx = nullptr;
   int rc = cs_create(&r->req.params, &ctx);
+  if (!rc)  // a mesh may turn out to need more than its admission counted
+    ctx->sv.reserve = [sv, r](size_t mesh_bytes, size_t state_bytes) {
+      std::lock_guard<std::mutex> lk(sv->mu);
+      if (!make_room(sv, mesh_bytes + state_bytes)) return false;
+      sv->reserved += mesh_bytes + state_bytes;
+      r->bytes += state_bytes;
+      (r->mesh_builder ? sv->meshes[r->mesh].bytes : r->bytes) += mesh_bytes;
+      return true;
+    };
   if (!rc && r->mesh_builder) {
     rc = cs_mesh_build(ctx);
     {
@@ -235,20 +258,6 @@ void run_request(cs_server* sv, int64_t id) {
 // state, plus its mesh unless that is cached (or being built).
 size_t admission_bytes(cs_server* sv, const Request& r) {
   return r.bytes + (sv->meshes.count(r.mesh) ? 0 : mesh_device_bytes(r.req.params));
-}
-
-// Frees cached meshes that no running solve uses, oldest key first, until
-// `need` more bytes fit in the budget; returns whether they do.
-bool make_room(cs_server* sv, size_t need) {
-  for (auto it = sv->meshes.begin(); sv->reserved + need > sv->budget && it != sv->meshes.end();) {
-    if (it->second.mesh && it->second.mesh.use_count() == 1) {
-      sv->reserved -= it->second.bytes;
-      it = sv->meshes.erase(it);
-    } else {
-      ++it;
-    }
-  }
-  return sv->reserved + need <= sv->budget;
 }
 
 // Admission: the oldest pending request starts when a slot is free and its

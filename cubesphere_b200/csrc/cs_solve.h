@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -109,6 +110,10 @@ struct Solve {
   cudaGraphExec_t graph_exec = nullptr;  // its executable form
   long long graph_kernels = 0;           // kernels in that graph
   double grid_frac = 1.0;                // share of the SMs a launch's grid is sized for (autotuned in batches)
+  // Asked before the mesh (first argument, bytes) or this solve (second) takes
+  // device memory that cs_estimate_device_bytes does not count; where it says no
+  // they do without.  Unset: the device's own room decides.
+  std::function<bool(size_t, size_t)> reserve;
   Prof prof;
   std::string err;
 };

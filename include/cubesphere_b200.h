@@ -434,7 +434,10 @@ int cs_snapshot_read_host(const char* path, const cs_params* p, double* U, doubl
  * needs its memory.  A request then runs cs_init_problem, cs_steps and
  * cs_diag; its result does not depend on what else runs (every kernel
  * is deterministic).  Latency is measured from submission to completion.
- * cs_estimate_device_bytes counts a solve's state and its mesh. */
+ * cs_estimate_device_bytes counts a solve's state and its mesh; a mesh that
+ * turns out too ill conditioned for the ADP inverse keeps the larger per-panel
+ * factors where the budget has room for them, and factors in every stage where
+ * not. */
 typedef struct cs_server cs_server;
 typedef struct cs_request {
   cs_params params;

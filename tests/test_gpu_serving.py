@@ -51,6 +51,36 @@ def test_result_is_the_same_alone_and_in_a_mix():
     assert st["zone_updates_per_s"] > 0
 
 
+def test_an_ill_conditioned_mesh_stays_within_the_budget():
+    """A mesh whose padding runs through r = 0 keeps per-panel ADP factors (1.3 GB
+    here) only where the server's budget has room for them; without it every
+    stage factors in place, with the same result to the parity tolerance."""
+    import torch
+
+    torch.cuda.set_device(0)
+    params, init = _req(48, 1, 3)
+    params.update(nghost=4)
+    need = cs.estimate_device_bytes(**params)
+    states = []
+    for budget in (need + (200 << 20), need + (2500 << 20)):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        srv = cs.Server(max_active=1, mem_fraction=budget / free, keep_state=True)
+        rid = srv.submit(2, params, init)
+        assert srv.wait(rid).status == 0
+        states.append(srv.state(rid, cs.make_params(**params)))
+        held = free - torch.cuda.mem_get_info()[0]  # the cached mesh and the solve's pool
+        factors = 6 * (48 + 4) ** 2 * (1 + 6) * 1296 * 8
+        assert (held > factors) == (budget > need + factors), (held, budget)
+        assert held <= budget, (held, budget)
+        srv.close()
+    s = cs.Solve(**params)
+    s.mesh_build(device=False)
+    for q in range(8):
+        a, b = (s.interior(x["U"][q]) for x in states)
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), q
+
+
 def test_request_larger_than_the_budget_is_refused():
     srv = cs.Server(max_active=2, mem_fraction=1e-6)
     rid = srv.submit(1, *_req(16, 8, 1))
