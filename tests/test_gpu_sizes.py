@@ -64,6 +64,28 @@ def test_precision_form_at_uneven_sizes(ntp, nr, ghosts, p2):
     assert max(face_b_errors(s, got, want).values()) <= 5e-6
 
 
+@pytest.mark.parametrize("name,ntp,nr,ghosts,kernel", [("shell16", 6, 1, 4, "k_adp_solve"), ("surface32", 12, 3, 4, "k_adp6")])
+def test_precision_form_on_ill_conditioned_meshes(name, ntp, nr, ghosts, kernel):
+    """The meshes at both sides of the choice between inverse and factors (max
+    |K| max |K^-1| of 1.4e9 and 2200), at the bound of the test above; measured
+    3e-7."""
+    pr = cs.preset(name)
+    pr["params"].update(ntp=ntp, nr=nr, nghost=ghosts)
+    out = []
+    for form in (0, cs.CS_FLAG_FP32):
+        s = cs.Solve(**pr["params"], flags=form)
+        s.mesh_build()
+        s.init_problem(**pr["init"])
+        s.profile_begin()
+        s.step(s.evaluate_timestep(1e30))
+        assert kernel in s.profile_end()
+        out.append(s.get_state())
+    want, got = out
+    for q in (0, 4, 5, 6, 7):
+        assert np.abs(zones(s, got["U"][q]) - zones(s, want["U"][q])).max() <= 5e-6 * np.abs(zones(s, want["U"][q])).max(), q
+    assert max(face_b_errors(s, got, want).values()) <= 5e-6
+
+
 def test_fp64_batches_give_each_members_own_result():
     """Members of different sizes side by side, many times: every state equals
     the member's run alone to the bit (an earlier pair of ADP kernels
