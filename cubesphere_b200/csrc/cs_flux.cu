@@ -363,19 +363,22 @@ __global__ void k_gather(Dims d, DGeom g, DStateT<R> s, Range3 r) {
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[c] = R(0.0);
     if (mask_at(g, d, p, i, j) == 1) {
-      const long long ox[2] = {d.idx(i - 1, j, k), d.idx(i, j, k)};
-      const long long oy[2] = {d.idx(i, j - 1, k), d.idx(i, j, k)};
-      const long long oz[2] = {d.idx(i, j, k - 1), d.idx(i, j, k)};
-      const long long* os[3] = {ox, oy, oz};
-      const bool first = k >= 0 && k <= d.nr + 1;  // not a second ghost
-      for (int dir = first ? 0 : 2; dir < 3; ++dir) {
-        const R* F = s.fcon[dir];
-        if (k >= 0)
+      const long long PS = (long long)NPANEL * d.S, o = (long long)p * d.S + d.idx(i, j, k);
+      const int dk = d.NI * d.NJ;
+      if (k >= 0 && k <= d.nr + 1) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) acc[c] = acc[c] - F[((long long)(8 + c) * NPANEL + p) * d.S + os[dir][0]];
-        if (k <= d.nr + 1)
+        for (int dir = 0; dir < 3; ++dir) {
+          const R *Fl = s.fcon[dir] + o, *Fr = Fl + 8 * PS - (dir == 0 ? 1 : (dir == 1 ? d.NI : dk));
 #pragma unroll
-          for (int c = 0; c < 8; ++c) acc[c] = acc[c] - F[((long long)c * NPANEL + p) * d.S + os[dir][1]];
+          for (int c = 0; c < 8; ++c) {
+            acc[c] = acc[c] - Fr[c * PS];
+            acc[c] = acc[c] - Fl[c * PS];
+          }
+        }
+      } else {  // a second ghost: its face toward the interior
+        const R* F = s.fcon[2] + o + (k < 0 ? 0 : 8 * PS - dk);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] = acc[c] - F[c * PS];
       }
     }
 #pragma unroll
