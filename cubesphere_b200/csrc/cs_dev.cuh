@@ -125,17 +125,33 @@ struct Range3 {
 template <typename R>
 __device__ __forceinline__ R sqr(R x) { return x * x; }
 
-// 1 / x for x of normal size by two Newton steps r += r (1 - x r) from the
-// hardware's approximation (more than 20 correct bits, so 40 and then all but
-// the rounding of the last step): 5 instructions where the IEEE quotient takes
-// over twice that, within 2 units in the last place.
-__device__ __forceinline__ double rcp_newton(double x) {
+// 1 / x for x of normal size (floored densities, lengths, areas, volumes) by two
+// Newton steps r += r (1 - x r) from the hardware's approximation (more than 20
+// correct bits, so 40 and then all but the rounding of the last step): 5
+// instructions where the IEEE quotient takes over twice that, within 2 units in
+// the last place.
+__device__ __forceinline__ double rcp_newton(double x, double& approx) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  approx = r;
   r = fma(fma(-x, r, 1.0), r, r);
   return fma(fma(-x, r, 1.0), r, r);
 }
+__device__ __forceinline__ double rcp_newton(double x) {
+  double approx;
+  return rcp_newton(x, approx);
+}
 __device__ __forceinline__ float rcp_newton(float x) { return 1.0f / x; }
+// The same where x may be 0 or have overflowed (a star density, a smoothness
+// indicator): the steps make a NaN of the quotients infinity and 0, which the
+// approximation already is.  A subnormal x gives infinity, one above 2^1022
+// gives 0.  The test is an integer one: the FP64 pipe is the busy one.
+__device__ __forceinline__ double rcp_any(double x) {
+  double approx;
+  const double r = rcp_newton(x, approx);
+  return (__double2hiint(r) & 0x7ff00000) != 0x7ff00000 ? r : approx;
+}
+__device__ __forceinline__ float rcp_any(float x) { return 1.0f / x; }
 
 // Conserved -> primitive with density/pressure floors and the entropy
 // fallback; updates ent and re-derives the total energy.  Returns the
@@ -243,7 +259,7 @@ __device__ __forceinline__ void d_hll(const PhysC& ph, R* VL, R* VR, R entL, R e
 #pragma unroll
   for (int c = 0; c < 8; ++c) Us[c] = t1 * UR[c] - t2 * UL[c] - t3 * (FR[c] - FL[c]);
   const R entU = t1 * entR - t2 * entL - t3 * (entR * VR[1] - entL * VL[1]);
-  const R peng = (R(ph.gamma) - R(1.0)) * (Us[4] - R(0.5) * (Us[1] * Us[1] + Us[2] * Us[2] + Us[3] * Us[3]) * rcp_newton(Us[0]) -
+  const R peng = (R(ph.gamma) - R(1.0)) * (Us[4] - R(0.5) * (Us[1] * Us[1] + Us[2] * Us[2] + Us[3] * Us[3]) * rcp_any(Us[0]) -
                                           R(ph.ob8pi) * (Us[5] * Us[5] + Us[6] * Us[6] + Us[7] * Us[7]));
   // The entropy pressure (a pow) is formed only where the floor needs it.
   if (peng <= R(ph.prsfloor)) {

@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(W7A_ZT * 3, sizeof(R) == 4 ? 8 : 6) k_weno_slo
 #pragma unroll
         for (int st = 0; st < 9; ++st) {
           const double x0 = X[0][st], x1 = X[1][st], x2 = X[2][st];
-          const double v = rcp_newton(x0 * x0 + x1 * x1 + x2 * x2 + ph.smallnum), v2 = v * v;
+          const double v = rcp_any(x0 * x0 + x1 * x1 + x2 * x2 + ph.smallnum), v2 = v * v;
           const double W = st < 8 ? v2 * v2 : 100.0 * (v2 * v2);
           sw = sw + W;
           t0 = t0 + W * x0;
@@ -1268,7 +1268,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
       for (int m = 0; m < 9; ++m) acc[c][m] = 0.0;
     }
     auto add = [&](int c, const R* X, double w0) {  // weighted modes of one stencil
-      const double v = rcp_newton(smooth(X) + ph.smallnum), v2 = v * v, W = w0 * (v2 * v2);
+      const double v = rcp_any(smooth(X) + ph.smallnum), v2 = v * v, W = w0 * (v2 * v2);
       sw[c] = sw[c] + W;
 #pragma unroll
       for (int m = 0; m < 9; ++m) acc[c][m] = acc[c][m] + W * (double)X[m];

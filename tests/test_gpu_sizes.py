@@ -329,3 +329,47 @@ def test_reciprocals_by_newton_steps_are_within_two_units():
     for sign, got in ((-1.0, out[:, 32]), (1.0, out[:, 33])):
         err = np.abs(sign * got - want) / want
         assert err.max() <= 4 * np.finfo(float).eps, float(err.max())
+
+
+def test_a_star_density_of_zero_matches_the_oracle():
+    """Two gases that leave each other at 2^60 with a jump in the transverse field:
+    the star density is exactly 0 and the star momentum is not, so the pressure
+    is -infinity and the entropy repair makes the energy infinite."""
+    from oracle import Oracle
+    c = np.zeros((1, 18))
+    c[0, [0, 8, 4, 12, 16, 17]] = 1.0
+    c[0, 1], c[0, 9] = -2.0 ** 60, 2.0 ** 60
+    c[0, [5, 13, 14]] = 1.0
+    got = cs.pointwise(2, c, ntp=8, nr=4)[0]
+    want = Oracle(params=cs.make_params(ntp=8, nr=4), mesh=False).pointwise(2, c)[0]
+    assert want[4] == want[12] == -np.inf
+    assert np.array_equal(np.isinf(got), np.isinf(want)) and np.array_equal(got[[4, 12]], want[[4, 12]])
+    on = np.isfinite(want)
+    assert np.abs(got[on] - want[on]).max() <= 1e-14 * np.abs(want[on]).max()
+
+
+@pytest.mark.parametrize("form", [0, cs.CS_FLAG_FP32])
+def test_smoothness_indicators_that_overflow_weigh_nothing(form):
+    """One zone so fast that the indicators of the stencils through it overflow:
+    its neighbours take their modes from the other stencils, finite where the
+    oracle's are (P2, whose modes are the weighted stencils' own)."""
+    from oracle import Oracle
+    from seeded_states import uniform_state
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=8, nr=6, gm=0.0)
+    s = cs.Solve(**pr["params"], flags=cs.CS_FLAG_P2 | form)
+    s.mesh_build()
+    st = uniform_state(s)
+    z = (2, s.G + 3, s.G + 4, s.G + 4)
+    v = 8e153 if not form else 1e18  # squares near the largest value of the state's type
+    st["U"][(1,) + z], st["U"][(4,) + z] = v, 0.5 * v * v + 1.5
+    o = Oracle(s)
+    V = []
+    for x in (s, o):
+        x.put_state(st)
+        x.fill_ghosts()
+        x.limit_all_slopes_p12()
+        V.append(zones(s, x.debug("V")))
+    if not form:
+        assert not np.isfinite(V[1]).all()
+    assert np.array_equal(np.isfinite(V[0]), np.isfinite(V[1]))
