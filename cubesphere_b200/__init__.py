@@ -587,7 +587,7 @@ class Server:
 
 def twod_rs_ez(kind: int, cases: np.ndarray) -> np.ndarray:
     """ESSz of the device multidimensional Riemann solver for each row of
-    `cases` (kind 4: 11 inputs, kind 3: 10 inputs; see cs_twod_rs_ez)."""
+    `cases` (kind 4: 11 inputs, kind 3: 10, kind 5: 7; see cs_twod_rs_ez)."""
     a = np.ascontiguousarray(cases, dtype=np.float64)
     out = np.zeros(a.shape[0])
     rc = load_library().cs_twod_rs_ez(kind, a.shape[0], _dptr(a), _dptr(out))

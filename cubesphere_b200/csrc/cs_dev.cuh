@@ -280,9 +280,9 @@ __device__ __forceinline__ void d_hll(const PhysC& ph, R* VL, R* VR, R entL, R e
   entF = right ? eL : (left ? eR : (SR * eL - SL * eR) * t3 + (entR - entL) * (SR * SL * t3));
 }
 
-// Multidimensional HLL solver for the induction equation with four states
-// (general branch reached when all four speeds straddle zero, which the
-// symmetrised LLF speeds always do).
+// Multidimensional HLL solver for the induction equation with four states, in
+// general: for known answers (the edge kernels evaluate its closed form at the
+// symmetrised LLF speeds, where all four straddle zero).
 __device__ __forceinline__ double d_rs4(double SR, double SL, double SU, double SD, double cos_t, double sin_t,
                                         double Ez, double BnU, double BnD, double ByR, double ByL) {
   const double EzRU = Ez, EzLU = Ez, EzLD = Ez, EzRD = Ez;

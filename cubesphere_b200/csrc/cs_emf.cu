@@ -267,8 +267,9 @@ void launch_edges(Solve& sv) {
 
 }  // namespace cs
 
-// Known-answer access to the two multidimensional Riemann solvers: one
-// thread per case evaluates the device function the edge kernels call.
+// Known-answer access to the multidimensional Riemann solvers, one thread a
+// case: the three-state solver and the four-state one's closed form, which
+// k_edges calls, and the four-state solver in general, which it does not.
 namespace {
 __global__ void k_twod_rs_ez(int n, int kind, const double* in, double* out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -276,6 +277,9 @@ __global__ void k_twod_rs_ez(int n, int kind, const double* in, double* out) {
   if (kind == 4) {
     const double* a = in + (long long)t * 11;
     out[t] = cs::d_rs4(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10]);
+  } else if (kind == 5) {
+    const double* a = in + (long long)t * 7;
+    out[t] = cs::llf_emf(a[0], a[1], a[2], a[3], a[4], a[5], a[6]);
   } else {
     const double* a = in + (long long)t * 10;
     out[t] = cs::d_rs3(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9]);
@@ -284,9 +288,9 @@ __global__ void k_twod_rs_ez(int n, int kind, const double* in, double* out) {
 }  // namespace
 
 extern "C" int cs_twod_rs_ez(int32_t kind, int32_t n, const double* in, double* out) {
-  if ((kind != 3 && kind != 4) || n < 0 || (n > 0 && (!in || !out))) return CS_ERR_ARG;
+  if (kind < 3 || kind > 5 || n < 0 || (n > 0 && (!in || !out))) return CS_ERR_ARG;
   if (n == 0) return CS_OK;
-  const size_t nin = (size_t)n * (kind == 4 ? 11 : 10);
+  const size_t nin = (size_t)n * (kind == 4 ? 11 : (kind == 5 ? 7 : 10));
   double *din = nullptr, *dout = nullptr;
   if (cudaMalloc(&din, nin * sizeof(double)) != cudaSuccess) return CS_ERR_CUDA;
   if (cudaMalloc(&dout, (size_t)n * sizeof(double)) != cudaSuccess) {

@@ -492,7 +492,10 @@ int cs_batch_destroy(cs_batch* b);
  * single Ez the edge kernels pass for all states: for kind 4, n cases of
  * (S_R, S_L, S_U, S_D, cos_t, sin_t, Ez, Bneta_U, Bneta_D, By_R, By_L); for
  * kind 3, n cases of (S_R1, S_L1, S_R2, S_L2, S_R3, S_L3, Ez, Bneta_1,
- * Bneta_2, Bneta_3).  out[n] = ESSz, evaluated on the current device. */
+ * Bneta_2, Bneta_3); for kind 5, the form of kind 4 at the symmetrised speeds
+ * S_R = S_U = -S_L = -S_D = S that the edge kernels evaluate, n cases of
+ * (S, sin_t, Ez, Bneta_U, Bneta_D, By_R, By_L).  out[n] = ESSz, evaluated on
+ * the current device. */
 int cs_twod_rs_ez(int32_t kind, int32_t n, const double* in, double* out);
 
 /* V_min_local / V_max_local of the last LIMIT_ALL_SLOPES_P12 of the context

@@ -95,3 +95,26 @@ def test_device_solvers_match_known_answers_and_oracle():
     assert got3[0] == pytest.approx(0.55, abs=1e-14)
     np.testing.assert_allclose(got4, want4, rtol=1e-12, atol=1e-13)
     np.testing.assert_allclose(got3, want3, rtol=1e-12, atol=1e-13)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not has_gpu(), reason="needs a CUDA device")
+def test_device_closed_form_of_the_edge_emfs_matches_the_oracles_four_state_solver():
+    """The function the edge kernels evaluate, on the device, against the oracle's
+    general solver at the symmetrised speeds.  Tolerance: 64 roundings of the
+    largest term, s |B| / sin^2 t or |E| (the general form divides by sin t
+    twice)."""
+    import cubesphere_b200 as cs
+
+    rng = np.random.default_rng(5)
+    cases, want, scale = [], [], []
+    for n in range(2000):
+        t = 0.5 * math.pi if n % 2 else rng.uniform(0.3, math.pi - 0.3)
+        c, sn = (0.0, 1.0) if n % 2 else (math.cos(t), math.sqrt(1.0 - math.cos(t) ** 2))
+        s, E = 10.0 ** rng.uniform(-6, 3), rng.normal() * 10.0 ** rng.uniform(-6, 2)
+        b = rng.normal(size=4) * 10.0 ** rng.uniform(-4, 2)
+        cases.append((s, sn, E, *b))
+        want.append(oracle.twod_rs_ez_4state(s, -s, s, -s, c, sn, E, E, E, E, *b))
+        scale.append(abs(E) + s * np.abs(b).max() / sn ** 2)
+    got = cs.twod_rs_ez(5, np.array(cases))
+    assert (np.abs(got - want) <= 64 * 2.0 ** -53 * np.array(scale)).all()
