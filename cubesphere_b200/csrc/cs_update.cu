@@ -188,6 +188,8 @@ __global__ void __launch_bounds__(TPB) k_update_zones(Dims d, PhysC ph, DGeom g,
         dU[2] += c * (-(gy * rho));
         dU[3] += c * (-(gz * rho));
         dU[4] += c * (-(gx * m1 + gy * m2 + gz * m3));
+#pragma unroll
+        for (int q = 1; q < 5; ++q) s.dUdt[q * PS + o] = dU[q];  // part of the rates from here on
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) U[q] = s.U0[q * PS + o] + dt0 * s.K1[q * PS + o];

@@ -147,6 +147,20 @@ def test_whole_steps_match_oracle(name, nsteps, flags, rk):
         check_state(s, s.get_state(), o.get_state())
 
 
+@pytest.mark.parametrize("rk", [cs.CS_RK2, cs.CS_SSPRK3, cs.CS_IMEX_RK2])
+def test_rates_read_after_each_stage_match_oracle(rk):
+    """dU/dt (with the gravity a stage adds to it) and the EMFs as they stand after
+    every stage of a step."""
+    s, o, st = make_pair("shell16", rk_scheme=rk)
+    dt = o.evaluate_timestep(1e30)
+    for irk in range(1, 4 if rk == cs.CS_SSPRK3 else 3):
+        s.stage(irk, dt)
+        o.stage(irk, dt)
+        for name in ("dUdt", "Efx", "Efy", "Efz"):
+            e = rel(zones(s, s.debug(name)), zones(s, o.debug(name)))
+            assert e <= TOL_WORK, (irk, name, e)
+
+
 def test_steps_keep_div_b_at_roundoff_across_panel_edges(shell16):
     """With panel-edge ownership (the default) CT keeps div B at round-off in
     every zone, including those next to panel edges and cube corners."""
