@@ -6,9 +6,8 @@
 // Follows LIMIT_ALL_SLOPES_P12
 // (pkg/inc/cubesphere/400riemann_integrate/421limit_all_slopes_p12.f) and
 // ENFORCE_PRESSURE_POSITIVITY_PRIM (440enforce_pressure_positivity_prim.f);
-// each kernel names the reference step it implements.  One thread per zone
-// or face; the ADP solve uses one warp per zone with the 36x36 KKT system
-// in shared memory.
+// each kernel names the reference step it implements.  STEPS 7.b and 9.c from
+// the resident row weights are in cs_weno.cu, STEP 8.d in cs_adp.cu.
 #include "cs_recon.cuh"
 
 namespace cs {
@@ -229,9 +228,7 @@ __global__ void k_flat_bc(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r, con
   }
 }
 
-// Central 18-zone stencil of STEP 7.b / 9.c: (neighbour w or -1 for self, dz).
-__constant__ int c_n18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {-1, 1}, {-1, -1}, {8, 0}, {9, 0},  {10, 0},
-                                 {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
+__constant__ Stencil18 c_n18 = stencil18();  // for run-time rows
 
 struct Nbr12 {
   int x[12], y[12];
@@ -391,8 +388,8 @@ template <typename R>
 __device__ __forceinline__ void w7b_row(const Dims& d, const PhysC& ph, const DGeom& g, int p, int i, int j, int k,
                                         const Nbr12& n, int rr, R cx, R cy, R cz, R l0, R obl0,
                                         const R* c0, R* A, long long& off) {
-  const int w = c_n18[rr][0], dz = c_n18[rr][1];
-  const int zx = w < 0 ? i : n.x[w], zy = w < 0 ? j : n.y[w], zz = k + dz;
+  const int w = c_n18.v[rr][0], dz = c_n18.v[rr][1];
+  const int zx = w == 12 ? i : n.x[w], zy = w == 12 ? j : n.y[w], zz = k + dz;
   off = d.idx(zx, zy, zz);
   const R x = (geoR<R>(g, d, CS_G_V_CEN, 0, p, zx, zy, zz) - cx) * obl0;
   const R y = (geoR<R>(g, d, CS_G_V_CEN, 1, p, zx, zy, zz) - cy) * obl0;
@@ -742,7 +739,6 @@ __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g
 #pragma unroll
         for (int m = 1; m < (c < 2 ? 10 : 4); ++m) dev = dev + fabs((double)v[m * ms]) * bb[m - 1];
         const double room = dev > 0.0 ? dev * (1.0 + 1e-12) + 1e-14 * (fabs(mean) + dev) : 0.0;
-        // written so that a NaN does not pass
         pass = pass && mean - room >= mn[c] && mean + room <= mx[c];
       }
       s.giveup[o] = pass ? 0 : positivity_shrink(d, ph, g, s, p, i, j, k, mn[0], mx[0], mn[1], mx[1], mn[2], mx[2]);
@@ -890,9 +886,6 @@ __global__ void k_efield_a(Dims d, DGeom g, DStateT<R> s, Range3 r, Range3 z) {
   }
 }
 
-// STEP 9.b (421:6840-8400): linear WENO slopes of the E point values.
-// Three blocks per SM (measured: faster than two at 255 registers, and than
-// four).
 // Row rr (0: the zone itself, 1..18: the STEP 7.b neighbours) of the
 // 19 x 10 interpolation least-squares matrix of STEP 9.c (421:8464-8620).
 template <typename R>
@@ -909,8 +902,8 @@ __device__ __forceinline__ void e9c_row(const Dims& d, const DGeom& g, int p, in
     for (int m = 4; m < 10; ++m) A[m] = R(0.0) * R(0.0) - c0[m];
     return;
   }
-  const int w = c_n18[rr - 1][0], dz = c_n18[rr - 1][1];
-  const int zx = w < 0 ? i : n.x[w], zy = w < 0 ? j : n.y[w], zz = k + dz;
+  const int w = c_n18.v[rr - 1][0], dz = c_n18.v[rr - 1][1];
+  const int zx = w == 12 ? i : n.x[w], zy = w == 12 ? j : n.y[w], zz = k + dz;
   off = d.idx(zx, zy, zz);
   const R x = (geoR<R>(g, d, CS_G_V_CEN, 0, p, zx, zy, zz) - cx) * obl0;
   const R y = (geoR<R>(g, d, CS_G_V_CEN, 1, p, zx, zy, zz) - cy) * obl0;
@@ -1144,10 +1137,6 @@ __global__ void k_ops_p2(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   }
 }
 
-// Central 18-zone stencil: (neighbour or 12 for the zone itself, dz).
-__constant__ int c_n18s[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {12, 1}, {12, -1}, {8, 0}, {9, 0},  {10, 0},
-                                  {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
-
 // STEP 7.a of LIMIT_ALL_SLOPES_P2.  A block takes 32 zones, a warp two of the 8
 // primitives.  For each of the eight one-sided stencils a thread forms its
 // primitives' modes from the resident inverse, their smoothness indicator over
@@ -1343,7 +1332,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
         for (int c = 0; c < 2; ++c) Y[c][m] = R(0.0);
 #pragma unroll 3
       for (int rr = 0; rr < 18; ++rr) {
-        const int off = nbo[c_n18s[rr][0]][lane] + c_n18s[rr][1] * plane;
+        const int off = nbo[c_n18.v[rr][0]][lane] + c_n18.v[rr][1] * plane;
         R v[2];
 #pragma unroll
         for (int c = 0; c < 2; ++c) v[c] = f[c * PS + off] - f0[c];
@@ -1389,8 +1378,7 @@ __global__ void __launch_bounds__(P2_THREADS, p2_blocks(sizeof(R))) k_p2_prim(Di
 template <bool kShared, typename R>
 __global__ void __launch_bounds__(32) k_p2_efield(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r) {
   constexpr int NM = 10, NR = 10;
-  constexpr int n18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {-1, 1}, {-1, -1}, {8, 0}, {9, 0},  {10, 0},
-                              {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
+  constexpr Stencil18 N18 = stencil18();
   const int lane = threadIdx.x;
   const long long nz = r.count(), npp = nz / 6, nw = kShared ? npp : nz;
   const long long ntile = kShared ? 6 * ((npp + 31) / 32) : (nz + 31) / 32;
@@ -1505,8 +1493,8 @@ __global__ void __launch_bounds__(32) k_p2_efield(Dims d, PhysC ph, DGeom g, DSt
 #pragma unroll
       for (int rr = 0; rr < NR + 9; ++rr) {
         const int ro = rr - 1;  // the zone itself first
-        const int w = ro < 0 ? -1 : n18[ro][0], dz = ro < 0 ? 0 : n18[ro][1];
-        const long long off = d.idx(w < 0 ? i : n.x[w], w < 0 ? j : n.y[w], k + dz);
+        const int w = ro < 0 ? 12 : N18.v[ro][0], dz = ro < 0 ? 0 : N18.v[ro][1];
+        const long long off = d.idx(w == 12 ? i : n.x[w], w == 12 ? j : n.y[w], k + dz);
         R Rv[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {

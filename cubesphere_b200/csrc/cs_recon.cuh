@@ -144,6 +144,16 @@ __device__ __forceinline__ void mrweno_hybrid(const R* X, const R* lin, const R*
   for (int a = 3; a < 9; ++a) out[a] = (Whi * Phi[a]) * x;
 }
 
+// The central 18-zone stencil of STEPS 7.b and 9.c: (neighbour in the plane, 12
+// for the zone's own column; radial offset).
+struct Stencil18 {
+  int v[18][2];
+};
+__host__ __device__ constexpr Stencil18 stencil18() {
+  return {{{0, 0},  {1, 0},  {2, 0},  {3, 0},  {12, 1}, {12, -1}, {8, 0}, {9, 0},  {10, 0},
+           {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}}};
+}
+
 // The line of p to L2.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

@@ -41,9 +41,7 @@ __global__ void __launch_bounds__(W7_THREADS, sizeof(R) == 4 ? 4 : 3) k_weno7b(D
                                                                                 Range3 r) {
   extern __shared__ __align__(128) unsigned char w7_raw[];
   W7Smem<R>& S = *reinterpret_cast<W7Smem<R>*>(w7_raw);
-  // central 18-zone stencil: (neighbour or 12 for the zone itself, dz)
-  constexpr int N18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {12, 1}, {12, -1}, {8, 0}, {9, 0},  {10, 0},
-                              {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
+  constexpr Stencil18 N18 = stencil18();
   const int tid = threadIdx.x;
   const long long nz = r.count(), npp = nz / 6, nw = kShared ? npp : nz;
   const unsigned ntile = (unsigned)(kShared ? 6 * ((npp + 31) / 32) : (nz + 31) / 32);
@@ -120,8 +118,8 @@ __global__ void __launch_bounds__(W7_THREADS, sizeof(R) == 4 ? 4 : 3) k_weno7b(D
     auto load_rows = [&](int c, R (&E)[2][W7_ROWS]) {
 #pragma unroll
       for (int rr = 0; rr < W7_ROWS; ++rr) {
-        const int n = N18[c * W7_ROWS + rr][0];
-        const int off = (n == 12 ? 0 : nbo[n == 12 ? 0 : n][lane]) + N18[c * W7_ROWS + rr][1] * plane;
+        const int n = N18.v[c * W7_ROWS + rr][0];
+        const int off = (n == 12 ? 0 : nbo[n == 12 ? 0 : n][lane]) + N18.v[c * W7_ROWS + rr][1] * plane;
         E[0][rr] = act ? v[off] : R(0.0);
         E[1][rr] = act ? v[PS + off] : R(0.0);
       }
@@ -229,8 +227,7 @@ __global__ void __launch_bounds__(E9_THREADS, sizeof(R) == 4 ? 8 : 6) k_efield_c
                                                                                  Range3 r, Range3 rs) {
   extern __shared__ __align__(128) unsigned char e9_raw[];
   E9Smem<R>& S = *reinterpret_cast<E9Smem<R>*>(e9_raw);
-  constexpr int N18[18][2] = {{0, 0},  {1, 0},  {2, 0},  {3, 0},  {12, 1}, {12, -1}, {8, 0}, {9, 0},  {10, 0},
-                              {11, 0}, {0, 1},  {1, 1},  {0, -1}, {1, -1}, {2, 1},   {3, 1}, {2, -1}, {3, -1}};
+  constexpr Stencil18 N18 = stencil18();
   const int tid = threadIdx.x;
   const long long nz = rs.count(), npp = nz / 6, nw = kShared ? npp : nz;
   const unsigned ntile = (unsigned)(kShared ? 6 * ((npp + 31) / 32) : (nz + 31) / 32);
@@ -297,7 +294,7 @@ __global__ void __launch_bounds__(E9_THREADS, sizeof(R) == 4 ? 8 : 6) k_efield_c
     R D[19];
 #pragma unroll
     for (int rr = 0; rr < 19; ++rr) {
-      const int n = rr ? N18[rr ? rr - 1 : 0][0] : 12, dz = rr ? N18[rr ? rr - 1 : 0][1] : 0;
+      const int n = rr ? N18.v[rr ? rr - 1 : 0][0] : 12, dz = rr ? N18.v[rr ? rr - 1 : 0][1] : 0;
       D[rr] = act ? f[(n == 12 ? 0 : nbo[n == 12 ? 0 : n][lane]) + dz * plane] : R(0.0);
     }
     R Y[10];
