@@ -755,8 +755,10 @@ int mesh_operators(Solve& sv, MeshRes& m, DStateT<R>& s) {
   // (2.8 KB per zone in FP64 per panel, 1.55 KB with STEP 9.c's shared).
   if (!(sv.p.flags & CS_FLAG_NO_OP_CACHE)) {
     // Panel-shared row weights where the mesh allows: STEP 9.c's always,
-    // STEP 7.b's in the precision form only (the FP64 k_weno7b, at its
-    // register limit, measured slower with them).
+    // STEP 7.b's in the precision form only.  In FP64 k_weno7b measured with
+    // panel 1's / with each panel's own: 8.55 / 8.37 ms of a 6 x 128^2 x 64 step,
+    // 1.22 / 1.16 of 6 x 64^2 x 32, 0.208 / 0.211 of 6 x 32^2 x 16: what L2 saves in
+    // HBM reads, six blocks waiting for one tile's words give back.
     LsqPanelMap qmap[6];
     const bool shared = !(sv.p.flags & CS_FLAG_LSQ_PER_PANEL) && lsq_panel_maps(m.host, qmap);
     m.m10_shared = shared;

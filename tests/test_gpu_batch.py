@@ -60,9 +60,9 @@ def test_batch_matches_each_solve_alone():
 def test_batch_is_reproducible_under_concurrency():
     """Members running side by side on the device must not change each
     other's results: four batched runs of the five members all equal the
-    solves run alone, bit for bit (a STEP 7.b kernel that split each
-    32-zone tile over four warps once made 15-25% of the member runs differ
-    in a few tiles)."""
+    solves run alone, bit for bit (member runs once differed in a few 32-zone
+    tiles, behind a ring of bulk copies whose stages were released without a
+    fence)."""
     want = alone(3)
     for rep in range(4):
         sols = [make(m) for m in MEMBERS]

@@ -316,3 +316,37 @@ def test_panel_sharded_steps_match_the_single_process_solve(name, flags, panel_r
         assert got_dts == dts, rank
         for k in want:
             assert np.array_equal(got[k], want[k][:, owned]), (rank, k)
+
+
+@pytest.mark.parametrize("ntp,nr,ghosts", [(5, 2, 3), (12, 4, 4), (9, 3, 5)])
+def test_every_ghost_beside_a_panel_is_filled_from_an_own_column(ntp, nr, ghosts):
+    """What lets a stage leave the ghosts beside a panel out: the fill sets every
+    active one of them, and every face of theirs, at all radial layers, and takes
+    each value from a panel's own column."""
+    pr = cs.preset("shell16")
+    pr["params"].update(ntp=ntp, nr=nr, nghost=ghosts)
+    s = cs.Solve(**pr["params"])
+    s.mesh_build(device=False)
+    src, dst, meta = (a.astype(np.int64) for a in s.fill_map())
+    G, N, NI, P = s.G, s.N, s.NI, 6 * s.box
+    mask = s.mask().reshape(6, s.NK, NI, NI) == 1
+    k, j, i = np.meshgrid(np.arange(s.NK) - G, np.arange(NI) - G, np.arange(NI) - G, indexing="ij")
+    zone = (i > -G) & (j > -G) & (k > -G)
+    own = lambda f, x, y: (x >= (f != 2)) & (x <= N) & (y >= (f != 3)) & (y <= N)  # noqa: E731
+    ghost = mask & zone & ~own(0, i, j)
+    for f in range(5):
+        to, so = dst[(meta & 7) == f], src[(meta & 7) == f]
+        sf = (meta[(meta & 7) == f] >> 5) & 7
+        filled = np.zeros((8 if f == 0 else 1) * P, bool)
+        filled[to] = True
+        filled = filled.reshape(-1, 6, s.NK, NI, NI).all(0)
+        if f < 2:
+            need = ghost
+        else:  # both faces of every such ghost that are not an own column's
+            low = np.roll(ghost, -1, axis={2: 3, 3: 2, 4: 1}[f])
+            need = (ghost | low) & ~own(f, i, j)
+        assert (filled | ~need).all(), f
+        active = need.reshape(-1)[to % P]
+        x, y = so % NI - G, so // NI % NI - G
+        from_own = np.where(sf == 2, own(2, x, y), np.where(sf == 3, own(3, x, y), own(0, x, y)))
+        assert from_own[active].all(), f
