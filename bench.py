@@ -70,19 +70,19 @@ ALGO_WORDS_PER_UNIT = {
 }
 
 # DRAM bytes per unit and launch (read + write) measured by ncu on the
-# shell32 case (units: 155,520 zones of the ADP and STEP 7.b ranges, 124,848 of
-# the flux and STEP 9.c ranges; 14 launches each), FP64 and precision form; the full
+# shell32 case (units: 171,072 zones of the ADP range, 155,520 of STEP 7.b's,
+# 124,848 of the flux and STEP 9.c ranges), FP64 and precision form; the full
 # shell128 launches are too large to capture, so roofline.traffic scales
 # these by the units of a full launch.
 MEASURED_TRAFFIC_PER_UNIT = {
-    "k_adp6": 1710.6,
-    "k_flux": 2251.2,
+    "k_adp6": 1744.4,
+    "k_flux": 2437.9,
     "k_weno7b": 2178.9,
     "k_efield_c": 487.6,
 }
 MEASURED_TRAFFIC_PER_UNIT_FP32 = {
-    "k_adp6": 948.3,
-    "k_flux": 1653.8,
+    "k_adp6": 957.0,
+    "k_flux": 1775.1,
     "k_weno7b": 441.4,
     "k_efield_c": 274.1,
 }
@@ -93,7 +93,7 @@ MEASURED_TRAFFIC_PER_UNIT_FP32 = {
 # FP64 FMA per clock x 2 x 1.965 GHz = 37.2 TFLOP/s, is kept for context.
 FP64_FLOP_PER_UNIT = {
     "k_adp6": 4455.1,
-    "k_flux": 14498.6,
+    "k_flux": 15096.6,
     "k_weno7b": 3900.7,
     "k_efield_c": 1780.4,
 }
@@ -732,9 +732,10 @@ def run_gpu(args):
     dom = max(prof.items(), key=lambda kv: kv[1][0])
     dname, (dms, dcount) = dom
     G, N, nr = s.G, s.N, s.nr
-    # zones of the kernel's range: layers around the interior
-    layers = {"k_weno7a": G - 1, "k_weno7b": G - 2, "k_adp6": 2, "k_faceB": 2, "k_positivity": G - 2}.get(dname, 1)
-    units = 6 * (N + 2 * layers) ** 2 * (nr + 2 * layers)
+    # zones of the kernel's range: layers beside the panel and beyond its radial ends
+    side, radial = {"k_weno7a": (G - 1, G - 1), "k_weno7b": (G - 2, G - 2), "k_adp6": (2, G - 1), "k_faceB": (2, G - 1),
+                    "k_positivity": (G - 1, G - 1)}.get(dname, (1, 1))
+    units = 6 * (N + 2 * side) ** 2 * (nr + 2 * radial)
     launch_s = dms / dcount / 1e3
     per_launch = stage_b * units
     achieved = per_launch / launch_s / 1e9

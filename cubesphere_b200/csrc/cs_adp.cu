@@ -546,7 +546,8 @@ __global__ void __launch_bounds__(ADPS_THREADS, 2) k_adp_solve(Dims d, PhysC ph,
 // a triangular solve reads 1296 words for one dependent one each.  The sums (60
 // registers a thread) leave two blocks an SM in FP64 and four in FP32, so what
 // is left is latency.  ms of a 6 x 128^2 x 64 step: 18.6 (FP32 15.0) for right-hand
-// sides in HBM and a substitution, 10.2 (8.7) for this.
+// sides in HBM and a substitution, 10.2 (8.7) for this on two layers around the
+// interior, 10.6 (9.0) on all radial layers that have faces.
 constexpr int ADP6_CONS = 6 * 32;
 constexpr int ADP6_THREADS = ADP6_CONS + 32;
 constexpr int ADP6_CH = 2 * ADP6_UNIT;  // words a ring stage

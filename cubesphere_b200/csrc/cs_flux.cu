@@ -39,7 +39,8 @@ constexpr int TPB = 128;
 // at the 20 warps its registers and shared memory allow.  ms of a 6 x 128^2 x
 // 64 step, FP64 / FP32: 29.5 / 19.8 with every thread forming its point's basis
 // per variable, 22.3 / 14.6 with the basis kept and two primitives a warp at a
-// time, 21.3 / 14.1 with four, 20.7 / 13.1 with the tiles in order (tile_blocks).
+// time, 21.3 / 14.1 with four, 20.7 / 13.1 with the tiles in order (tile_blocks),
+// 21.7 / 13.3 since it forms the second radial faces beyond the ends too.
 constexpr int FLUX_FACES = 32;
 // Registers / occupancy: 4 blocks per SM suit the FP64 instantiation, 7 the
 // FP32 one (measured on the 6 x 128^2 x 64 shell).

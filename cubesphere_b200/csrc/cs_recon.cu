@@ -763,7 +763,8 @@ __global__ void __launch_bounds__(TPB, 5) k_positivity(Dims d, PhysC ph, DGeom g
 // face normal is one vector on x- and y-faces, so there each side's modes are
 // first contracted with it (10 values, one polynomial); on z-faces, where it
 // varies over the points, the components are taken one after another.  ms of a
-// 6 x 128^2 x 64 step, that / this: 7.7 / 5.6 (FP32 7.4 / 3.9).
+// 6 x 128^2 x 64 step, that / this: 7.7 / 5.6 (FP32 7.4 / 3.9); 5.8
+// (4.0) since the third radial layer of ghosts is one of its zones.
 template <typename R>
 __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 4) k_faceB(Dims d, PhysC ph, DGeom g, DStateT<R> s, Range3 r0, Range3 r1, Range3 r2) {
   const unsigned nt0 = (unsigned)((r0.count() + TPB - 1) / TPB), nt1 = (unsigned)((r1.count() + TPB - 1) / TPB),

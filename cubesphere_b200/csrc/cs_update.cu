@@ -107,7 +107,7 @@ __global__ void k_pad_radial(Dims d, DGeom g, DStateT<R> s, int bc_lower, int bc
 // What one pass of the update does besides U += scale dt dU/dt.  A stage's save,
 // combine and restore need no passes of their own: with them, the copies and the
 // gravity a 6 x 32^2 x 1 step was 111 launches, now 73.  Both updates are bound by
-// HBM on large meshes (1.1 and 0.9 ms of a 6 x 128^2 x 64 step):
+// HBM on large meshes (1.3 and 1.0 ms of a 6 x 128^2 x 64 step):
 //   UP_PLAIN  nothing (the routine by itself)
 //   UP_SAVE   first stage: also saves the state
 //   UP_MEAN   (x + x0) / 2 first (RK2's second stage)
