@@ -71,7 +71,7 @@ struct MeshRes {
   bool p2_shared = false;  // op_p2v / op_p2e are panel 1's only
   void* adp_lu = nullptr;   // per-panel factors (FP64) or the panel-shared inverse (state's type)
   int8_t* adp_piv = nullptr;
-  int8_t* adp_pmap = nullptr;  // ADP factors shared by the panels: per panel [unknown map][sign]
+  int8_t* adp_pmap = nullptr;  // inverse shared by the panels: per panel [unknown map][sign]
   std::vector<void*> allocs;
   size_t bytes = 0;     // device bytes held
   bool on_device = false;
